@@ -7,6 +7,7 @@
 #include <string>
 
 #include "../../include/pdb200.h"
+#include "mesh_fft.hpp"
 
 namespace pdb {
 
@@ -168,11 +169,14 @@ struct pd_mesh {
     float *gridB = nullptr;    // potential grid
     float *field[3] = {nullptr, nullptr, nullptr};  // ik field grids
     cufftComplex *spec = nullptr;
-    cufftComplex *scratch = nullptr;                // ik
+    cufftComplex *scratch = nullptr;                // ik: one field spectrum (cuFFT) or all three
     float *G = nullptr;        // nmodes
     float *Vc = nullptr;       // 6 nmodes (row c: c * nmodes + m)
     double *acc = nullptr;     // 7
     float4 *packed = nullptr;  // particles packed in the caller's order (SoA entry points)
+    int route = 0;             // FFT_PLANES / FFT_LINES: this library's transforms; FFT_CUFFT: the plans below
+    pdb::FftMesh fft{};
+    float2 *tw[3] = {nullptr, nullptr, nullptr};    // twiddle tables per axis
     cufftHandle fwd = 0, bwd = 0;
     bool plans = false;
     void *work = nullptr;
@@ -269,8 +273,8 @@ int bmesh_pack_launch(const BMeshView &v, const float *x, const float *y, const 
 int bmesh_spread_launch(const BMeshView &v, const long long *st, cudaStream_t s);
 // spec *= G over every replica's modes; clears the charge grids for the next spread.
 int bmesh_solve_launch(const BMeshView &v, const long long *st, cudaStream_t s);
-// AD gather joined with the pair forces already stored in f: f += mesh force, the closing half kick
-// when kick.on, and with energy epot += q phi / 2 - half_c_self q^2.
+// AD gather joined with the pair forces stored by position: f = pair + mesh force, the closing half kick
+// when kick.on, and with energy epot = pair energy + q phi / 2 - half_c_self q^2.
 int bmesh_gather_launch(const BMeshView &v, float *fx, float *fy, float *fz, float *epot, int energy,
                         const BMeshKick &kick, float half_c_self, const long long *st, cudaStream_t s);
 

@@ -461,6 +461,44 @@ static void refresh_background(pd_mesh *m) {
 
 static WindowPoly window_poly(const pd_mesh *m) { return WindowPoly{m->wpoly, m->wdeg}; }
 
+// Charge grid -> potential grid (or the ik fields, and the potential with energy): forward transform,
+// influence multiply, inverse transforms; the charge grid is left zero.
+static int mesh_solve_grids(pd_mesh *m, int energy, cudaStream_t s, cudaEvent_t ev_r2c) {
+    const bool ik = m->p.kind == PD_MESH_P3M_IK;
+    int rc;
+    if (m->route != FFT_CUFFT) {
+        if ((rc = fft_forward(m->fft, m->route, s))) return rc;
+        if (ev_r2c) PD_CUDA(cudaEventRecord(ev_r2c, s));
+        if (energy) PD_CUDA(cudaMemsetAsync(m->acc, 0, 7 * sizeof(double), s));
+        if ((rc = fft_solve(m->fft, ik, energy, m->Vc, m->acc, s))) return rc;
+        return fft_inverse(m->fft, m->route, ik ? (energy ? 4 : 3) : 1, s);
+    }
+    PD_CUFFT(cufftSetStream(m->fwd, s));
+    PD_CUFFT(cufftExecR2C(m->fwd, m->gridA, m->spec));
+    if (ev_r2c) PD_CUDA(cudaEventRecord(ev_r2c, s));
+    if (energy) PD_CUDA(cudaMemsetAsync(m->acc, 0, 7 * sizeof(double), s));
+    const int blocks = (m->nmodes + 255) / 256;
+    if (energy)
+        k_solve<true><<<blocks, 256, 0, s>>>((float2 *)m->spec, m->G, m->Vc, m->acc, m->K1, m->K1h, m->nmodes, m->gridA,
+                                             m->nnodes);
+    else
+        k_solve<false><<<blocks, 256, 0, s>>>((float2 *)m->spec, m->G, m->Vc, m->acc, m->K1, m->K1h, m->nmodes,
+                                              m->gridA, m->nnodes);
+    PD_LAUNCHED();
+    PD_CUFFT(cufftSetStream(m->bwd, s));
+    if (ik) {
+        for (int d = 0; d < 3; ++d) {
+            k_ik_field<<<blocks, 256, 0, s>>>((float2 *)m->scratch, (const float2 *)m->spec, m->K1, m->K2, m->K3,
+                                              (float)m->box[d], d);
+            PD_LAUNCHED();
+            PD_CUFFT(cufftExecC2R(m->bwd, m->scratch, m->field[d]));
+        }
+        if (!energy) return PD_OK;
+    }
+    PD_CUFFT(cufftExecC2R(m->bwd, m->spec, m->gridB));
+    return PD_OK;
+}
+
 // Fill m->self_tab (T = m->self_T) for the current box and influence function (host boundary: runs on
 // the legacy stream and waits for it).  Leaves the charge grid zero, as every transform does.
 static int compute_self_table(pd_mesh *m) {
@@ -468,13 +506,8 @@ static int compute_self_table(pd_mesh *m) {
     cudaStream_t s = 0;
     k_unit_node<<<1, 1, 0, s>>>(m->gridA);
     PD_LAUNCHED();
-    PD_CUFFT(cufftSetStream(m->fwd, s));
-    PD_CUFFT(cufftExecR2C(m->fwd, m->gridA, m->spec));
-    k_solve<false><<<(m->nmodes + 255) / 256, 256, 0, s>>>((float2 *)m->spec, m->G, m->Vc, m->acc, m->K1, m->K1h,
-                                                            m->nmodes, m->gridA, m->nnodes);
-    PD_LAUNCHED();
-    PD_CUFFT(cufftSetStream(m->bwd, s));
-    PD_CUFFT(cufftExecC2R(m->bwd, m->spec, m->gridB));
+    int rc;
+    if ((rc = mesh_solve_grids(m, 0, s, nullptr))) return rc;
     const int T = m->self_T, cells = T * T * T;
     const float s1 = (float)(m->K1 / m->box[0]), s2 = (float)(m->K2 / m->box[1]), s3 = (float)(m->K3 / m->box[2]);
 #define PD_ST(PP)                                                                                             \
@@ -505,33 +538,7 @@ int mesh_transform_packed(pd_mesh *m, const float4 *xq, int nchunks, const int *
                                      window_poly(m), s);
     PD_LAUNCHED();
     if (ev_spread) PD_CUDA(cudaEventRecord(ev_spread, s));
-    PD_CUFFT(cufftSetStream(m->fwd, s));
-    PD_CUFFT(cufftExecR2C(m->fwd, m->gridA, m->spec));
-    if (ev_r2c) PD_CUDA(cudaEventRecord(ev_r2c, s));
-    if (energy) PD_CUDA(cudaMemsetAsync(m->acc, 0, 7 * sizeof(double), s));
-    const int blocks = (m->nmodes + 255) / 256;
-    if (energy)
-        k_solve<true><<<blocks, 256, 0, s>>>((float2 *)m->spec, m->G, m->Vc, m->acc, m->K1, m->K1h, m->nmodes, m->gridA,
-                                             m->nnodes);
-    else
-        k_solve<false><<<blocks, 256, 0, s>>>((float2 *)m->spec, m->G, m->Vc, m->acc, m->K1, m->K1h, m->nmodes,
-                                              m->gridA, m->nnodes);
-    PD_LAUNCHED();
-    PD_CUFFT(cufftSetStream(m->bwd, s));
-    if (m->p.kind == PD_MESH_P3M_IK) {
-        const float L[3] = {Lx, Ly, Lz};
-        for (int d = 0; d < 3; ++d) {
-            k_ik_field<<<blocks, 256, 0, s>>>((float2 *)m->scratch, (const float2 *)m->spec, m->K1, m->K2, m->K3, L[d], d);
-            PD_LAUNCHED();
-            PD_CUFFT(cufftExecC2R(m->bwd, m->scratch, m->field[d]));
-        }
-        if (energy) {
-            PD_CUFFT(cufftExecC2R(m->bwd, m->spec, m->gridB));
-        }
-    } else {
-        PD_CUFFT(cufftExecC2R(m->bwd, m->spec, m->gridB));
-    }
-    return PD_OK;
+    return mesh_solve_grids(m, energy, s, ev_r2c);
 }
 
 int mesh_store_virial(pd_mesh *m, float *vglobal6, cudaStream_t s) {
@@ -610,6 +617,7 @@ static void free_mesh(pd_mesh *m) {
     dfree(m->packed);
     dfree(m->self_tab);
     m->self_T = 0;
+    for (int d = 0; d < 3; ++d) dfree(m->tw[d]);
     dfree(m->xq);
     dfree(m->wchi);
     dfree(m->wpoly);
@@ -657,6 +665,51 @@ int copy_prolate(pd_mesh *m, const pd_prolate *w) {
     return PD_OK;
 }
 
+// cuFFT plans with a library-owned work area (Solver.jl:48-49: plan_rfft / plan_brfft), for meshes with an
+// axis that this library's transforms do not take.
+int make_plans(pd_mesh *m) {
+    size_t ws1 = 0, ws2 = 0;
+    PD_CHECK(cufftCreate(&m->fwd) == CUFFT_SUCCESS && cufftCreate(&m->bwd) == CUFFT_SUCCESS, PD_ECUFFT,
+             "cufftCreate failed");
+    m->plans = true;
+    PD_CHECK(cufftSetAutoAllocation(m->fwd, 0) == CUFFT_SUCCESS && cufftSetAutoAllocation(m->bwd, 0) == CUFFT_SUCCESS &&
+                 cufftMakePlan3d(m->fwd, m->K3, m->K2, m->K1, CUFFT_R2C, &ws1) == CUFFT_SUCCESS &&
+                 cufftMakePlan3d(m->bwd, m->K3, m->K2, m->K1, CUFFT_C2R, &ws2) == CUFFT_SUCCESS,
+             PD_ECUFFT, "cuFFT plan creation failed for mesh %d x %d x %d", m->K1, m->K2, m->K3);
+    m->work_size = std::max(ws1, ws2);
+    PD_CHECK(m->work_size == 0 || cudaMalloc(&m->work, m->work_size) == cudaSuccess, PD_ENOMEM,
+             "cuFFT work area allocation failed");
+    cufftSetWorkArea(m->fwd, m->work);
+    cufftSetWorkArea(m->bwd, m->work);
+    return PD_OK;
+}
+
+// Twiddle tables and the transform description of a mesh on this library's transforms.
+int make_transforms(pd_mesh *m) {
+    int rc;
+    if ((rc = fft_init())) return rc;
+    FftMesh &f = m->fft;
+    for (int d = 0; d < 3; ++d) {
+        if ((rc = fft_twiddles(f.ax[d].n, &m->tw[d]))) return rc;
+        f.ax[d].w = m->tw[d];
+    }
+    f.grid = m->gridA;
+    f.spec = (float2 *)m->spec;
+    f.G = m->G;
+    if (m->p.kind == PD_MESH_P3M_IK) {
+        for (int d = 0; d < 3; ++d) {
+            f.zspec[d] = (float2 *)m->scratch + (size_t)d * m->nmodes;
+            f.out[d] = m->field[d];
+        }
+        f.zspec[3] = f.spec;
+        f.out[3] = m->gridB;
+    } else {
+        f.zspec[0] = f.spec;
+        f.out[0] = m->gridB;
+    }
+    return PD_OK;
+}
+
 int mesh_create(pd_mesh **out, const pd_mesh_params *p, const pd_prolate *w, const double box[3]) {
     const bool esp = w != nullptr;
     for (int d = 0; d < 3; ++d)
@@ -673,6 +726,7 @@ int mesh_create(pd_mesh **out, const pd_mesh_params *p, const pd_prolate *w, con
     m->nnodes = (int)nnodes;
     m->nmodes = (int)nmodes;
     const bool ik = p->kind == PD_MESH_P3M_IK;
+    m->route = fft_route(p->mesh, &m->fft);
     int rc;
     if ((rc = dalloc(&m->gridA, (size_t)nnodes)) || (rc = dalloc(&m->gridB, (size_t)nnodes)) ||
         (rc = dalloc(&m->spec, (size_t)nmodes)) || (rc = dalloc(&m->G, (size_t)nmodes)) ||
@@ -683,7 +737,8 @@ int mesh_create(pd_mesh **out, const pd_mesh_params *p, const pd_prolate *w, con
     }
     if (ik) {
         if ((rc = dalloc(&m->field[0], (size_t)nnodes)) || (rc = dalloc(&m->field[1], (size_t)nnodes)) ||
-            (rc = dalloc(&m->field[2], (size_t)nnodes)) || (rc = dalloc(&m->scratch, (size_t)nmodes))) {
+            (rc = dalloc(&m->field[2], (size_t)nnodes)) ||
+            (rc = dalloc(&m->scratch, (size_t)nmodes * (m->route == FFT_CUFFT ? 1 : 3)))) {
             free_mesh(m);
             delete m;
             return rc;
@@ -698,30 +753,11 @@ int mesh_create(pd_mesh **out, const pd_mesh_params *p, const pd_prolate *w, con
     cudaMemset(m->gridA, 0, sizeof(float) * (size_t)nnodes);
     cudaMemset(m->gridB, 0, sizeof(float) * (size_t)nnodes);
     cudaMemset(m->acc, 0, 8 * sizeof(double));
-    // cuFFT plans with a library-owned work area (Solver.jl:48-49: plan_rfft / plan_brfft)
-    size_t ws1 = 0, ws2 = 0;
-    bool ok = cufftCreate(&m->fwd) == CUFFT_SUCCESS && cufftCreate(&m->bwd) == CUFFT_SUCCESS;
-    if (ok) {
-        m->plans = true;
-        ok = cufftSetAutoAllocation(m->fwd, 0) == CUFFT_SUCCESS && cufftSetAutoAllocation(m->bwd, 0) == CUFFT_SUCCESS &&
-             cufftMakePlan3d(m->fwd, m->K3, m->K2, m->K1, CUFFT_R2C, &ws1) == CUFFT_SUCCESS &&
-             cufftMakePlan3d(m->bwd, m->K3, m->K2, m->K1, CUFFT_C2R, &ws2) == CUFFT_SUCCESS;
-    }
-    if (!ok) {
-        set_error("cuFFT plan creation failed for mesh %d x %d x %d", m->K1, m->K2, m->K3);
+    if (m->route == FFT_CUFFT ? (rc = make_plans(m)) : (rc = make_transforms(m))) {
         free_mesh(m);
         delete m;
-        return PD_ECUFFT;
+        return rc;
     }
-    m->work_size = std::max(ws1, ws2);
-    if (m->work_size > 0 && cudaMalloc(&m->work, m->work_size) != cudaSuccess) {
-        set_error("cuFFT work area allocation failed");
-        free_mesh(m);
-        delete m;
-        return PD_ENOMEM;
-    }
-    cufftSetWorkArea(m->fwd, m->work);
-    cufftSetWorkArea(m->bwd, m->work);
     if ((esp && (rc = copy_prolate(m, w))) || (rc = pd_mesh_set_box(m, box))) {
         free_mesh(m);
         delete m;
@@ -780,7 +816,11 @@ int pd_mesh_set_box(pd_mesh *m, const double box[3]) {
     PD_CHECK(m && box, PD_EINVAL, "pd_mesh_set_box: null argument");
     for (int d = 0; d < 3; ++d)
         PD_CHECK(std::isfinite(box[d]) && box[d] > 0, PD_EINVAL, "box lengths must be finite and positive");
-    for (int d = 0; d < 3; ++d) m->box[d] = box[d];
+    for (int d = 0; d < 3; ++d) {
+        m->box[d] = box[d];
+        m->fft.kd[d] = (float)(2.0 * M_PI / box[d]);
+    }
+    ++m->epoch;   // captured steps hold the old wave-vector units
     int rc = compute_influence(m);
     if (rc) return rc;
     refresh_background(m);
