@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
+#include "rows.cuh"
 
 #include <algorithm>
 #include <numeric>
@@ -43,7 +44,6 @@ using namespace pdb;
 namespace pdb {
 
 constexpr int B_THREADS = 256;
-constexpr int BROWS_WARPS = 4, BROWS_CAP = 640;
 
 struct BatchRep {
     float L[3];
@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, float *__restr
                                                            const int *__restrict__ rep_of,
                                                            const BatchRep *__restrict__ reps,
                                                            const float4 *__restrict__ ref, float threshold,
+                                                           const int *__restrict__ pos_of, float4 *__restrict__ xq,
                                                            unsigned *__restrict__ rep_dmax, int *__restrict__ rep_flag,
                                                            int nrep, long long *__restrict__ st,
                                                            cudaGraphConditionalHandle h) {
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, float *__restr
             x[i] = p[0];
             y[i] = p[1];
             z[i] = p[2];
+            if (pos_of) xq[pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);   // packed for the pair pass
         }
         v = ell_displacement<3>(p, ref[i], L, st[E_VALID] != 0);
     }
@@ -186,164 +188,37 @@ __global__ void k_batch_bin(const float *__restrict__ x, const float *__restrict
     atomicAdd(&cell_count[c], 1);
 }
 
-// Rows, one warp per global cell: the replica's stencil (same visiting order as the single-system
-// row kernels) staged in shared memory once per cell, each lane taking up to M particles of the cell
-// (lane, lane + 32, ...), so a cell of up to 32 M particles stages its candidates once.
-// The candidates come from the packed coordinates in cell order (xq, packed after the sort of this
-// rebuild), so a stencil row's candidates are one contiguous, coalesced float4 run.  Rows, their
-// lengths and their entries are in cell order (positions in `sorted`), so the row stores of a warp and
-// the pair kernel's row loads are contiguous and neighbours' packed records sit close together; a
-// particle's entries are appended in the candidates' visiting order, as in the single-system kernels.
-template <int M>   // particles per lane (1, 2 or 4), from the batch's mean cell occupancy
-__global__ void __launch_bounds__(32 * BROWS_WARPS) k_batch_rows(
-    const float4 *__restrict__ xq, int n, int ncell, const int *__restrict__ cell_rep,
+// Rows of the flagged replicas' cells, nsplit warps per global cell (rows.cuh): rows, their lengths and their
+// entries are in cell order (positions in `sorted`).
+__global__ void __launch_bounds__(32 * ROWS_WARPS) k_batch_rows(
+    const float4 *__restrict__ xq, int ncell, int nsplit, const int *__restrict__ cell_rep,
     const BatchRep *__restrict__ reps, const int *__restrict__ rep_flag, const int *__restrict__ sorted,
     const int *__restrict__ cell_off, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts,
     float4 *__restrict__ ref, long long *__restrict__ st) {
     if (!ell_requested(st)) return;
     extern __shared__ float4 batch_stage[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x * BROWS_WARPS + w;
-    float4 *sw = batch_stage + w * BROWS_CAP;
+    const int w = threadIdx.x >> 5;
+    const int item = blockIdx.x * ROWS_WARPS + w, c = item / nsplit;
     unsigned fmax = 0;
-    if (c < ncell && rep_flag[__ldg(cell_rep + c)]) {   // warp-uniform; only replicas being rebuilt
-        const BatchRep &R = reps[__ldg(cell_rep + c)];
-        const float Lx = R.L[0], Ly = R.L[1], Lz = R.L[2];
-        const int nx = R.nx, ny = R.ny, nz = R.nz, base = R.cell_base;
-        const float hLx = 0.5f * Lx, hLy = 0.5f * Ly, hLz = 0.5f * Lz;
-        const float rl = sqrtf(rl2);
-        const float hx = Lx / (float)nx, hy = Ly / (float)ny, hz = Lz / (float)nz;
-        const int Sx = ell_reach(rl, Lx, nx), Sy = ell_reach(rl, Ly, ny), Sz = ell_reach(rl, Lz, nz);
-        const int lc = c - base;
-        const int cx = lc % nx, tmp = lc / nx, cy = tmp % ny, cz = tmp / ny;
-        const int p0 = cell_off[c], pn = cell_off[c + 1] - p0;
-        for (int pg = 0; pg < pn; pg += 32 * M) {
-            int kp[M], found[M];
-            bool has[M];
-            float xi[M], yi[M], zi[M];
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-                has[m] = pg + lane + 32 * m < pn;
-                kp[m] = p0 + pg + lane + 32 * m;   // this lane's m-th particle: its position in cell order
-                const float4 v = has[m] ? xq[kp[m]] : make_float4(0.f, 0.f, 0.f, 0.f);
-                xi[m] = v.x;
-                yi[m] = v.y;
-                zi[m] = v.z;
-                found[m] = 0;
-            }
-            // bounding box of this group's particles: a candidate farther than the list radius from the
-            // box is farther from every particle of the group, so it is not staged (a conservative
-            // margin keeps rounding from dropping a candidate that the exact test would accept)
-            float blo[3] = {INFINITY, INFINITY, INFINITY}, bhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-                if (!has[m]) continue;
-                blo[0] = fminf(blo[0], xi[m]);
-                blo[1] = fminf(blo[1], yi[m]);
-                blo[2] = fminf(blo[2], zi[m]);
-                bhi[0] = fmaxf(bhi[0], xi[m]);
-                bhi[1] = fmaxf(bhi[1], yi[m]);
-                bhi[2] = fmaxf(bhi[2], zi[m]);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    blo[d] = fminf(blo[d], __shfl_xor_sync(0xffffffffu, blo[d], off));
-                    bhi[d] = fmaxf(bhi[d], __shfl_xor_sync(0xffffffffu, bhi[d], off));
-                }
-            }
-            const float bcx = 0.5f * (blo[0] + bhi[0]), bcy = 0.5f * (blo[1] + bhi[1]), bcz = 0.5f * (blo[2] + bhi[2]);
-            const float bhx = 0.5f * (bhi[0] - blo[0]), bhy = 0.5f * (bhi[1] - blo[1]), bhz = 0.5f * (bhi[2] - blo[2]);
-            const float rbox = rl * 1.0001f + 1e-3f;
-            const float rbox2 = rbox * rbox;
-            int fill = 0;
-            // scan of the staged candidates by every particle of the lane (one body, expanded where a
-            // full stage buffer is flushed and at the end, so the per-particle counters stay in registers)
-#define PD_BATCH_ROWS_SCAN                                                            \
-    do {                                                                              \
-        __syncwarp();                                                                 \
-        for (int t = 0; t < fill; ++t) {                                              \
-            const float4 cj = sw[t];                                                  \
-            const int kc = __float_as_int(cj.w);                                      \
-            _Pragma("unroll") for (int m = 0; m < M; ++m) {                           \
-                if (!has[m] || kc == kp[m]) continue;                                 \
-                const float dx = mic_fast(cj.x - xi[m], hLx, Lx);                     \
-                const float dy = mic_fast(cj.y - yi[m], hLy, Ly);                     \
-                const float dz = mic_fast(cj.z - zi[m], hLz, Lz);                     \
-                const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));                 \
-                if (r2 <= rl2) {                                                      \
-                    if (found[m] < cap) rows[(size_t)found[m] * n + kp[m]] = kc;      \
-                    ++found[m];                                                       \
-                }                                                                     \
-            }                                                                         \
-        }                                                                             \
-        __syncwarp();                                                                 \
-        fill = 0;                                                                     \
-    } while (0)
-            for (int oz = -Sz; oz <= Sz; ++oz) {
-                int cz2 = cz + oz;
-                cz2 -= cz2 >= nz ? nz : 0;
-                cz2 += cz2 < 0 ? nz : 0;
-                const float gz = (float)max(abs(oz) - 1, 0) * hz;
-                for (int oy = -Sy; oy <= Sy; ++oy) {
-                    int cy2 = cy + oy;
-                    cy2 -= cy2 >= ny ? ny : 0;
-                    cy2 += cy2 < 0 ? ny : 0;
-                    const float gy = (float)max(abs(oy) - 1, 0) * hy;
-                    const float g2 = fmaf(gy, gy, gz * gz);
-                    if (g2 > rl2) continue;
-                    const int row = base + (cz2 * ny + cy2) * nx;
-                    int a1, b1, a2, b2;
-                    ell_row_ranges(cx, g2, rl2, hx, Sx, nx, a1, b1, a2, b2);
-                    for (int part = 0; part < 2; ++part) {
-                        if (part == 1 && a2 > b2) break;
-                        const int ka = cell_off[row + (part ? a2 : a1)], kb = cell_off[row + (part ? b2 : b1) + 1];
-                        for (int k0 = ka; k0 < kb; k0 += 32) {
-                            const bool in = lane < kb - k0;
-                            float4 v = in ? xq[k0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-                            const float ex = fmaxf(fabsf(mic_fast(v.x - bcx, hLx, Lx)) - bhx, 0.f);
-                            const float ey = fmaxf(fabsf(mic_fast(v.y - bcy, hLy, Ly)) - bhy, 0.f);
-                            const float ez = fmaxf(fabsf(mic_fast(v.z - bcz, hLz, Lz)) - bhz, 0.f);
-                            const bool keep = in && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= rbox2;
-                            const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                            const int nk = __popc(bal);
-                            if (fill + nk > BROWS_CAP) PD_BATCH_ROWS_SCAN;
-                            if (keep) {   // staged in the candidates' order
-                                v.w = __int_as_float(k0 + lane);
-                                sw[fill + __popc(bal & ((1u << lane) - 1u))] = v;
-                            }
-                            fill += nk;
-                        }
-                    }
-                }
-            }
-            PD_BATCH_ROWS_SCAN;
-#undef PD_BATCH_ROWS_SCAN
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-                if (has[m]) {
-                    counts[kp[m]] = found[m];
-                    ref[sorted[kp[m]]] = make_float4(xi[m], yi[m], zi[m], 0.f);
-                }
-                fmax = max(fmax, (unsigned)found[m]);
-            }
+    if (c < ncell) {
+        const int r = __ldg(cell_rep + c);
+        if (rep_flag[r]) {   // warp-uniform; only replicas being rebuilt
+            const BatchRep &R = reps[r];
+            const RowGrid g{{R.L[0], R.L[1], R.L[2]}, R.nx, R.ny, R.nz, R.cell_base};
+            fmax = cell_rows<3>(g, c - g.base, item - c * nsplit, nsplit, xq, sorted, cell_off, rl2, cap, rows, counts,
+                                ref, batch_stage + w * ROWS_CAP);
         }
     }
-    if (ell_block_max_last(fmax, st, E_RMAX, E_TICKET_R)) {
-        const long long largest = st[E_RMAX];
-        st[E_RMAX] = 0;
-        st[E_TICKET_R] = 0;
-        st[E_REQUIRED] = largest;
-        if (largest > cap) {
-            st[E_ERROR] = E_ERR_CAPACITY;
-            st[E_VALID] = 0;
-        } else {
-            st[E_VALID] = 1;
-            st[E_LAST_BUILD] = st[E_STEP];
-            st[E_BUILDS] += 1;
-        }
-    }
+    if (ell_block_max_last(fmax, st, E_RMAX, E_TICKET_R)) rows_commit(st, cap);
+}
+
+// The rows in the exported layout (slot t of position k at t n + k) for callers that read them.
+__global__ void k_batch_export(const int *__restrict__ rows, const int *__restrict__ counts, int n, int cap,
+                               int *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int c = min(counts[k], cap);
+    for (int t = 0; t < c; ++t) out[(size_t)t * n + k] = rows[(size_t)k * cap + t];
 }
 
 // Packed coordinates (and charges, when q is given) in cell order: xq[k] = (x, y, z, q) of particle
@@ -352,11 +227,12 @@ __global__ void __launch_bounds__(32 * BROWS_WARPS) k_batch_rows(
 template <bool REBUILD>
 __global__ void k_batch_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                              const float *__restrict__ q, const int *__restrict__ sorted, int n,
-                             float4 *__restrict__ xq, const long long *__restrict__ st) {
+                             int *__restrict__ pos_of, float4 *__restrict__ xq, const long long *__restrict__ st) {
     if (REBUILD ? !ell_requested(st) : st[E_VALID] == 0) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = sorted[k];
+    if (REBUILD) pos_of[i] = k;
     xq[k] = make_float4(x[i], y[i], z[i], q ? q[i] : 0.f);
 }
 
@@ -378,94 +254,101 @@ struct BatchCoul {
 };
 
 // Row pair kernel over all replicas: the model of particle i's replica (LJ or WCA, the ELL route's
-// UniformLJ / UniformWCA arithmetic), forces stored, optional energy (half of each pair), the
-// closing half kick fused.  The packed coordinates are refreshed by the pack of the same stage.
+// UniformLJ / UniformWCA arithmetic), forces stored, optional energy (half of each pair).  G lanes per row.
+// The packed coordinates are refreshed by the pack of the same stage.
 // COUL: the packed records carry the charges (xq.w) and the pair adds the Coulomb polynomial term,
 // evaluated with NP coefficients (the fitted ones, zeros above them); one reciprocal square root
 // serves both terms.
-template <int G, bool ENERGY, bool COUL, int NP = BATCH_NP>
-__global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restrict__ xq, int n,
+// SLOT: forces (and the energy) are stored by position in fc, one coalesced record, for the kernel that carries
+// them to particle order with the closing half kick (k_batch_finish, or the charged replicas' gather).
+template <int G, bool ENERGY, bool COUL, bool SLOT, int NP = BATCH_NP>
+__global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restrict__ xq, int n, int cap,
                                                            const int *__restrict__ rows,
                                                            const int *__restrict__ counts,
                                                            const int *__restrict__ sorted,
                                                            const int *__restrict__ rep_of,
                                                            const BatchRep *__restrict__ reps, float *__restrict__ fx,
                                                            float *__restrict__ fy, float *__restrict__ fz,
-                                                           float *__restrict__ epot, BatchKick kick,
-                                                           long long *__restrict__ st, int advance,
+                                                           float *__restrict__ epot, float4 *__restrict__ fc,
+                                                           BatchKick kick, long long *__restrict__ st, int advance,
                                                            const __grid_constant__ BatchCoul cp) {
     if (st[E_VALID] == 0) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = tid / G, lane = tid % G;   // position in cell order
     const int i = k < n ? sorted[k] : -1;
     float a[3] = {0.f, 0.f, 0.f}, e = 0.f;
-    if (k < n) {
-        const BatchRep &R = reps[__ldg(rep_of + i)];
-        const float Lx = R.L[0], Ly = R.L[1], Lz = R.L[2];
-        const float hLx = 0.5f * Lx, hLy = 0.5f * Ly, hLz = 0.5f * Lz;
-        const float eps = R.eps, sig2 = R.sig2, rc2 = R.rc2;
-        const float eoff = R.kind == PD_PAIR_WCA ? R.eps : -R.eshift;
-        const float4 pi = xq[k];
-        const int cnt = counts[k];
-        const float cqi = COUL ? cp.C * pi.w : 0.f;
-        const float cut2 = COUL ? fmaxf(rc2, cp.rc2) : rc2;
-        auto pair = [&](float4 pj) {
-            const float dx = periodic_delta(pi.x, pj.x, hLx, Lx);
-            const float dy = periodic_delta(pi.y, pj.y, hLy, Ly);
-            const float dz = periodic_delta(pi.z, pj.z, hLz, Lz);
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            if (COUL) {
-                if (!(r2 > 0.f && r2 < cut2)) return;
-                const float rinv = rsqrtf(r2);
-                const float ir2 = rinv * rinv;
-                float fr = 0.f;
-                if (r2 < rc2) {
-                    const float s2 = sig2 * ir2;
-                    const float s6 = s2 * s2 * s2;
-                    const float s12 = s6 * s6;
-                    fr = 24.f * eps * (2.f * s12 - s6) * ir2;
-                    if (ENERGY) e += 0.5f * (4.f * eps * (s12 - s6) + eoff);
-                }
-                if (r2 < cp.rc2) {
-                    const float x = fmaf(r2, cp.sx, -1.f);
-                    float pf = cp.pf[NP - 1];
+    const BatchRep &R = reps[k < n ? __ldg(rep_of + i) : 0];
+    const float L[3] = {R.L[0], R.L[1], R.L[2]};
+    const float rc2 = R.rc2;
+    const LjRow lj = lj_row(R.eps, R.sig2, rc2, R.kind == PD_PAIR_WCA ? R.eps : -R.eshift);
+    const float4 pi = k < n ? xq[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int cnt = k < n ? counts[k] : 0;
+    const float cqi = COUL ? cp.C * pi.w : 0.f;
+    const float cut2 = COUL ? fmaxf(rc2, cp.rc2) : rc2;
+    f2 npf[COUL ? NP : 1];   // minus the force polynomial
+    if (COUL) {
 #pragma unroll
-                    for (int t = NP - 2; t >= 0; --t) pf = fmaf(pf, x, cp.pf[t]);
-                    const float cq = cqi * pj.w;
-                    fr = fmaf(cq, rinv * ir2 - pf, fr);
-                    if (ENERGY) {
-                        float pe = cp.pe[NP - 1];
-#pragma unroll
-                        for (int t = NP - 2; t >= 0; --t) pe = fmaf(pe, x, cp.pe[t]);
-                        e = fmaf(0.5f * cq, rinv + pe - cp.eshift, e);
-                    }
-                }
-                a[0] = fmaf(fr, dx, a[0]);
-                a[1] = fmaf(fr, dy, a[1]);
-                a[2] = fmaf(fr, dz, a[2]);
-                return;
-            }
-            if (r2 > 0.f && r2 < rc2) {
-                const float ir2 = 1.f / r2;
-                const float s2 = sig2 * ir2;
-                const float s6 = s2 * s2 * s2;
-                const float s12 = s6 * s6;
-                const float fr = 24.f * eps * (2.f * s12 - s6) * ir2;
-                a[0] += fr * dx;
-                a[1] += fr * dy;
-                a[2] += fr * dz;
-                if (ENERGY) e += 0.5f * (4.f * eps * (s12 - s6) + eoff);
-            }
-        };
-        int slot = lane;
-        for (; slot + G < cnt; slot += 2 * G) {
-            const float4 p1 = xq[rows[(size_t)slot * n + k]];
-            const float4 p2 = xq[rows[(size_t)(slot + G) * n + k]];
-            pair(p1);
-            pair(p2);
-        }
-        for (; slot < cnt; slot += G) pair(xq[rows[(size_t)slot * n + k]]);
+        for (int t = 0; t < NP; ++t) npf[t] = pk_held(-cp.pf[t]);
     }
+    auto walk = [&](auto wrap) {
+        constexpr bool WRAP = decltype(wrap)::value;
+        walk_row<G, true>(rows + (size_t)k * cap, 1, lane, cnt, k, xq, [&](const float4 &pa, const float4 &pb) {
+            float dx[2], dy[2], dz[2], r2[2], f[2], u[2];
+            pair_delta<3, WRAP>(pi, pa, L, dx[0], dy[0], dz[0]);
+            pair_delta<3, WRAP>(pi, pb, L, dx[1], dy[1], dz[1]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) r2[c] = fmaf(dx[c], dx[c], fmaf(dy[c], dy[c], dz[c] * dz[c]));
+            const f2 r22 = pk(r2[0], r2[1]);
+            f2 fr, un, rinv, ir2;
+            if (COUL) {
+                rinv = pk(rsqrt_fast(r2[0]), rsqrt_fast(r2[1]));
+                ir2 = mul2(rinv, rinv);
+            } else {
+                ir2 = rcp2(r22);
+            }
+            lj_two<ENERGY>(lj, ir2, fr, un);
+            unpk(fr, f[0], f[1]);
+            if (ENERGY) unpk(un, u[0], u[1]);
+            bool in[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                in[c] = r2[c] > 0.f && r2[c] < rc2;
+                f[c] = in[c] ? f[c] : 0.f;
+                if (ENERGY) e += in[c] ? 0.5f * u[c] : 0.f;
+            }
+            if (COUL) {
+                const f2 x = fma2(r22, pk(cp.sx), pk(-1.f));
+                f2 g = npf[NP - 1];
+#pragma unroll
+                for (int t = NP - 2; t >= 0; --t) g = fma2(g, x, npf[t]);
+                float q[2], h[2];
+                unpk(fma2(rinv, ir2, g), h[0], h[1]);
+                unpk(mul2(pk(cqi), pk(pa.w, pb.w)), q[0], q[1]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    in[c] = r2[c] > 0.f && r2[c] < cp.rc2;
+                    f[c] = fmaf(q[c], in[c] ? h[c] : 0.f, f[c]);
+                }
+                if (ENERGY) {
+                    f2 pe = pk(cp.pe[NP - 1]);
+#pragma unroll
+                    for (int t = NP - 2; t >= 0; --t) pe = fma2(pe, x, pk(cp.pe[t]));
+                    unpk(add2(add2(rinv, pe), pk(-cp.eshift)), h[0], h[1]);
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) e = fmaf(0.5f * q[c], in[c] ? h[c] : 0.f, e);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                a[0] = fmaf(f[c], dx[c], a[0]);
+                a[1] = fmaf(f[c], dy[c], a[1]);
+                a[2] = fmaf(f[c], dz[c], a[2]);
+            }
+        });
+    };
+    // the margin keeps the faces farther than the cutoff by more than the coordinates' rounding
+    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, 1.001f * sqrtf(cut2)))) walk(std::false_type{});
+    else walk(std::true_type{});
 #pragma unroll
     for (int off = G / 2; off > 0; off >>= 1) {
 #pragma unroll
@@ -473,15 +356,44 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
         if (ENERGY) e += __shfl_down_sync(0xffffffffu, e, off, G);
     }
     if (lane == 0 && k < n) {
-        fx[i] = a[0];
-        fy[i] = a[1];
-        fz[i] = a[2];
-        if (ENERGY) epot[i] = e;
+        if (SLOT) {
+            fc[k] = make_float4(a[0], a[1], a[2], e);
+        } else {
+            fx[i] = a[0];
+            fy[i] = a[1];
+            fz[i] = a[2];
+            if (ENERGY) epot[i] = e;
+            if (kick.on) {
+                const float c = kick.half_dt * kick.inv_mass[i];
+                kick.vx[i] = fmaf(c, a[0], kick.vx[i]);
+                kick.vy[i] = fmaf(c, a[1], kick.vy[i]);
+                kick.vz[i] = fmaf(c, a[2], kick.vz[i]);
+            }
+        }
+    }
+    if (advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
+}
+
+// Positions' forces to particle order, with the closing half kick when there is one.
+template <bool ENERGY>
+__global__ void __launch_bounds__(B_THREADS) k_batch_finish(const float4 *__restrict__ fc,
+                                                            const int *__restrict__ pos_of, int n,
+                                                            float *__restrict__ fx, float *__restrict__ fy,
+                                                            float *__restrict__ fz, float *__restrict__ epot,
+                                                            BatchKick kick, long long *__restrict__ st, int advance) {
+    if (st[E_VALID] == 0) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        const float4 f = fc[pos_of[i]];
+        fx[i] = f.x;
+        fy[i] = f.y;
+        fz[i] = f.z;
+        if (ENERGY) epot[i] = f.w;
         if (kick.on) {
             const float c = kick.half_dt * kick.inv_mass[i];
-            kick.vx[i] = fmaf(c, a[0], kick.vx[i]);
-            kick.vy[i] = fmaf(c, a[1], kick.vy[i]);
-            kick.vz[i] = fmaf(c, a[2], kick.vz[i]);
+            kick.vx[i] = fmaf(c, f.x, kick.vx[i]);
+            kick.vy[i] = fmaf(c, f.y, kick.vy[i]);
+            kick.vz[i] = fmaf(c, f.z, kick.vz[i]);
         }
     }
     if (advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
@@ -491,6 +403,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
 
 struct pd_batch {
     int nrep = 0, n = 0, ncell = 0, cap = 0, lanes = 4;
+    double mean_row = 0.0;           // expected entries per row at the replicas' densities
     float rl2 = 0.f, threshold = 0.f;
     std::vector<BatchRep> hreps;
     std::vector<int> first;
@@ -501,7 +414,9 @@ struct pd_batch {
     long long *st = nullptr;
     int *cell_of = nullptr, *cell_count = nullptr, *cell_off = nullptr, *sorted = nullptr, *tmp = nullptr;
     int *rows = nullptr, *counts = nullptr;
-    float4 *ref = nullptr, *xq = nullptr;
+    int *pos_of = nullptr, *scan_part = nullptr;   // inverse of sorted; tile sums of the cell scan
+    int *xrows = nullptr;            // rows in the exported layout, kept current once pd_batch_rows was called
+    float4 *ref = nullptr, *xq = nullptr, *fc = nullptr;
     // bound state (pd_batch_bind)
     pd_md_state state;
     bool bound = false;
@@ -533,6 +448,12 @@ struct pd_batch {
         cufftHandle fwd, bwd;
     };
     std::vector<FftGroup> groups;
+    // every replica's mesh on this library's transforms: three launches for the whole set (fft.tab set);
+    // otherwise the cuFFT groups
+    FftBatch fft{};
+    FftMesh *fft_tab = nullptr;
+    int2 *fft_planes = nullptr, *fft_cols = nullptr;
+    std::vector<float2 *> twiddles;
     // the mesh sizes' transforms run on NFFT streams at once, group g on stream g % NFFT with that
     // stream's own cuFFT work area
     static constexpr int NFFT = 4;
@@ -560,6 +481,12 @@ static void batch_free_mesh(pd_batch *b) {
         if (g.bwd) cufftDestroy(g.bwd);
     }
     b->groups.clear();
+    for (auto &w : b->twiddles) dfree(w);
+    b->twiddles.clear();
+    dfree(b->fft_tab);
+    dfree(b->fft_planes);
+    dfree(b->fft_cols);
+    b->fft = FftBatch{};
     batch_free_chunks(b);
     dfree(b->mreps);
     dfree(b->gridA);
@@ -605,6 +532,10 @@ static void batch_free(pd_batch *b) {
     dfree(b->counts);
     dfree(b->ref);
     dfree(b->xq);
+    dfree(b->fc);
+    dfree(b->pos_of);
+    dfree(b->scan_part);
+    dfree(b->xrows);
 }
 
 static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, const float *z, cudaStream_t s) {
@@ -613,43 +544,47 @@ static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, con
                                              b->cell_count, b->st);
     PD_LAUNCHED();
     int rc;
-    if ((rc = ell_sort_cells_launch(b->cell_of, b->n, b->ncell, b->cell_count, b->cell_off, b->sorted, b->tmp, b->st,
-                                    s)))
+    if ((rc = ell_sort_launch(b->cell_of, b->n, b->ncell, b->cell_count, b->cell_off, b->scan_part, b->sorted, b->tmp,
+                              b->st, s)))
         return rc;
-    k_batch_pack<true><<<(b->n + B_THREADS - 1) / B_THREADS, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n,
-                                                                                b->xq, b->st);
+    k_batch_pack<true><<<blocks, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
     PD_LAUNCHED();
-    // particles per lane: enough lanes for a cell of 1.3x the mean occupancy
-    const double occ = 1.3 * (double)b->n / (double)std::max(b->ncell, 1);
-    const dim3 grid((b->ncell + BROWS_WARPS - 1) / BROWS_WARPS), block(32 * BROWS_WARPS);
-    const size_t shm = sizeof(float4) * BROWS_WARPS * BROWS_CAP;
-    if (occ <= 32.0)
-        k_batch_rows<1><<<grid, block, shm, s>>>(b->xq, b->n, b->ncell, b->cell_rep, b->reps, b->rep_flag, b->sorted,
-                                                 b->cell_off, b->rl2, b->cap, b->rows, b->counts, b->ref, b->st);
-    else if (occ <= 64.0)
-        k_batch_rows<2><<<grid, block, shm, s>>>(b->xq, b->n, b->ncell, b->cell_rep, b->reps, b->rep_flag, b->sorted,
-                                                 b->cell_off, b->rl2, b->cap, b->rows, b->counts, b->ref, b->st);
-    else
-        k_batch_rows<4><<<grid, block, shm, s>>>(b->xq, b->n, b->ncell, b->cell_rep, b->reps, b->rep_flag, b->sorted,
-                                                 b->cell_off, b->rl2, b->cap, b->rows, b->counts, b->ref, b->st);
+    // few cells: several warps per cell, until the chip has about 16 warps per SM
+    int nsplit = 1;
+    while (nsplit < 8 && (long long)b->ncell * nsplit < 148 * 16) nsplit *= 2;
+    const int grid = (int)(((long long)b->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
+    k_batch_rows<<<grid, 32 * ROWS_WARPS, sizeof(float4) * ROWS_WARPS * ROWS_CAP, s>>>(
+        b->xq, b->ncell, nsplit, b->cell_rep, b->reps, b->rep_flag, b->sorted, b->cell_off, b->rl2, b->cap, b->rows,
+        b->counts, b->ref, b->st);
     PD_LAUNCHED();
+    if (b->xrows) {
+        k_batch_export<<<blocks, B_THREADS, 0, s>>>(b->rows, b->counts, b->n, b->cap, b->xrows);
+        PD_LAUNCHED();
+    }
     return PD_OK;
 }
 
+// Lanes per row: the caller's choice, but at least as many as fill 32-byte sectors of the row-major rows where
+// the rows are that long (walking them with fewer lanes reads each sector several times).
+static int batch_lanes(const pd_batch *b) { return std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8); }
+
 template <bool COUL, int NP = BATCH_NP>
 static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, float *epot, int energy,
-                               const BatchKick &kick, int advance, cudaStream_t s) {
-    const int G = b->lanes;
+                               const BatchKick &kick, int advance, bool slot, cudaStream_t s) {
+    const int G = batch_lanes(b);
     const int blocks = (int)(((long long)b->n * G + B_THREADS - 1) / B_THREADS);
-#define PD_BP(GG)                                                                                                      \
-    if (energy)                                                                                                        \
-        k_batch_pairs<GG, true, COUL, NP><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->rows, b->counts, b->sorted,   \
-                                                                        b->rep_of, b->reps, fx, fy, fz, epot, kick,    \
-                                                                        b->st, advance, b->cp);                        \
-    else                                                                                                               \
-        k_batch_pairs<GG, false, COUL, NP><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->rows, b->counts, b->sorted,  \
-                                                                         b->rep_of, b->reps, fx, fy, fz, epot, kick,   \
-                                                                         b->st, advance, b->cp);
+#define PD_BP2(GG, EE, SS)                                                                                            \
+    k_batch_pairs<GG, EE, COUL, SS, NP><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->cap, b->rows, b->counts,         \
+                                                                     b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, \
+                                                                     b->fc, kick, b->st, advance, b->cp)
+#define PD_BP(GG)                                                                                                     \
+    if (slot) {                                                                                                       \
+        if (energy) PD_BP2(GG, true, true);                                                                           \
+        else PD_BP2(GG, false, true);                                                                                 \
+    } else if constexpr (!COUL) {                                                                                     \
+        if (energy) PD_BP2(GG, true, false);                                                                          \
+        else PD_BP2(GG, false, false);                                                                                \
+    }
     switch (G) {
         case 1: PD_BP(1) break;
         case 2: PD_BP(2) break;
@@ -657,6 +592,7 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
         default: PD_BP(8) break;
     }
 #undef PD_BP
+#undef PD_BP2
 }
 
 static BMeshView batch_mesh_view(const pd_batch *b) {
@@ -671,6 +607,7 @@ static BMeshView batch_mesh_view(const pd_batch *b) {
     v.slot_src = b->slot_src;
     v.mq = b->mq;
     v.mid = b->mid;
+    v.fc = b->fc;
     v.gridA = b->gridA;
     v.gridB = b->gridB;
     v.spec = b->spec;
@@ -713,21 +650,38 @@ static int batch_mesh_transform(pd_batch *b, cudaStream_t s) {
     const BMeshView v = batch_mesh_view(b);
     int rc;
     if ((rc = bmesh_spread_launch(v, b->st, s))) return rc;
+    if (b->fft.tab) return fft_batch(b->fft, b->st, s);
     if ((rc = batch_fft_all(b, true, s))) return rc;
     if ((rc = bmesh_solve_launch(v, b->st, s))) return rc;
     return batch_fft_all(b, false, s);
 }
 
-// The force pass: pack, then the row pair kernel; with charges and meshes the pair kernel runs on s
+// From this size the pair kernel stores its forces by position and k_batch_finish carries them to particle order:
+// below it the extra launch costs more than the scattered stores.
+constexpr int BATCH_SLOT_MIN = 32768;
+
+// The force pass: pack (unless the drift has packed the coordinates), then the row pair kernel; with charges and meshes the pair kernel runs on s
 // while the mesh branch runs on the batch's mesh stream (forked and joined by events, so the same
 // code is captured into the step graph), and the gather joins both and applies the closing kick.
 static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const float *z, float *fx, float *fy,
-                              float *fz, float *epot, int energy, BatchKick kick, int advance, cudaStream_t s) {
+                              float *fz, float *epot, int energy, BatchKick kick, int advance, bool packed,
+                              cudaStream_t s) {
     if (!b->coul) {
-        k_batch_pack<false><<<(b->n + B_THREADS - 1) / B_THREADS, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n,
-                                                                                     b->xq, b->st);
+        const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
+        if (!packed) {
+            k_batch_pack<false><<<blocks, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
+            PD_LAUNCHED();
+        }
+        const bool slot = b->n >= BATCH_SLOT_MIN;
+        launch_batch_pairs<false>(b, fx, fy, fz, epot, energy, kick, slot ? 0 : advance, slot, s);
         PD_LAUNCHED();
-        launch_batch_pairs<false>(b, fx, fy, fz, epot, energy, kick, advance, s);
+        if (!slot) return PD_OK;
+        if (energy)
+            k_batch_finish<true><<<blocks, B_THREADS, 0, s>>>(b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
+                                                              advance);
+        else
+            k_batch_finish<false><<<blocks, B_THREADS, 0, s>>>(b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
+                                                               advance);
         PD_LAUNCHED();
         return PD_OK;
     }
@@ -744,9 +698,9 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
     nokick.on = 0;
     // the polynomial's coefficient bucket: the fitted force coefficients, and the energy's with energy
     if (std::max(b->coul_nf, energy ? b->coul_ne : 0) <= 14)
-        launch_batch_pairs<true, 14>(b, fx, fy, fz, epot, energy, nokick, advance, s);
+        launch_batch_pairs<true, 14>(b, fx, fy, fz, epot, energy, nokick, advance, true, s);
     else
-        launch_batch_pairs<true, BATCH_NP>(b, fx, fy, fz, epot, energy, nokick, advance, s);
+        launch_batch_pairs<true, BATCH_NP>(b, fx, fy, fz, epot, energy, nokick, advance, true, s);
     PD_LAUNCHED();
     PD_CUDA(cudaStreamWaitEvent(s, b->ev_join, 0));
     BMeshKick mk;
@@ -770,12 +724,14 @@ static int batch_enqueue_step(pd_batch *b, float dt, cudaStream_t s, int cond) {
         PD_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
         k_batch_drift<true, true><<<blocks, B_THREADS, 0, s>>>(b->n, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy, S.fz,
                                                                S.inv_mass, dt, b->rep_of, b->reps, b->ref,
-                                                               b->threshold, b->rep_dmax, b->rep_flag, b->nrep,
+                                                               b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
+                                                               b->rep_dmax, b->rep_flag, b->nrep,
                                                                b->st, h);
     } else {
         k_batch_drift<true, false><<<blocks, B_THREADS, 0, s>>>(b->n, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy,
                                                                 S.fz, S.inv_mass, dt, b->rep_of, b->reps, b->ref,
-                                                                b->threshold, b->rep_dmax, b->rep_flag, b->nrep,
+                                                                b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
+                                                                b->rep_dmax, b->rep_flag, b->nrep,
                                                                 b->st, 0);
     }
     PD_LAUNCHED();
@@ -795,7 +751,7 @@ static int batch_enqueue_step(pd_batch *b, float dt, cudaStream_t s, int cond) {
     kick.inv_mass = S.inv_mass;
     kick.half_dt = 0.5f * dt;
     kick.on = 1;
-    return batch_pairs_launch(b, S.x, S.y, S.z, S.fx, S.fy, S.fz, S.epot, 0, kick, 1, s);
+    return batch_pairs_launch(b, S.x, S.y, S.z, S.fx, S.fy, S.fz, S.epot, 0, kick, 1, true, s);
 }
 
 }  // namespace pdb
@@ -852,6 +808,7 @@ int pd_batch_create(pd_batch **out, const pd_batch_replica *reps, int nrep, floa
         b->hreps.push_back(h);
         b->box.insert(b->box.end(), R.box, R.box + 3);
         b->first.push_back(b->n);
+        b->mean_row += (double)R.n * R.n / (R.box[0] * R.box[1] * R.box[2]) * 4.18879 * (double)rl * rl * rl;
         b->n += R.n;
         const int nc = ng[0] * ng[1] * ng[2];
         b->ncell += nc;
@@ -860,13 +817,15 @@ int pd_batch_create(pd_batch **out, const pd_batch_replica *reps, int nrep, floa
     }
     int rc;
     const size_t n = (size_t)b->n;
+    b->mean_row /= b->n;
     if ((rc = dalloc(&b->reps, (size_t)nrep)) || (rc = dalloc(&b->rep_of, n)) ||
         (rc = dalloc(&b->cell_rep, (size_t)b->ncell)) || (rc = dalloc(&b->st, (size_t)E_LEN)) ||
         (rc = dalloc(&b->rep_flag, (size_t)nrep)) || (rc = dalloc(&b->rep_dmax, (size_t)nrep)) ||
         (rc = dalloc(&b->cell_of, n)) || (rc = dalloc(&b->cell_count, (size_t)b->ncell)) ||
         (rc = dalloc(&b->cell_off, (size_t)b->ncell + 1)) || (rc = dalloc(&b->sorted, n)) ||
         (rc = dalloc(&b->tmp, n)) || (rc = dalloc(&b->rows, n * (size_t)cap)) || (rc = dalloc(&b->counts, n)) ||
-        (rc = dalloc(&b->ref, n)) || (rc = dalloc(&b->xq, n))) {
+        (rc = dalloc(&b->ref, n)) || (rc = dalloc(&b->xq, n)) || (rc = dalloc(&b->fc, n)) ||
+        (rc = dalloc(&b->pos_of, n)) || (rc = dalloc(&b->scan_part, ell_scan_part_len(b->ncell)))) {
         batch_free(b);
         delete b;
         return rc;
@@ -883,6 +842,8 @@ int pd_batch_create(pd_batch **out, const pd_batch_replica *reps, int nrep, floa
         cudaMemset(b->cell_count, 0, sizeof(int) * (size_t)b->ncell) != cudaSuccess ||
         cudaMemset(b->rep_flag, 0, sizeof(int) * (size_t)nrep) != cudaSuccess ||
         cudaMemset(b->rep_dmax, 0, sizeof(unsigned) * (size_t)nrep) != cudaSuccess ||
+        cudaMemset(b->scan_part, 0, sizeof(int) * ell_scan_part_len(b->ncell)) != cudaSuccess ||
+        cudaMemcpy(b->pos_of, iota.data(), sizeof(int) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(b->cell_of, 0, sizeof(int) * n) != cudaSuccess ||
         cudaMemset(b->counts, 0, sizeof(int) * n) != cudaSuccess ||
         cudaMemset(b->ref, 0, sizeof(float4) * n) != cudaSuccess ||
@@ -922,8 +883,8 @@ int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z,
     cudaStream_t s = (cudaStream_t)sp;
     k_batch_drift<false, false><<<(b->n + B_THREADS - 1) / B_THREADS, B_THREADS, 0, s>>>(
         b->n, const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
-        nullptr, nullptr, nullptr, nullptr, 0.f, b->rep_of, b->reps, b->ref, b->threshold, b->rep_dmax, b->rep_flag,
-        b->nrep, b->st, 0);
+        nullptr, nullptr, nullptr, nullptr, 0.f, b->rep_of, b->reps, b->ref, b->threshold, nullptr, nullptr, b->rep_dmax,
+        b->rep_flag, b->nrep, b->st, 0);
     PD_LAUNCHED();
     return batch_rebuild_launch(b, x, y, z, s);
 }
@@ -934,7 +895,7 @@ int pd_batch_forces(pd_batch *b, const float *x, const float *y, const float *z,
     PD_CHECK(!energy || epot, PD_EINVAL, "pd_batch_forces: energy needs epot");
     BatchKick kick;
     memset(&kick, 0, sizeof kick);
-    return batch_pairs_launch(b, x, y, z, fx, fy, fz, epot, energy, kick, 0, (cudaStream_t)sp);
+    return batch_pairs_launch(b, x, y, z, fx, fy, fz, epot, energy, kick, 0, false, (cudaStream_t)sp);
 }
 
 int pd_batch_status(pd_batch *b, pd_ell_stats *out) {
@@ -1079,6 +1040,106 @@ static int batch_layout_chunks(pd_batch *b, int chunk) {
     return PD_OK;
 }
 
+// One batched cuFFT plan per mesh size, spread over the FFT streams.
+static int batch_make_plans(pd_batch *b, int prio_hi) {
+    size_t wmax = 0;
+    for (auto &g : b->groups) {
+        int n[3] = {g.K3, g.K2, g.K1};
+        const int K1h = g.K1 / 2 + 1;
+        const int nn = g.K1 * g.K2 * g.K3, nm = K1h * g.K2 * g.K3;
+        size_t w1 = 0, w2 = 0;
+        PD_CHECK(cufftCreate(&g.fwd) == CUFFT_SUCCESS && cufftCreate(&g.bwd) == CUFFT_SUCCESS, PD_ECUFFT,
+                 "batched mesh: cufftCreate failed");
+        PD_CHECK(cufftSetAutoAllocation(g.fwd, 0) == CUFFT_SUCCESS && cufftSetAutoAllocation(g.bwd, 0) == CUFFT_SUCCESS,
+                 PD_ECUFFT, "batched mesh: cufftSetAutoAllocation failed");
+        PD_CHECK(cufftMakePlanMany(g.fwd, 3, n, nullptr, 1, nn, nullptr, 1, nm, CUFFT_R2C, g.count, &w1) ==
+                         CUFFT_SUCCESS &&
+                     cufftMakePlanMany(g.bwd, 3, n, nullptr, 1, nm, nullptr, 1, nn, CUFFT_C2R, g.count, &w2) ==
+                         CUFFT_SUCCESS,
+                 PD_ECUFFT, "batched mesh: plan of %d meshes %dx%dx%d failed", g.count, g.K1, g.K2, g.K3);
+        wmax = std::max(wmax, std::max(w1, w2));
+    }
+    for (int k = 0; k < pd_batch::NFFT; ++k) {
+        PD_CUDA(cudaMalloc(&b->fft_work[k], std::max<size_t>(wmax, 256)));
+        PD_CUDA(cudaStreamCreateWithPriority(&b->fft_stream[k], cudaStreamNonBlocking, prio_hi));
+        PD_CUDA(cudaEventCreateWithFlags(&b->ev_fft[k], cudaEventDisableTiming));
+    }
+    PD_CUDA(cudaEventCreateWithFlags(&b->ev_fft_fork, cudaEventDisableTiming));
+    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
+        auto &g = b->groups[gi];
+        void *w = b->fft_work[gi % pd_batch::NFFT];
+        PD_CHECK(cufftSetWorkArea(g.fwd, w) == CUFFT_SUCCESS && cufftSetWorkArea(g.bwd, w) == CUFFT_SUCCESS,
+                 PD_ECUFFT, "batched mesh: cufftSetWorkArea failed");
+    }
+    return PD_OK;
+}
+
+// Every replica's mesh on this library's transforms, when every mesh's planes fit in shared memory:
+// the table of meshes and the work of every CTA, the replicas' planes largest first.
+static int batch_make_transforms(pd_batch *b) {
+    std::vector<FftMesh> tab((size_t)b->nrep);
+    for (int r = 0; r < b->nrep; ++r) {
+        const BMeshRep &R = b->hmreps[(size_t)r];
+        const int K[3] = {R.K1, R.K2, R.K3};
+        if (fft_route(K, &tab[(size_t)r]) != FFT_PLANES) return PD_OK;
+    }
+    for (const FftMesh &m : tab)   // two buffers for all where one plane needs them
+        if (fft_plane_smem(m, false) > FFT_PLANE_SMEM_MAX && !fft_plane_inplace(m)) return PD_OK;
+    int rc;
+    if ((rc = fft_init())) return rc;
+    std::vector<int> lens;
+    FftBatch f{};
+    f.inplace = true;
+    for (const FftMesh &m : tab) f.inplace = f.inplace && fft_plane_inplace(m);
+    std::vector<int> order((size_t)b->nrep);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+        return (long long)b->hmreps[(size_t)p].K1 * b->hmreps[(size_t)p].K2 >
+               (long long)b->hmreps[(size_t)q].K1 * b->hmreps[(size_t)q].K2;
+    });
+    std::vector<int2> planes, cols;
+    for (int r : order) {
+        const BMeshRep &R = b->hmreps[(size_t)r];
+        FftMesh &m = tab[(size_t)r];
+        for (int d = 0; d < 3; ++d) {
+            const int n = m.ax[d].n;
+            size_t k = 0;
+            while (k < lens.size() && lens[k] != n) ++k;
+            if (k == lens.size()) {
+                float2 *w = nullptr;
+                if ((rc = fft_twiddles(n, &w))) return rc;
+                b->twiddles.push_back(w);
+                lens.push_back(n);
+            }
+            m.ax[d].w = b->twiddles[k];
+        }
+        m.grid = b->gridA + R.grid;
+        m.spec = b->spec + R.modes;
+        m.G = b->G + R.modes;
+        m.zspec[0] = m.spec;
+        m.out[0] = b->gridB + R.grid;
+        f.plane_threads = std::max(f.plane_threads, fft_plane_threads(m));
+        f.plane_smem = std::max(f.plane_smem, fft_plane_smem(m, f.inplace));
+        f.line_threads = std::max(f.line_threads, fft_line_threads(m.ax[2]));
+        f.line_smem = std::max(f.line_smem, fft_line_smem(m.ax[2]));
+        for (int z = 0; z < R.K3; ++z) planes.push_back(make_int2(r, z));
+        for (int c = 0; c < R.K2 * R.K1h; c += FFT_LINES_C) cols.push_back(make_int2(r, c));
+    }
+    f.nplanes = (int)planes.size();
+    f.ncols = (int)cols.size();
+    if ((rc = dalloc(&b->fft_tab, tab.size())) || (rc = dalloc(&b->fft_planes, planes.size())) ||
+        (rc = dalloc(&b->fft_cols, cols.size())))
+        return rc;
+    PD_CUDA(cudaMemcpy(b->fft_tab, tab.data(), sizeof(FftMesh) * tab.size(), cudaMemcpyHostToDevice));
+    PD_CUDA(cudaMemcpy(b->fft_planes, planes.data(), sizeof(int2) * planes.size(), cudaMemcpyHostToDevice));
+    PD_CUDA(cudaMemcpy(b->fft_cols, cols.data(), sizeof(int2) * cols.size(), cudaMemcpyHostToDevice));
+    f.tab = b->fft_tab;
+    f.planes = b->fft_planes;
+    f.cols = b->fft_cols;
+    b->fft = f;
+    return PD_OK;
+}
+
 static int batch_set_mesh(pd_batch *b, int kind, int order, double alpha, double C, const int *meshes) {
     const int nrep = b->nrep;
     std::vector<int> idx((size_t)nrep);
@@ -1158,39 +1219,12 @@ static int batch_set_mesh(pd_batch *b, int kind, int order, double alpha, double
         pd_mesh_destroy(m);
         PD_CHECK(err == cudaSuccess, PD_ECUDA, "batched mesh: influence copy failed: %s", cudaGetErrorString(err));
     }
-    size_t wmax = 0;
-    for (auto &g : b->groups) {
-        int n[3] = {g.K3, g.K2, g.K1};
-        const int K1h = g.K1 / 2 + 1;
-        const int nn = g.K1 * g.K2 * g.K3, nm = K1h * g.K2 * g.K3;
-        size_t w1 = 0, w2 = 0;
-        PD_CHECK(cufftCreate(&g.fwd) == CUFFT_SUCCESS && cufftCreate(&g.bwd) == CUFFT_SUCCESS, PD_ECUFFT,
-                 "batched mesh: cufftCreate failed");
-        PD_CHECK(cufftSetAutoAllocation(g.fwd, 0) == CUFFT_SUCCESS && cufftSetAutoAllocation(g.bwd, 0) == CUFFT_SUCCESS,
-                 PD_ECUFFT, "batched mesh: cufftSetAutoAllocation failed");
-        PD_CHECK(cufftMakePlanMany(g.fwd, 3, n, nullptr, 1, nn, nullptr, 1, nm, CUFFT_R2C, g.count, &w1) ==
-                         CUFFT_SUCCESS &&
-                     cufftMakePlanMany(g.bwd, 3, n, nullptr, 1, nm, nullptr, 1, nn, CUFFT_C2R, g.count, &w2) ==
-                         CUFFT_SUCCESS,
-                 PD_ECUFFT, "batched mesh: plan of %d meshes %dx%dx%d failed", g.count, g.K1, g.K2, g.K3);
-        wmax = std::max(wmax, std::max(w1, w2));
-    }
     // the mesh branch is the longer of the two branches of the force pass: its streams get the high
     // priority, so its kernels' blocks are scheduled ahead of the pair kernel's
     int prio_lo = 0, prio_hi = 0;
     cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
-    for (int k = 0; k < pd_batch::NFFT; ++k) {
-        PD_CUDA(cudaMalloc(&b->fft_work[k], std::max<size_t>(wmax, 256)));
-        PD_CUDA(cudaStreamCreateWithPriority(&b->fft_stream[k], cudaStreamNonBlocking, prio_hi));
-        PD_CUDA(cudaEventCreateWithFlags(&b->ev_fft[k], cudaEventDisableTiming));
-    }
-    PD_CUDA(cudaEventCreateWithFlags(&b->ev_fft_fork, cudaEventDisableTiming));
-    for (size_t gi = 0; gi < b->groups.size(); ++gi) {
-        auto &g = b->groups[gi];
-        void *w = b->fft_work[gi % pd_batch::NFFT];
-        PD_CHECK(cufftSetWorkArea(g.fwd, w) == CUFFT_SUCCESS && cufftSetWorkArea(g.bwd, w) == CUFFT_SUCCESS,
-                 PD_ECUFFT, "batched mesh: cufftSetWorkArea failed");
-    }
+    if ((rc = batch_make_transforms(b))) return rc;
+    if (!b->fft.tab && (rc = batch_make_plans(b, prio_hi))) return rc;
     PD_CUDA(cudaStreamCreateWithPriority(&b->mesh_stream, cudaStreamNonBlocking, prio_hi));
     PD_CUDA(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
     PD_CUDA(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
@@ -1249,7 +1283,18 @@ int pd_batch_mesh_info(pd_batch *b, int *groups, long long *nodes, long long *mo
 
 int pd_batch_rows(pd_batch *b, int **rows, int **counts, int **order) {
     PD_CHECK(b && rows && counts, PD_EINVAL, "pd_batch_rows: null argument");
-    *rows = b->rows;
+    if (!b->xrows) {   // from now on every rebuild refreshes them: a captured step is captured again
+        const int rc = dalloc(&b->xrows, (size_t)b->n * b->cap);
+        if (rc) return rc;
+        PD_CUDA(cudaMemset(b->xrows, 0xff, sizeof(int) * (size_t)b->n * b->cap));
+        PD_CUDA(cudaDeviceSynchronize());   // a build may be in flight on another stream
+        k_batch_export<<<(b->n + B_THREADS - 1) / B_THREADS, B_THREADS>>>(b->rows, b->counts, b->n, b->cap, b->xrows);
+        PD_LAUNCHED();
+        PD_CUDA(cudaDeviceSynchronize());
+        if (b->exec) cudaGraphExecDestroy(b->exec);
+        b->exec = nullptr;
+    }
+    *rows = b->xrows;
     *counts = b->counts;
     if (order) *order = b->sorted;
     return PD_OK;

@@ -85,11 +85,13 @@ __global__ void __launch_bounds__(256) k_bsolve(float2 *__restrict__ spec, const
 
 // AD gather of one chunk (the sums of _gather_ad_lines_sums, MeshKernels.jl:281-311, and
 // _gather_ad_lines_kernel!, :313-333) from the replica's potential grid, joined with the pair force
-// already stored for the particle: F = F_pair - q grad(phi) K / L, then the closing half kick.  Each
+// of the particle's position: F = F_pair - q grad(phi) K / L, then the closing half kick.  Each
 // particle's TP threads share the z planes of its stencil.
 template <int P, int CH, int TP, bool ENERGY>
 __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const float4 *__restrict__ mq,
                                                                       const int *__restrict__ mid,
+                                                                      const int *__restrict__ slot_src,
+                                                                      const float4 *__restrict__ fc,
                                                                       const int *__restrict__ chunk_rep,
                                                                       const BMeshRep *__restrict__ reps,
                                                                       const float *__restrict__ gridB,
@@ -115,10 +117,11 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const fl
     // the pair force and the velocity are fetched now, so that their latency overlaps the brick
     float fpx = 0.f, fpy = 0.f, fpz = 0.f, pvx = 0.f, pvy = 0.f, pvz = 0.f, pim = 0.f, ep = 0.f;
     if (h == 0 && id >= 0) {
-        fpx = fx[id];
-        fpy = fy[id];
-        fpz = fz[id];
-        if (ENERGY) ep = epot[id];
+        const float4 f = fc[slot_src[e]];
+        fpx = f.x;
+        fpy = f.y;
+        fpz = f.z;
+        if (ENERGY) ep = f.w;
         if (kick.on) {
             pvx = kick.vx[id];
             pvy = kick.vy[id];
@@ -272,10 +275,10 @@ template <int P, int CH, int TP>
 static void gather_pc(const BMeshView &v, float *fx, float *fy, float *fz, float *epot, int energy,
                       const BMeshKick &kick, float half_c_self, const long long *st, cudaStream_t s) {
     if (energy)
-        k_bgather<P, CH, TP, true><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.chunk_rep, v.reps, v.gridB, fx, fy,
+        k_bgather<P, CH, TP, true><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
                                                                 fz, epot, kick, half_c_self, st);
     else
-        k_bgather<P, CH, TP, false><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.chunk_rep, v.reps, v.gridB, fx, fy,
+        k_bgather<P, CH, TP, false><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
                                                                  fz, epot, kick, half_c_self, st);
 }
 

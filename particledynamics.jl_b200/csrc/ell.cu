@@ -9,18 +9,16 @@
 // src/nonbonded/LJELLEngineKernels.jl) and its Langevin BAOAB kernels
 // (src/engine/Langevin.jl, src/engine/Philox.jl).  The layout is this
 // library's own:
-//   * the rows are slot-major (slot t of particle i at t * N + i, the
-//     reference's _ell_index), so the row loads of consecutive particles
-//     coalesce;
-//   * particles inside a cell are ordered by id, so rows (and the summation
-//     order of the pair kernel) are reproducible;
-//   * rows are built by one thread per particle in cell order (neighbouring
-//     threads share candidate cells), and the last block to finish commits
-//     the capacity check;
+//   * particles are taken in cell order (by cell, by id inside a cell, so that rows and pair sums
+//     are reproducible), rows and their entries are cell-order positions (rows.cuh);
+//     pd_ell_rows exports them by particle id, slot t of particle i at t * N + i (the
+//     reference's _ell_index);
+//   * the last block of a row build commits the capacity check;
 //   * the displacement maximum and the rebuild decision run in one kernel
 //     (the last block decides), fused with the drift in the step engine;
 //   * the pair kernel reads packed (x, y, z, 0) coordinates, G lanes per row
-//     reduced by shuffles, with the closing half kick fused in the step.
+//     reduced by shuffles; the closing half kick is fused into it for small systems and
+//     runs in particle order after it for large ones.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -28,6 +26,7 @@
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
+#include "rows.cuh"
 
 using namespace pdb;
 
@@ -84,7 +83,8 @@ __global__ void k_ell_bin(const float *__restrict__ x, const float *__restrict__
 }
 
 // Exclusive scan of the cell histogram into cell_off (ncell + 1 entries); the histogram is
-// reset to zero for use as scatter cursors.  One CTA, chunks staged in shared memory.
+// reset to zero for use as scatter cursors.  One CTA, chunks staged in shared memory: the histograms of up
+// to SCAN_ONE_BLOCK cells (two launches cost more than a second chunk there).
 __global__ void __launch_bounds__(1024) k_ell_scan(int *__restrict__ cell_count, int *__restrict__ cell_off,
                                                    int ncell, const long long *__restrict__ st) {
     if (!ell_requested(st)) return;
@@ -143,6 +143,91 @@ __global__ void __launch_bounds__(1024) k_ell_scan(int *__restrict__ cell_count,
     if (t == 0) cell_off[ncell] = carry;
 }
 
+// The same scan by SCAN_TILE cells per CTA: the tiles' sums (the last block to report scans them into the
+// tiles' offsets), then the cells' offsets.  One CTA took 306 us for the 506 944 cells of a million 2D disks.
+constexpr int SCAN_ONE_BLOCK = 2 * ELL_SCAN_CHUNK, SCAN_TILE = 4096, SCAN_THREADS = 512;
+
+__device__ __forceinline__ int block_exclusive(int v, int *sh, int &total) {   // SCAN_THREADS threads
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int inc = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += y;
+    }
+    if (lane == 31) sh[w] = inc;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+    for (int k = 0; k < SCAN_THREADS / 32; ++k) {
+        const int s = sh[k];
+        before += k < w ? s : 0;
+        total += s;
+    }
+    __syncthreads();
+    return before + inc - v;
+}
+
+// part: ntile sums, then the total, then the ticket (zero between scans)
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restrict__ cell_count, int ncell,
+                                                            int *__restrict__ part, int ntile,
+                                                            const long long *__restrict__ st) {
+    if (!ell_requested(st)) return;
+    __shared__ int sh[SCAN_THREADS / 32];
+    __shared__ bool last;
+    const int c0 = blockIdx.x * SCAN_TILE;
+    int v = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_TILE / SCAN_THREADS; ++k) {
+        const int c = c0 + k * SCAN_THREADS + threadIdx.x;
+        v += c < ncell ? cell_count[c] : 0;
+    }
+    int total;
+    block_exclusive(v, sh, total);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = total;
+        __threadfence();
+        last = atomicAdd(&part[ntile + 1], 1) == ntile - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    volatile int *vp = part;
+    int carry = 0;
+    for (int t0 = 0; t0 < ntile; t0 += SCAN_THREADS) {
+        const int t = t0 + threadIdx.x, x = t < ntile ? vp[t] : 0;
+        int sum;
+        const int ex = block_exclusive(x, sh, sum);
+        if (t < ntile) vp[t] = carry + ex;
+        carry += sum;
+    }
+    if (threadIdx.x == 0) {
+        vp[ntile] = carry;
+        vp[ntile + 1] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(int *__restrict__ cell_count, int *__restrict__ cell_off,
+                                                             int ncell, const int *__restrict__ part, int ntile,
+                                                             const long long *__restrict__ st) {
+    if (!ell_requested(st)) return;
+    __shared__ int sh[SCAN_THREADS / 32];
+    int at = part[blockIdx.x];
+#pragma unroll 1
+    for (int k = 0; k < SCAN_TILE / SCAN_THREADS; ++k) {
+        const int c = blockIdx.x * SCAN_TILE + k * SCAN_THREADS + threadIdx.x;
+        const int v = c < ncell ? cell_count[c] : 0;
+        int total;
+        const int ex = block_exclusive(v, sh, total);
+        if (c < ncell) {
+            cell_off[c] = at + ex;
+            cell_count[c] = 0;
+        }
+        at += total;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) cell_off[ncell] = part[ntile];
+}
+
 // _kernel_scatter_by_cell! (DenseNeighborCUDA.jl:61-72): atomic cursors per cell.
 __global__ void k_ell_scatter(const int *__restrict__ cell_of, int n, const int *__restrict__ cell_off,
                               int *__restrict__ cursor, int *__restrict__ sorted, const long long *__restrict__ st) {
@@ -182,38 +267,55 @@ __global__ void k_ell_cellsort(const int *__restrict__ cell_off, int ncell, int 
     for (int k = lane; k < n; k += 32) sorted[a + k] = tmp[a + k];
 }
 
-// Row construction (_kernel_neighbors3g!, DeviceNeighborCUDA.jl:510-559; 2D _kernel_neighbors2!,
-// DenseNeighborCUDA.jl:77-123): thread t takes particle sorted[t] and walks the cell-row stencil
-// (z, then y offsets; x cells in range order), keeping j != i with r^2 <= r_list^2 (nearest
-// image by one conditional shift).  Rows past the capacity are counted but not stored.  The
-// build reference coordinates are refreshed; the last block commits (_device_commit_kernel!,
-// DeviceNeighborCUDA.jl:345-404).
+// The same order for sparse cells, one thread per cell: insertion by id (a warp per cell left 30 lanes idle,
+// 72 us for the 506 944 cells of a million 2D disks).
+__global__ void k_ell_cellsort_sparse(const int *__restrict__ cell_off, int ncell, int *__restrict__ sorted,
+                                      int *__restrict__ cell_count, const long long *__restrict__ st) {
+    if (!ell_requested(st)) return;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncell) return;
+    cell_count[c] = 0;
+    const int a = cell_off[c], b = cell_off[c + 1];
+    for (int k = a + 1; k < b; ++k) {
+        const int id = sorted[k];
+        int j = k;
+        for (; j > a && sorted[j - 1] > id; --j) sorted[j] = sorted[j - 1];
+        sorted[j] = id;
+    }
+}
+
+// Row construction for sparse cells and small boxes (_kernel_neighbors3g!, DeviceNeighborCUDA.jl:510-559; 2D
+// _kernel_neighbors2!, DenseNeighborCUDA.jl:77-123): thread k takes the particle at cell-order position k and
+// walks the cell-row stencil (z, then y offsets; x cells in range order), keeping the other particles with
+// r^2 <= r_list^2 (nearest image by one conditional shift).  Rows past the capacity are counted but not
+// stored.  The build reference coordinates are refreshed; the last block commits.
 template <int D, bool ALLPAIRS>
 __global__ void __launch_bounds__(ELL_THREADS) k_ell_rows(
-    const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, int n,
-    const int *__restrict__ sorted, const int *__restrict__ cell_of, const int *__restrict__ cell_off, float Lx,
-    float Ly, float Lz, int nx, int ny, int nz, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts,
-    float4 *__restrict__ ref, long long *__restrict__ st) {
+    const float4 *__restrict__ xq, int n, const int *__restrict__ sorted, const int *__restrict__ cell_of,
+    const int *__restrict__ cell_off, float Lx, float Ly, float Lz, int nx, int ny, int nz, float rl2, int cap,
+    int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref, long long *__restrict__ st) {
     if (!ell_requested(st)) return;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int found = 0;
-    if (t < n) {
-        const int i = ALLPAIRS ? t : sorted[t];
-        const float xi = x[i], yi = y[i], zi = D == 3 ? z[i] : 0.f;
+    if (k < n) {
+        const int i = sorted[k];
+        const float4 me = xq[k];
+        const float xi = me.x, yi = me.y, zi = D == 3 ? me.z : 0.f;
         const float hLx = 0.5f * Lx, hLy = 0.5f * Ly, hLz = 0.5f * Lz;
         auto visit = [&](int j) {
-            if (j == i) return;
-            const float dx = mic_fast(x[j] - xi, hLx, Lx);
-            const float dy = mic_fast(y[j] - yi, hLy, Ly);
+            if (j == k) return;
+            const float4 cj = __ldg(xq + j);
+            const float dx = mic_fast(cj.x - xi, hLx, Lx);
+            const float dy = mic_fast(cj.y - yi, hLy, Ly);
             float r2;
             if (D == 3) {
-                const float dz = mic_fast(z[j] - zi, hLz, Lz);
+                const float dz = mic_fast(cj.z - zi, hLz, Lz);
                 r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             } else {
                 r2 = fmaf(dx, dx, dy * dy);
             }
             if (r2 <= rl2) {
-                if (found < cap) rows[(size_t)found * n + i] = j;
+                if (found < cap) rows[(size_t)found * n + k] = j;
                 ++found;
             }
         };
@@ -241,181 +343,66 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_rows(
                     const int row = (cz2 * ny + cy2) * nx;
                     int a1, b1, a2, b2;
                     ell_row_ranges(cx, g2, rl2, hx, Sx, nx, a1, b1, a2, b2);
-                    for (int k = cell_off[row + a1]; k < cell_off[row + b1 + 1]; ++k) visit(sorted[k]);
+                    for (int j = cell_off[row + a1], e = cell_off[row + b1 + 1]; j < e; ++j) visit(j);
                     if (a2 <= b2)
-                        for (int k = cell_off[row + a2]; k < cell_off[row + b2 + 1]; ++k) visit(sorted[k]);
+                        for (int j = cell_off[row + a2], e = cell_off[row + b2 + 1]; j < e; ++j) visit(j);
                 }
             }
         }
-        counts[i] = found;
+        counts[k] = found;
         ref[i] = make_float4(xi, yi, zi, 0.f);
     }
-    if (ell_block_max_last((unsigned)found, st, E_RMAX, E_TICKET_R)) {
-        // commit: the largest row against the capacity
-        const long long largest = st[E_RMAX];
-        st[E_RMAX] = 0;
-        st[E_TICKET_R] = 0;
-        st[E_REQUIRED] = largest;
-        if (largest > cap) {
-            st[E_ERROR] = E_ERR_CAPACITY;
-            st[E_VALID] = 0;
-        } else {
-            st[E_VALID] = 1;
-            st[E_LAST_BUILD] = st[E_STEP];
-            st[E_BUILDS] += 1;
-        }
-    }
+    if (ell_block_max_last((unsigned)found, st, E_RMAX, E_TICKET_R)) rows_commit(st, cap);
 }
 
-// Row construction, cell-staged: one warp per cell.  The warp walks the same stencil segments
-// in the same order as k_ell_rows (z, then y offsets; x cells in range order; each cell's
-// particles in id order), stages the candidates (x, y, z, id) in shared memory once for the
-// whole cell, and every lane (a particle of the cell) scans them with the same arithmetic as
-// k_ell_rows, so the rows are identical entry by entry.  Chunks of ROWS_CAP candidates are
-// scanned in turn when the stencil holds more.
-constexpr int ROWS_WARPS = 4, ROWS_CAP = 640;   // 40 KB of staging per block (below the 48 KB default)
-constexpr int ROWS_MIN_PER_CELL = 8;            // mean cell occupancy from which the cell-staged kernel is used
-
+// Row construction for dense cells: one warp per cell, or nsplit warps where the grid has few cells (each
+// stages the stencil for its share of the cell's particles).
 template <int D>
 __global__ void __launch_bounds__(32 * ROWS_WARPS) k_ell_rows_cells(
-    const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, int n,
-    const int *__restrict__ sorted, const int *__restrict__ cell_off, float Lx, float Ly, float Lz, int nx, int ny,
-    int nz, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref,
+    const float4 *__restrict__ xq, const int *__restrict__ sorted, const int *__restrict__ cell_off, RowGrid g,
+    int nsplit, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref,
     long long *__restrict__ st) {
     if (!ell_requested(st)) return;
     extern __shared__ float4 ell_stage[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ncell = nx * ny * nz;
-    const int c = blockIdx.x * ROWS_WARPS + w;
-    float4 *sw = ell_stage + w * ROWS_CAP;
+    const int w = threadIdx.x >> 5;
+    const int item = blockIdx.x * ROWS_WARPS + w, c = item / nsplit;
     unsigned fmax = 0;
-    if (c < ncell) {   // warp-uniform
-        const float hLx = 0.5f * Lx, hLy = 0.5f * Ly, hLz = 0.5f * Lz;
-        const float rl = sqrtf(rl2);
-        const float hx = Lx / (float)nx, hy = Ly / (float)ny, hz = Lz / (float)nz;
-        const int Sx = ell_reach(rl, Lx, nx), Sy = ell_reach(rl, Ly, ny);
-        const int Sz = D == 3 ? ell_reach(rl, Lz, nz) : 0;
-        const int cx = c % nx, tmp = c / nx, cy = tmp % ny, cz = tmp / ny;
-        const int p0 = cell_off[c], pn = cell_off[c + 1] - p0;
-        for (int pg = 0; pg < pn; pg += 32) {
-            const bool has = pg + lane < pn;
-            const int i = has ? sorted[p0 + pg + lane] : -1;
-            const float xi = has ? x[i] : 0.f, yi = has ? y[i] : 0.f, zi = (has && D == 3) ? z[i] : 0.f;
-            // bounding box of this group's particles: a candidate farther than the list radius from the
-            // box is farther from every particle of the group and is not staged (a conservative margin
-            // keeps rounding from dropping a candidate that the exact test below would accept)
-            float bl[3] = {has ? xi : INFINITY, has ? yi : INFINITY, has ? zi : INFINITY};
-            float bh[3] = {has ? xi : -INFINITY, has ? yi : -INFINITY, has ? zi : -INFINITY};
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    bl[d] = fminf(bl[d], __shfl_xor_sync(0xffffffffu, bl[d], off));
-                    bh[d] = fmaxf(bh[d], __shfl_xor_sync(0xffffffffu, bh[d], off));
-                }
-            }
-            const float bcx = 0.5f * (bl[0] + bh[0]), bcy = 0.5f * (bl[1] + bh[1]), bcz = 0.5f * (bl[2] + bh[2]);
-            const float bhx = 0.5f * (bh[0] - bl[0]), bhy = 0.5f * (bh[1] - bl[1]), bhz = 0.5f * (bh[2] - bl[2]);
-            const float rbox = rl * 1.0001f + 1e-3f;
-            const float rbox2 = rbox * rbox;
-            int found = 0;
-            int fill = 0;
-            auto scan = [&]() {
-                __syncwarp();
-                if (has) {
-                    for (int t = 0; t < fill; ++t) {
-                        const float4 cj = sw[t];
-                        const int j = __float_as_int(cj.w);
-                        if (j == i) continue;
-                        const float dx = mic_fast(cj.x - xi, hLx, Lx);
-                        const float dy = mic_fast(cj.y - yi, hLy, Ly);
-                        float r2;
-                        if (D == 3) {
-                            const float dz = mic_fast(cj.z - zi, hLz, Lz);
-                            r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        } else {
-                            r2 = fmaf(dx, dx, dy * dy);
-                        }
-                        if (r2 <= rl2) {
-                            if (found < cap) rows[(size_t)found * n + i] = j;
-                            ++found;
-                        }
-                    }
-                }
-                __syncwarp();
-                fill = 0;
-            };
-            auto stage = [&](int ka, int kb) {
-                for (int k0 = ka; k0 < kb; k0 += 32) {
-                    const bool in = lane < kb - k0;
-                    const int j = in ? sorted[k0 + lane] : 0;
-                    const float cx3 = in ? x[j] : 0.f, cy3 = in ? y[j] : 0.f, cz3 = (in && D == 3) ? z[j] : 0.f;
-                    const float ex = fmaxf(fabsf(mic_fast(cx3 - bcx, hLx, Lx)) - bhx, 0.f);
-                    const float ey = fmaxf(fabsf(mic_fast(cy3 - bcy, hLy, Ly)) - bhy, 0.f);
-                    const float ez = D == 3 ? fmaxf(fabsf(mic_fast(cz3 - bcz, hLz, Lz)) - bhz, 0.f) : 0.f;
-                    const bool keep = in && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= rbox2;
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                    const int nk = __popc(bal);
-                    if (fill + nk > ROWS_CAP) scan();
-                    if (keep)   // staged in the candidates' order
-                        sw[fill + __popc(bal & ((1u << lane) - 1u))] = make_float4(cx3, cy3, cz3, __int_as_float(j));
-                    fill += nk;
-                }
-            };
-            for (int oz = -Sz; oz <= Sz; ++oz) {
-                int cz2 = cz + oz;
-                cz2 -= cz2 >= nz ? nz : 0;
-                cz2 += cz2 < 0 ? nz : 0;
-                const float gz = (float)max(abs(oz) - 1, 0) * hz;
-                for (int oy = -Sy; oy <= Sy; ++oy) {
-                    int cy2 = cy + oy;
-                    cy2 -= cy2 >= ny ? ny : 0;
-                    cy2 += cy2 < 0 ? ny : 0;
-                    const float gy = (float)max(abs(oy) - 1, 0) * hy;
-                    const float g2 = fmaf(gy, gy, gz * gz);
-                    if (g2 > rl2) continue;
-                    const int row = (cz2 * ny + cy2) * nx;
-                    int a1, b1, a2, b2;
-                    ell_row_ranges(cx, g2, rl2, hx, Sx, nx, a1, b1, a2, b2);
-                    stage(cell_off[row + a1], cell_off[row + b1 + 1]);
-                    if (a2 <= b2) stage(cell_off[row + a2], cell_off[row + b2 + 1]);
-                }
-            }
-            scan();
-            if (has) {
-                counts[i] = found;
-                ref[i] = make_float4(xi, yi, zi, 0.f);
-            }
-            fmax = max(fmax, (unsigned)found);
-        }
-    }
-    if (ell_block_max_last(fmax, st, E_RMAX, E_TICKET_R)) {
-        const long long largest = st[E_RMAX];
-        st[E_RMAX] = 0;
-        st[E_TICKET_R] = 0;
-        st[E_REQUIRED] = largest;
-        if (largest > cap) {
-            st[E_ERROR] = E_ERR_CAPACITY;
-            st[E_VALID] = 0;
-        } else {
-            st[E_VALID] = 1;
-            st[E_LAST_BUILD] = st[E_STEP];
-            st[E_BUILDS] += 1;
-        }
-    }
+    if (c < g.nx * g.ny * g.nz)
+        fmax = cell_rows<D>(g, c, item - c * nsplit, nsplit, xq, sorted, cell_off, rl2, cap, rows, counts, ref,
+                            ell_stage + w * ROWS_CAP);
+    if (ell_block_max_last(fmax, st, E_RMAX, E_TICKET_R)) rows_commit(st, cap);
 }
 
-// Packed coordinates (x, y, z, 0) for the pair kernel's 16-byte neighbour loads.
-template <int D>
+// Packed coordinates (x, y, z, 0) in cell order.  REBUILD: inside a rebuild, after the sort (the particles'
+// positions in the new order are written too); otherwise the pack of a force evaluation.
+template <int D, bool REBUILD>
 __global__ void k_ell_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-                           int n, float4 *__restrict__ xq) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) xq[i] = make_float4(x[i], y[i], D == 3 ? z[i] : 0.f, 0.f);
+                           const int *__restrict__ sorted, int n, int *__restrict__ pos_of, float4 *__restrict__ xq,
+                           const long long *__restrict__ st) {
+    if (REBUILD && !ell_requested(st)) return;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int i = sorted[k];
+    xq[k] = make_float4(x[i], y[i], D == 3 ? z[i] : 0.f, 0.f);
+    if (REBUILD) pos_of[i] = k;
+}
+
+// The rows by particle id, slot t of particle i at t n + i, for callers that read them (pd_ell_rows): entry t
+// of position k at k sk + t st_.
+__global__ void k_ell_export(const int *__restrict__ rows, const int *__restrict__ counts,
+                             const int *__restrict__ sorted, int n, int cap, size_t sk, size_t st_,
+                             int *__restrict__ orows, int *__restrict__ ocounts) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int i = sorted[k], c = counts[k];
+    ocounts[i] = c;
+    for (int t = 0; t < min(c, cap); ++t) orows[(size_t)t * n + i] = sorted[rows[k * sk + t * st_]];
 }
 
 struct EllModel {
     int kind;        // PD_PAIR_LJ or PD_PAIR_WCA
     float eps, sig2, rc2, eshift;
+    float rc_clear;  // a particle farther than this from every face has no pair across one
 };
 
 struct EllKick {     // closing half kick fused into the pair kernel (step engine)
@@ -427,72 +414,88 @@ struct EllKick {     // closing half kick fused into the pair kernel (step engin
 };
 
 // Row pair kernel (_pair_cooperative_kernel!, PairTraversal.jl:66-125, with the UniformLJ /
-// UniformWCA models of PairModels.jl:13-49): G lanes per particle stride its row; per pair the
+// UniformWCA models of PairModels.jl:13-49): G lanes per cell-order position walk its row; per pair the
 // compensated periodic difference, nested multiply-add r^2, f/r = 24 eps (2 s12 - s6) / r^2 and
 // u = 4 eps (s12 - s6) - shift (LJ) or + eps (WCA) inside (0, rc^2); each row gets half of every
-// pair energy and half of its dyadic virial.  Forces are stored (not added).
-template <int D, int G, bool ENERGY, bool KICK>
+// pair energy and half of its dyadic virial.  Forces are stored (not added): by particle (OUT_FORCE), by
+// particle with the closing half kick (OUT_KICK), or by position for k_ell_finish (OUT_SLOT): a particle's
+// force and velocity are nine scattered 32-byte sectors, a position's force is one coalesced record.
+enum { OUT_FORCE = 0, OUT_KICK = 1, OUT_SLOT = 2 };
+
+__device__ __forceinline__ void ell_kick(const EllKick &kick, int i, int D, const float *a) {
+    const float im = kick.inv_mass ? kick.inv_mass[i] : kick.inv_mass_uniform;
+    const float c = kick.half_dt * im;
+    const float v0 = fmaf(c, a[0], kick.vx[i]), v1 = fmaf(c, a[1], kick.vy[i]);
+    const float v2 = D == 3 ? fmaf(c, a[2], kick.vz[i]) : 0.f;
+    kick.vx[i] = v0;
+    kick.vy[i] = v1;
+    if (D == 3) kick.vz[i] = v2;
+    if (kick.dU) {   // _b2_kernel! (Langevin.jl:141-160): power v.f and kinetic energy after B2
+        kick.dU[i] += v0 * a[0] + v1 * a[1] + v2 * a[2];
+        kick.ekin[i] = 0.5f * (v0 * v0 + v1 * v1 + v2 * v2) / im;
+    }
+}
+
+template <int D, int G, bool UNIT, bool ENERGY, int OUT>
 __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restrict__ xq, int n,
                                                            const int *__restrict__ rows,
-                                                           const int *__restrict__ counts, float Lx, float Ly,
-                                                           float Lz, EllModel m, float *__restrict__ fx,
-                                                           float *__restrict__ fy, float *__restrict__ fz,
-                                                           float *__restrict__ epot, float *__restrict__ vir,
+                                                           const int *__restrict__ counts,
+                                                           const int *__restrict__ sorted, size_t sk, size_t slot_stride,
+                                                           float Lx, float Ly, float Lz, EllModel m,
+                                                           float *__restrict__ fx, float *__restrict__ fy,
+                                                           float *__restrict__ fz, float *__restrict__ epot,
+                                                           float *__restrict__ vir, float4 *__restrict__ fc,
                                                            EllKick kick, long long *__restrict__ st) {
     if (st[E_VALID] == 0) return;   // _device_if_valid!: no valid list, no forces
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = tid / G, lane = tid % G;
-    const float hLx = 0.5f * Lx, hLy = 0.5f * Ly, hLz = 0.5f * Lz;
+    const int k = tid / G, lane = tid % G;
+    const float L[3] = {Lx, Ly, Lz};
     constexpr int NV = D == 3 ? 6 : 3;
     float a[3] = {0.f, 0.f, 0.f}, e = 0.f, w[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) w[k] = 0.f;
-    if (i < n) {
-        const float4 pi = xq[i];
-        const int cnt = counts[i];
-        auto pair = [&](float4 pj) {
-            const float dx = periodic_delta(pi.x, pj.x, hLx, Lx);
-            const float dy = periodic_delta(pi.y, pj.y, hLy, Ly);
-            const float dz = D == 3 ? periodic_delta(pi.z, pj.z, hLz, Lz) : 0.f;
-            const float r2 = D == 3 ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : fmaf(dx, dx, dy * dy);
-            if (r2 > 0.f && r2 < m.rc2) {
-                const float ir2 = 1.f / r2;
-                const float s2 = m.sig2 * ir2;
-                const float s6 = s2 * s2 * s2;
-                const float s12 = s6 * s6;
-                const float fr = 24.f * m.eps * (2.f * s12 - s6) * ir2;
-                const float fxv = fr * dx, fyv = fr * dy, fzv = fr * dz;
-                a[0] += fxv;
-                a[1] += fyv;
-                if (D == 3) a[2] += fzv;
+    for (int t = 0; t < NV; ++t) w[t] = 0.f;
+    const float4 pi = k < n ? xq[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int cnt = k < n ? counts[k] : 0;
+    const LjRow lj = lj_row(m.eps, m.sig2, m.rc2, m.kind == PD_PAIR_WCA ? m.eps : -m.eshift);
+    auto walk = [&](auto wrap) {
+        constexpr bool WRAP = decltype(wrap)::value;
+        walk_row<G, UNIT>(rows + k * sk, slot_stride, lane, cnt, k, xq, [&](const float4 &pa, const float4 &pb) {
+            float dx[2], dy[2], dz[2], r2[2], f[2], u[2];
+            pair_delta<D, WRAP>(pi, pa, L, dx[0], dy[0], dz[0]);
+            pair_delta<D, WRAP>(pi, pb, L, dx[1], dy[1], dz[1]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                r2[c] = D == 3 ? fmaf(dx[c], dx[c], fmaf(dy[c], dy[c], dz[c] * dz[c])) : fmaf(dx[c], dx[c], dy[c] * dy[c]);
+            f2 fr, un;
+            lj_two<ENERGY>(lj, rcp2(pk(r2[0], r2[1])), fr, un);
+            unpk(fr, f[0], f[1]);
+            if (ENERGY) unpk(un, u[0], u[1]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const bool in = r2[c] > 0.f && r2[c] < lj.rc2;
+                const float fv = in ? f[c] : 0.f;
+                a[0] = fmaf(fv, dx[c], a[0]);
+                a[1] = fmaf(fv, dy[c], a[1]);
+                if (D == 3) a[2] = fmaf(fv, dz[c], a[2]);
                 if (ENERGY) {
-                    const float u = 4.f * m.eps * (s12 - s6) + (m.kind == PD_PAIR_WCA ? m.eps : -m.eshift);
-                    e += 0.5f * u;
+                    e += in ? 0.5f * u[c] : 0.f;
+                    const float hx = 0.5f * fv * dx[c], hy = 0.5f * fv * dy[c];
+                    w[0] = fmaf(hx, dx[c], w[0]);
+                    w[1] = fmaf(hy, dy[c], w[1]);
                     if (D == 3) {
-                        w[0] += 0.5f * dx * fxv;
-                        w[1] += 0.5f * dy * fyv;
-                        w[2] += 0.5f * dz * fzv;
-                        w[3] += 0.5f * dx * fyv;
-                        w[4] += 0.5f * dx * fzv;
-                        w[5] += 0.5f * dy * fzv;
+                        w[2] = fmaf(0.5f * fv * dz[c], dz[c], w[2]);
+                        w[3] = fmaf(hx, dy[c], w[3]);
+                        w[4] = fmaf(hx, dz[c], w[4]);
+                        w[5] = fmaf(hy, dz[c], w[5]);
                     } else {
-                        w[0] += 0.5f * dx * fxv;
-                        w[1] += 0.5f * dy * fyv;
-                        w[2] += 0.5f * dx * fyv;
+                        w[2] = fmaf(hx, dy[c], w[2]);
                     }
                 }
             }
-        };
-        int slot = lane;
-        // two neighbours per iteration: both loads in flight before either is used
-        for (; slot + G < cnt; slot += 2 * G) {
-            const float4 p1 = xq[rows[(size_t)slot * n + i]];
-            const float4 p2 = xq[rows[(size_t)(slot + G) * n + i]];
-            pair(p1);
-            pair(p2);
-        }
-        for (; slot < cnt; slot += G) pair(xq[rows[(size_t)slot * n + i]]);
-    }
+        });
+    };
+    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<D>(pi, L, m.rc_clear))) walk(std::false_type{});
+    else walk(std::true_type{});
     // every lane reaches every shuffle
 #pragma unroll
     for (int off = G / 2; off > 0; off >>= 1) {
@@ -501,31 +504,44 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
         if (ENERGY) {
             e += __shfl_down_sync(0xffffffffu, e, off, G);
 #pragma unroll
-            for (int k = 0; k < NV; ++k) w[k] += __shfl_down_sync(0xffffffffu, w[k], off, G);
+            for (int t = 0; t < NV; ++t) w[t] += __shfl_down_sync(0xffffffffu, w[t], off, G);
         }
     }
-    if (lane == 0 && i < n) {
+    if (lane == 0 && k < n) {
+        if (OUT == OUT_SLOT) {
+            fc[k] = make_float4(a[0], a[1], a[2], 0.f);
+        } else {
+            const int i = sorted[k];
+            fx[i] = a[0];
+            fy[i] = a[1];
+            if (D == 3) fz[i] = a[2];
+            if (ENERGY) {
+                epot[i] = e;
+#pragma unroll
+                for (int t = 0; t < NV; ++t) vir[(size_t)i * NV + t] = w[t];
+            }
+            if (OUT == OUT_KICK) ell_kick(kick, i, D, a);
+        }
+    }
+    if (OUT == OUT_KICK && kick.advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
+}
+
+// Positions' forces to particle order, with the closing half kick when there is one.
+template <int D, bool KICK>
+__global__ void __launch_bounds__(ELL_THREADS) k_ell_finish(const float4 *__restrict__ fc,
+                                                            const int *__restrict__ pos_of, int n,
+                                                            float *__restrict__ fx, float *__restrict__ fy,
+                                                            float *__restrict__ fz, EllKick kick,
+                                                            long long *__restrict__ st) {
+    if (st[E_VALID] == 0) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        const float4 f = fc[pos_of[i]];
+        const float a[3] = {f.x, f.y, f.z};
         fx[i] = a[0];
         fy[i] = a[1];
         if (D == 3) fz[i] = a[2];
-        if (ENERGY) {
-            epot[i] = e;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) vir[(size_t)i * NV + k] = w[k];
-        }
-        if (KICK) {
-            const float im = kick.inv_mass ? kick.inv_mass[i] : kick.inv_mass_uniform;
-            const float c = kick.half_dt * im;
-            const float v0 = fmaf(c, a[0], kick.vx[i]), v1 = fmaf(c, a[1], kick.vy[i]);
-            const float v2 = D == 3 ? fmaf(c, a[2], kick.vz[i]) : 0.f;
-            kick.vx[i] = v0;
-            kick.vy[i] = v1;
-            if (D == 3) kick.vz[i] = v2;
-            if (kick.dU) {   // _b2_kernel! (Langevin.jl:141-160): power v.f and kinetic energy after B2
-                kick.dU[i] += v0 * a[0] + v1 * a[1] + v2 * a[2];
-                kick.ekin[i] = 0.5f * (v0 * v0 + v1 * v1 + v2 * v2) / im;
-            }
-        }
+        if (KICK) ell_kick(kick, i, D, a);
     }
     if (KICK && kick.advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
 }
@@ -548,13 +564,26 @@ struct pd_ell {
     int cap = 0;
     long long *st = nullptr;
     int *cell_of = nullptr, *cell_count = nullptr, *cell_off = nullptr, *sorted = nullptr, *tmp = nullptr;
+    int *pos_of = nullptr;              // inverse of sorted
+    int *scan_part = nullptr;           // tile sums of the cell scan
     int *rows = nullptr, *counts = nullptr;
-    float4 *ref = nullptr, *xq = nullptr;
+    bool dense = false;                 // row-major rows, built by warps (rows.cuh); otherwise slot-major
+    int *xrows = nullptr, *xcounts = nullptr;   // rows by particle id, kept current once pd_ell_rows was called
+    float4 *ref = nullptr, *xq = nullptr, *fc = nullptr;
 };
 
 namespace pdb {
 
+// From this size the pair kernel stores its forces by position and k_ell_finish carries them to particle
+// order: below it the extra launch costs more than the scattered stores.
+constexpr int ELL_SLOT_MIN = 32768;
+
 static void ell_free(pd_ell *e) {
+    dfree(e->pos_of);
+    dfree(e->scan_part);
+    dfree(e->xrows);
+    dfree(e->xcounts);
+    dfree(e->fc);
     dfree(e->st);
     dfree(e->cell_of);
     dfree(e->cell_count);
@@ -574,7 +603,58 @@ EllModel ell_model(const pd_ell *e) {
     m.sig2 = e->p.sigma * e->p.sigma;
     m.rc2 = e->p.rc2;
     m.eshift = e->p.eshift;
+    m.rc_clear = 1.001f * std::sqrt(e->p.rc2);   // above the cutoff by more than the coordinates' rounding
     return m;
+}
+
+static size_t scan_part_len(int ncell) { return (size_t)(ncell + SCAN_TILE - 1) / SCAN_TILE + 2; }
+
+// The counting sort of particles into cells, shared with the batched replicas: exclusive scan of
+// the histogram (which becomes the scatter cursors), the scatter, id order inside each cell; every
+// kernel returns at once unless st asks for a rebuild.  part: ell_scan_part_len(ncell) ints, zero at first.
+int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
+                    int *tmp, long long *st, cudaStream_t s) {
+    const int blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
+    if (ncell <= SCAN_ONE_BLOCK) {
+        k_ell_scan<<<1, 1024, 0, s>>>(cell_count, cell_off, ncell, st);
+        PD_LAUNCHED();
+    } else {
+        const int ntile = (ncell + SCAN_TILE - 1) / SCAN_TILE;
+        k_scan_sums<<<ntile, SCAN_THREADS, 0, s>>>(cell_count, ncell, part, ntile, st);
+        PD_LAUNCHED();
+        k_scan_apply<<<ntile, SCAN_THREADS, 0, s>>>(cell_count, cell_off, ncell, part, ntile, st);
+        PD_LAUNCHED();
+    }
+    k_ell_scatter<<<blocks, ELL_THREADS, 0, s>>>(cell_of, n, cell_off, cell_count, sorted, st);
+    PD_LAUNCHED();
+    if (n >= ROWS_MIN_PER_CELL * (long long)ncell)
+        k_ell_cellsort<<<(int)(((long long)ncell * 32 + 255) / 256), 256, 0, s>>>(cell_off, ncell, sorted, tmp,
+                                                                                  cell_count, st);
+    else
+        k_ell_cellsort_sparse<<<(ncell + 127) / 128, 128, 0, s>>>(cell_off, ncell, sorted, cell_count, st);
+    PD_LAUNCHED();
+    return PD_OK;
+}
+
+size_t ell_scan_part_len(int ncell) { return scan_part_len(ncell); }
+
+EllRowsView ell_rows_view(const pd_ell *e) {
+    EllRowsView v;
+    v.rows = e->rows;
+    v.counts = e->counts;
+    v.sorted = e->sorted;
+    v.cap = e->cap;
+    v.sk = e->dense ? (size_t)e->cap : 1;
+    v.st = e->dense ? 1 : (size_t)e->n;
+    return v;
+}
+
+static int ell_export_launch(pd_ell *e, cudaStream_t s) {
+    const EllRowsView v = ell_rows_view(e);
+    k_ell_export<<<(e->n + ELL_THREADS - 1) / ELL_THREADS, ELL_THREADS, 0, s>>>(v.rows, v.counts, v.sorted, e->n, v.cap,
+                                                                                 v.sk, v.st, e->xrows, e->xcounts);
+    PD_LAUNCHED();
+    return PD_OK;
 }
 
 // Decision + flag-gated rebuild kernels on stream s (the rebuild returns at once unless the
@@ -582,6 +662,7 @@ EllModel ell_model(const pd_ell *e) {
 int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int n = e->n, blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
     const float Lx = e->L[0], Ly = e->L[1], Lz = e->L[2];
+    int rc;
     if (!e->allpairs) {
         if (e->dim == 3)
             k_ell_bin<3><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
@@ -590,54 +671,41 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
             k_ell_bin<2><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
                                                         e->cell_count, e->st);
         PD_LAUNCHED();
-        k_ell_scan<<<1, 1024, 0, s>>>(e->cell_count, e->cell_off, e->ncell, e->st);
-        PD_LAUNCHED();
-        k_ell_scatter<<<blocks, ELL_THREADS, 0, s>>>(e->cell_of, n, e->cell_off, e->cell_count, e->sorted, e->st);
-        PD_LAUNCHED();
-        k_ell_cellsort<<<(int)(((long long)e->ncell * 32 + 255) / 256), 256, 0, s>>>(e->cell_off, e->ncell, e->sorted,
-                                                                                    e->tmp, e->cell_count, e->st);
-        PD_LAUNCHED();
+        if ((rc = ell_sort_launch(e->cell_of, n, e->ncell, e->cell_count, e->cell_off, e->scan_part, e->sorted, e->tmp,
+                                  e->st, s)))
+            return rc;
     }
-#define PD_ELL_ROWS(DD, AP)                                                                                           \
-    k_ell_rows<DD, AP><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, n, e->sorted, e->cell_of, e->cell_off, Lx, Ly, Lz,    \
-                                                      e->nx, e->ny, e->nz, e->rl2, e->cap, e->rows, e->counts, e->ref, \
-                                                      e->st)
-#define PD_ELL_ROWS_CELLS(DD)                                                                                         \
-    k_ell_rows_cells<DD><<<(e->ncell + ROWS_WARPS - 1) / ROWS_WARPS, 32 * ROWS_WARPS,                                \
-                           sizeof(float4) * ROWS_WARPS * ROWS_CAP, s>>>(x, y, z, n, e->sorted, e->cell_off, Lx, Ly,  \
-                                                                        Lz, e->nx, e->ny, e->nz, e->rl2, e->cap,     \
-                                                                        e->rows, e->counts, e->ref, e->st)
-    // a warp per cell pays off once cells hold enough particles to occupy its lanes
-    const bool cells = !e->allpairs && n >= ROWS_MIN_PER_CELL * e->ncell;
-    if (e->dim == 3) {
+    if (e->dim == 3)
+        k_ell_pack<3, true><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
+    else
+        k_ell_pack<2, true><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
+    PD_LAUNCHED();
+#define PD_ELL_ROWS(DD, AP)                                                                                          \
+    k_ell_rows<DD, AP><<<blocks, ELL_THREADS, 0, s>>>(e->xq, n, e->sorted, e->cell_of, e->cell_off, Lx, Ly, Lz, e->nx, \
+                                                      e->ny, e->nz, e->rl2, e->cap, e->rows, e->counts, e->ref, e->st)
+    if (e->dense) {
+        const RowGrid g{{Lx, Ly, Lz}, e->nx, e->ny, e->nz, 0};
+        // few cells: several warps per cell, until the chip has about 16 warps per SM
+        int nsplit = 1;
+        while (nsplit < 8 && (long long)e->ncell * nsplit < 148 * 16) nsplit *= 2;
+        const int grid = (int)(((long long)e->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
+        const size_t shm = sizeof(float4) * ROWS_WARPS * ROWS_CAP;
+        if (e->dim == 3)
+            k_ell_rows_cells<3><<<grid, 32 * ROWS_WARPS, shm, s>>>(e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
+                                                                   e->cap, e->rows, e->counts, e->ref, e->st);
+        else
+            k_ell_rows_cells<2><<<grid, 32 * ROWS_WARPS, shm, s>>>(e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
+                                                                   e->cap, e->rows, e->counts, e->ref, e->st);
+    } else if (e->dim == 3) {
         if (e->allpairs) PD_ELL_ROWS(3, true);
-        else if (cells) PD_ELL_ROWS_CELLS(3);
         else PD_ELL_ROWS(3, false);
     } else {
         if (e->allpairs) PD_ELL_ROWS(2, true);
-        else if (cells) PD_ELL_ROWS_CELLS(2);
         else PD_ELL_ROWS(2, false);
     }
 #undef PD_ELL_ROWS
-#undef PD_ELL_ROWS_CELLS
     PD_LAUNCHED();
-    return PD_OK;
-}
-
-// The counting sort of particles into cells, shared with the batched replicas: exclusive scan of
-// the histogram (which becomes the scatter cursors), the scatter, id order inside each cell; every
-// kernel returns at once unless st asks for a rebuild.
-int ell_sort_cells_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *sorted, int *tmp,
-                          long long *st, cudaStream_t s) {
-    const int blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
-    k_ell_scan<<<1, 1024, 0, s>>>(cell_count, cell_off, ncell, st);
-    PD_LAUNCHED();
-    k_ell_scatter<<<blocks, ELL_THREADS, 0, s>>>(cell_of, n, cell_off, cell_count, sorted, st);
-    PD_LAUNCHED();
-    k_ell_cellsort<<<(int)(((long long)ncell * 32 + 255) / 256), 256, 0, s>>>(cell_off, ncell, sorted, tmp, cell_count,
-                                                                             st);
-    PD_LAUNCHED();
-    return PD_OK;
+    return e->xrows ? ell_export_launch(e, s) : PD_OK;
 }
 
 int ell_decide_launch(pd_ell *e, const float *x, const float *y, const float *z, cudaStream_t s) {
@@ -652,40 +720,47 @@ int ell_decide_launch(pd_ell *e, const float *x, const float *y, const float *z,
     return PD_OK;
 }
 
-template <int D, int G>
+template <int D, int G, bool UNIT>
 static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
                         const EllKick &kick, cudaStream_t s) {
     const int blocks = (int)(((long long)e->n * G + ELL_THREADS - 1) / ELL_THREADS);
     const EllModel m = ell_model(e);
-    if (kick.vx) {
-        if (energy)
-            k_ell_pairs<D, G, true, true><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, e->rows, e->counts, e->L[0],
-                                                                         e->L[1], e->L[2], m, fx, fy, fz, epot, vir,
-                                                                         kick, e->st);
-        else
-            k_ell_pairs<D, G, false, true><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, e->rows, e->counts, e->L[0],
-                                                                          e->L[1], e->L[2], m, fx, fy, fz, epot, vir,
-                                                                          kick, e->st);
+    const EllRowsView v = ell_rows_view(e);
+#define PD_ELL_PAIRS(EN, OO)                                                                                      \
+    k_ell_pairs<D, G, UNIT, EN, OO><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, v.rows, v.counts, v.sorted, v.sk, v.st, \
+                                                             e->L[0], e->L[1], e->L[2], m, fx, fy, fz, epot, vir, \
+                                                             e->fc, kick, e->st)
+    if (energy) {
+        if (kick.vx) PD_ELL_PAIRS(true, OUT_KICK);
+        else PD_ELL_PAIRS(true, OUT_FORCE);
+    } else if (e->n < ELL_SLOT_MIN) {
+        if (kick.vx) PD_ELL_PAIRS(false, OUT_KICK);
+        else PD_ELL_PAIRS(false, OUT_FORCE);
     } else {
-        if (energy)
-            k_ell_pairs<D, G, true, false><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, e->rows, e->counts, e->L[0],
-                                                                          e->L[1], e->L[2], m, fx, fy, fz, epot, vir,
-                                                                          kick, e->st);
-        else
-            k_ell_pairs<D, G, false, false><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, e->rows, e->counts, e->L[0],
-                                                                           e->L[1], e->L[2], m, fx, fy, fz, epot, vir,
-                                                                           kick, e->st);
+        PD_ELL_PAIRS(false, OUT_SLOT);
+        const int fb = (e->n + ELL_THREADS - 1) / ELL_THREADS;
+        count_launch();
+        if (kick.vx) k_ell_finish<D, true><<<fb, ELL_THREADS, 0, s>>>(e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
+        else k_ell_finish<D, false><<<fb, ELL_THREADS, 0, s>>>(e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
     }
+#undef PD_ELL_PAIRS
 }
 
+// Lanes per row: slot-major rows take the engine's choice; row-major rows at least 8, so that a step of the
+// walk reads whole 32-byte sectors, and a whole warp per row where the rows alone would leave SMs idle.
 template <int D>
 static void ell_pairs_d(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
                         const EllKick &kick, cudaStream_t s) {
+    if (e->dense) {
+        if (e->n < 16384) ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
+        else ell_pairs_g<D, 8, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
+        return;
+    }
     switch (e->lanes) {
-        case 1: ell_pairs_g<D, 1>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        case 2: ell_pairs_g<D, 2>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        case 4: ell_pairs_g<D, 4>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        default: ell_pairs_g<D, 8>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        case 1: ell_pairs_g<D, 1, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        case 2: ell_pairs_g<D, 2, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        case 4: ell_pairs_g<D, 4, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        default: ell_pairs_g<D, 8, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
     }
 }
 
@@ -700,18 +775,14 @@ int ell_pairs_launch(pd_ell *e, float *fx, float *fy, float *fz, float *epot, fl
 
 int ell_pack_launch(pd_ell *e, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int blocks = (e->n + ELL_THREADS - 1) / ELL_THREADS;
-    if (e->dim == 3) k_ell_pack<3><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->n, e->xq);
-    else k_ell_pack<2><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->n, e->xq);
+    if (e->dim == 3)
+        k_ell_pack<3, false><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
+    else
+        k_ell_pack<2, false><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
     PD_LAUNCHED();
     return PD_OK;
 }
 
-long long *ell_state(pd_ell *e) { return e->st; }
-float4 *ell_packed(pd_ell *e) { return e->xq; }
-float4 *ell_ref(pd_ell *e) { return e->ref; }
-float ell_threshold(const pd_ell *e) { return e->threshold; }
-int ell_dim(const pd_ell *e) { return e->dim; }
-int ell_capacity(const pd_ell *e) { return e->cap; }
 
 static int ell_alloc_rows(pd_ell *e, int cap) {
     PD_CHECK(cap > 0, PD_EINVAL, "Invalid ELL capacity");
@@ -721,6 +792,11 @@ static int ell_alloc_rows(pd_ell *e, int cap) {
     int rc = dalloc(&e->rows, (size_t)e->n * cap);
     if (rc) return rc;
     PD_CUDA(cudaMemset(e->rows, 0xff, sizeof(int) * (size_t)e->n * cap));
+    if (e->xrows) {
+        dfree(e->xrows);
+        if ((rc = dalloc(&e->xrows, (size_t)e->n * cap))) return rc;
+        PD_CUDA(cudaMemset(e->xrows, 0xff, sizeof(int) * (size_t)e->n * cap));
+    }
     e->cap = cap;
     return PD_OK;
 }
@@ -772,6 +848,8 @@ int pd_ell_create(pd_ell **out, const pd_ell_params *p, const double box[3]) {
     e->nz = ng[2];
     if (e->allpairs) e->nx = e->ny = e->nz = 1;
     e->ncell = e->nx * e->ny * e->nz;
+    // a warp per cell pays off once cells hold enough particles to share its stage
+    e->dense = !e->allpairs && e->n >= (long long)ROWS_MIN_PER_CELL * e->ncell;
     // lanes per row: the expected row length at this density
     if (p->lanes) {
         e->lanes = p->lanes;
@@ -787,14 +865,22 @@ int pd_ell_create(pd_ell **out, const pd_ell_params *p, const double box[3]) {
         (rc = dalloc(&e->cell_count, (size_t)e->ncell)) || (rc = dalloc(&e->cell_off, (size_t)e->ncell + 1)) ||
         (rc = dalloc(&e->sorted, (size_t)e->n)) || (rc = dalloc(&e->tmp, (size_t)e->n)) ||
         (rc = dalloc(&e->counts, (size_t)e->n)) || (rc = dalloc(&e->ref, (size_t)e->n)) ||
-        (rc = dalloc(&e->xq, (size_t)e->n)) || (rc = ell_alloc_rows(e, p->cap))) {
+        (rc = dalloc(&e->xq, (size_t)e->n)) || (rc = dalloc(&e->pos_of, (size_t)e->n)) ||
+        (rc = dalloc(&e->scan_part, scan_part_len(e->ncell))) ||
+        (rc = dalloc(&e->fc, e->n < ELL_SLOT_MIN ? 1 : (size_t)e->n)) || (rc = ell_alloc_rows(e, p->cap))) {
         ell_free(e);
         delete e;
         return rc;
     }
     long long init[E_LEN] = {0};
     init[E_INTERVAL] = p->interval;
-    if (cudaMemcpy(e->st, init, sizeof init, cudaMemcpyHostToDevice) != cudaSuccess ||
+    // the identity order until the first build (and for good in small boxes, whose rows take all pairs)
+    std::vector<int> ident((size_t)e->n);
+    for (int i = 0; i < e->n; ++i) ident[(size_t)i] = i;
+    if (cudaMemcpy(e->sorted, ident.data(), sizeof(int) * (size_t)e->n, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(e->pos_of, ident.data(), sizeof(int) * (size_t)e->n, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemset(e->scan_part, 0, sizeof(int) * scan_part_len(e->ncell)) != cudaSuccess ||
+        cudaMemcpy(e->st, init, sizeof init, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(e->cell_count, 0, sizeof(int) * (size_t)e->ncell) != cudaSuccess ||
         cudaMemset(e->counts, 0, sizeof(int) * (size_t)e->n) != cudaSuccess ||
         cudaMemset(e->ref, 0, sizeof(float4) * (size_t)e->n) != cudaSuccess) {
@@ -862,8 +948,21 @@ int pd_ell_status(pd_ell *e, pd_ell_stats *out) {
 
 int pd_ell_rows(pd_ell *e, int **rows, int **counts) {
     PD_CHECK(e && rows && counts, PD_EINVAL, "pd_ell_rows: null argument");
-    *rows = e->rows;
-    *counts = e->counts;
+    if (!e->xrows) {   // from now on every rebuild refreshes them (captured steps are captured again)
+        int rc;
+        if ((rc = dalloc(&e->xcounts, (size_t)e->n)) || (rc = dalloc(&e->xrows, (size_t)e->n * e->cap))) {
+            dfree(e->xcounts);
+            return rc;
+        }
+        PD_CUDA(cudaMemset(e->xrows, 0xff, sizeof(int) * (size_t)e->n * e->cap));
+        PD_CUDA(cudaMemset(e->xcounts, 0, sizeof(int) * (size_t)e->n));
+        PD_CUDA(cudaDeviceSynchronize());   // a build may be in flight on another stream
+        int rc2 = ell_export_launch(e, 0);
+        if (rc2) return rc2;
+        PD_CUDA(cudaDeviceSynchronize());
+    }
+    *rows = e->xrows;
+    *counts = e->xcounts;
     return PD_OK;
 }
 
@@ -943,7 +1042,9 @@ struct EllStepArgs {
     float kick;               // BAOAB / BAOA: the B1 kick length, dt (BAOAB) or 2 dt (BAOA, no B2)
     float *dq, *dU, *ekin;    // Langevin bookkeeping (heat, work of the forces, kinetic energy), or null
     float4 *xq;
+    const int *pos_of;
     const float4 *ref;
+    const int *rows, *xrows;  // not read by the drift: part of the key that captured steps are matched on
     float threshold;
 };
 
@@ -1033,7 +1134,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_drift(EllStepArgs a, long l
             a.z[i] = p[2];
             a.vz[i] = v[2];
         }
-        a.xq[i] = make_float4(p[0], p[1], p[2], 0.f);
+        a.xq[a.pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);
         disp = ell_displacement<D>(p, a.ref[i], a.L, true);
     }
     if (ell_block_max_last(__float_as_uint(disp), st, E_DMAX, E_TICKET_D)) {
@@ -1128,6 +1229,9 @@ static EllStepArgs ell_step_args(pd_ell_md *md, float dt, float gamma, float kT,
         a.ekin = md->ekin;
     }
     a.xq = e->xq;
+    a.pos_of = e->pos_of;
+    a.rows = e->rows;
+    a.xrows = e->xrows;
     a.ref = e->ref;
     a.threshold = e->threshold;
     if (md->f0) {

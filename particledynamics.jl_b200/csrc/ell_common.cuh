@@ -137,4 +137,24 @@ __device__ __forceinline__ int ell_reach(float rl, float L, int n) {
     return min(max(1, (int)ceilf(rl * (float)n / L - 1e-5f)), (n - 1) / 2);
 }
 
+// ------------------------------------------------------------------ host side of ell.cu
+
+// The rows of an ELL engine: entry t of cell-order position k at rows[k sk + t st], positions as entries.
+struct EllRowsView {
+    const int *rows, *counts, *sorted;
+    int cap;
+    size_t sk, st;
+};
+
+}  // namespace pdb
+
+struct pd_ell;
+
+namespace pdb {
+
+EllRowsView ell_rows_view(const ::pd_ell *e);
+int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
+                    int *tmp, long long *st, cudaStream_t s);
+size_t ell_scan_part_len(int ncell);
+
 }  // namespace pdb

@@ -222,15 +222,12 @@ int cluster_exceptions_launch(pd_cluster *c, int energy, cudaStream_t s);
 void cluster_free_exceptions(pd_cluster *c);
 int cluster_set_word(pd_cluster *c, int word, int value, cudaStream_t s);
 // ELL, network and learned-correction internals used by the learned form and the step engine.
-int ell_capacity(const pd_ell *e);
 int mlp_forward_launch(const pd_mlp *q, const void *X, int n, float *s, const float4 *V, float4 *corr,
                        cudaStream_t st);
 int learned_correction_launch(pd_learned *h, const pd_mlp *net, const float *x, const float *y, const float *z,
                               const float *q, const int *type, float4 *corr, cudaStream_t s);
 const float4 *learned_corr(const pd_learned *h);
 const float4 *learned_radial(const pd_learned *h);
-int ell_sort_cells_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *sorted, int *tmp,
-                          long long *st, cudaStream_t s);
 
 // Batched meshes of charged replicas (batch_mesh.cu).  Replica r's real grids start at float
 // `grid` of the concatenated grids and its half spectrum (and influence function) at complex mode
@@ -253,6 +250,7 @@ struct BMeshView {
     const int *slot_src;         // nchunk * chunk: cell-order position or -1
     float4 *mq;                  // nchunk * chunk: (x, y, z, q) of the slot's particle
     int *mid;                    // nchunk * chunk: particle index or -1
+    const float4 *fc;            // pair force and energy by cell-order position
     float *gridA, *gridB;        // charge grids (zero between steps), potential grids
     float2 *spec;
     const float *G;

@@ -24,6 +24,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "ell_common.cuh"
 #include "internal.hpp"
 
 using namespace pdb;
@@ -69,15 +70,16 @@ __device__ __forceinline__ float mic_d(float d, float L) {
     return d;
 }
 
-// Packed neighbour record (x, y, z, q) with the species in the lowest mantissa bit of q (a change
+// Packed neighbour record (x, y, z, q), in the rows' cell order, with the species in the lowest mantissa bit of q (a change
 // of at most one ulp of the charge), so that a row entry costs one 16-byte gather.
 __global__ void k_desc_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-                            const float *__restrict__ q, const int *__restrict__ type, int n,
-                            float4 *__restrict__ xq) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+                            const float *__restrict__ q, const int *__restrict__ type,
+                            const int *__restrict__ sorted, int n, float4 *__restrict__ xq) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int i = sorted[k];
     const int s1 = (type != nullptr && type[i] > 1) ? 1 : 0;
-    xq[i] = make_float4(x[i], y[i], z[i], __int_as_float((__float_as_int(q[i]) & ~1) | s1));
+    xq[k] = make_float4(x[i], y[i], z[i], __int_as_float((__float_as_int(q[i]) & ~1) | s1));
 }
 
 // Sum over the G consecutive lanes of a particle's group (butterfly: every lane gets the total).
@@ -93,15 +95,16 @@ __device__ __forceinline__ float group_sum(float v) {
 // of the group stores the g-th 16-byte chunk of the particle's BF16 features.
 template <bool BASIS, int G>
 __global__ void __launch_bounds__(DESC_THREADS, 4) k_descriptors(const float4 *__restrict__ xq, int n,
-                                                              const int *__restrict__ rows,
-                                                              const int *__restrict__ counts, int cap, DescParams p,
+                                                              EllRowsView rv, DescParams p,
                                                               __nv_bfloat16 *__restrict__ X, float4 *__restrict__ V,
                                                               float4 *__restrict__ Vb) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = tid / G, g = tid % G;
-    const bool live = i < n;   // whole groups are live or not (G divides the warp)
+    const int pos = tid / G, g = tid % G;   // cell-order position
+    const bool live = pos < n;   // whole groups are live or not (G divides the warp)
     if (__all_sync(0xffffffffu, !live)) return;
-    const int ii = live ? i : 0;
+    const int ii = live ? pos : 0;
+    const int i = rv.sorted[ii];
+    const int *row = rv.rows + ii * rv.sk;
     const float4 pi = xq[ii];
     const float xi = pi.x, yi = pi.y, zi = pi.z, qi = pi.w;
     float a0[DESC_F], a1[DESC_F];
@@ -111,15 +114,15 @@ __global__ void __launch_bounds__(DESC_THREADS, 4) k_descriptors(const float4 *_
     float bx[PD_LEARNED_MAX_RADIAL], by[PD_LEARNED_MAX_RADIAL], bz[PD_LEARNED_MAX_RADIAL];
 #pragma unroll
     for (int m = 0; m < PD_LEARNED_MAX_RADIAL; ++m) bx[m] = by[m] = bz[m] = 0.f;
-    const int cnt = live ? min(counts[ii], cap) : 0;
+    const int cnt = live ? min(rv.counts[ii], rv.cap) : 0;
     // one entry ahead: the row index and the neighbour record of the next entry are in flight
     // while this one is evaluated
-    int jn = g < cnt ? __ldg(rows + (size_t)g * n + ii) : ii;
+    int jn = g < cnt ? __ldg(row + g * rv.st) : ii;
     float4 pn = __ldg(xq + jn);
     for (int t = g; t < cnt; t += G) {
         const float4 pj = pn;
         if (t + G < cnt) {
-            jn = __ldg(rows + (size_t)(t + G) * n + ii);
+            jn = __ldg(row + (t + G) * rv.st);
             pn = __ldg(xq + jn);
         }
         const float dx = mic_d(xi - pj.x, p.Lx);
@@ -252,18 +255,16 @@ static int descriptors_launch(pd_learned *h, const float *x, const float *y, con
                               const int *type, __nv_bfloat16 *X, float4 *V, float4 *Vb, cudaStream_t s) {
     int rc;
     if ((rc = pd_ell_update(h->ell, x, y, z, (pd_stream_t)s))) return rc;
-    int *rows = nullptr, *counts = nullptr;
-    if ((rc = pd_ell_rows(h->ell, &rows, &counts))) return rc;
-    const int cap = ell_capacity(h->ell);
+    const EllRowsView rv = ell_rows_view(h->ell);
     const DescParams d = desc_params(h);
-    k_desc_pack<<<(h->n + 255) / 256, 256, 0, s>>>(x, y, z, q, type, h->n, h->xq);
+    k_desc_pack<<<(h->n + 255) / 256, 256, 0, s>>>(x, y, z, q, type, rv.sorted, h->n, h->xq);
     PD_LAUNCHED();
     constexpr int G = DESC_LANES;
     const int blocks = (int)(((long long)h->n * G + DESC_THREADS - 1) / DESC_THREADS);
     if (Vb)
-        k_descriptors<true, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rows, counts, cap, d, X, V, Vb);
+        k_descriptors<true, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rv, d, X, V, Vb);
     else
-        k_descriptors<false, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rows, counts, cap, d, X, V, Vb);
+        k_descriptors<false, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rv, d, X, V, Vb);
     PD_LAUNCHED();
     return PD_OK;
 }

@@ -1,0 +1,108 @@
+"""Cell-order rows: row layouts, builds and force outputs at the sizes where their rules switch, against the
+FP64 pair sums and the neighbour-row oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _fluid(n, rho, seed, dim=3):
+    """A jittered lattice of n particles at density rho, in random order."""
+    rng = np.random.default_rng(seed)
+    L = (n / rho) ** (1.0 / dim)
+    m = int(np.ceil(n ** (1.0 / dim) - 1e-9))
+    g = np.stack(np.meshgrid(*[np.arange(m)] * dim, indexing="ij"), -1).reshape(-1, dim)
+    pos = (g[rng.permutation(len(g))[:n]] + 0.5 + rng.uniform(-0.12, 0.12, (n, dim))) * (L / m) - L / 2
+    return pos.astype(np.float32).astype(float), (float(np.float32(L)),) * dim
+
+
+# 3D, dense cells: a warp per row and several warps per cell; 8 lanes, direct stores; 8 lanes, forces by position.
+# Sparse cells: one thread per row, direct and by position; 2D: the one-block and the tiled cell scan.
+CASES = [(3, 1500, 0.8), (3, 17000, 0.8), (3, 33000, 0.8), (3, 9000, 0.08), (3, 40000, 0.08), (2, 9000, 0.85),
+         (2, 60000, 0.85)]
+
+
+@pytest.mark.parametrize("dim,n,rho", CASES)
+def test_forces_and_rows(pd, ora, cuda, dim, n, rho):
+    import torch
+    pos, box = _fluid(n, rho, 5 + n, dim)
+    rc, skin = 2.5, 0.3
+    eng = pd.ELLEngine(n, box, dim=dim, model="lj", cutoff=rc, skin=skin, capacity=160)
+    p3 = pos if dim == 3 else np.concatenate([pos, np.zeros((n, 1))], 1)
+    b3 = box if dim == 3 else (*box, 50.0)
+    ref = ora.pairs_cells(p3, b3, kind=1, sigma=1.0, eps=1.0, rc_lj=rc)
+    x = [torch.tensor(np.ascontiguousarray(pos[:, d]), dtype=torch.float32, device="cuda") for d in range(dim)]
+    x += [None] * (3 - dim)
+    f = [torch.zeros(n, device="cuda") for _ in range(dim)] + [None] * (3 - dim)
+    e, w = torch.zeros(n, device="cuda"), torch.zeros((n, 6 if dim == 3 else 3), device="cuda")
+    eng.update(*x)
+    eng.forces(*x, *f)
+    torch.cuda.synchronize()
+    F = torch.stack(f[:dim], 1).double().cpu().numpy()
+    assert np.linalg.norm(F - ref["F"][:, :dim]) < 2e-5 * np.linalg.norm(ref["F"])   # the FP32 bound of the route
+    eng.forces(*x, *f, epot=e, vir=w, energy=True)
+    torch.cuda.synchronize()
+    assert abs(float(e.double().sum()) - ref["E"].sum()) < 2e-5 * np.abs(ref["E"]).sum()
+    W = ref["W"].sum(0) if dim == 3 else ref["W"].sum(0)[[0, 1, 3]]
+    assert np.max(np.abs(w.double().sum(0).cpu().numpy() - W)) < 2e-5 * np.abs(W[:2]).sum()
+    rows, counts = eng.rows_host()
+    rl, sample = rc + skin, np.random.default_rng(1).integers(0, n, 300)
+    L = np.array(b3)
+    for i in sample:
+        d = p3 - p3[i]
+        d -= L * np.round(d / L)
+        r = np.sqrt((d * d).sum(1))
+        inner, outer = set(np.nonzero(r <= rl * (1 - 1e-5))[0]) - {i}, set(np.nonzero(r <= rl * (1 + 1e-5))[0]) - {i}
+        got = set(rows[i].tolist())
+        assert len(got) == counts[i] and inner <= got <= outer
+    eng.close()
+
+
+def test_exported_rows_follow_rebuilds(pd, cuda):
+    """Rows read once stay current through later rebuilds, in eager updates and in captured steps."""
+    import torch
+    pos, box = _fluid(5000, 0.8, 3)
+    system = pd.ParticleSystem(pos, box, velocities=np.random.default_rng(2).normal(size=pos.shape))
+    force = pd.LennardJones(epsilon=1.0, sigma=1.0, cutoff=2.5, neighborlist=pd.CellList(buffer=0.3, capacity=160))
+    sim = pd.Simulation(system, pd.Integrator(dt=0.005, forces=[force]))
+    st = sim.state
+    st.step(2)
+    st.synchronize()
+    st.ell.rows_host()
+    st.ell.request(stream=st.stream)
+    st.step(1)
+    st.synchronize()
+    rows, counts = st.ell.rows_host()
+    p = st.positions()
+    L = np.array(box)
+    for i in range(0, 5000, 97):
+        d = p - p[i]
+        d -= L * np.round(d / L)
+        r = np.sqrt((d * d).sum(1))
+        got = set(rows[i].tolist())
+        assert len(got) == counts[i]
+        assert set(np.nonzero(r <= 2.8 * (1 - 1e-5))[0]) - {i} <= got <= set(np.nonzero(r <= 2.8 * (1 + 1e-5))[0]) - {i}
+
+
+@pytest.mark.parametrize("nrep,n_hi", [(3, 1500), (12, 6000)])
+def test_batch_outputs_match_single_systems(pd, cuda, nrep, n_hi):
+    """Batched forces by particle (small batch) and by position (from 32 768 particles), and 8 captured steps."""
+    import torch
+    specs = pd.synthetic.replica_set(nrep, n_lo=1200 if nrep < 5 else 3000, n_hi=n_hi, seed=21)
+    systems = pd.batch.make_systems(specs)
+    b = pd.batch.BatchedReplicas(systems, skin=0.3, cap=160, lanes=1)
+    b.evaluate()
+    b.step(8, 0.004)
+    b.synchronize()
+    assert b.status()["error"] == 0 and (b.n >= 32768) == (nrep > 5)
+    for k, s in enumerate(systems):
+        t = [b.replica(k, a).clone() for a in (b.x, b.y, b.z)]
+        kw = dict(model="lj", cutoff=2.5) if s["kind"] == "lj" else dict(model="wca")
+        eng = pd.ELLEngine(s["n"], s["box"], skin=0.3, capacity=160, **kw)
+        f = [torch.zeros(s["n"], device="cuda") for _ in range(3)]
+        eng.update(*t)
+        eng.forces(*t, *f)
+        torch.cuda.synchronize()
+        for a, c in zip((b.fx, b.fy, b.fz), f):
+            assert float((b.replica(k, a) - c).norm()) < 1e-5 * float(torch.stack(f).norm())
+        eng.close()
