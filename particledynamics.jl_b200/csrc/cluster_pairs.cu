@@ -1,8 +1,8 @@
 // Cluster-pair pass (tiles without exclusion masks) and slot scatter of libpdb200.
 //
 // Semantics: _cluster_pair_kernel! and _scatter_kernel! of src/clusterpairs/Kernels.jl
-// (ParticleDynamics.jl); the kernel itself is in cluster_pairs.cuh.
-#include "cluster_pairs.cuh"
+// (ParticleDynamics.jl); the kernels are in pair_tiles.cuh.
+#include "pair_tiles.cuh"
 
 using namespace pdb;
 
@@ -52,7 +52,7 @@ __global__ void k_scatter(const int *__restrict__ perm, int nslot, const int *__
 
 int cluster_pairs_launch(pd_cluster *c, int energy, cudaStream_t s) {
     if (c->nexc > 0) return cluster_pairs_launch_excl(c, energy, s);
-    pairs_dispatch<false>(c, energy, s);
+    tiles_dispatch(c, energy, s);
     PD_LAUNCHED();
     return PD_OK;
 }

@@ -1,0 +1,428 @@
+// Fused cluster-pair kernels of the plain pair pass (no exclusion masks), two j-atoms per thread in packed FP32.
+//
+// Semantics: _cluster_pair_kernel! of src/clusterpairs/Kernels.jl with the pair physics of pair_force
+// (src/clusterpairs/PairFunctor.jl:127-156).  One CTA of 1, 2 or 4 warps per super-cluster part; lane
+// (ti, q) = (lane & 7, lane >> 3) pairs i-atom ti of the entry's i-clusters with j-atoms q and q + 4 of its
+// j-cluster.  The two pairs are the two halves of packed FP32 registers: the kernel is bound by instruction
+// issue, and a packed multiply-add issues once for both.  A tile whose entry names only one j half computes both
+// and masks the other, which costs what one half cost in scalar code.
+//
+// k_pairs_force keeps the i-forces of the eight i-clusters in registers; j-forces are reduced over the 8 ti
+// lanes by shuffles.  k_pairs_energy has ten sums per i-atom (force, energy, virial): it loops over the
+// i-clusters and keeps their sums in shared memory, private to each thread, because the body unrolled eight times
+// ran out of instruction cache and registers (24 002 ions: 135 us, 6.9 of 10 stalled warps without an
+// instruction, 158 registers).
+#pragma once
+#include "cluster_pairs.cuh"
+#include "packed2.cuh"
+
+namespace pdb {
+
+
+
+template <int NP>
+__device__ __forceinline__ f2 horner2(const f2 (&c)[NP], f2 x) {
+    f2 acc = c[NP - 1];
+#pragma unroll
+    for (int k = NP - 2; k >= 0; --k) acc = fma2(acc, x, c[k]);
+    return acc;
+}
+
+// Constants of the pair physics as held register pairs.
+struct TileConst {
+    f2 c6m, c12m, c6n, c12, esh, sx, one_n, eshift;   // -6 c6, 12 c12, -c6, c12, -e_shift; 2 / r_c^2, -1, -shift
+};
+template <int LJK, bool COUL, bool ENERGY>
+__device__ __forceinline__ TileConst tile_const(const PairParams &pp) {
+    TileConst c;
+    if (LJK == PD_LJ_UNIFORM) {
+        c.c6m = pk_held(-6.f * pp.c6);
+        c.c12m = pk_held(12.f * pp.c12);
+        if (ENERGY) {
+            c.c6n = pk_held(-pp.c6);
+            c.c12 = pk_held(pp.c12);
+            c.esh = pk_held(-pp.esh);
+        }
+    }
+    if (COUL) {
+        c.sx = pk_held(pp.sx);
+        c.one_n = pk_held(-1.f);
+        if (ENERGY) c.eshift = pk_held(-pp.eshift);
+    }
+    return c;
+}
+
+// Differences i - j of both halves (the compensated periodic difference on marked tiles).
+__device__ __forceinline__ void tile_delta(const float4 &pi, const float4 &ja, const float4 &jb, f2 njx, f2 njy, f2 njz,
+                                           bool pbc, const PairParams &pp, f2 &dx, f2 &dy, f2 &dz) {
+    if (pbc) {
+        const float hx = 0.5f * pp.Lx, hy = 0.5f * pp.Ly, hz = 0.5f * pp.Lz;
+        dx = pk(periodic_delta(pi.x, ja.x, hx, pp.Lx), periodic_delta(pi.x, jb.x, hx, pp.Lx));
+        dy = pk(periodic_delta(pi.y, ja.y, hy, pp.Ly), periodic_delta(pi.y, jb.y, hy, pp.Ly));
+        dz = pk(periodic_delta(pi.z, ja.z, hz, pp.Lz), periodic_delta(pi.z, jb.z, hz, pp.Lz));
+    } else {
+        dx = add2(pk(pi.x), njx);
+        dy = add2(pk(pi.y), njy);
+        dz = add2(pk(pi.z), njz);
+    }
+}
+
+// f / r (and with ENERGY the pair energy) of both halves; keep*: the half counts (its bit is set and the pair is
+// not the self tile's masked triangle).  Padding atoms sit far away with zero charge: exact zeros.
+template <int LJK, bool COUL, bool ENERGY, int NP>
+__device__ __forceinline__ void tile_pair(f2 dx, f2 dy, f2 dz, float qi, f2 qj, const float4 &ta, const float4 &tb,
+                                          bool keepa, bool keepb, const f2 (&cpf)[NP], const f2 (&cpe)[NP],
+                                          const TileConst &tc, const PairParams &pp, f2 &f, f2 &en) {
+    const f2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+    float ra, rb;
+    unpk(r2, ra, rb);
+    const f2 rinv = pk(rsqrt_fast(ra), rsqrt_fast(rb));
+    const f2 rinv2 = mul2(rinv, rinv);
+    float fa = 0.f, fb = 0.f, ea = 0.f, eb = 0.f;
+    if (LJK != PD_LJ_NONE) {
+        constexpr bool tab = LJK == PD_LJ_TABLE;
+        const float la = tab ? ta.z : pp.lrc2, lb = tab ? tb.z : pp.lrc2;
+        const f2 c6m = tab ? pk(-6.f * ta.x, -6.f * tb.x) : tc.c6m, c12m = tab ? pk(12.f * ta.y, 12.f * tb.y) : tc.c12m;
+        const f2 ir6 = mul2(mul2(rinv2, rinv2), rinv2);
+        float xa, xb;
+        unpk(mul2(mul2(fma2(c12m, ir6, c6m), ir6), rinv2), xa, xb);
+        const bool ina = ra < la && keepa, inb = rb < lb && keepb;
+        fa = ina ? xa : 0.f;
+        fb = inb ? xb : 0.f;
+        if (ENERGY) {
+            const f2 c6n = tab ? pk(-ta.x, -tb.x) : tc.c6n, c12 = tab ? pk(ta.y, tb.y) : tc.c12;
+            const f2 esh = tab ? pk(-ta.w, -tb.w) : tc.esh;
+            unpk(add2(mul2(fma2(c12, ir6, c6n), ir6), esh), xa, xb);
+            ea = ina ? xa : 0.f;
+            eb = inb ? xb : 0.f;
+        }
+    }
+    f = pk(fa, fb);
+    en = pk(ea, eb);
+    if (COUL) {
+        const bool ina = ra < pp.rc2 && keepa, inb = rb < pp.rc2 && keepb;
+        const f2 x = fma2(r2, tc.sx, tc.one_n);
+        const f2 cq = mul2(pk(qi), qj);
+        const f2 fq = add2(mul2(rinv, rinv2), horner2(cpf, x));   // the coefficients come negated
+        float xa, xb;
+        unpk(fq, xa, xb);
+        f = fma2(cq, pk(ina ? xa : 0.f, inb ? xb : 0.f), f);
+        if (ENERGY) {
+            const f2 eq = add2(add2(rinv, horner2(cpe, x)), tc.eshift);
+            unpk(eq, xa, xb);
+            en = fma2(cq, pk(ina ? xa : 0.f, inb ? xb : 0.f), en);
+        }
+    }
+}
+
+// The entry loop's registers: the current entry's word and j-atoms, the next one's in flight.
+struct TileEntry {
+    uint2 ent;
+    float4 pa, pb;
+    int ta, tb;
+};
+
+template <int LJK>
+__device__ __forceinline__ void load_entry(TileEntry &t, const uint2 *__restrict__ cjw, const float4 *__restrict__ xq,
+                                           const int *__restrict__ ts, int e, int q) {
+    t.ent = cjw[e];
+    t.pa = xq[(int)t.ent.x * 8 + q];
+    t.pb = xq[(int)t.ent.x * 8 + q + 4];
+    if (LJK == PD_LJ_TABLE) {
+        t.ta = ts[(int)t.ent.x * 8 + q];
+        t.tb = ts[(int)t.ent.x * 8 + q + 4];
+    }
+}
+
+template <int LJK, bool COUL, int NP>
+__global__ void __launch_bounds__(128) k_pairs_force(const float4 *__restrict__ xq, const int *__restrict__ ts,
+                                                     const uint2 *__restrict__ cjw, const int *__restrict__ scio,
+                                                     const int *__restrict__ nw, const int *__restrict__ counts,
+                                                     const float *__restrict__ lj_table, float4 *__restrict__ fc,
+                                                     int nsplit, const __grid_constant__ PairParams pp) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nwarp = blockDim.x >> 5;
+    const int ti = lane & 7, q = lane >> 3;
+    const int S = blockIdx.x / nsplit, part = blockIdx.x % nsplit;
+    if (S >= counts[W_NS] || counts[W_ERR] != 0) return;
+    __shared__ float4 sxq[SUPER];
+    __shared__ int sty[SUPER];
+    __shared__ float4 stab[LJK == PD_LJ_TABLE ? PD_MAX_TYPES * PD_MAX_TYPES : 1];
+    for (int k = tid; k < SUPER; k += blockDim.x) {
+        float4 v = xq[S * SUPER + k];
+        if (COUL) v.w *= pp.C;
+        sxq[k] = v;
+        if (LJK == PD_LJ_TABLE) sty[k] = (ts[S * SUPER + k] - 1) * pp.ntypes;
+    }
+    if (LJK == PD_LJ_TABLE)
+        for (int k = tid; k < pp.ntypes * pp.ntypes; k += blockDim.x)
+            stab[k] = reinterpret_cast<const float4 *>(lj_table)[k];
+    __syncthreads();
+    f2 cpf[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) cpf[k] = pk_held(COUL ? -pp.pf[k] : 0.f);
+    const TileConst tc = tile_const<LJK, COUL, false>(pp);
+    float fxi[8], fyi[8], fzi[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) fxi[a] = fyi[a] = fzi[a] = 0.f;
+    const int e0 = scio[S], ne = nw[S];
+    const int ea = e0 + (int)(((long long)ne * part) / nsplit);
+    const int eb = e0 + (int)(((long long)ne * (part + 1)) / nsplit);
+    const bool gta = q > ti, gtb = q + 4 > ti;
+    int e = ea + w;
+    TileEntry nx;
+    nx.ta = nx.tb = 1;
+    if (e < eb) load_entry<LJK>(nx, cjw, xq, ts, e, q);
+    for (; e < eb; e += nwarp) {
+        const TileEntry cur = nx;
+        if (e + nwarp < eb) load_entry<LJK>(nx, cjw, xq, ts, e + nwarp, q);
+        // the entry is the same for every lane; the warp reduction makes that visible to the
+        // compiler, so the branches on its bits below are uniform
+        const uint32_t word = __reduce_or_sync(0xffffffffu, cur.ent.y);
+        const bool pbc = (word >> 16) & 1u;   // tile may cross a box face before the next prune
+        const int cj = (int)__reduce_or_sync(0xffffffffu, cur.ent.x);
+        const int da = cj - S * 8;   // index of the i-cluster that is the j-cluster itself, if in [0, 8)
+        const f2 njx = pk(-cur.pa.x, -cur.pb.x), njy = pk(-cur.pa.y, -cur.pb.y), njz = pk(-cur.pa.z, -cur.pb.z);
+        const f2 qj = pk(cur.pa.w, cur.pb.w);
+        f2 Jx = pk(0.f), Jy = pk(0.f), Jz = pk(0.f);   // minus the j-atoms' forces
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            if (((word | (word >> 8)) >> a) & 1u) {
+                const float4 pi = sxq[a * 8 + ti];
+                const bool self = da == a;
+                const bool ka = ((word >> a) & 1u) && (!self || gta), kb = ((word >> (a + 8)) & 1u) && (!self || gtb);
+                float4 ta4 = make_float4(0.f, 0.f, 0.f, 0.f), tb4 = ta4;
+                if (LJK == PD_LJ_TABLE) {
+                    const int tyi = sty[a * 8 + ti];
+                    ta4 = stab[tyi + (cur.ta - 1)];
+                    tb4 = stab[tyi + (cur.tb - 1)];
+                }
+                f2 dx, dy, dz, f, en;
+                tile_delta(pi, cur.pa, cur.pb, njx, njy, njz, pbc, pp, dx, dy, dz);
+                tile_pair<LJK, COUL, false, NP>(dx, dy, dz, pi.w, qj, ta4, tb4, ka, kb, cpf, cpf, tc, pp, f, en);
+                Jx = fma2(f, dx, Jx);
+                Jy = fma2(f, dy, Jy);
+                Jz = fma2(f, dz, Jz);
+                float fa, fb, da_, db_;
+                unpk(f, fa, fb);
+                unpk(dx, da_, db_);
+                fxi[a] = fmaf(fb, db_, fmaf(fa, da_, fxi[a]));
+                unpk(dy, da_, db_);
+                fyi[a] = fmaf(fb, db_, fmaf(fa, da_, fyi[a]));
+                unpk(dz, da_, db_);
+                fzi[a] = fmaf(fb, db_, fmaf(fa, da_, fzi[a]));
+            }
+        }
+        float xa, xb, ya, yb, za, zb;
+        unpk(Jx, xa, xb);
+        unpk(Jy, ya, yb);
+        unpk(Jz, za, zb);
+        const float rA = reduce3(-xa, -ya, -za, ti), rB = reduce3(-xb, -yb, -zb, ti);
+        if (ti < 3) {
+            red_add(reinterpret_cast<float *>(&fc[cj * 8 + q]) + ti, rA);
+            red_add(reinterpret_cast<float *>(&fc[cj * 8 + q + 4]) + ti, rB);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        fxi[a] = reduce_i(fxi[a]);
+        fyi[a] = reduce_i(fyi[a]);
+        fzi[a] = reduce_i(fzi[a]);
+    }
+    if (lane < 8) {
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+            red_add_v4(reinterpret_cast<float *>(&fc[S * SUPER + a * 8 + lane]), fxi[a], fyi[a], fzi[a], 0.f);
+    }
+}
+
+template <int LJK, bool COUL, int NP>
+__global__ void __launch_bounds__(64) k_pairs_energy(const float4 *__restrict__ xq, const int *__restrict__ ts,
+                                                     const uint2 *__restrict__ cjw, const int *__restrict__ scio,
+                                                     const int *__restrict__ nw, const int *__restrict__ counts,
+                                                     const float *__restrict__ lj_table, float4 *__restrict__ fc,
+                                                     float *__restrict__ vc, int nslot, int nsplit,
+                                                     const __grid_constant__ PairParams pp) {
+    constexpr int NT = 64;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int ti = lane & 7, q = lane >> 3;
+    const int S = blockIdx.x / nsplit, part = blockIdx.x % nsplit;
+    if (S >= counts[W_NS] || counts[W_ERR] != 0) return;
+    __shared__ float4 sxq[SUPER];
+    __shared__ int sty[SUPER];
+    __shared__ float4 stab[LJK == PD_LJ_TABLE ? PD_MAX_TYPES * PD_MAX_TYPES : 1];
+    // per thread and i-cluster: force and energy, then the virial (xx, yy, zz, xy), then (xz, yz)
+    __shared__ float4 sf[8][NT], sv[8][NT];
+    __shared__ float2 sw[8][NT];
+    for (int k = tid; k < SUPER; k += NT) {
+        float4 v = xq[S * SUPER + k];
+        if (COUL) v.w *= pp.C;
+        sxq[k] = v;
+        if (LJK == PD_LJ_TABLE) sty[k] = (ts[S * SUPER + k] - 1) * pp.ntypes;
+    }
+    if (LJK == PD_LJ_TABLE)
+        for (int k = tid; k < pp.ntypes * pp.ntypes; k += NT) stab[k] = reinterpret_cast<const float4 *>(lj_table)[k];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        sf[a][tid] = sv[a][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        sw[a][tid] = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    f2 cpf[NP], cpe[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        cpf[k] = pk(COUL ? -pp.pf[k] : 0.f);
+        cpe[k] = pk(COUL ? pp.pe[k] : 0.f);
+    }
+    const TileConst tc = tile_const<LJK, COUL, true>(pp);
+    const int e0 = scio[S], ne = nw[S];
+    const int ea = e0 + (int)(((long long)ne * part) / nsplit);
+    const int eb = e0 + (int)(((long long)ne * (part + 1)) / nsplit);
+    const bool gta = q > ti, gtb = q + 4 > ti;
+    int e = ea + w;
+    TileEntry nx;
+    nx.ta = nx.tb = 1;
+    if (e < eb) load_entry<LJK>(nx, cjw, xq, ts, e, q);
+    for (; e < eb; e += NT / 32) {
+        const TileEntry cur = nx;
+        if (e + NT / 32 < eb) load_entry<LJK>(nx, cjw, xq, ts, e + NT / 32, q);
+        const uint32_t word = __reduce_or_sync(0xffffffffu, cur.ent.y);
+        const bool pbc = (word >> 16) & 1u;
+        const int cj = (int)__reduce_or_sync(0xffffffffu, cur.ent.x);
+        const int da = cj - S * 8;
+        const f2 njx = pk(-cur.pa.x, -cur.pb.x), njy = pk(-cur.pa.y, -cur.pb.y), njz = pk(-cur.pa.z, -cur.pb.z);
+        const f2 qj = pk(cur.pa.w, cur.pb.w);
+        f2 J[10];   // minus the j-atoms' force, then energy and virial
+#pragma unroll
+        for (int k = 0; k < 10; ++k) J[k] = pk(0.f);
+        uint32_t left = (word | (word >> 8)) & 0xffu;
+#pragma unroll 1
+        while (left) {
+            const int a = __ffs(left) - 1;
+            left &= left - 1;
+            const float4 pi = sxq[a * 8 + ti];
+            const bool self = da == a;
+            const bool ka = ((word >> a) & 1u) && (!self || gta), kb = ((word >> (a + 8)) & 1u) && (!self || gtb);
+            float4 ta4 = make_float4(0.f, 0.f, 0.f, 0.f), tb4 = ta4;
+            if (LJK == PD_LJ_TABLE) {
+                const int tyi = sty[a * 8 + ti];
+                ta4 = stab[tyi + (cur.ta - 1)];
+                tb4 = stab[tyi + (cur.tb - 1)];
+            }
+            f2 dx, dy, dz, f, en;
+            tile_delta(pi, cur.pa, cur.pb, njx, njy, njz, pbc, pp, dx, dy, dz);
+            tile_pair<LJK, COUL, true, NP>(dx, dy, dz, pi.w, qj, ta4, tb4, ka, kb, cpf, cpe, tc, pp, f, en);
+            const f2 fx = mul2(f, dx), fy = mul2(f, dy), fz = mul2(f, dz);
+            en = mul2(pk(0.5f), en);
+            J[0] = add2(J[0], fx);
+            J[1] = add2(J[1], fy);
+            J[2] = add2(J[2], fz);
+            J[3] = add2(J[3], en);
+            const f2 hx = mul2(pk(0.5f), fx), hy = mul2(pk(0.5f), fy), hz = mul2(pk(0.5f), fz);
+            const f2 v[6] = {mul2(hx, dx), mul2(hy, dy), mul2(hz, dz), mul2(hx, dy), mul2(hx, dz), mul2(hy, dz)};
+#pragma unroll
+            for (int k = 0; k < 6; ++k) J[4 + k] = add2(J[4 + k], v[k]);
+            float xa, xb;
+            float4 s = sf[a][tid];
+            unpk(fx, xa, xb);
+            s.x += xa + xb;
+            unpk(fy, xa, xb);
+            s.y += xa + xb;
+            unpk(fz, xa, xb);
+            s.z += xa + xb;
+            unpk(en, xa, xb);
+            s.w += xa + xb;
+            sf[a][tid] = s;
+            s = sv[a][tid];
+            unpk(v[0], xa, xb);
+            s.x += xa + xb;
+            unpk(v[1], xa, xb);
+            s.y += xa + xb;
+            unpk(v[2], xa, xb);
+            s.z += xa + xb;
+            unpk(v[3], xa, xb);
+            s.w += xa + xb;
+            sv[a][tid] = s;
+            float2 s2 = sw[a][tid];
+            unpk(v[4], xa, xb);
+            s2.x += xa + xb;
+            unpk(v[5], xa, xb);
+            s2.y += xa + xb;
+            sw[a][tid] = s2;
+        }
+        float A[10], B[10];
+#pragma unroll
+        for (int k = 0; k < 10; ++k) unpk(J[k], A[k], B[k]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float *Z = h ? B : A;
+            const int js = cj * 8 + q + 4 * h;
+            const float r = reduce3(-Z[0], -Z[1], -Z[2], ti);
+            const float rv1 = reduce3(Z[4], Z[5], Z[6], ti), rv2 = reduce3(Z[7], Z[8], Z[9], ti);
+            const float ej = sum8(Z[3]);
+            if (ti < 3) {
+                red_add(reinterpret_cast<float *>(&fc[js]) + ti, r);
+                red_add(&vc[(size_t)ti * nslot + js], rv1);
+                red_add(&vc[(size_t)(ti + 3) * nslot + js], rv2);
+            }
+            if (ti == 0) red_add(reinterpret_cast<float *>(&fc[js]) + 3, ej);
+        }
+    }
+    // i-sums: each of the CTA's threads adds up one i-atom's columns (two warps x four q)
+    __syncthreads();
+    {
+        const int a = tid >> 3, t = tid & 7, ai = S * SUPER + tid;   // 64 threads, 64 i-atoms
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f), v = f;
+        float2 x = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < NT / 8; ++c) {
+            const float4 f1 = sf[a][c * 8 + t], v1 = sv[a][c * 8 + t];
+            const float2 x1 = sw[a][c * 8 + t];
+            f = make_float4(f.x + f1.x, f.y + f1.y, f.z + f1.z, f.w + f1.w);
+            v = make_float4(v.x + v1.x, v.y + v1.y, v.z + v1.z, v.w + v1.w);
+            x = make_float2(x.x + x1.x, x.y + x1.y);
+        }
+        red_add_v4(reinterpret_cast<float *>(&fc[ai]), f.x, f.y, f.z, f.w);
+        red_add(&vc[(size_t)0 * nslot + ai], v.x);
+        red_add(&vc[(size_t)1 * nslot + ai], v.y);
+        red_add(&vc[(size_t)2 * nslot + ai], v.z);
+        red_add(&vc[(size_t)3 * nslot + ai], v.w);
+        red_add(&vc[(size_t)4 * nslot + ai], x.x);
+        red_add(&vc[(size_t)5 * nslot + ai], x.y);
+    }
+}
+
+template <int LJK, bool COUL, int NP>
+static void launch_tiles(pd_cluster *c, int energy, cudaStream_t s) {
+    if (energy)
+        k_pairs_energy<LJK, COUL, NP><<<c->nsmax * c->nsplit, 64, 0, s>>>(c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts,
+                                                                       c->lj_table, c->fc, c->vc, c->nslot, c->nsplit,
+                                                                       c->pp);
+    else
+        k_pairs_force<LJK, COUL, NP><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
+            c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts, c->lj_table, c->fc, c->nsplit, c->pp);
+}
+
+// Coefficient buckets: the fitted degrees are even, so their counts are odd (13 at the usual Gaussian splits).
+template <int LJK>
+static void launch_tiles_poly(pd_cluster *c, int energy, cudaStream_t s) {
+    const PairParams &pp = c->pp;
+    const int n = !pp.coulomb ? 0 : energy ? (pp.nf > pp.ne ? pp.nf : pp.ne) : pp.nf;
+    if (n == 0) launch_tiles<LJK, false, 1>(c, energy, s);
+    else if (n <= 9) launch_tiles<LJK, true, 9>(c, energy, s);
+    else if (n <= 11) launch_tiles<LJK, true, 11>(c, energy, s);
+    else if (n <= 13) launch_tiles<LJK, true, 13>(c, energy, s);
+    else if (n <= 15) launch_tiles<LJK, true, 15>(c, energy, s);
+    else if (n <= 17) launch_tiles<LJK, true, 17>(c, energy, s);
+    else if (n <= 20) launch_tiles<LJK, true, 20>(c, energy, s);
+    else launch_tiles<LJK, true, 32>(c, energy, s);
+}
+
+static void tiles_dispatch(pd_cluster *c, int energy, cudaStream_t s) {
+    switch (c->pp.lj_kind) {
+        case PD_LJ_NONE: launch_tiles_poly<PD_LJ_NONE>(c, energy, s); break;
+        case PD_LJ_UNIFORM: launch_tiles_poly<PD_LJ_UNIFORM>(c, energy, s); break;
+        default: launch_tiles_poly<PD_LJ_TABLE>(c, energy, s); break;
+    }
+}
+
+}  // namespace pdb
