@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const fl
     const int K1 = R.K1, K2 = R.K2, K3 = R.K3;
     __shared__ __align__(16) float tile[BTILE];
     __shared__ unsigned rowbase[ROWS_MAX];
-    __shared__ int sm[10];
+    __shared__ int sm[BRICK_WORDS];
     const int t = threadIdx.x, p = t & (CH - 1), h = t / CH;
     const int e = c * CH + p;
     const float4 v = mq[e];
@@ -138,17 +138,11 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const fl
     }
     int d1 = 0, d2 = 0, d3 = 0;
     Brick b;
-    chunk_brick<P, NT, BTILE>(charged, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
+    chunk_brick<P, CH, NT, BTILE>(charged, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
     float phi = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
     if (b.fits) {
-        if (b.vec) {
-            float4 *tile4 = reinterpret_cast<float4 *>(tile);
-            for_brick<NT>(b, rowbase, K1, [&](int kt, size_t kg) {
-                tile4[kt] = __ldg(reinterpret_cast<const float4 *>(grid + kg));
-            });
-        } else {
-            for_brick<NT>(b, rowbase, K1, [&](int kt, size_t kg) { tile[kt] = __ldg(grid + kg); });
-        }
+        load_brick<NT>(b, rowbase, K1, grid, tile);
+        brick_wait();
         __syncthreads();
         if (charged) {
 #pragma unroll

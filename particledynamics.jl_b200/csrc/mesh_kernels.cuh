@@ -135,10 +135,13 @@ __device__ __forceinline__ int wrap_node(int n, int K) {
     return n < 0 ? n + K : n;
 }
 
-// Signed offset of node k from the reference node r on a periodic axis of K nodes, in [-K/2, K/2).
+// Signed offset of node k from the reference node r on a periodic axis of K nodes, in [-K/2, K/2); stencil
+// bases lie in [-K, K), so their difference is within two periods.
 __device__ __forceinline__ int signed_offset(int k, int r, int K) {
-    int d = (k - r) % K;
-    if (d < 0) d += K;
+    int d = k - r;
+    d += d < 0 ? K : 0;
+    d += d < 0 ? K : 0;
+    d -= d >= K ? K : 0;
     if (d >= (K + 1) / 2) d -= K;
     return d;
 }
@@ -161,63 +164,96 @@ struct Brick {
 
 constexpr int ROWS_MAX = 512;   // brick rows tabulated in shared memory
 
-// NT: threads of the CTA that moves the brick (two per particle of the chunk); TILE: floats of the
-// shared brick.
-template <int P, int NT = MESH_THREADS, int TILE = TILE_MAX>
+// floor(n / K) for |n| < 2^18, 1 <= K <= 2^10 with inv = 1 / K: (n + 1/2) / K lies at least 1 / 2K from an integer,
+// above the product's rounding error.  (Larger axes take the integer division.)
+__device__ __forceinline__ int floor_div(int n, int K, float inv) {
+    if (K > 1024) return (n - (n < 0 ? K - 1 : 0)) / K;
+    return (int)floorf(((float)n + 0.5f) * inv);
+}
+
+constexpr int BRICK_WORDS = 40;   // shared words of chunk_brick: 4 per reporting warp, 6 per reporting warp
+
+// CH: particles of the chunk (threads t and t + CH, ... share particle t); NT: threads of the CTA; TILE: floats
+// of the shared brick.  The chunk's bounding box comes from warp reductions (the warps of the first CH threads
+// report, every thread combines): bound by latency, as one CTA's chunk is all that many SMs have.
+template <int P, int CH, int NT, int TILE = TILE_MAX>
 __device__ __forceinline__ void chunk_brick(bool valid, int k1, int k2, int k3, int K1, int K2, int K3, int &d1,
-                                            int &d2, int &d3, Brick &b, int *sm /* >= 10 ints */,
+                                            int &d2, int &d3, Brick &b, int *sm /* BRICK_WORDS ints */,
                                             unsigned *rowbase) {
-    // sm[0] first valid, sm[1..3] ref, sm[4..6] min, sm[7..9] max
-    const int t = threadIdx.x;
-    if (t == 0) {
-        sm[0] = 1 << 30;
-        sm[4] = sm[5] = sm[6] = 1 << 30;
-        sm[7] = sm[8] = sm[9] = -(1 << 30);
+    constexpr int NW = CH / 32;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    // reference: the stencil base of the first valid particle
+    const unsigned bal = __ballot_sync(0xffffffffu, valid);
+    const int src = bal ? __ffs(bal) - 1 : 0;
+    const int r1 = __shfl_sync(0xffffffffu, k1, src), r2 = __shfl_sync(0xffffffffu, k2, src),
+              r3 = __shfl_sync(0xffffffffu, k3, src);
+    if (w < NW && lane == 0) {
+        sm[4 * w] = bal != 0;
+        sm[4 * w + 1] = r1;
+        sm[4 * w + 2] = r2;
+        sm[4 * w + 3] = r3;
     }
     __syncthreads();
-    if (valid) atomicMin(&sm[0], t);
-    __syncthreads();
-    if (valid && sm[0] == t) {
-        sm[1] = k1;
-        sm[2] = k2;
-        sm[3] = k3;
+    int any = 0, ref[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = NW - 1; k >= 0; --k) {
+        if (sm[4 * k]) {
+            any = 1;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) ref[d] = sm[4 * k + 1 + d];
+        }
     }
-    __syncthreads();
-    const bool any = sm[0] < (1 << 30);
+    int lo[3] = {1 << 30, 1 << 30, 1 << 30}, hi[3] = {-(1 << 30), -(1 << 30), -(1 << 30)};
     if (valid) {
-        d1 = signed_offset(k1, sm[1], K1);
-        d2 = signed_offset(k2, sm[2], K2);
-        d3 = signed_offset(k3, sm[3], K3);
-        atomicMin(&sm[4], d1);
-        atomicMin(&sm[5], d2);
-        atomicMin(&sm[6], d3);
-        atomicMax(&sm[7], d1);
-        atomicMax(&sm[8], d2);
-        atomicMax(&sm[9], d3);
+        d1 = signed_offset(k1, ref[0], K1);
+        d2 = signed_offset(k2, ref[1], K2);
+        d3 = signed_offset(k3, ref[2], K3);
+        lo[0] = hi[0] = d1;
+        lo[1] = hi[1] = d2;
+        lo[2] = hi[2] = d3;
+    }
+    int *mm = sm + 4 * NW;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int l = __reduce_min_sync(0xffffffffu, lo[d]), h = __reduce_max_sync(0xffffffffu, hi[d]);
+        if (w < NW && lane == 0) {
+            mm[6 * w + d] = l;
+            mm[6 * w + 3 + d] = h;
+        }
     }
     __syncthreads();
     b.vec = (K1 & 3) == 0;
     if (any) {
-        int o1 = sm[1] + sm[4], e1 = sm[7] - sm[4] + P;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = mm[d];
+            hi[d] = mm[3 + d];
+#pragma unroll
+            for (int k = 1; k < NW; ++k) {
+                lo[d] = min(lo[d], mm[6 * k + d]);
+                hi[d] = max(hi[d], mm[6 * k + 3 + d]);
+            }
+        }
+        int o1 = ref[0] + lo[0], e1 = hi[0] - lo[0] + P;
         int shift = 0;
         if (b.vec) {
-            shift = ((o1 % 4) + 4) % 4;
+            shift = o1 & 3;
             o1 -= shift;
             e1 = (e1 + shift + 3) & ~3;
         }
         b.o1 = o1;
-        b.o2 = sm[2] + sm[5];
-        b.o3 = sm[3] + sm[6];
+        b.o2 = ref[1] + lo[1];
+        b.o3 = ref[2] + lo[2];
         b.e1 = e1;
-        b.e2 = sm[8] - sm[5] + P;
-        b.e3 = sm[9] - sm[6] + P;
+        b.e2 = hi[1] - lo[1] + P;
+        b.e3 = hi[2] - lo[2] + P;
         const long long nodes = (long long)b.e1 * b.e2 * b.e3;
         b.fits = nodes <= TILE && b.e1 <= NT && (!b.vec || b.e1 <= K1) &&
                  (long long)b.e2 * b.e3 <= ROWS_MAX;
         if (valid) {
-            d1 += shift - sm[4];
-            d2 -= sm[5];
-            d3 -= sm[6];
+            d1 += shift - lo[0];
+            d2 -= lo[1];
+            d3 -= lo[2];
         }
     } else {
         b.o1 = b.o2 = b.o3 = 0;
@@ -226,16 +262,20 @@ __device__ __forceinline__ void chunk_brick(bool valid, int k1, int k2, int k3, 
     }
     if (b.fits) {
         const int nrows = b.e2 * b.e3;
-        for (int r = threadIdx.x; r < nrows; r += blockDim.x) {
-            const int l2 = r % b.e2, l3 = r / b.e2;
-            rowbase[r] = (unsigned)(((size_t)wrap_node(b.o3 + l3, K3) * K2 + wrap_node(b.o2 + l2, K2)) * K1);
+        const float ie2 = 1.f / (float)max(b.e2, 1), iK2 = 1.f / (float)K2, iK3 = 1.f / (float)K3;
+        for (int r = threadIdx.x; r < nrows; r += NT) {
+            const int l3 = floor_div(r, b.e2, ie2), l2 = r - l3 * b.e2;
+            int n2 = b.o2 + l2, n3 = b.o3 + l3;
+            n2 -= floor_div(n2, K2, iK2) * K2;
+            n3 -= floor_div(n3, K3, iK3) * K3;
+            rowbase[r] = (unsigned)(((size_t)n3 * K2 + n2) * K1);
         }
     }
     __syncthreads();
 }
 
 // Move a brick between shared memory and the global grid: lanes are laid out as
-// (row, x vector) with MESH_THREADS / nv rows in flight, nv = vectors (or nodes)
+// (row, x vector) with NT / nv rows in flight, nv = vectors (or nodes)
 // per row; visit(tile_element, global_node) gets the first node of each
 // 4-node vector (vec) or single node.
 template <int NT = MESH_THREADS, typename F>
@@ -243,14 +283,33 @@ __device__ __forceinline__ void for_brick(const Brick &b, const unsigned *rowbas
     const int per = b.vec ? 4 : 1;
     const int nv = b.e1 / per;
     if (nv == 0) return;
-    const int rpi = NT / nv;
+    const float inv = 1.f / (float)nv;
+    const int rpi = floor_div(NT, nv, inv);   // nv <= NT
     const int t = threadIdx.x;
-    const int r0 = t / nv, v = t - r0 * nv;
+    const int r0 = floor_div(t, nv, inv), v = t - r0 * nv;
     if (r0 >= rpi) return;
-    const int x0 = wrap_node(b.o1 + per * v, K1);
+    int x0 = b.o1 + per * v;
+    x0 -= floor_div(x0, K1, 1.f / (float)K1) * K1;
     const int nrows = b.e2 * b.e3;
     for (int r = r0; r < nrows; r += rpi) visit(r * nv + v, (size_t)rowbase[r] + x0);
 }
+
+// Stage a brick of the grid in shared memory with asynchronous copies: every row's copy is in flight at once (plain
+// loads went one row of a thread after another, a memory latency each).  The caller waits with brick_wait().
+template <int NT = MESH_THREADS>
+__device__ __forceinline__ void load_brick(const Brick &b, const unsigned *rowbase, int K1,
+                                           const float *__restrict__ grid, float *tile) {
+    const unsigned base = (unsigned)__cvta_generic_to_shared(tile);
+    if (b.vec)
+        for_brick<NT>(b, rowbase, K1, [&](int kt, size_t kg) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + 16u * kt), "l"(grid + kg) : "memory");
+        });
+    else
+        for_brick<NT>(b, rowbase, K1, [&](int kt, size_t kg) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(base + 4u * kt), "l"(grid + kg) : "memory");
+        });
+}
+__device__ __forceinline__ void brick_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // z planes of a particle's stencil taken by its thread h of TP: the two halves of the stencil (TP = 2),
 // or every TP-th plane (TP = 4).
@@ -268,7 +327,7 @@ __device__ __forceinline__ void spread_chunk(const float4 *__restrict__ chunk, f
     constexpr int NT = TP * CH;
     __shared__ __align__(16) float tile[TILE];
     __shared__ unsigned rowbase[ROWS_MAX];
-    __shared__ int sm[10];
+    __shared__ int sm[BRICK_WORDS];
     const int t = threadIdx.x, p = t & (CH - 1), h = t / CH;
     const float4 v = chunk[p];
     const bool valid = v.w != 0.f && isfinite(v.x) && isfinite(v.y) && isfinite(v.z);
@@ -281,8 +340,7 @@ __device__ __forceinline__ void spread_chunk(const float4 *__restrict__ chunk, f
     }
     int d1 = 0, d2 = 0, d3 = 0;
     Brick b;
-    // both halves of a particle take part (their min/max contributions are identical)
-    chunk_brick<P, NT, TILE>(valid, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
+    chunk_brick<P, CH, NT, TILE>(valid, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
 
     if (b.fits) {
         // The brick accumulates in 32-bit fixed point: integer shared-memory reductions are native
@@ -436,7 +494,7 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_gather(const
     if (c >= nchunks) return;
     __shared__ __align__(16) float tile[TILE_MAX];
     __shared__ unsigned rowbase[ROWS_MAX];
-    __shared__ int sm[10];
+    __shared__ int sm[BRICK_WORDS];
     __shared__ float part[MESH_CHUNK][4];
     const int t = threadIdx.x, p = t & (MESH_CHUNK - 1), h = t >> 6;
     const int e = c * MESH_CHUNK + p;
@@ -469,7 +527,7 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_gather(const
     }
     int d1 = 0, d2 = 0, d3 = 0;
     Brick b;
-    chunk_brick<P>(charged, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
+    chunk_brick<P, MESH_CHUNK, MESH_THREADS>(charged, k1, k2, k3, K1, K2, K3, d1, d2, d3, b, sm, rowbase);
     constexpr int PH = (P + 1) / 2;
     constexpr int NG = IK ? (ENERGY ? 4 : 3) : 1;   // grids read one after another
 
@@ -479,14 +537,8 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_gather(const
         for (int gi = 0; gi < NG; ++gi) {
             const float *grid = grids.g[gi];
             if (gi > 0) __syncthreads();   // every thread is done with the previous grid's brick
-            if (b.vec) {
-                float4 *tile4 = reinterpret_cast<float4 *>(tile);
-                for_brick(b, rowbase, K1, [&](int kt, size_t kg) {
-                    tile4[kt] = __ldg(reinterpret_cast<const float4 *>(grid + kg));
-                });
-            } else {
-                for_brick(b, rowbase, K1, [&](int kt, size_t kg) { tile[kt] = __ldg(grid + kg); });
-            }
+            load_brick(b, rowbase, K1, grid, tile);
+            brick_wait();
             __syncthreads();
             if (charged) {
                 float acc = 0.f;
@@ -538,14 +590,8 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_gather(const
         }
     } else if (b.fits) {
         const float *grid = grids.g[0];
-        if (b.vec) {
-            float4 *tile4 = reinterpret_cast<float4 *>(tile);
-            for_brick(b, rowbase, K1, [&](int kt, size_t kg) {
-                tile4[kt] = __ldg(reinterpret_cast<const float4 *>(grid + kg));
-            });
-        } else {
-            for_brick(b, rowbase, K1, [&](int kt, size_t kg) { tile[kt] = __ldg(grid + kg); });
-        }
+        load_brick(b, rowbase, K1, grid, tile);
+        brick_wait();
         __syncthreads();
         if (charged) {
 #pragma unroll
