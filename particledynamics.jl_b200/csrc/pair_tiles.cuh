@@ -53,27 +53,6 @@ __device__ __forceinline__ TileConst tile_const(const PairParams &pp) {
 }
 
 // Differences i - j of both halves (the compensated periodic difference on marked tiles).
-__device__ __forceinline__ void tile_delta2(f2 x2, f2 y2, f2 z2, const float4 &ja, const float4 &jb, f2 njx, f2 njy, f2 njz,
-                                           bool pbc, const PairParams &pp, f2 &dx, f2 &dy, f2 &dz) {
-    dx = add2(x2, njx);
-    dy = add2(y2, njy);
-    dz = add2(z2, njz);
-    if (pbc) {
-        const float hx = 0.5f * pp.Lx, hy = 0.5f * pp.Ly, hz = 0.5f * pp.Lz;
-        float px, py, pz, t0, t1;
-        unpk(x2, px, t0); unpk(y2, py, t0); unpk(z2, pz, t0);
-#ifdef TV_PBC
-        float a0, a1, b0, b1, c0, c1;
-        unpk(dx, a0, a1); unpk(dy, b0, b1); unpk(dz, c0, c1);
-        const bool far = fmaxf(fabsf(a0), fabsf(a1)) > hx || fmaxf(fabsf(b0), fabsf(b1)) > hy || fmaxf(fabsf(c0), fabsf(c1)) > hz;
-        if (!__any_sync(0xffffffffu, far)) return;
-#endif
-        dx = pk(periodic_delta(px, ja.x, hx, pp.Lx), periodic_delta(px, jb.x, hx, pp.Lx));
-        dy = pk(periodic_delta(py, ja.y, hy, pp.Ly), periodic_delta(py, jb.y, hy, pp.Ly));
-        dz = pk(periodic_delta(pz, ja.z, hz, pp.Lz), periodic_delta(pz, jb.z, hz, pp.Lz));
-        (void)t1;
-    }
-}
 __device__ __forceinline__ void tile_delta(const float4 &pi, const float4 &ja, const float4 &jb, f2 njx, f2 njy, f2 njz,
                                            bool pbc, const PairParams &pp, f2 &dx, f2 &dy, f2 &dz) {
     if (pbc) {
@@ -91,7 +70,7 @@ __device__ __forceinline__ void tile_delta(const float4 &pi, const float4 &ja, c
 // f / r (and with ENERGY the pair energy) of both halves; keep*: the half counts (its bit is set and the pair is
 // not the self tile's masked triangle).  Padding atoms sit far away with zero charge: exact zeros.
 template <int LJK, bool COUL, bool ENERGY, int NP>
-__device__ __forceinline__ void tile_pair(f2 dx, f2 dy, f2 dz, f2 qi, f2 qj, const float4 &ta, const float4 &tb,
+__device__ __forceinline__ void tile_pair(f2 dx, f2 dy, f2 dz, float qi, f2 qj, const float4 &ta, const float4 &tb,
                                           bool keepa, bool keepb, const f2 (&cpf)[NP], const f2 (&cpe)[NP],
                                           const TileConst &tc, const PairParams &pp, f2 &f, f2 &en) {
     const f2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
@@ -123,7 +102,7 @@ __device__ __forceinline__ void tile_pair(f2 dx, f2 dy, f2 dz, f2 qi, f2 qj, con
     if (COUL) {
         const bool ina = ra < pp.rc2 && keepa, inb = rb < pp.rc2 && keepb;
         const f2 x = fma2(r2, tc.sx, tc.one_n);
-        const f2 cq = mul2(qi, qj);
+        const f2 cq = mul2(pk(qi), qj);
         const f2 fq = add2(mul2(rinv, rinv2), horner2(cpf, x));   // the coefficients come negated
         float xa, xb;
         unpk(fq, xa, xb);
@@ -155,13 +134,8 @@ __device__ __forceinline__ void load_entry(TileEntry &t, const uint2 *__restrict
     }
 }
 
-#ifdef TV_LB
-#define TVLB __launch_bounds__(128, TV_LB)
-#else
-#define TVLB __launch_bounds__(128)
-#endif
 template <int LJK, bool COUL, int NP>
-__global__ void TVLB k_pairs_force(const float4 *__restrict__ xq, const int *__restrict__ ts,
+__global__ void __launch_bounds__(128) k_pairs_force(const float4 *__restrict__ xq, const int *__restrict__ ts,
                                                      const uint2 *__restrict__ cjw, const int *__restrict__ scio,
                                                      const int *__restrict__ nw, const int *__restrict__ counts,
                                                      const float *__restrict__ lj_table, float4 *__restrict__ fc,
@@ -170,37 +144,22 @@ __global__ void TVLB k_pairs_force(const float4 *__restrict__ xq, const int *__r
     const int ti = lane & 7, q = lane >> 3;
     const int S = blockIdx.x / nsplit, part = blockIdx.x % nsplit;
     if (S >= counts[W_NS] || counts[W_ERR] != 0) return;
-#ifdef TV_DUP
-    __shared__ float4 sxq[2 * SUPER];
-#else
     __shared__ float4 sxq[SUPER];
-#endif
-#ifdef TV_SM
-    __shared__ float4 scoef[(NP + 1) / 2];
-    for (int k = tid; k < (NP + 1) / 2; k += blockDim.x) { const float c0 = -pp.pf[2*k], c1 = 2*k+1<NP ? -pp.pf[2*k+1] : 0.f; scoef[k] = make_float4(c0,c0,c1,c1); }
-#endif
     __shared__ int sty[SUPER];
     __shared__ float4 stab[LJK == PD_LJ_TABLE ? PD_MAX_TYPES * PD_MAX_TYPES : 1];
     for (int k = tid; k < SUPER; k += blockDim.x) {
         float4 v = xq[S * SUPER + k];
         if (COUL) v.w *= pp.C;
-#ifdef TV_DUP
-        sxq[2 * k] = make_float4(v.x, v.x, v.y, v.y);
-        sxq[2 * k + 1] = make_float4(v.z, v.z, v.w, v.w);
-#else
         sxq[k] = v;
-#endif
         if (LJK == PD_LJ_TABLE) sty[k] = (ts[S * SUPER + k] - 1) * pp.ntypes;
     }
     if (LJK == PD_LJ_TABLE)
         for (int k = tid; k < pp.ntypes * pp.ntypes; k += blockDim.x)
             stab[k] = reinterpret_cast<const float4 *>(lj_table)[k];
     __syncthreads();
-#ifndef TV_SM
     f2 cpf[NP];
 #pragma unroll
     for (int k = 0; k < NP; ++k) cpf[k] = pk_held(COUL ? -pp.pf[k] : 0.f);
-#endif
     const TileConst tc = tile_const<LJK, COUL, false>(pp);
     float fxi[8], fyi[8], fzi[8];
 #pragma unroll
@@ -228,13 +187,7 @@ __global__ void TVLB k_pairs_force(const float4 *__restrict__ xq, const int *__r
 #pragma unroll
         for (int a = 0; a < 8; ++a) {
             if (((word | (word >> 8)) >> a) & 1u) {
-#ifdef TV_DUP
-                const float4 p0 = sxq[2 * (a * 8 + ti)], p1 = sxq[2 * (a * 8 + ti) + 1];
-                const f2 x2 = pk(p0.x, p0.y), y2 = pk(p0.z, p0.w), z2 = pk(p1.x, p1.y), qi2 = pk(p1.z, p1.w);
-#else
                 const float4 pi = sxq[a * 8 + ti];
-                const f2 qi2 = pk(pi.w);
-#endif
                 const bool self = da == a;
                 const bool ka = ((word >> a) & 1u) && (!self || gta), kb = ((word >> (a + 8)) & 1u) && (!self || gtb);
                 float4 ta4 = make_float4(0.f, 0.f, 0.f, 0.f), tb4 = ta4;
@@ -244,17 +197,8 @@ __global__ void TVLB k_pairs_force(const float4 *__restrict__ xq, const int *__r
                     tb4 = stab[tyi + (cur.tb - 1)];
                 }
                 f2 dx, dy, dz, f, en;
-#ifdef TV_DUP
-                tile_delta2(x2, y2, z2, cur.pa, cur.pb, njx, njy, njz, pbc, pp, dx, dy, dz);
-#else
                 tile_delta(pi, cur.pa, cur.pb, njx, njy, njz, pbc, pp, dx, dy, dz);
-#endif
-#ifdef TV_SM
-                f2 cpf[NP];
-#pragma unroll
-                for (int k = 0; k < (NP + 1) / 2; ++k) { const float4 c4 = scoef[k]; cpf[2*k] = pk(c4.x, c4.y); if (2*k+1<NP) cpf[2*k+1] = pk(c4.z, c4.w); }
-#endif
-                tile_pair<LJK, COUL, false, NP>(dx, dy, dz, qi2, qj, ta4, tb4, ka, kb, cpf, cpf, tc, pp, f, en);
+                tile_pair<LJK, COUL, false, NP>(dx, dy, dz, pi.w, qj, ta4, tb4, ka, kb, cpf, cpf, tc, pp, f, en);
                 Jx = fma2(f, dx, Jx);
                 Jy = fma2(f, dy, Jy);
                 Jz = fma2(f, dz, Jz);
@@ -366,7 +310,7 @@ __global__ void __launch_bounds__(64) k_pairs_energy(const float4 *__restrict__ 
             }
             f2 dx, dy, dz, f, en;
             tile_delta(pi, cur.pa, cur.pb, njx, njy, njz, pbc, pp, dx, dy, dz);
-            tile_pair<LJK, COUL, true, NP>(dx, dy, dz, pk(pi.w), qj, ta4, tb4, ka, kb, cpf, cpe, tc, pp, f, en);
+            tile_pair<LJK, COUL, true, NP>(dx, dy, dz, pi.w, qj, ta4, tb4, ka, kb, cpf, cpe, tc, pp, f, en);
             const f2 fx = mul2(f, dx), fy = mul2(f, dy), fz = mul2(f, dz);
             en = mul2(pk(0.5f), en);
             J[0] = add2(J[0], fx);
