@@ -87,7 +87,7 @@ __global__ void k_ell_bin(const float *__restrict__ x, const float *__restrict__
 // to SCAN_ONE_BLOCK cells (two launches cost more than a second chunk there).
 __global__ void __launch_bounds__(1024) k_ell_scan(int *__restrict__ cell_count, int *__restrict__ cell_off,
                                                    int ncell, const long long *__restrict__ st) {
-    if (!ell_requested(st)) return;
+    if (st && !ell_requested(st)) return;
     __shared__ int sb[ELL_SCAN_CHUNK + ELL_SCAN_CHUNK / 32];
     __shared__ int warp_tot[32];
     __shared__ int s_next;
@@ -172,7 +172,7 @@ __device__ __forceinline__ int block_exclusive(int v, int *sh, int &total) {   /
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restrict__ cell_count, int ncell,
                                                             int *__restrict__ part, int ntile,
                                                             const long long *__restrict__ st) {
-    if (!ell_requested(st)) return;
+    if (st && !ell_requested(st)) return;
     __shared__ int sh[SCAN_THREADS / 32];
     __shared__ bool last;
     const int c0 = blockIdx.x * SCAN_TILE;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restric
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(int *__restrict__ cell_count, int *__restrict__ cell_off,
                                                              int ncell, const int *__restrict__ part, int ntile,
                                                              const long long *__restrict__ st) {
-    if (!ell_requested(st)) return;
+    if (st && !ell_requested(st)) return;
     __shared__ int sh[SCAN_THREADS / 32];
     int at = part[blockIdx.x];
 #pragma unroll 1
@@ -609,12 +609,7 @@ EllModel ell_model(const pd_ell *e) {
 
 static size_t scan_part_len(int ncell) { return (size_t)(ncell + SCAN_TILE - 1) / SCAN_TILE + 2; }
 
-// The counting sort of particles into cells, shared with the batched replicas: exclusive scan of
-// the histogram (which becomes the scatter cursors), the scatter, id order inside each cell; every
-// kernel returns at once unless st asks for a rebuild.  part: ell_scan_part_len(ncell) ints, zero at first.
-int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
-                    int *tmp, long long *st, cudaStream_t s) {
-    const int blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
+int cell_scan_launch(int *cell_count, int *cell_off, int ncell, int *part, const long long *st, cudaStream_t s) {
     if (ncell <= SCAN_ONE_BLOCK) {
         k_ell_scan<<<1, 1024, 0, s>>>(cell_count, cell_off, ncell, st);
         PD_LAUNCHED();
@@ -625,6 +620,17 @@ int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *
         k_scan_apply<<<ntile, SCAN_THREADS, 0, s>>>(cell_count, cell_off, ncell, part, ntile, st);
         PD_LAUNCHED();
     }
+    return PD_OK;
+}
+
+// The counting sort of particles into cells, shared with the batched replicas: exclusive scan of
+// the histogram (which becomes the scatter cursors), the scatter, id order inside each cell; every
+// kernel returns at once unless st asks for a rebuild.  part: ell_scan_part_len(ncell) ints, zero at first.
+int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
+                    int *tmp, long long *st, cudaStream_t s) {
+    const int blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
+    const int rc = cell_scan_launch(cell_count, cell_off, ncell, part, st, s);
+    if (rc) return rc;
     k_ell_scatter<<<blocks, ELL_THREADS, 0, s>>>(cell_of, n, cell_off, cell_count, sorted, st);
     PD_LAUNCHED();
     if (n >= ROWS_MIN_PER_CELL * (long long)ncell)

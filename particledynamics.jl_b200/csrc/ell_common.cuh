@@ -155,6 +155,9 @@ namespace pdb {
 EllRowsView ell_rows_view(const ::pd_ell *e);
 int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
                     int *tmp, long long *st, cudaStream_t s);
+// Exclusive scan of a histogram into ncell + 1 offsets, the histogram set to zero; part: ell_scan_part_len(ncell)
+// ints, zero before the first call.  st: an ELL state that gates the kernels, or null.
+int cell_scan_launch(int *cell_count, int *cell_off, int ncell, int *part, const long long *st, cudaStream_t s);
 size_t ell_scan_part_len(int ncell);
 
 }  // namespace pdb

@@ -1,0 +1,44 @@
+"""The mesh's own order of unordered charges: one chunk and one more, ragged counts, a flat box, gathers at moved
+positions and of another count, against the FP64 oracle's mesh sum."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,L", [(64, (14.0, 15.0, 16.0)), (65, (14.0, 15.0, 16.0)), (1501, (14.0, 15.0, 16.0)),
+                                 (20011, (40.0, 44.0, 12.0)), (3000, (9.0, 9.0, 70.0))])
+def test_unordered_charges(pd, ora, cuda, n, L):
+    import torch
+    rng = np.random.default_rng(n)
+    mesh = tuple(int(2 * np.ceil(l / 2)) for l in L)
+    R = (rng.random((n, 3)) * np.array(L) - np.array(L) / 2).astype(np.float32).astype(float)
+    q = rng.standard_normal(n)
+    q = (q - q.mean()).astype(np.float32).astype(float)
+    spec = pd.ElectrostaticsSpec(coulomb_prefactor=1.7, real_cutoff=4.0, alpha=0.9, influence="spme", order=5, mesh=mesh,
+                                 net_charge="background")
+    s = pd.ElectrostaticsSolver(spec, L, q)
+    t = [torch.tensor(np.ascontiguousarray(a), dtype=torch.float32, device="cuda") for a in (*R.T, q)]
+    f = [torch.zeros(n, device="cuda") for _ in range(4)]
+    s.transform(*t, energy=True)
+    s.gather(*t, *f[:3], f[3], energy=True, set=True)
+    torch.cuda.synchronize()
+    ref = ora.mesh(R, q, L, mesh, 5, kind="spme", alpha=0.9, C=1.7, background=True)
+    F = torch.stack(f[:3], 1).double().cpu().numpy()
+    assert np.linalg.norm(F - ref["F"]) < 1e-5 * np.linalg.norm(ref["F"])   # the FP32 mesh bound
+    assert np.linalg.norm(f[3].double().cpu().numpy() - ref["E"]) < 1e-5 * np.linalg.norm(ref["E"])
+    # the same potential gathered with an explicit order, and at other positions, does not depend on the order
+    perm = torch.tensor(rng.permutation(n), dtype=torch.int32, device="cuda")
+    moved = [(a + 0.37).contiguous() for a in t[:3]] + [t[3]]
+    out = []
+    for order in (None, perm):
+        g = [torch.zeros(n, device="cuda") for _ in range(3)]
+        s.gather(*moved, *g, order=order, set=True)
+        out.append(torch.stack(g))
+    assert float((out[0] - out[1]).norm()) < 1e-6 * float(out[1].norm())
+    half = n // 2   # fewer particles than the transform's
+    g, h = ([torch.zeros(half, device="cuda") for _ in range(3)] for _ in range(2))
+    m2 = [a[:half].contiguous() for a in moved]
+    s.gather(*m2, *g, set=True)
+    assert float((torch.stack(g) - out[1][:, :half]).norm()) < 1e-6 * float(out[1].norm())
+    s.close()
