@@ -1083,21 +1083,18 @@ static int batch_make_transforms(pd_batch *b) {
         const int K[3] = {R.K1, R.K2, R.K3};
         if (fft_route(K, &tab[(size_t)r]) != FFT_PLANES) return PD_OK;
     }
-    for (const FftMesh &m : tab)   // two buffers for all where one plane needs them
-        if (fft_plane_smem(m, false) > FFT_PLANE_SMEM_MAX && !fft_plane_inplace(m)) return PD_OK;
     int rc;
     if ((rc = fft_init())) return rc;
     std::vector<int> lens;
     FftBatch f{};
-    f.inplace = true;
-    for (const FftMesh &m : tab) f.inplace = f.inplace && fft_plane_inplace(m);
     std::vector<int> order((size_t)b->nrep);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
         return (long long)b->hmreps[(size_t)p].K1 * b->hmreps[(size_t)p].K2 >
                (long long)b->hmreps[(size_t)q].K1 * b->hmreps[(size_t)q].K2;
     });
-    std::vector<int2> planes, cols;
+    std::vector<int2> planes[4], cols;
+    FftBatch::Class cls[4] = {};
     for (int r : order) {
         const BMeshRep &R = b->hmreps[(size_t)r];
         FftMesh &m = tab[(size_t)r];
@@ -1118,20 +1115,29 @@ static int batch_make_transforms(pd_batch *b) {
         m.G = b->G + R.modes;
         m.zspec[0] = m.spec;
         m.out[0] = b->gridB + R.grid;
-        f.plane_threads = std::max(f.plane_threads, fft_plane_threads(m));
-        f.plane_smem = std::max(f.plane_smem, fft_plane_smem(m, f.inplace));
+        const int c = fft_plane_class(m);
+        cls[c].inplace = c < 3;
+        cls[c].threads = std::max(cls[c].threads, fft_plane_threads(m));
+        cls[c].smem = std::max(cls[c].smem, fft_plane_smem(m, c < 3));
         f.line_threads = std::max(f.line_threads, fft_line_threads(m.ax[2]));
         f.line_smem = std::max(f.line_smem, fft_line_smem(m.ax[2]));
-        for (int z = 0; z < R.K3; ++z) planes.push_back(make_int2(r, z));
-        for (int c = 0; c < R.K2 * R.K1h; c += FFT_LINES_C) cols.push_back(make_int2(r, c));
+        for (int z = 0; z < R.K3; ++z) planes[c].push_back(make_int2(r, z));
+        for (int k = 0; k < R.K2 * R.K1h; k += FFT_LINES_C) cols.push_back(make_int2(r, k));
     }
-    f.nplanes = (int)planes.size();
+    std::vector<int2> all;
+    for (int c = 3; c >= 0; --c) {   // the largest planes first
+        if (planes[c].empty()) continue;
+        cls[c].first = (int)all.size();
+        cls[c].count = (int)planes[c].size();
+        f.cls[f.nclass++] = cls[c];
+        all.insert(all.end(), planes[c].begin(), planes[c].end());
+    }
     f.ncols = (int)cols.size();
-    if ((rc = dalloc(&b->fft_tab, tab.size())) || (rc = dalloc(&b->fft_planes, planes.size())) ||
+    if ((rc = dalloc(&b->fft_tab, tab.size())) || (rc = dalloc(&b->fft_planes, all.size())) ||
         (rc = dalloc(&b->fft_cols, cols.size())))
         return rc;
     PD_CUDA(cudaMemcpy(b->fft_tab, tab.data(), sizeof(FftMesh) * tab.size(), cudaMemcpyHostToDevice));
-    PD_CUDA(cudaMemcpy(b->fft_planes, planes.data(), sizeof(int2) * planes.size(), cudaMemcpyHostToDevice));
+    PD_CUDA(cudaMemcpy(b->fft_planes, all.data(), sizeof(int2) * all.size(), cudaMemcpyHostToDevice));
     PD_CUDA(cudaMemcpy(b->fft_cols, cols.data(), sizeof(int2) * cols.size(), cudaMemcpyHostToDevice));
     f.tab = b->fft_tab;
     f.planes = b->fft_planes;

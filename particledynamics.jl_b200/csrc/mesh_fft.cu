@@ -336,13 +336,18 @@ __device__ __forceinline__ void lines_z(const FftMesh &m, int col0, float2 *S, c
 
 // ------------------------------------------------------------------ kernels: one mesh
 
-template <bool INPLACE>
-__global__ void __launch_bounds__(FFT_PLANE_THREADS) k_plane_forward(const __grid_constant__ FftMesh m) {
+// Planes come in three CTA sizes (up to 256, 512 or FFT_PLANE_THREADS threads): the registers are capped so that
+// four, two or one of them share an SM, as a plane alone leaves most of an SM waiting on its own barriers (12 melts of
+// 3 600 to 12 000 ions, 10 steps: 926 us with one size, 814 with three).
+constexpr int fft_plane_blocks(int maxt) { return maxt <= 256 ? 4 : maxt <= 512 ? 2 : 1; }
+
+template <bool INPLACE, int MAXT>
+__global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_plane_forward(const __grid_constant__ FftMesh m) {
     extern __shared__ float2 fft_smem[];
     plane_forward<INPLACE>(m, blockIdx.x, fft_smem);
 }
-template <bool INPLACE>
-__global__ void __launch_bounds__(FFT_PLANE_THREADS) k_plane_inverse(const __grid_constant__ FftMesh m) {
+template <bool INPLACE, int MAXT>
+__global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_plane_inverse(const __grid_constant__ FftMesh m) {
     extern __shared__ float2 fft_smem[];
     plane_inverse<INPLACE>(m, blockIdx.x, blockIdx.y, fft_smem);
 }
@@ -436,8 +441,8 @@ __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_LINES_C) k_lines_y(const __
 
 // blocks[i] = (mesh, plane or first column); every kernel returns while the rows are invalid, as the other
 // stages of the batched step do.
-template <bool INPLACE>
-__global__ void __launch_bounds__(FFT_PLANE_THREADS) k_bplane_forward(const FftMesh *__restrict__ tab,
+template <bool INPLACE, int MAXT>
+__global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_bplane_forward(const FftMesh *__restrict__ tab,
                                                                      const int2 *__restrict__ blocks,
                                                                      const long long *__restrict__ st) {
     if (st[E_VALID] == 0) return;
@@ -448,8 +453,8 @@ __global__ void __launch_bounds__(FFT_PLANE_THREADS) k_bplane_forward(const FftM
     __syncthreads();
     plane_forward<INPLACE>(m, w.y, fft_smem);
 }
-template <bool INPLACE>
-__global__ void __launch_bounds__(FFT_PLANE_THREADS) k_bplane_inverse(const FftMesh *__restrict__ tab,
+template <bool INPLACE, int MAXT>
+__global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_bplane_inverse(const FftMesh *__restrict__ tab,
                                                                      const int2 *__restrict__ blocks,
                                                                      const long long *__restrict__ st) {
     if (st[E_VALID] == 0) return;
@@ -525,15 +530,21 @@ int fft_plane_threads(const FftMesh &m) {
     return std::min(FFT_PLANE_THREADS, ((items + rounds - 1) / rounds + 31) / 32 * 32);
 }
 
+int fft_plane_class(const FftMesh &m) {
+    const int nt = fft_plane_threads(m);
+    return !fft_plane_inplace(m) ? 3 : nt <= 256 ? 0 : nt <= 512 ? 1 : 2;
+}
+
 int fft_line_threads(const FftAxis &a) { return FFT_LINES_C * std::max(a.a, a.b); }
 size_t fft_line_smem(const FftAxis &a) { return sizeof(float2) * (size_t)a.n * FFT_LINES_C; }
 
 int fft_init() {
     const int most = (int)FFT_PLANE_SMEM_MAX;
-    const void *fns[] = {(const void *)k_plane_forward<true>,   (const void *)k_plane_forward<false>,
-                         (const void *)k_plane_inverse<true>,   (const void *)k_plane_inverse<false>,
-                         (const void *)k_bplane_forward<true>,  (const void *)k_bplane_forward<false>,
-                         (const void *)k_bplane_inverse<true>,  (const void *)k_bplane_inverse<false>};
+#define PD_PLANE_SIZES(K) (const void *)K<true, 256>, (const void *)K<true, 512>, (const void *)K<true, FFT_PLANE_THREADS>, \
+                          (const void *)K<false, FFT_PLANE_THREADS>
+    const void *fns[] = {PD_PLANE_SIZES(k_plane_forward), PD_PLANE_SIZES(k_plane_inverse),
+                         PD_PLANE_SIZES(k_bplane_forward), PD_PLANE_SIZES(k_bplane_inverse)};
+#undef PD_PLANE_SIZES
     for (const void *f : fns) PD_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     const int line = 2 * FFT_RADIX_MAX * FFT_RADIX_MAX * FFT_LINES_C * (int)sizeof(float2);   // two exchanges (ik)
     PD_CUDA(cudaFuncSetAttribute((const void *)k_lines_z<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, line));
@@ -546,13 +557,23 @@ static size_t fft_rows_smem(const FftMesh &m) {
     return sizeof(float2) * FFT_ROW_PAIRS * ((size_t)X.a * (X.b | 1) + std::max(X.n, 2 * m.K1h));
 }
 
+#define PD_UNPAREN(...) __VA_ARGS__
+// A plane kernel in the CTA size of nt threads (two buffers: always the largest).
+#define PD_PLANE_LAUNCH(K, inplace, nt, grid, shm, s, args)                                \
+    do {                                                                                   \
+        if (!(inplace)) K<false, FFT_PLANE_THREADS><<<grid, nt, shm, s>>>(PD_UNPAREN args);            \
+        else if ((nt) <= 256) K<true, 256><<<grid, nt, shm, s>>>(PD_UNPAREN args);                     \
+        else if ((nt) <= 512) K<true, 512><<<grid, nt, shm, s>>>(PD_UNPAREN args);                     \
+        else K<true, FFT_PLANE_THREADS><<<grid, nt, shm, s>>>(PD_UNPAREN args);                        \
+    } while (0)
+
 int fft_forward(const FftMesh &m, int route, cudaStream_t s) {
     if (route == FFT_PLANES) {
         const bool in = fft_plane_inplace(m);
         const int nt = fft_plane_threads(m);
         const size_t shm = fft_plane_smem(m, in);
-        if (in) k_plane_forward<true><<<m.ax[2].n, nt, shm, s>>>(m);
-        else k_plane_forward<false><<<m.ax[2].n, nt, shm, s>>>(m);
+        const dim3 g(m.ax[2].n);
+        PD_PLANE_LAUNCH(k_plane_forward, in, nt, g, shm, s, (m));
         PD_LAUNCHED();
         return PD_OK;
     }
@@ -585,8 +606,8 @@ int fft_inverse(const FftMesh &m, int route, int nout, cudaStream_t s) {
         const bool in = fft_plane_inplace(m);
         const int nt = fft_plane_threads(m);
         const size_t shm = fft_plane_smem(m, in);
-        if (in) k_plane_inverse<true><<<dim3(m.ax[2].n, nout), nt, shm, s>>>(m);
-        else k_plane_inverse<false><<<dim3(m.ax[2].n, nout), nt, shm, s>>>(m);
+        const dim3 g(m.ax[2].n, nout);
+        PD_PLANE_LAUNCH(k_plane_inverse, in, nt, g, shm, s, (m));
         PD_LAUNCHED();
         return PD_OK;
     }
@@ -594,21 +615,24 @@ int fft_inverse(const FftMesh &m, int route, int nout, cudaStream_t s) {
     k_lines_y<true><<<g, fft_line_threads(m.ax[1]), fft_line_smem(m.ax[1]), s>>>(m);
     PD_LAUNCHED();
     const int pairs = (m.ax[1].n + 1) / 2 * m.ax[2].n;
-    k_rows_inverse<<<dim3((pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, nout), FFT_RADIX_MAX * FFT_ROW_PAIRS,
-                     fft_rows_smem(m), s>>>(m);
+    k_rows_inverse<<<dim3((pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, nout), FFT_RADIX_MAX * FFT_ROW_PAIRS, fft_rows_smem(m), s>>>(m);
     PD_LAUNCHED();
     return PD_OK;
 }
 
 int fft_batch(const FftBatch &f, const long long *st, cudaStream_t s) {
-    if (f.inplace) k_bplane_forward<true><<<f.nplanes, f.plane_threads, f.plane_smem, s>>>(f.tab, f.planes, st);
-    else k_bplane_forward<false><<<f.nplanes, f.plane_threads, f.plane_smem, s>>>(f.tab, f.planes, st);
-    PD_LAUNCHED();
+    for (int c = 0; c < f.nclass; ++c) {
+        const FftBatch::Class &k = f.cls[c];
+        PD_PLANE_LAUNCH(k_bplane_forward, k.inplace, k.threads, k.count, k.smem, s, (f.tab, f.planes + k.first, st));
+        PD_LAUNCHED();
+    }
     k_blines_z<<<f.ncols, f.line_threads, f.line_smem, s>>>(f.tab, f.cols, st);
     PD_LAUNCHED();
-    if (f.inplace) k_bplane_inverse<true><<<f.nplanes, f.plane_threads, f.plane_smem, s>>>(f.tab, f.planes, st);
-    else k_bplane_inverse<false><<<f.nplanes, f.plane_threads, f.plane_smem, s>>>(f.tab, f.planes, st);
-    PD_LAUNCHED();
+    for (int c = 0; c < f.nclass; ++c) {
+        const FftBatch::Class &k = f.cls[c];
+        PD_PLANE_LAUNCH(k_bplane_inverse, k.inplace, k.threads, k.count, k.smem, s, (f.tab, f.planes + k.first, st));
+        PD_LAUNCHED();
+    }
     return PD_OK;
 }
 

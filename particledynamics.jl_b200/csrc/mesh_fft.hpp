@@ -32,15 +32,22 @@ struct FftMesh {
     float kd[3];        // ik: 2 pi / L per axis
 };
 
-// Batched meshes: a table of meshes and the (mesh, plane) and (mesh, first column) of every CTA.
+// Batched meshes: a table of meshes and the (mesh, plane) and (mesh, first column) of every CTA; the planes
+// by CTA size (one launch each way per class).
 struct FftBatch {
+    struct Class {
+        int first, count, threads;
+        size_t smem;
+        bool inplace;
+    };
     const FftMesh *tab;
     const int2 *planes, *cols;
-    int nplanes, ncols;
-    int plane_threads, line_threads;
-    size_t plane_smem, line_smem;
-    bool inplace;        // every plane's passes have a thread per item
+    int ncols, line_threads;
+    size_t line_smem;
+    int nclass;
+    Class cls[4];   // up to 256, 512 and FFT_PLANE_THREADS threads in place, then two buffers
 };
+int fft_plane_class(const FftMesh &m);
 
 // Route of a mesh; fills the axes' factors (twiddle tables stay null).
 int fft_route(const int K[3], FftMesh *m);
@@ -57,7 +64,7 @@ size_t fft_line_smem(const FftAxis &a);
 int fft_forward(const FftMesh &m, int route, cudaStream_t s);
 int fft_solve(const FftMesh &m, bool ik, bool energy, const float *Vc, double *acc, cudaStream_t s);
 int fft_inverse(const FftMesh &m, int route, int nout, cudaStream_t s);
-// The whole transform pair of every batched mesh: three launches.
+// The whole transform pair of every batched mesh: three launches per class and z lines.
 int fft_batch(const FftBatch &f, const long long *st, cudaStream_t s);
 
 }  // namespace pdb
