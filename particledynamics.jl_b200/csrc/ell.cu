@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_rows(
 // Row construction for dense cells: one warp per cell, or nsplit warps where the grid has few cells (each
 // stages the stencil for its share of the cell's particles).
 template <int D>
-__global__ void __launch_bounds__(32 * ROWS_WARPS) k_ell_rows_cells(
+__global__ void __launch_bounds__(32 * ROWS_WARPS, ROWS_BLOCKS) k_ell_rows_cells(
     const float4 *__restrict__ xq, const int *__restrict__ sorted, const int *__restrict__ cell_off, RowGrid g,
     int nsplit, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref,
     long long *__restrict__ st) {

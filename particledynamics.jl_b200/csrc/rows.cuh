@@ -15,7 +15,8 @@
 
 namespace pdb {
 
-constexpr int ROWS_WARPS = 4, ROWS_CAP = 640;   // 40 KB of staging per block (below the 48 KB default)
+constexpr int ROWS_WARPS = 4, ROWS_CAP = 512;   // 32 KB of staging per block: six blocks share an SM
+constexpr int ROWS_BLOCKS = 6;
 constexpr int ROWS_MIN_PER_CELL = 8;            // mean cell occupancy from which the cell-staged build is used
 constexpr int ROWS_GROUP = 4;                   // particles tested against each staged candidate register
 
@@ -33,7 +34,7 @@ struct RowGrid {
 // ROWS_GROUP particles: the accepted ones are appended in visiting order by ballot.  Bound by the issue of the
 // tests (12 instructions per 32 candidates and particle); a lane-per-particle scan of the same stage left the
 // lanes beyond the cell's particles idle and scattered its row stores (1 048 576 LJ atoms, 19 per cell: 3.34 ms
-// per build).  NOWRAP: no pair of the stencil crosses a periodic face, the nearest-image shift is the identity.
+// per build, now 0.56).  NOWRAP: no pair of the stencil crosses a periodic face, the nearest-image shift is the identity.
 template <int D, bool WRAP>
 __device__ __forceinline__ void rows_test(const RowGrid &g, float4 *sw, int fill, int np, float xi, float yi, float zi,
                                           int k0, float rl2, int cap, int *__restrict__ rows, int &found) {
@@ -46,8 +47,10 @@ __device__ __forceinline__ void rows_test(const RowGrid &g, float4 *sw, int fill
     for (int m0 = 0; m0 < np; m0 += ROWS_GROUP) {
         float px[ROWS_GROUP], py[ROWS_GROUP], pz[ROWS_GROUP];
         int base[ROWS_GROUP];
+        int *row[ROWS_GROUP];
 #pragma unroll
         for (int m = 0; m < ROWS_GROUP; ++m) {
+            row[m] = rows + (size_t)(k0 + m0 + m) * cap;
             const int src = (m0 + m) & 31;
             px[m] = __shfl_sync(0xffffffffu, xi, src);
             py[m] = __shfl_sync(0xffffffffu, yi, src);
@@ -71,7 +74,7 @@ __device__ __forceinline__ void rows_test(const RowGrid &g, float4 *sw, int fill
                 const bool hit = r2 <= rl2 && kc != k;
                 const unsigned bal = __ballot_sync(0xffffffffu, hit);
                 const int at = base[m] + __popc(bal & lt);
-                if (hit && at < cap) rows[(size_t)k * cap + at] = kc;
+                if (hit && at < cap) row[m][at] = kc;
                 base[m] += __popc(bal);
             }
         }
@@ -127,41 +130,72 @@ __device__ __forceinline__ unsigned cell_rows(const RowGrid &g, int c, int split
             else rows_test<D, true>(g, sw, fill, np, me.x, me.y, me.z, p0 + pg, rl2, cap, rows, found);
             fill = 0;
         };
-        for (int oz = -Sz; oz <= Sz; ++oz) {
-            int cz2 = cz + oz;
-            cz2 -= cz2 >= nz ? nz : 0;
-            cz2 += cz2 < 0 ? nz : 0;
-            const float gz = (float)max(abs(oz) - 1, 0) * hz;
-            for (int oy = -Sy; oy <= Sy; ++oy) {
-                int cy2 = cy + oy;
+        // The stencil's runs of candidates (positions [ka, kb), two per (oz, oy) row at the periodic seam) are
+        // looked up at once, lane 2 r + part holding one run, and then walked as one sequence: a lane's candidate
+        // needs no load that waits for another run's.
+        const int nrow = (2 * Sz + 1) * (2 * Sy + 1);
+        for (int r0 = 0; r0 < nrow; r0 += 16) {
+            int ka = 0, len = 0;
+            const int r = r0 + (lane >> 1);
+            if (r < nrow) {
+                const int oz = r / (2 * Sy + 1) - Sz, oy = r % (2 * Sy + 1) - Sy;
+                int cz2 = cz + oz, cy2 = cy + oy;
+                cz2 -= cz2 >= nz ? nz : 0;
+                cz2 += cz2 < 0 ? nz : 0;
                 cy2 -= cy2 >= ny ? ny : 0;
                 cy2 += cy2 < 0 ? ny : 0;
-                const float gy = (float)max(abs(oy) - 1, 0) * hy;
+                const float gz = (float)max(abs(oz) - 1, 0) * hz, gy = (float)max(abs(oy) - 1, 0) * hy;
                 const float g2 = fmaf(gy, gy, gz * gz);
-                if (g2 > rl2) continue;
-                const int row = g.base + (cz2 * ny + cy2) * nx;
-                int a1, b1, a2, b2;
-                ell_row_ranges(cx, g2, rl2, hx, Sx, nx, a1, b1, a2, b2);
-                for (int part = 0; part < 2; ++part) {
-                    if (part == 1 && a2 > b2) break;
-                    const int ka = cell_off[row + (part ? a2 : a1)], kb = cell_off[row + (part ? b2 : b1) + 1];
-                    for (int k0 = ka; k0 < kb; k0 += 32) {
-                        const bool in = lane < kb - k0;
-                        float4 v = in ? xq[k0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float ex = fmaxf(fabsf(mic_fast(v.x - bcx, hLx, Lx)) - bhx, 0.f);
-                        const float ey = fmaxf(fabsf(mic_fast(v.y - bcy, hLy, Ly)) - bhy, 0.f);
-                        const float ez = D == 3 ? fmaxf(fabsf(mic_fast(v.z - bcz, hLz, Lz)) - bhz, 0.f) : 0.f;
-                        const bool keep = in && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= rbox2;
-                        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                        const int nk = __popc(bal);
-                        if (fill + nk > ROWS_CAP) scan();
-                        if (keep) {   // staged in the candidates' order
-                            v.w = __int_as_float(k0 + lane);
-                            sw[fill + __popc(bal & ((1u << lane) - 1u))] = v;
-                        }
-                        fill += nk;
+                if (g2 <= rl2) {
+                    int a1, b1, a2, b2;
+                    ell_row_ranges(cx, g2, rl2, hx, Sx, nx, a1, b1, a2, b2);
+                    const bool second = lane & 1;
+                    if (!second || a2 <= b2) {
+                        const int *off = cell_off + g.base + (cz2 * ny + cy2) * nx;
+                        ka = off[second ? a2 : a1];
+                        len = off[(second ? b2 : b1) + 1] - ka;
                     }
                 }
+            }
+            int end = len;   // inclusive prefix over the runs
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += y;
+            }
+            const int total = __shfl_sync(0xffffffffu, end, 31);
+            const int shift = ka - (end - len);   // candidate c of this run sits at position c + shift
+            auto position = [&](int c) {          // of candidate c (c < total): the first run ending past it
+                int run = 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int e = __shfl_sync(0xffffffffu, end, run + o - 1);
+                    run += c >= e ? o : 0;
+                }
+                return c + __shfl_sync(0xffffffffu, shift, run);
+            };
+            int kn = position(min(lane, max(total - 1, 0)));
+            float4 vn = lane < total ? xq[kn] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c0 = 0; c0 < total; c0 += 32) {
+                const bool in = c0 + lane < total;
+                float4 v = vn;
+                const int kc = kn;
+                if (c0 + 32 < total) {   // the next 32 candidates are in flight while these are tested
+                    kn = position(min(c0 + 32 + lane, total - 1));
+                    vn = xq[kn];
+                }
+                const float ex = fmaxf(fabsf(mic_fast(v.x - bcx, hLx, Lx)) - bhx, 0.f);
+                const float ey = fmaxf(fabsf(mic_fast(v.y - bcy, hLy, Ly)) - bhy, 0.f);
+                const float ez = D == 3 ? fmaxf(fabsf(mic_fast(v.z - bcz, hLz, Lz)) - bhz, 0.f) : 0.f;
+                const bool keep = in && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= rbox2;
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                const int nk = __popc(bal);
+                if (fill + nk > ROWS_CAP) scan();
+                if (keep) {   // staged in the candidates' order
+                    v.w = __int_as_float(kc);
+                    sw[fill + __popc(bal & ((1u << lane) - 1u))] = v;
+                }
+                fill += nk;
             }
         }
         scan();
