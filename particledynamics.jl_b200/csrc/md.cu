@@ -402,17 +402,31 @@ int pd_md_evaluate(pd_md *md, int energy, pd_stream_t sp) {
     const float *q = c->p.coulomb ? st.q : nullptr;
     int rc, h[W_LEN];
     if ((rc = cluster_decide_launch(c, st.x, st.y, st.z, 0, s))) return rc;
-    if ((rc = cluster_read_counts(c, h, s))) return rc;
+    // With a list there is a slot order, and any slot order will do for the mesh: its transform starts before
+    // the host knows whether the list is kept, and runs while the decision is read back.
+    const bool early = c->have_build;
+    if (early) {
+        if ((rc = pd_cluster_pack(c, st.x, st.y, st.z, q, st.type, sp))) return rc;
+        if ((rc = fork_mesh(md, energy, s))) return rc;
+    }
+    // after an early start, what refuses the evaluation still leaves the mesh's work ordered before the stream's next
+    auto refused = [&](int code) {
+        if (early && md->m) cudaStreamWaitEvent(s, md->ev_join, 0);
+        return code;
+    };
+    if ((rc = cluster_read_counts(c, h, s))) return refused(rc);
     if (h[W_BUILD] || !c->have_build) {
+        // the build packs the slots anew: after the spread has read them
+        if (early && md->m) PD_CUDA(cudaStreamWaitEvent(s, md->ev_spread, 0));
         for (int attempt = 0; attempt < 8; ++attempt) {
-            if ((rc = cluster_build_launch(c, st.x, st.y, st.z, q, st.type, 0, s))) return rc;
-            if ((rc = cluster_read_counts(c, h, s))) return rc;
+            if ((rc = cluster_build_launch(c, st.x, st.y, st.z, q, st.type, 0, s))) return refused(rc);
+            if ((rc = cluster_read_counts(c, h, s))) return refused(rc);
             if (h[W_ERR] == 0) break;
             if (h[W_ERR] == PD_ENONFINITE) {
                 set_error("Cluster-pair list: non-finite coordinates");
-                return PD_ENONFINITE;
+                return refused(PD_ENONFINITE);
             }
-            if ((rc = pd_cluster_grow(c))) return rc;
+            if ((rc = pd_cluster_grow(c))) return refused(rc);
             // the graphs captured the old entry storage
             for (int k = 0; k < 2; ++k)
                 if (md->exec[k]) {
@@ -420,14 +434,15 @@ int pd_md_evaluate(pd_md *md, int energy, pd_stream_t sp) {
                     md->exec[k] = nullptr;
                 }
         }
-        PD_CHECK(h[W_ERR] == 0, PD_ECAPACITY, "outer list still overflows after growth");
+        if (h[W_ERR] != 0) {
+            set_error("outer list still overflows after growth");
+            return refused(PD_ECAPACITY);
+        }
         c->have_build = true;
         if ((rc = cluster_set_word(c, W_PRUNE, 1, s))) return rc;
-    } else {
-        if ((rc = pd_cluster_pack(c, st.x, st.y, st.z, q, st.type, sp))) return rc;
     }
     if ((rc = fork_learned(md, s))) return rc;
-    if ((rc = fork_mesh(md, energy, s))) return rc;
+    if (!early && (rc = fork_mesh(md, energy, s))) return rc;
     if ((rc = cluster_prune_launch(c, 1, s))) return rc;
     return enqueue_forces(md, energy, 0.f, s);
 }
