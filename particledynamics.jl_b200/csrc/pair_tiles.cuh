@@ -13,6 +13,8 @@
 // ran out of instruction cache and registers (24 002 ions: 135 us, 6.9 of 10 stalled warps without an
 // instruction, 158 registers).
 #pragma once
+#include <algorithm>
+
 #include "cluster_pairs.cuh"
 #include "packed2.cuh"
 
@@ -393,9 +395,11 @@ __global__ void __launch_bounds__(64) k_pairs_energy(const float4 *__restrict__ 
 
 template <int LJK, bool COUL, int NP>
 static void launch_tiles(pd_cluster *c, int energy, cudaStream_t s) {
+    // the energy pass has two warps per part: as many warps as the force pass
+    const int eparts = std::max(1, c->nsplit * c->pair_warps / 2);
     if (energy)
-        k_pairs_energy<LJK, COUL, NP><<<c->nsmax * c->nsplit, 64, 0, s>>>(c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts,
-                                                                       c->lj_table, c->fc, c->vc, c->nslot, c->nsplit,
+        k_pairs_energy<LJK, COUL, NP><<<c->nsmax * eparts, 64, 0, s>>>(c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts,
+                                                                       c->lj_table, c->fc, c->vc, c->nslot, eparts,
                                                                        c->pp);
     else
         k_pairs_force<LJK, COUL, NP><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
