@@ -374,6 +374,104 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
     if (advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
 }
 
+// The uncharged pair pass with one lane per row: a thread adds its row's terms in row order, so the sums are those
+// of the row order itself.  A warp's 32 rows are read eight entries at a time by eight lanes each (whole sectors of
+// the row-major rows) and turned around in shared memory.  96 replicas, 568 986 atoms: 158 us (eight lanes per row:
+// 133 us, slot-major rows read entry by entry: 225 us).
+constexpr int SEQ_E = 8;   // entries per turn
+template <bool ENERGY, bool SLOT>
+__global__ void __launch_bounds__(B_THREADS, 3) k_batch_pairs_seq(const float4 *__restrict__ xq, int n, int cap,
+                                                               const int *__restrict__ rows,
+                                                               const int *__restrict__ counts,
+                                                               const int *__restrict__ sorted,
+                                                               const int *__restrict__ rep_of,
+                                                               const BatchRep *__restrict__ reps,
+                                                               float *__restrict__ fx, float *__restrict__ fy,
+                                                               float *__restrict__ fz, float *__restrict__ epot,
+                                                               float4 *__restrict__ fc, BatchKick kick,
+                                                               long long *__restrict__ st, int advance) {
+    if (st[E_VALID] == 0) return;
+    __shared__ int turn[B_THREADS / 32][32 * (SEQ_E + 1)];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int *mine = turn[threadIdx.x >> 5];
+    const bool live = k < n;
+    const int i = live ? sorted[k] : -1;
+    const BatchRep &R = reps[live ? __ldg(rep_of + i) : 0];
+    const float L[3] = {R.L[0], R.L[1], R.L[2]};
+    const LjRow lj = lj_row(R.eps, R.sig2, R.rc2, R.kind == PD_PAIR_WCA ? R.eps : -R.eshift);
+    const float4 pi = live ? xq[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int cnt = live ? counts[k] : 0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    float a[3] = {0.f, 0.f, 0.f}, e = 0.f;
+    // lane reads entry c0 + (lane & 7) of rows (lane >> 3) + 4 u, u < 8; past a row's end its own position
+    int at[SEQ_E], rc[SEQ_E];
+    const int k0 = k - lane, er = lane & (SEQ_E - 1);
+#pragma unroll
+    for (int u = 0; u < SEQ_E; ++u) rc[u] = __shfl_sync(0xffffffffu, cnt, (lane >> 3) + 4 * u);
+    auto fetch = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < SEQ_E; ++u) {
+            const int r = k0 + (lane >> 3) + 4 * u, t = c0 + er;
+            at[u] = t < rc[u] ? __ldg(rows + (size_t)r * cap + t) : min(r, n - 1);
+        }
+    };
+    auto walk = [&](auto wrap) {
+        constexpr bool WRAP = decltype(wrap)::value;
+        fetch(0);
+        for (int c0 = 0; c0 < most; c0 += SEQ_E) {
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < SEQ_E; ++u) mine[((lane >> 3) + 4 * u) * (SEQ_E + 1) + er] = at[u];
+            __syncwarp();
+            float4 p[SEQ_E];
+#pragma unroll
+            for (int u = 0; u < SEQ_E; ++u) p[u] = __ldg(xq + mine[lane * (SEQ_E + 1) + u]);
+            if (c0 + SEQ_E < most) fetch(c0 + SEQ_E);
+#pragma unroll
+            for (int u = 0; u < SEQ_E; u += 2) {
+                float dx[2], dy[2], dz[2], r2[2], f[2], v[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    pair_delta<3, WRAP>(pi, p[u + c], L, dx[c], dy[c], dz[c]);
+                    r2[c] = fmaf(dx[c], dx[c], fmaf(dy[c], dy[c], dz[c] * dz[c]));
+                }
+                f2 fr, un;
+                lj_two<ENERGY>(lj, rcp2(pk(r2[0], r2[1])), fr, un);
+                unpk(fr, f[0], f[1]);
+                if (ENERGY) unpk(un, v[0], v[1]);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const bool in = r2[c] > 0.f && r2[c] < lj.rc2;
+                    const float fv = in ? f[c] : 0.f;
+                    a[0] = fmaf(fv, dx[c], a[0]);
+                    a[1] = fmaf(fv, dy[c], a[1]);
+                    a[2] = fmaf(fv, dz[c], a[2]);
+                    if (ENERGY) e += in ? 0.5f * v[c] : 0.f;
+                }
+            }
+        }
+    };
+    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, 1.001f * sqrtf(lj.rc2)))) walk(std::false_type{});
+    else walk(std::true_type{});
+    if (live) {
+        if (SLOT) {
+            fc[k] = make_float4(a[0], a[1], a[2], e);
+        } else {
+            fx[i] = a[0];
+            fy[i] = a[1];
+            fz[i] = a[2];
+            if (ENERGY) epot[i] = e;
+            if (kick.on) {
+                const float c = kick.half_dt * kick.inv_mass[i];
+                kick.vx[i] = fmaf(c, a[0], kick.vx[i]);
+                kick.vy[i] = fmaf(c, a[1], kick.vy[i]);
+                kick.vz[i] = fmaf(c, a[2], kick.vz[i]);
+            }
+        }
+    }
+    if (advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
+}
+
 // Positions' forces to particle order, with the closing half kick when there is one.
 template <bool ENERGY>
 __global__ void __launch_bounds__(B_THREADS) k_batch_finish(const float4 *__restrict__ fc,
@@ -538,6 +636,8 @@ static void batch_free(pd_batch *b) {
     dfree(b->xrows);
 }
 
+static int batch_blocks(const pd_batch *b) { return (b->n + B_THREADS - 1) / B_THREADS; }
+
 static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
     k_batch_bin<<<blocks, B_THREADS, 0, s>>>(x, y, z, b->n, b->rep_of, b->reps, b->rep_flag, b->cell_of,
@@ -564,15 +664,29 @@ static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, con
     return PD_OK;
 }
 
-// Lanes per row: the caller's choice, but at least as many as fill 32-byte sectors of the row-major rows where
-// the rows are that long (walking them with fewer lanes reads each sector several times).
-static int batch_lanes(const pd_batch *b) { return std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8); }
-
 template <bool COUL, int NP = BATCH_NP>
 static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, float *epot, int energy,
                                const BatchKick &kick, int advance, bool slot, cudaStream_t s) {
-    const int G = batch_lanes(b);
+    // Charged rows are long and every choice below 8 lanes reads their sectors several times; uncharged rows take
+    // the caller's choice.
+    const int G = COUL ? std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8) : b->lanes;
     const int blocks = (int)(((long long)b->n * G + B_THREADS - 1) / B_THREADS);
+    if constexpr (!COUL) {
+        if (G == 1) {
+#define PD_BS(EE, SS)                                                                                               \
+    k_batch_pairs_seq<EE, SS><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->cap, b->rows, b->counts,     \
+                   b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, b->fc, kick, b->st, advance)
+            if (slot) {
+                if (energy) PD_BS(true, true);
+                else PD_BS(false, true);
+            } else {
+                if (energy) PD_BS(true, false);
+                else PD_BS(false, false);
+            }
+#undef PD_BS
+            return;
+        }
+    }
 #define PD_BP2(GG, EE, SS)                                                                                            \
     k_batch_pairs<GG, EE, COUL, SS, NP><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->cap, b->rows, b->counts,         \
                                                                      b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, \
@@ -586,7 +700,9 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
         else PD_BP2(GG, false, false);                                                                                \
     }
     switch (G) {
-        case 1: PD_BP(1) break;
+        case 1:
+            if constexpr (COUL) { PD_BP(1) }
+            break;
         case 2: PD_BP(2) break;
         case 4: PD_BP(4) break;
         default: PD_BP(8) break;

@@ -752,14 +752,23 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
 #undef PD_ELL_PAIRS
 }
 
-// Lanes per row: slot-major rows take the engine's choice; row-major rows at least 8, so that a step of the
-// walk reads whole 32-byte sectors, and a whole warp per row where the rows alone would leave SMs idle.
 template <int D>
 static void ell_pairs_d(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
                         const EllKick &kick, cudaStream_t s) {
     if (e->dense) {
-        if (e->n < 16384) ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
-        else ell_pairs_g<D, 8, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
+        // the caller's lanes, or a whole warp per row where the rows alone leave SMs idle (4000 LJ atoms: 63 blocks
+        // of four lanes per row, 16 us; 500 blocks of a warp, 8 us); a million atoms take 4 and 8 lanes alike and 16
+        // a third longer
+        if (e->p.lanes == 0 && e->n < 16384) {
+            ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
+            return;
+        }
+        switch (e->lanes) {
+            case 1: ell_pairs_g<D, 1, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+            case 2: ell_pairs_g<D, 2, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+            case 4: ell_pairs_g<D, 4, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+            default: ell_pairs_g<D, 8, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        }
         return;
     }
     switch (e->lanes) {
