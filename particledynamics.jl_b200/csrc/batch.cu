@@ -97,7 +97,7 @@ __device__ void batch_decide(long long *st, unsigned *rep_dmax, int *rep_flag, i
 // Half kick, drift, wrap and displacement (DRIFT), or the displacement of the current coordinates
 // alone; per-replica displacement maxima, the decision by the last block.
 template <bool DRIFT, bool COND>
-__global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, float *__restrict__ x, float *__restrict__ y,
+__global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, int items, float *__restrict__ x, float *__restrict__ y,
                                                            float *__restrict__ z, float *__restrict__ vx,
                                                            float *__restrict__ vy, float *__restrict__ vz,
                                                            const float *__restrict__ fx, const float *__restrict__ fy,
@@ -114,41 +114,46 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, float *__restr
         if (COND && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
         return;
     }
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float v = 0.f;
-    int r = -1;
-    if (i < n) {
-        r = __ldg(rep_of + i);
-        const BatchRep &R = reps[r];
-        const float L[3] = {R.L[0], R.L[1], R.L[2]};
-        float p[3] = {x[i], y[i], z[i]};
-        if (DRIFT) {
-            const float c = 0.5f * dt * inv_mass[i];
-            const float u[3] = {fmaf(c, fx[i], vx[i]), fmaf(c, fy[i], vy[i]), fmaf(c, fz[i], vz[i])};
-            vx[i] = u[0];
-            vy[i] = u[1];
-            vz[i] = u[2];
+    unsigned most = 0;
+    // `items` rounds per block: the fence and the ticket come once for all of them
+    for (int it = 0; it < items; ++it) {
+        const int i = (blockIdx.x * items + it) * B_THREADS + threadIdx.x;
+        float v = 0.f;
+        int r = -1;
+        if (i < n) {
+            r = __ldg(rep_of + i);
+            const BatchRep &R = reps[r];
+            const float L[3] = {R.L[0], R.L[1], R.L[2]};
+            float p[3] = {x[i], y[i], z[i]};
+            if (DRIFT) {
+                const float c = 0.5f * dt * inv_mass[i];
+                const float u[3] = {fmaf(c, fx[i], vx[i]), fmaf(c, fy[i], vy[i]), fmaf(c, fz[i], vz[i])};
+                vx[i] = u[0];
+                vy[i] = u[1];
+                vz[i] = u[2];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) p[d] = wrap_centred(fmaf(dt, u[d], p[d]), L[d]);
-            x[i] = p[0];
-            y[i] = p[1];
-            z[i] = p[2];
-            if (pos_of) xq[pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);   // packed for the pair pass
+                for (int d = 0; d < 3; ++d) p[d] = wrap_centred(fmaf(dt, u[d], p[d]), L[d]);
+                x[i] = p[0];
+                y[i] = p[1];
+                z[i] = p[2];
+                if (pos_of) xq[pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);   // packed for the pair pass
+            }
+            v = ell_displacement<3>(p, ref[i], L, st[E_VALID] != 0);
         }
-        v = ell_displacement<3>(p, ref[i], L, st[E_VALID] != 0);
-    }
-    // per-replica maximum: one atomic per warp where the warp's particles share a replica
-    const unsigned bits = __float_as_uint(v);
-    const int r0 = __shfl_sync(0xffffffffu, r, 0);
-    if (__all_sync(0xffffffffu, r == r0)) {
-        const unsigned m = __reduce_max_sync(0xffffffffu, bits);
-        if ((threadIdx.x & 31) == 0 && r0 >= 0) atomicMax(rep_dmax + r0, m);
-    } else if (r >= 0) {
-        atomicMax(rep_dmax + r, bits);
+        // per-replica maximum: one atomic per warp where the warp's particles share a replica
+        const unsigned bits = __float_as_uint(v);
+        most = max(most, bits);
+        const int r0 = __shfl_sync(0xffffffffu, r, 0);
+        if (__all_sync(0xffffffffu, r == r0)) {
+            const unsigned m = __reduce_max_sync(0xffffffffu, bits);
+            if ((threadIdx.x & 31) == 0 && r0 >= 0) atomicMax(rep_dmax + r0, m);
+        } else if (r >= 0) {
+            atomicMax(rep_dmax + r, bits);
+        }
     }
     __threadfence();   // the per-replica maxima are visible before this block's ticket
     __shared__ bool last_block;
-    const bool t0last = ell_block_max_last(bits, st, E_DMAX, E_TICKET_D);
+    const bool t0last = ell_block_max_last(most, st, E_DMAX, E_TICKET_D);
     if (threadIdx.x == 0) last_block = t0last;
     __syncthreads();
     if (last_block) {
@@ -831,20 +836,20 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
 
 static int batch_enqueue_step(pd_batch *b, float dt, cudaStream_t s, int cond) {
     const pd_md_state &S = b->state;
-    const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
+    const int blocks = batch_blocks(b), items = drift_items(blocks);
     cudaGraphConditionalHandle h = 0;
     if (cond) {
         cudaStreamCaptureStatus status;
         cudaGraph_t g = nullptr;
         PD_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr));
         PD_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-        k_batch_drift<true, true><<<blocks, B_THREADS, 0, s>>>(b->n, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy, S.fz,
+        k_batch_drift<true, true><<<(blocks + items - 1) / items, B_THREADS, 0, s>>>(b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy, S.fz,
                                                                S.inv_mass, dt, b->rep_of, b->reps, b->ref,
                                                                b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
                                                                b->rep_dmax, b->rep_flag, b->nrep,
                                                                b->st, h);
     } else {
-        k_batch_drift<true, false><<<blocks, B_THREADS, 0, s>>>(b->n, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy,
+        k_batch_drift<true, false><<<(blocks + items - 1) / items, B_THREADS, 0, s>>>(b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy,
                                                                 S.fz, S.inv_mass, dt, b->rep_of, b->reps, b->ref,
                                                                 b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
                                                                 b->rep_dmax, b->rep_flag, b->nrep,
@@ -997,8 +1002,8 @@ int pd_batch_set_lanes(pd_batch *b, int lanes) {
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t sp) {
     PD_CHECK(b && x && y && z, PD_EINVAL, "pd_batch_update: null argument");
     cudaStream_t s = (cudaStream_t)sp;
-    k_batch_drift<false, false><<<(b->n + B_THREADS - 1) / B_THREADS, B_THREADS, 0, s>>>(
-        b->n, const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
+    k_batch_drift<false, false><<<(batch_blocks(b) + drift_items(batch_blocks(b)) - 1) / drift_items(batch_blocks(b)), B_THREADS, 0, s>>>(
+        b->n, drift_items(batch_blocks(b)), const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, 0.f, b->rep_of, b->reps, b->ref, b->threshold, nullptr, nullptr, b->rep_dmax,
         b->rep_flag, b->nrep, b->st, 0);
     PD_LAUNCHED();

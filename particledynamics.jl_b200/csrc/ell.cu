@@ -1075,13 +1075,16 @@ __device__ __forceinline__ float wrap_half(float x, float L) {
 // Philox noise keyed on the particle and the device step), the pack of the new coordinates, the
 // displacement maximum and, in the last block, the rebuild decision.
 template <int D, int MODE, bool COND>
-__global__ void __launch_bounds__(ELL_THREADS) k_ell_drift(EllStepArgs a, long long *__restrict__ st,
+__global__ void __launch_bounds__(ELL_THREADS) k_ell_drift(EllStepArgs a, int items, long long *__restrict__ st,
                                                            cudaGraphConditionalHandle h) {
     if (st[E_ERROR] != 0) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = st[E_VALID] != 0;
     float disp = 0.f;
-    if (i < a.n && valid) {
+    // `items` rounds per block: the block's report of its maximum (a fence and an atomic whose answer it waits for)
+    // comes once for all of them
+    for (int it = 0; it < items && valid; ++it) {
+        const int i = (blockIdx.x * items + it) * ELL_THREADS + threadIdx.x;
+        if (i >= a.n) break;
         const float im = a.inv_mass ? a.inv_mass[i] : a.inv_mass_uniform;
         float p[3] = {a.x[i], a.y[i], D == 3 ? a.z[i] : 0.f};
         float v[3] = {a.vx[i], a.vy[i], D == 3 ? a.vz[i] : 0.f};
@@ -1150,7 +1153,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_drift(EllStepArgs a, long l
             a.vz[i] = v[2];
         }
         a.xq[a.pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);
-        disp = ell_displacement<D>(p, a.ref[i], a.L, true);
+        disp = fmaxf(disp, ell_displacement<D>(p, a.ref[i], a.L, true));
     }
     if (ell_block_max_last(__float_as_uint(disp), st, E_DMAX, E_TICKET_D)) {
         const float largest = __uint_as_float((unsigned)st[E_DMAX]);
@@ -1262,6 +1265,7 @@ static EllStepArgs ell_step_args(pd_ell_md *md, float dt, float gamma, float kT,
 static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int energy, cudaStream_t s, int cond) {
     pd_ell *e = md->e;
     const int blocks = (e->n + ELL_THREADS - 1) / ELL_THREADS;
+    const int items = drift_items(blocks);
     cudaGraphConditionalHandle h = 0;
     if (cond) {
         cudaStreamCaptureStatus status;
@@ -1269,7 +1273,7 @@ static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int e
         PD_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr));
         PD_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     }
-#define PD_ELL_DRIFT(DD, MM, CC) k_ell_drift<DD, MM, CC><<<blocks, ELL_THREADS, 0, s>>>(a, e->st, h)
+#define PD_ELL_DRIFT(DD, MM, CC) k_ell_drift<DD, MM, CC><<<(blocks + items - 1) / items, ELL_THREADS, 0, s>>>(a, items, e->st, h)
 #define PD_ELL_DRIFT_D(DD)                                                        \
     if (mode == 0) { if (cond) PD_ELL_DRIFT(DD, 0, true); else PD_ELL_DRIFT(DD, 0, false); } \
     else if (mode == 1) { if (cond) PD_ELL_DRIFT(DD, 1, true); else PD_ELL_DRIFT(DD, 1, false); } \

@@ -137,6 +137,10 @@ __device__ __forceinline__ int ell_reach(float rl, float L, int n) {
     return min(max(1, (int)ceilf(rl * (float)n / L - 1e-5f)), (n - 1) / 2);
 }
 
+// Rounds per block of a drift kernel of `blocks` blocks of 256 particles: one while the blocks are about a wave
+// (148 SMs, five blocks each), up to four beyond.
+inline int drift_items(int blocks) { return blocks <= 740 ? 1 : blocks <= 1480 ? 2 : 4; }
+
 // ------------------------------------------------------------------ host side of ell.cu
 
 // The rows of an ELL engine: entry t of cell-order position k at rows[k sk + t st], positions as entries.
