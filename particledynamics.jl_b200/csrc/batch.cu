@@ -30,6 +30,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
@@ -110,6 +111,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_drift(int n, int items, flo
                                                            unsigned *__restrict__ rep_dmax, int *__restrict__ rep_flag,
                                                            int nrep, long long *__restrict__ st,
                                                            cudaGraphConditionalHandle h) {
+    chain_begin();
     if (st[E_ERROR] != 0) {
         if (COND && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
         return;
@@ -170,6 +172,7 @@ __global__ void k_batch_bin(const float *__restrict__ x, const float *__restrict
                             int n, const int *__restrict__ rep_of, const BatchRep *__restrict__ reps,
                             const int *__restrict__ rep_flag, int *__restrict__ cell_of, int *__restrict__ cell_count,
                             const long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS, ROWS_BLOCKS) k_batch_rows(
     const BatchRep *__restrict__ reps, const int *__restrict__ rep_flag, const int *__restrict__ sorted,
     const int *__restrict__ cell_off, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts,
     float4 *__restrict__ ref, long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     extern __shared__ float4 batch_stage[];
     const int w = threadIdx.x >> 5;
@@ -233,6 +237,7 @@ template <bool REBUILD>
 __global__ void k_batch_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                              const float *__restrict__ q, const int *__restrict__ sorted, int n,
                              int *__restrict__ pos_of, float4 *__restrict__ xq, const long long *__restrict__ st) {
+    chain_begin();
     if (REBUILD ? !ell_requested(st) : st[E_VALID] == 0) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -277,6 +282,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
                                                            float *__restrict__ epot, float4 *__restrict__ fc,
                                                            BatchKick kick, long long *__restrict__ st, int advance,
                                                            const __grid_constant__ BatchCoul cp) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = tid / G, lane = tid % G;   // position in cell order
@@ -395,6 +401,7 @@ __global__ void __launch_bounds__(B_THREADS, 3) k_batch_pairs_seq(const float4 *
                                                                float *__restrict__ fz, float *__restrict__ epot,
                                                                float4 *__restrict__ fc, BatchKick kick,
                                                                long long *__restrict__ st, int advance) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     __shared__ int turn[B_THREADS / 32][32 * (SEQ_E + 1)];
     const int k = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
@@ -484,6 +491,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_finish(const float4 *__rest
                                                             float *__restrict__ fx, float *__restrict__ fy,
                                                             float *__restrict__ fz, float *__restrict__ epot,
                                                             BatchKick kick, long long *__restrict__ st, int advance) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
@@ -645,20 +653,20 @@ static int batch_blocks(const pd_batch *b) { return (b->n + B_THREADS - 1) / B_T
 
 static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
-    k_batch_bin<<<blocks, B_THREADS, 0, s>>>(x, y, z, b->n, b->rep_of, b->reps, b->rep_flag, b->cell_of,
+    launch_chained(k_batch_bin, blocks, B_THREADS, 0, s, x, y, z, b->n, b->rep_of, b->reps, b->rep_flag, b->cell_of,
                                              b->cell_count, b->st);
     PD_LAUNCHED();
     int rc;
     if ((rc = ell_sort_launch(b->cell_of, b->n, b->ncell, b->cell_count, b->cell_off, b->scan_part, b->sorted, b->tmp,
                               b->st, s)))
         return rc;
-    k_batch_pack<true><<<blocks, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
+    launch_chained(k_batch_pack<true>, blocks, B_THREADS, 0, s, x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
     PD_LAUNCHED();
     // few cells: several warps per cell, until the chip has about 16 warps per SM
     int nsplit = 1;
     while (nsplit < 8 && (long long)b->ncell * nsplit < 148 * 16) nsplit *= 2;
     const int grid = (int)(((long long)b->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
-    k_batch_rows<<<grid, 32 * ROWS_WARPS, sizeof(float4) * ROWS_WARPS * ROWS_CAP, s>>>(
+    launch_chained(k_batch_rows, grid, 32 * ROWS_WARPS, sizeof(float4) * ROWS_WARPS * ROWS_CAP, s, 
         b->xq, b->ncell, nsplit, b->cell_rep, b->reps, b->rep_flag, b->sorted, b->cell_off, b->rl2, b->cap, b->rows,
         b->counts, b->ref, b->st);
     PD_LAUNCHED();
@@ -679,7 +687,7 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
     if constexpr (!COUL) {
         if (G == 1) {
 #define PD_BS(EE, SS)                                                                                               \
-    k_batch_pairs_seq<EE, SS><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->cap, b->rows, b->counts,     \
+    launch_chained(k_batch_pairs_seq<EE, SS>, blocks, B_THREADS, 0, s, b->xq, b->n, b->cap, b->rows, b->counts,     \
                    b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, b->fc, kick, b->st, advance)
             if (slot) {
                 if (energy) PD_BS(true, true);
@@ -693,7 +701,7 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
         }
     }
 #define PD_BP2(GG, EE, SS)                                                                                            \
-    k_batch_pairs<GG, EE, COUL, SS, NP><<<blocks, B_THREADS, 0, s>>>(b->xq, b->n, b->cap, b->rows, b->counts,         \
+    launch_chained(k_batch_pairs<GG, EE, COUL, SS, NP>, blocks, B_THREADS, 0, s, b->xq, b->n, b->cap, b->rows, b->counts,         \
                                                                      b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, \
                                                                      b->fc, kick, b->st, advance, b->cp)
 #define PD_BP(GG)                                                                                                     \
@@ -790,7 +798,7 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
     if (!b->coul) {
         const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
         if (!packed) {
-            k_batch_pack<false><<<blocks, B_THREADS, 0, s>>>(x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
+            launch_chained(k_batch_pack<false>, blocks, B_THREADS, 0, s, x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
             PD_LAUNCHED();
         }
         const bool slot = b->n >= BATCH_SLOT_MIN;
@@ -798,10 +806,10 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
         PD_LAUNCHED();
         if (!slot) return PD_OK;
         if (energy)
-            k_batch_finish<true><<<blocks, B_THREADS, 0, s>>>(b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
+            launch_chained(k_batch_finish<true>, blocks, B_THREADS, 0, s, b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
                                                               advance);
         else
-            k_batch_finish<false><<<blocks, B_THREADS, 0, s>>>(b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
+            launch_chained(k_batch_finish<false>, blocks, B_THREADS, 0, s, b->fc, b->pos_of, b->n, fx, fy, fz, epot, kick, b->st,
                                                                advance);
         PD_LAUNCHED();
         return PD_OK;
@@ -843,13 +851,13 @@ static int batch_enqueue_step(pd_batch *b, float dt, cudaStream_t s, int cond) {
         cudaGraph_t g = nullptr;
         PD_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr));
         PD_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-        k_batch_drift<true, true><<<(blocks + items - 1) / items, B_THREADS, 0, s>>>(b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy, S.fz,
+        launch_chained(k_batch_drift<true, true>, (blocks + items - 1) / items, B_THREADS, 0, s, b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy, S.fz,
                                                                S.inv_mass, dt, b->rep_of, b->reps, b->ref,
                                                                b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
                                                                b->rep_dmax, b->rep_flag, b->nrep,
                                                                b->st, h);
     } else {
-        k_batch_drift<true, false><<<(blocks + items - 1) / items, B_THREADS, 0, s>>>(b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy,
+        launch_chained(k_batch_drift<true, false>, (blocks + items - 1) / items, B_THREADS, 0, s, b->n, items, S.x, S.y, S.z, S.vx, S.vy, S.vz, S.fx, S.fy,
                                                                 S.fz, S.inv_mass, dt, b->rep_of, b->reps, b->ref,
                                                                 b->threshold, b->coul ? nullptr : b->pos_of, b->xq,
                                                                 b->rep_dmax, b->rep_flag, b->nrep,
@@ -1002,7 +1010,7 @@ int pd_batch_set_lanes(pd_batch *b, int lanes) {
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t sp) {
     PD_CHECK(b && x && y && z, PD_EINVAL, "pd_batch_update: null argument");
     cudaStream_t s = (cudaStream_t)sp;
-    k_batch_drift<false, false><<<(batch_blocks(b) + drift_items(batch_blocks(b)) - 1) / drift_items(batch_blocks(b)), B_THREADS, 0, s>>>(
+    launch_chained(k_batch_drift<false, false>, (batch_blocks(b) + drift_items(batch_blocks(b)) - 1) / drift_items(batch_blocks(b)), B_THREADS, 0, s,
         b->n, drift_items(batch_blocks(b)), const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, 0.f, b->rep_of, b->reps, b->ref, b->threshold, nullptr, nullptr, b->rep_dmax,
         b->rep_flag, b->nrep, b->st, 0);

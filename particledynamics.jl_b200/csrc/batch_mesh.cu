@@ -33,6 +33,7 @@ __global__ void k_bmesh_pack(const float *__restrict__ x, const float *__restric
                              const float *__restrict__ q, const int *__restrict__ sorted,
                              const int *__restrict__ slot_src, int nslots, float4 *__restrict__ xq,
                              float4 *__restrict__ mq, int *__restrict__ mid, const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslots) return;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bspread(const fl
                                                                       const BMeshRep *__restrict__ reps,
                                                                       float *__restrict__ gridA,
                                                                       const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     const int c = blockIdx.x;
     const BMeshRep R = reps[chunk_rep[c]];
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const fl
                                                                       float *__restrict__ epot, BMeshKick kick,
                                                                       float half_c_self,
                                                                       const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     constexpr int NT = TP * CH;
     const int c = blockIdx.x;
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bgather(const fl
 int bmesh_pack_launch(const BMeshView &v, const float *x, const float *y, const float *z, const float *q,
                       const int *sorted, float4 *xq, const long long *st, cudaStream_t s) {
     const int nslots = v.nchunk * v.chunk;
-    k_bmesh_pack<<<(nslots + 255) / 256, 256, 0, s>>>(x, y, z, q, sorted, v.slot_src, nslots, xq, v.mq, v.mid, st);
+    launch_chained(k_bmesh_pack, (nslots + 255) / 256, 256, 0, s, x, y, z, q, sorted, v.slot_src, nslots, xq, v.mq, v.mid, st);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -239,11 +242,11 @@ int bmesh_pack_launch(const BMeshView &v, const float *x, const float *y, const 
 template <int P>
 static void spread_p(const BMeshView &v, const long long *st, cudaStream_t s) {
     if (v.chunk == 32)
-        k_bspread<P, 32, 2><<<v.nchunk, 64, 0, s>>>(v.mq, v.chunk_rep, v.reps, v.gridA, st);
+        launch_chained(k_bspread<P, 32, 2>, v.nchunk, 64, 0, s, v.mq, v.chunk_rep, v.reps, v.gridA, st);
     else if (v.tpi == 4)
-        k_bspread<P, 64, 4><<<v.nchunk, 256, 0, s>>>(v.mq, v.chunk_rep, v.reps, v.gridA, st);
+        launch_chained(k_bspread<P, 64, 4>, v.nchunk, 256, 0, s, v.mq, v.chunk_rep, v.reps, v.gridA, st);
     else
-        k_bspread<P, 64, 2><<<v.nchunk, 128, 0, s>>>(v.mq, v.chunk_rep, v.reps, v.gridA, st);
+        launch_chained(k_bspread<P, 64, 2>, v.nchunk, 128, 0, s, v.mq, v.chunk_rep, v.reps, v.gridA, st);
 }
 
 int bmesh_spread_launch(const BMeshView &v, const long long *st, cudaStream_t s) {
@@ -269,10 +272,10 @@ template <int P, int CH, int TP>
 static void gather_pc(const BMeshView &v, float *fx, float *fy, float *fz, float *epot, int energy,
                       const BMeshKick &kick, float half_c_self, const long long *st, cudaStream_t s) {
     if (energy)
-        k_bgather<P, CH, TP, true><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
+        launch_chained(k_bgather<P, CH, TP, true>, v.nchunk, TP * CH, 0, s, v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
                                                                 fz, epot, kick, half_c_self, st);
     else
-        k_bgather<P, CH, TP, false><<<v.nchunk, TP * CH, 0, s>>>(v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
+        launch_chained(k_bgather<P, CH, TP, false>, v.nchunk, TP * CH, 0, s, v.mq, v.mid, v.slot_src, v.fc, v.chunk_rep, v.reps, v.gridB, fx, fy,
                                                                  fz, epot, kick, half_c_self, st);
 }
 

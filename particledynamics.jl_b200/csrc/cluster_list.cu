@@ -18,6 +18,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -574,6 +575,7 @@ __global__ void __launch_bounds__(256) k_prune(const float4 *__restrict__ xq, co
                                                const int *__restrict__ xid,
                                                const unsigned long long *__restrict__ xmask,
                                                int *__restrict__ wxid) {
+    chain_begin();
     if (gated && counts[W_PRUNE] == 0) return;
     if (counts[W_ERR] != 0) return;
     const int S = blockIdx.x;
@@ -794,6 +796,7 @@ __global__ void __launch_bounds__(256) k_displacement(const float *__restrict__ 
                                                       const float4 *__restrict__ rb, const float4 *__restrict__ rp,
                                                       float Lx, float Ly, float Lz, float tb2, float tp2,
                                                       int *__restrict__ counts) {
+    chain_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     float ra = 0.f, rbv = 0.f;
     if (i < n) {
@@ -835,6 +838,7 @@ __global__ void __launch_bounds__(256) k_displacement(const float *__restrict__ 
 
 // Device build/prune decision (_decide_kernel!, Engine.jl:301-324).
 __global__ void k_decide(int *__restrict__ counts, int nstlist, int nstprune) {
+    chain_begin();
     float anyr = __int_as_float(counts[W_FLAG_ANY]);
     float br = __int_as_float(counts[W_FLAG_BUILD]);
     bool build, prune;
@@ -868,6 +872,7 @@ __global__ void k_pack(const int *__restrict__ perm, int nslot, const float *__r
                        const float *__restrict__ y, const float *__restrict__ z, const float *__restrict__ q,
                        const int *__restrict__ type, float Lx, float Ly, float Lz, float4 *__restrict__ xq,
                        int *__restrict__ ts) {
+    chain_begin();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslot) return;
     int i = perm[s];
@@ -1069,7 +1074,7 @@ int cluster_build_launch(pd_cluster *c, const float *x, const float *y, const fl
 int cluster_prune_launch(pd_cluster *c, int conditional, cudaStream_t s) {
     const double rp = c->p.rmax + c->p.prune_buffer;
     const float rp2 = (float)rp * (float)rp;
-    k_prune<<<c->nsmax, 256, 0, s>>>(c->xq, c->perm, c->scio, c->cjo, c->cjw, c->nw, c->ref_prune, c->L[0], c->L[1],
+    launch_chained(k_prune, c->nsmax, 256, 0, s, c->xq, c->perm, c->scio, c->cjo, c->cjw, c->nw, c->ref_prune, c->L[0], c->L[1],
                                      c->L[2], rp2, (float)c->p.prune_buffer, c->counts, conditional ? 1 : 0,
                                      c->nexc > 0 ? c->xid : nullptr, c->xmask, c->nexc > 0 ? c->wxid : nullptr);
     PD_LAUNCHED();
@@ -1078,10 +1083,10 @@ int cluster_prune_launch(pd_cluster *c, int conditional, cudaStream_t s) {
 
 int cluster_decide_launch(pd_cluster *c, const float *x, const float *y, const float *z, int fixed, cudaStream_t s) {
     const float hb = (float)(0.5 * c->p.skin), hp = (float)(0.5 * c->p.prune_buffer);
-    k_displacement<<<(c->n + 255) / 256, 256, 0, s>>>(x, y, z, c->n, c->ref_build, c->ref_prune, c->L[0], c->L[1],
+    launch_chained(k_displacement, (c->n + 255) / 256, 256, 0, s, x, y, z, c->n, c->ref_build, c->ref_prune, c->L[0], c->L[1],
                                                       c->L[2], hb * hb, hp * hp, c->counts);
     PD_LAUNCHED();
-    k_decide<<<1, 1, 0, s>>>(c->counts, fixed ? c->p.nstlist : 0, c->p.nstprune);
+    launch_chained(k_decide, 1, 1, 0, s, c->counts, fixed ? c->p.nstlist : 0, c->p.nstprune);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -1368,7 +1373,7 @@ int pd_cluster_build(pd_cluster *c, const float *x, const float *y, const float 
 int pd_cluster_pack(pd_cluster *c, const float *x, const float *y, const float *z, const float *q, const int *type,
                     pd_stream_t s) {
     PD_CHECK(c && x && y && z, PD_EINVAL, "pd_cluster_pack: null argument");
-    k_pack<<<(c->nslot + 255) / 256, 256, 0, (cudaStream_t)s>>>(c->perm, c->nslot, x, y, z, q, type, c->L[0], c->L[1],
+    launch_chained(k_pack, (c->nslot + 255) / 256, 256, 0, (cudaStream_t)s, c->perm, c->nslot, x, y, z, q, type, c->L[0], c->L[1],
                                                                   c->L[2], c->xq, c->ts);
     PD_LAUNCHED();
     return PD_OK;

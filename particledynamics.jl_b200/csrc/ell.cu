@@ -23,6 +23,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_decide(const float *__restr
                                                             const float *__restrict__ z, const float4 *__restrict__ ref,
                                                             int n, float Lx, float Ly, float Lz, float threshold,
                                                             long long *__restrict__ st) {
+    chain_begin();
     if (st[E_ERROR] != 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const float L[3] = {Lx, Ly, Lz};
@@ -60,6 +62,7 @@ template <int D>
 __global__ void k_ell_bin(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, int n,
                           float Lx, float Ly, float Lz, int nx, int ny, int nz, int *__restrict__ cell_of,
                           int *__restrict__ cell_count, const long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -87,6 +90,7 @@ __global__ void k_ell_bin(const float *__restrict__ x, const float *__restrict__
 // to SCAN_ONE_BLOCK cells (two launches cost more than a second chunk there).
 __global__ void __launch_bounds__(1024) k_ell_scan(int *__restrict__ cell_count, int *__restrict__ cell_off,
                                                    int ncell, const long long *__restrict__ st) {
+    chain_begin();
     if (st && !ell_requested(st)) return;
     __shared__ int sb[ELL_SCAN_CHUNK + ELL_SCAN_CHUNK / 32];
     __shared__ int warp_tot[32];
@@ -172,6 +176,7 @@ __device__ __forceinline__ int block_exclusive(int v, int *sh, int &total) {   /
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restrict__ cell_count, int ncell,
                                                             int *__restrict__ part, int ntile,
                                                             const long long *__restrict__ st) {
+    chain_begin();
     if (st && !ell_requested(st)) return;
     __shared__ int sh[SCAN_THREADS / 32];
     __shared__ bool last;
@@ -210,6 +215,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int *__restric
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(int *__restrict__ cell_count, int *__restrict__ cell_off,
                                                              int ncell, const int *__restrict__ part, int ntile,
                                                              const long long *__restrict__ st) {
+    chain_begin();
     if (st && !ell_requested(st)) return;
     __shared__ int sh[SCAN_THREADS / 32];
     int at = part[blockIdx.x];
@@ -231,6 +237,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(int *__restrict__ c
 // _kernel_scatter_by_cell! (DenseNeighborCUDA.jl:61-72): atomic cursors per cell.
 __global__ void k_ell_scatter(const int *__restrict__ cell_of, int n, const int *__restrict__ cell_off,
                               int *__restrict__ cursor, int *__restrict__ sorted, const long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -243,6 +250,7 @@ __global__ void k_ell_scatter(const int *__restrict__ cell_of, int n, const int 
 // The cell's scatter cursor is reset to zero for the next build's histogram.
 __global__ void k_ell_cellsort(const int *__restrict__ cell_off, int ncell, int *__restrict__ sorted,
                                int *__restrict__ tmp, int *__restrict__ cell_count, const long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (c >= ncell) return;   // uniform per warp
@@ -271,6 +279,7 @@ __global__ void k_ell_cellsort(const int *__restrict__ cell_off, int ncell, int 
 // 72 us for the 506 944 cells of a million 2D disks).
 __global__ void k_ell_cellsort_sparse(const int *__restrict__ cell_off, int ncell, int *__restrict__ sorted,
                                       int *__restrict__ cell_count, const long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncell) return;
@@ -294,6 +303,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_rows(
     const float4 *__restrict__ xq, int n, const int *__restrict__ sorted, const int *__restrict__ cell_of,
     const int *__restrict__ cell_off, float Lx, float Ly, float Lz, int nx, int ny, int nz, float rl2, int cap,
     int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref, long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int found = 0;
@@ -362,6 +372,7 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS, ROWS_BLOCKS) k_ell_rows_cells
     const float4 *__restrict__ xq, const int *__restrict__ sorted, const int *__restrict__ cell_off, RowGrid g,
     int nsplit, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts, float4 *__restrict__ ref,
     long long *__restrict__ st) {
+    chain_begin();
     if (!ell_requested(st)) return;
     extern __shared__ float4 ell_stage[];
     const int w = threadIdx.x >> 5;
@@ -379,6 +390,7 @@ template <int D, bool REBUILD>
 __global__ void k_ell_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                            const int *__restrict__ sorted, int n, int *__restrict__ pos_of, float4 *__restrict__ xq,
                            const long long *__restrict__ st) {
+    chain_begin();
     if (REBUILD && !ell_requested(st)) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -446,6 +458,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
                                                            float *__restrict__ fz, float *__restrict__ epot,
                                                            float *__restrict__ vir, float4 *__restrict__ fc,
                                                            EllKick kick, long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;   // _device_if_valid!: no valid list, no forces
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = tid / G, lane = tid % G;
@@ -533,6 +546,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_finish(const float4 *__rest
                                                             float *__restrict__ fx, float *__restrict__ fy,
                                                             float *__restrict__ fz, EllKick kick,
                                                             long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
@@ -611,13 +625,13 @@ static size_t scan_part_len(int ncell) { return (size_t)(ncell + SCAN_TILE - 1) 
 
 int cell_scan_launch(int *cell_count, int *cell_off, int ncell, int *part, const long long *st, cudaStream_t s) {
     if (ncell <= SCAN_ONE_BLOCK) {
-        k_ell_scan<<<1, 1024, 0, s>>>(cell_count, cell_off, ncell, st);
+        launch_chained(k_ell_scan, 1, 1024, 0, s, cell_count, cell_off, ncell, st);
         PD_LAUNCHED();
     } else {
         const int ntile = (ncell + SCAN_TILE - 1) / SCAN_TILE;
-        k_scan_sums<<<ntile, SCAN_THREADS, 0, s>>>(cell_count, ncell, part, ntile, st);
+        launch_chained(k_scan_sums, ntile, SCAN_THREADS, 0, s, cell_count, ncell, part, ntile, st);
         PD_LAUNCHED();
-        k_scan_apply<<<ntile, SCAN_THREADS, 0, s>>>(cell_count, cell_off, ncell, part, ntile, st);
+        launch_chained(k_scan_apply, ntile, SCAN_THREADS, 0, s, cell_count, cell_off, ncell, part, ntile, st);
         PD_LAUNCHED();
     }
     return PD_OK;
@@ -631,13 +645,13 @@ int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *
     const int blocks = (n + ELL_THREADS - 1) / ELL_THREADS;
     const int rc = cell_scan_launch(cell_count, cell_off, ncell, part, st, s);
     if (rc) return rc;
-    k_ell_scatter<<<blocks, ELL_THREADS, 0, s>>>(cell_of, n, cell_off, cell_count, sorted, st);
+    launch_chained(k_ell_scatter, blocks, ELL_THREADS, 0, s, cell_of, n, cell_off, cell_count, sorted, st);
     PD_LAUNCHED();
     if (n >= ROWS_MIN_PER_CELL * (long long)ncell)
-        k_ell_cellsort<<<(int)(((long long)ncell * 32 + 255) / 256), 256, 0, s>>>(cell_off, ncell, sorted, tmp,
+        launch_chained(k_ell_cellsort, (int)(((long long)ncell * 32 + 255) / 256), 256, 0, s, cell_off, ncell, sorted, tmp,
                                                                                   cell_count, st);
     else
-        k_ell_cellsort_sparse<<<(ncell + 127) / 128, 128, 0, s>>>(cell_off, ncell, sorted, cell_count, st);
+        launch_chained(k_ell_cellsort_sparse, (ncell + 127) / 128, 128, 0, s, cell_off, ncell, sorted, cell_count, st);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -671,10 +685,10 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
     int rc;
     if (!e->allpairs) {
         if (e->dim == 3)
-            k_ell_bin<3><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
+            launch_chained(k_ell_bin<3>, blocks, ELL_THREADS, 0, s, x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
                                                         e->cell_count, e->st);
         else
-            k_ell_bin<2><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
+            launch_chained(k_ell_bin<2>, blocks, ELL_THREADS, 0, s, x, y, z, n, Lx, Ly, Lz, e->nx, e->ny, e->nz, e->cell_of,
                                                         e->cell_count, e->st);
         PD_LAUNCHED();
         if ((rc = ell_sort_launch(e->cell_of, n, e->ncell, e->cell_count, e->cell_off, e->scan_part, e->sorted, e->tmp,
@@ -682,12 +696,12 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
             return rc;
     }
     if (e->dim == 3)
-        k_ell_pack<3, true><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
+        launch_chained(k_ell_pack<3, true>, blocks, ELL_THREADS, 0, s, x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
     else
-        k_ell_pack<2, true><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
+        launch_chained(k_ell_pack<2, true>, blocks, ELL_THREADS, 0, s, x, y, z, e->sorted, n, e->pos_of, e->xq, e->st);
     PD_LAUNCHED();
 #define PD_ELL_ROWS(DD, AP)                                                                                          \
-    k_ell_rows<DD, AP><<<blocks, ELL_THREADS, 0, s>>>(e->xq, n, e->sorted, e->cell_of, e->cell_off, Lx, Ly, Lz, e->nx, \
+    launch_chained(k_ell_rows<DD, AP>, blocks, ELL_THREADS, 0, s, e->xq, n, e->sorted, e->cell_of, e->cell_off, Lx, Ly, Lz, e->nx, \
                                                       e->ny, e->nz, e->rl2, e->cap, e->rows, e->counts, e->ref, e->st)
     if (e->dense) {
         const RowGrid g{{Lx, Ly, Lz}, e->nx, e->ny, e->nz, 0};
@@ -697,10 +711,10 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
         const int grid = (int)(((long long)e->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
         const size_t shm = sizeof(float4) * ROWS_WARPS * ROWS_CAP;
         if (e->dim == 3)
-            k_ell_rows_cells<3><<<grid, 32 * ROWS_WARPS, shm, s>>>(e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
+            launch_chained(k_ell_rows_cells<3>, grid, 32 * ROWS_WARPS, shm, s, e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
                                                                    e->cap, e->rows, e->counts, e->ref, e->st);
         else
-            k_ell_rows_cells<2><<<grid, 32 * ROWS_WARPS, shm, s>>>(e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
+            launch_chained(k_ell_rows_cells<2>, grid, 32 * ROWS_WARPS, shm, s, e->xq, e->sorted, e->cell_off, g, nsplit, e->rl2,
                                                                    e->cap, e->rows, e->counts, e->ref, e->st);
     } else if (e->dim == 3) {
         if (e->allpairs) PD_ELL_ROWS(3, true);
@@ -717,10 +731,10 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
 int ell_decide_launch(pd_ell *e, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int blocks = (e->n + ELL_THREADS - 1) / ELL_THREADS;
     if (e->dim == 3)
-        k_ell_decide<3><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->ref, e->n, e->L[0], e->L[1], e->L[2], e->threshold,
+        launch_chained(k_ell_decide<3>, blocks, ELL_THREADS, 0, s, x, y, z, e->ref, e->n, e->L[0], e->L[1], e->L[2], e->threshold,
                                                        e->st);
     else
-        k_ell_decide<2><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->ref, e->n, e->L[0], e->L[1], e->L[2], e->threshold,
+        launch_chained(k_ell_decide<2>, blocks, ELL_THREADS, 0, s, x, y, z, e->ref, e->n, e->L[0], e->L[1], e->L[2], e->threshold,
                                                        e->st);
     PD_LAUNCHED();
     return PD_OK;
@@ -733,7 +747,7 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
     const EllModel m = ell_model(e);
     const EllRowsView v = ell_rows_view(e);
 #define PD_ELL_PAIRS(EN, OO)                                                                                      \
-    k_ell_pairs<D, G, UNIT, EN, OO><<<blocks, ELL_THREADS, 0, s>>>(e->xq, e->n, v.rows, v.counts, v.sorted, v.sk, v.st, \
+    launch_chained(k_ell_pairs<D, G, UNIT, EN, OO>, blocks, ELL_THREADS, 0, s, e->xq, e->n, v.rows, v.counts, v.sorted, v.sk, v.st, \
                                                              e->L[0], e->L[1], e->L[2], m, fx, fy, fz, epot, vir, \
                                                              e->fc, kick, e->st)
     if (energy) {
@@ -746,8 +760,8 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
         PD_ELL_PAIRS(false, OUT_SLOT);
         const int fb = (e->n + ELL_THREADS - 1) / ELL_THREADS;
         count_launch();
-        if (kick.vx) k_ell_finish<D, true><<<fb, ELL_THREADS, 0, s>>>(e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
-        else k_ell_finish<D, false><<<fb, ELL_THREADS, 0, s>>>(e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
+        if (kick.vx) launch_chained(k_ell_finish<D, true>, fb, ELL_THREADS, 0, s, e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
+        else launch_chained(k_ell_finish<D, false>, fb, ELL_THREADS, 0, s, e->fc, e->pos_of, e->n, fx, fy, fz, kick, e->st);
     }
 #undef PD_ELL_PAIRS
 }
@@ -791,9 +805,9 @@ int ell_pairs_launch(pd_ell *e, float *fx, float *fy, float *fz, float *epot, fl
 int ell_pack_launch(pd_ell *e, const float *x, const float *y, const float *z, cudaStream_t s) {
     const int blocks = (e->n + ELL_THREADS - 1) / ELL_THREADS;
     if (e->dim == 3)
-        k_ell_pack<3, false><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
+        launch_chained(k_ell_pack<3, false>, blocks, ELL_THREADS, 0, s, x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
     else
-        k_ell_pack<2, false><<<blocks, ELL_THREADS, 0, s>>>(x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
+        launch_chained(k_ell_pack<2, false>, blocks, ELL_THREADS, 0, s, x, y, z, e->sorted, e->n, e->pos_of, e->xq, e->st);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -1077,6 +1091,7 @@ __device__ __forceinline__ float wrap_half(float x, float L) {
 template <int D, int MODE, bool COND>
 __global__ void __launch_bounds__(ELL_THREADS) k_ell_drift(EllStepArgs a, int items, long long *__restrict__ st,
                                                            cudaGraphConditionalHandle h) {
+    chain_begin();
     if (st[E_ERROR] != 0) return;
     const bool valid = st[E_VALID] != 0;
     float disp = 0.f;
@@ -1273,7 +1288,7 @@ static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int e
         PD_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr));
         PD_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     }
-#define PD_ELL_DRIFT(DD, MM, CC) k_ell_drift<DD, MM, CC><<<(blocks + items - 1) / items, ELL_THREADS, 0, s>>>(a, items, e->st, h)
+#define PD_ELL_DRIFT(DD, MM, CC) launch_chained(k_ell_drift<DD, MM, CC>, (blocks + items - 1) / items, ELL_THREADS, 0, s, a, items, e->st, h)
 #define PD_ELL_DRIFT_D(DD)                                                        \
     if (mode == 0) { if (cond) PD_ELL_DRIFT(DD, 0, true); else PD_ELL_DRIFT(DD, 0, false); } \
     else if (mode == 1) { if (cond) PD_ELL_DRIFT(DD, 1, true); else PD_ELL_DRIFT(DD, 1, false); } \

@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
@@ -75,6 +76,7 @@ __device__ __forceinline__ float mic_d(float d, float L) {
 __global__ void k_desc_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                             const float *__restrict__ q, const int *__restrict__ type,
                             const int *__restrict__ sorted, int n, float4 *__restrict__ xq) {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = sorted[k];
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(DESC_THREADS, 4) k_descriptors(const float4 *_
                                                               EllRowsView rv, DescParams p,
                                                               __nv_bfloat16 *__restrict__ X, float4 *__restrict__ V,
                                                               float4 *__restrict__ Vb) {
+    chain_begin();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int pos = tid / G, g = tid % G;   // cell-order position
     const bool live = pos < n;   // whole groups are live or not (G divides the warp)
@@ -257,14 +260,14 @@ static int descriptors_launch(pd_learned *h, const float *x, const float *y, con
     if ((rc = pd_ell_update(h->ell, x, y, z, (pd_stream_t)s))) return rc;
     const EllRowsView rv = ell_rows_view(h->ell);
     const DescParams d = desc_params(h);
-    k_desc_pack<<<(h->n + 255) / 256, 256, 0, s>>>(x, y, z, q, type, rv.sorted, h->n, h->xq);
+    launch_chained(k_desc_pack, (h->n + 255) / 256, 256, 0, s, x, y, z, q, type, rv.sorted, h->n, h->xq);
     PD_LAUNCHED();
     constexpr int G = DESC_LANES;
     const int blocks = (int)(((long long)h->n * G + DESC_THREADS - 1) / DESC_THREADS);
     if (Vb)
-        k_descriptors<true, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rv, d, X, V, Vb);
+        launch_chained(k_descriptors<true, G>, blocks, DESC_THREADS, 0, s, h->xq, h->n, rv, d, X, V, Vb);
     else
-        k_descriptors<false, G><<<blocks, DESC_THREADS, 0, s>>>(h->xq, h->n, rv, d, X, V, Vb);
+        launch_chained(k_descriptors<false, G>, blocks, DESC_THREADS, 0, s, h->xq, h->n, rv, d, X, V, Vb);
     PD_LAUNCHED();
     return PD_OK;
 }

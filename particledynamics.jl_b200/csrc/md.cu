@@ -18,6 +18,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(256) k_kick_drift(int n, float *__restrict__ x
                                                     const float4 *__restrict__ rp, float tb2, float tp2,
                                                     int *__restrict__ counts, int nstlist, int nstprune,
                                                     cudaGraphConditionalHandle hb) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float ra = 0.f, rbv = 0.f;
     if (i < n) {
@@ -173,6 +175,7 @@ __global__ void k_scatter_kick(const int *__restrict__ perm, int nslot, const in
                                float *__restrict__ fz, float *__restrict__ vx, float *__restrict__ vy,
                                float *__restrict__ vz, const float *__restrict__ inv_mass, float inv_mass_uniform,
                                float half_dt, float *__restrict__ epot, float *__restrict__ vir6) {
+    chain_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nslot || s >= counts[W_NS] * SUPER) return;
     const int i = perm[s];
@@ -267,11 +270,11 @@ static int enqueue_forces(pd_md *md, int energy, float half_dt, cudaStream_t s) 
     } else {
         const int blocks = (c->nslot + 255) / 256;
         if (energy)
-            k_scatter_kick<true><<<blocks, 256, 0, s>>>(c->perm, c->nslot, c->counts, c->fc, c->vc, c->xq,
+            launch_chained(k_scatter_kick<true>, blocks, 256, 0, s, c->perm, c->nslot, c->counts, c->fc, c->vc, c->xq,
                                                         md->half_c_self, st.fx, st.fy, st.fz, st.vx, st.vy, st.vz,
                                                         st.inv_mass, st.inv_mass_uniform, half_dt, st.epot, st.vir6);
         else
-            k_scatter_kick<false><<<blocks, 256, 0, s>>>(c->perm, c->nslot, c->counts, c->fc, c->vc, c->xq,
+            launch_chained(k_scatter_kick<false>, blocks, 256, 0, s, c->perm, c->nslot, c->counts, c->fc, c->vc, c->xq,
                                                          md->half_c_self, st.fx, st.fy, st.fz, st.vx, st.vy, st.vz,
                                                          st.inv_mass, st.inv_mass_uniform, half_dt, st.epot,
                                                          st.vir6);
@@ -308,7 +311,7 @@ static int enqueue_step(pd_md *md, float dt, int energy, cudaStream_t s, int con
         PD_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &g, nullptr, nullptr));
         cudaGraphConditionalHandle hbuild;
         PD_CUDA(cudaGraphConditionalHandleCreate(&hbuild, g, 0, cudaGraphCondAssignDefault));
-        k_kick_drift<true><<<kb, 256, 0, s>>>(st.n, st.x, st.y, st.z, st.vx, st.vy, st.vz, st.fx, st.fy, st.fz,
+        launch_chained(k_kick_drift<true>, kb, 256, 0, s, st.n, st.x, st.y, st.z, st.vx, st.vy, st.vz, st.fx, st.fy, st.fz,
                                               st.inv_mass, st.inv_mass_uniform, dt, md->L[0], md->L[1], md->L[2], q,
                                               c->slot_of, c->xq, c->ref_build, c->ref_prune, hb * hb, hp * hp,
                                               c->counts, c->p.nstlist, c->p.nstprune, hbuild);
@@ -319,7 +322,7 @@ static int enqueue_step(pd_md *md, float dt, int energy, cudaStream_t s, int con
              })))
             return rc;
     } else {
-        k_kick_drift<false><<<kb, 256, 0, s>>>(st.n, st.x, st.y, st.z, st.vx, st.vy, st.vz, st.fx, st.fy, st.fz,
+        launch_chained(k_kick_drift<false>, kb, 256, 0, s, st.n, st.x, st.y, st.z, st.vx, st.vy, st.vz, st.fx, st.fy, st.fz,
                                                st.inv_mass, st.inv_mass_uniform, dt, md->L[0], md->L[1], md->L[2], q,
                                                c->slot_of, c->xq, c->ref_build, c->ref_prune, hb * hb, hp * hp,
                                                c->counts, c->p.nstlist, c->p.nstprune, 0);

@@ -18,6 +18,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
@@ -144,6 +145,7 @@ __global__ void k_unit_node(float *grid) { grid[0] = 1.f; }
 __global__ void k_pack_order(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                              const float *__restrict__ q, const int *__restrict__ order, int n, int ntot,
                              float4 *__restrict__ out) {
+    chain_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntot) return;
     if (t < n) {
@@ -161,6 +163,7 @@ __global__ void k_pack_order(const float *__restrict__ x, const float *__restric
 __global__ void k_order_bin(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, int n,
                             float Lx, float Ly, float Lz, int ncx, int ncy, int nzb, int *__restrict__ bin,
                             int *__restrict__ rank, int *__restrict__ count) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     auto slot = [](float v, float L, int nb) {
@@ -181,12 +184,14 @@ __global__ void k_order_bin(const float *__restrict__ x, const float *__restrict
 
 __global__ void k_order_scatter(const int *__restrict__ bin, const int *__restrict__ rank, const int *__restrict__ off,
                                 int n, int *__restrict__ order) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) order[off[bin[i]] + rank[i]] = i;
 }
 
 // Global virial plus background (_store_global_virial_kernel!, Solver.jl:382-388).
 __global__ void k_store_virial(float *vg, const double *acc, double ubg) {
+    chain_begin();
     const int i = threadIdx.x;
     if (i < 6) vg[i] = (float)(acc[i + 1] + (i < 3 ? ubg : 0.0));
 }
@@ -575,7 +580,7 @@ int mesh_transform_packed(pd_mesh *m, const float4 *xq, int nchunks, const int *
 
 int mesh_store_virial(pd_mesh *m, float *vglobal6, cudaStream_t s) {
     if (!vglobal6) return PD_OK;
-    k_store_virial<<<1, 32, 0, s>>>(vglobal6, m->acc, m->ubg);
+    launch_chained(k_store_virial, 1, 32, 0, s, vglobal6, m->acc, m->ubg);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -928,18 +933,18 @@ int pd_mesh_transform(pd_mesh *m, const float *x, const float *y, const float *z
     m->sort_n = 0;
     if (!order && n > MESH_CHUNK) {
         const int blocks = (n + 255) / 256;
-        k_order_bin<<<blocks, 256, 0, st>>>(x, y, z, n, (float)m->box[0], (float)m->box[1], (float)m->box[2], m->ncx,
+        launch_chained(k_order_bin, blocks, 256, 0, st, x, y, z, n, (float)m->box[0], (float)m->box[1], (float)m->box[2], m->ncx,
                                             m->ncy, m->nzb, m->bin, m->rank, m->bin_count);
         PD_LAUNCHED();
         const int rc = cell_scan_launch(m->bin_count, m->bin_off, m->nbin, m->scan_part, nullptr, st);
         if (rc) return rc;
-        k_order_scatter<<<blocks, 256, 0, st>>>(m->bin, m->rank, m->bin_off, n, m->order);
+        launch_chained(k_order_scatter, blocks, 256, 0, st, m->bin, m->rank, m->bin_off, n, m->order);
         PD_LAUNCHED();
         m->sort_n = n;
         order = m->order;
     }
     if (ntot > 0) {
-        k_pack_order<<<(ntot + 255) / 256, 256, 0, st>>>(x, y, z, q, order, n, ntot, m->packed);
+        launch_chained(k_pack_order, (ntot + 255) / 256, 256, 0, st, x, y, z, q, order, n, ntot, m->packed);
         PD_LAUNCHED();
     }
     return mesh_transform_packed(m, m->packed, nchunks, nullptr, energy, st);
@@ -955,7 +960,7 @@ int pd_mesh_gather(pd_mesh *m, const float *x, const float *y, const float *z, c
     if (!order && n > 0 && n == m->sort_n) order = m->order;   // a permutation, whatever the positions are now
     // the packed staging buffer holds the particles of the last transform; refresh it (positions may differ)
     if (n > 0) {
-        k_pack_order<<<(nchunks * MESH_CHUNK + 255) / 256, 256, 0, st>>>(x, y, z, q, order, n, nchunks * MESH_CHUNK,
+        launch_chained(k_pack_order, (nchunks * MESH_CHUNK + 255) / 256, 256, 0, st, x, y, z, q, order, n, nchunks * MESH_CHUNK,
                                                                          m->packed);
         PD_LAUNCHED();
     }

@@ -2,6 +2,7 @@
 #include <cmath>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "ell_common.cuh"
 #include "internal.hpp"
@@ -343,11 +344,13 @@ constexpr int fft_plane_blocks(int maxt) { return maxt <= 256 ? 4 : maxt <= 512 
 
 template <bool INPLACE, int MAXT>
 __global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_plane_forward(const __grid_constant__ FftMesh m) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     plane_forward<INPLACE>(m, blockIdx.x, fft_smem);
 }
 template <bool INPLACE, int MAXT>
 __global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_plane_inverse(const __grid_constant__ FftMesh m) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     plane_inverse<INPLACE>(m, blockIdx.x, blockIdx.y, fft_smem);
 }
@@ -355,6 +358,7 @@ template <bool ENERGY, bool IK>
 __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_LINES_C) k_lines_z(const __grid_constant__ FftMesh m,
                                                                        const float *__restrict__ Vc,
                                                                        double *__restrict__ acc) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     lines_z<ENERGY, IK>(m, blockIdx.x * FFT_LINES_C, fft_smem, Vc, acc);
 }
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_LINES_C) k_lines_z(const __
 constexpr int FFT_ROW_PAIRS = 8;
 
 __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_ROW_PAIRS) k_rows_forward(const __grid_constant__ FftMesh m) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     const FftAxis X = m.ax[0];
     const int K1 = X.n, K2 = m.ax[1].n, K1h = m.K1h, P = (K2 + 1) >> 1, bp = X.b | 1, xa = X.a, xb = X.b;
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_ROW_PAIRS) k_rows_forward(c
 }
 
 __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_ROW_PAIRS) k_rows_inverse(const __grid_constant__ FftMesh m) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     const FftAxis X = m.ax[0];
     const int K1 = X.n, K2 = m.ax[1].n, K1h = m.K1h, P = (K2 + 1) >> 1, bp = X.b | 1, xa = X.a, xb = X.b;
@@ -431,6 +437,7 @@ __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_ROW_PAIRS) k_rows_inverse(c
 // y lines of one z plane, in place.
 template <bool INVERSE>
 __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_LINES_C) k_lines_y(const __grid_constant__ FftMesh m) {
+    chain_begin();
     extern __shared__ float2 fft_smem[];
     const int K1h = m.K1h, c0 = blockIdx.x * FFT_LINES_C;
     float2 *base = (INVERSE ? m.zspec[blockIdx.z] : m.spec) + (size_t)blockIdx.y * m.ax[1].n * K1h + c0;
@@ -445,6 +452,7 @@ template <bool INPLACE, int MAXT>
 __global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_bplane_forward(const FftMesh *__restrict__ tab,
                                                                      const int2 *__restrict__ blocks,
                                                                      const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     extern __shared__ float2 fft_smem[];
     __shared__ FftMesh m;
@@ -457,6 +465,7 @@ template <bool INPLACE, int MAXT>
 __global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_bplane_inverse(const FftMesh *__restrict__ tab,
                                                                      const int2 *__restrict__ blocks,
                                                                      const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     extern __shared__ float2 fft_smem[];
     __shared__ FftMesh m;
@@ -468,6 +477,7 @@ __global__ void __launch_bounds__(MAXT, fft_plane_blocks(MAXT)) k_bplane_inverse
 __global__ void __launch_bounds__(FFT_RADIX_MAX *FFT_LINES_C) k_blines_z(const FftMesh *__restrict__ tab,
                                                                         const int2 *__restrict__ blocks,
                                                                         const long long *__restrict__ st) {
+    chain_begin();
     if (st[E_VALID] == 0) return;
     extern __shared__ float2 fft_smem[];
     __shared__ FftMesh m;
@@ -561,10 +571,10 @@ static size_t fft_rows_smem(const FftMesh &m) {
 // A plane kernel in the CTA size of nt threads (two buffers: always the largest).
 #define PD_PLANE_LAUNCH(K, inplace, nt, grid, shm, s, args)                                \
     do {                                                                                   \
-        if (!(inplace)) K<false, FFT_PLANE_THREADS><<<grid, nt, shm, s>>>(PD_UNPAREN args);            \
-        else if ((nt) <= 256) K<true, 256><<<grid, nt, shm, s>>>(PD_UNPAREN args);                     \
-        else if ((nt) <= 512) K<true, 512><<<grid, nt, shm, s>>>(PD_UNPAREN args);                     \
-        else K<true, FFT_PLANE_THREADS><<<grid, nt, shm, s>>>(PD_UNPAREN args);                        \
+        if (!(inplace)) launch_chained(K<false, FFT_PLANE_THREADS>, grid, nt, shm, s, PD_UNPAREN args);            \
+        else if ((nt) <= 256) launch_chained(K<true, 256>, grid, nt, shm, s, PD_UNPAREN args);                     \
+        else if ((nt) <= 512) launch_chained(K<true, 512>, grid, nt, shm, s, PD_UNPAREN args);                     \
+        else launch_chained(K<true, FFT_PLANE_THREADS>, grid, nt, shm, s, PD_UNPAREN args);                        \
     } while (0)
 
 int fft_forward(const FftMesh &m, int route, cudaStream_t s) {
@@ -578,10 +588,10 @@ int fft_forward(const FftMesh &m, int route, cudaStream_t s) {
         return PD_OK;
     }
     const int pairs = (m.ax[1].n + 1) / 2 * m.ax[2].n;
-    k_rows_forward<<<(pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, FFT_RADIX_MAX * FFT_ROW_PAIRS, fft_rows_smem(m), s>>>(m);
+    launch_chained(k_rows_forward, (pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, FFT_RADIX_MAX * FFT_ROW_PAIRS, fft_rows_smem(m), s, m);
     PD_LAUNCHED();
     const dim3 g((m.K1h + FFT_LINES_C - 1) / FFT_LINES_C, m.ax[2].n);
-    k_lines_y<false><<<g, fft_line_threads(m.ax[1]), fft_line_smem(m.ax[1]), s>>>(m);
+    launch_chained(k_lines_y<false>, g, fft_line_threads(m.ax[1]), fft_line_smem(m.ax[1]), s, m);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -591,11 +601,11 @@ int fft_solve(const FftMesh &m, bool ik, bool energy, const float *Vc, double *a
     const int threads = fft_line_threads(m.ax[2]);
     const size_t shm = fft_line_smem(m.ax[2]) * (ik ? 2 : 1);
     if (ik) {
-        if (energy) k_lines_z<true, true><<<blocks, threads, shm, s>>>(m, Vc, acc);
-        else k_lines_z<false, true><<<blocks, threads, shm, s>>>(m, Vc, acc);
+        if (energy) launch_chained(k_lines_z<true, true>, blocks, threads, shm, s, m, Vc, acc);
+        else launch_chained(k_lines_z<false, true>, blocks, threads, shm, s, m, Vc, acc);
     } else {
-        if (energy) k_lines_z<true, false><<<blocks, threads, shm, s>>>(m, Vc, acc);
-        else k_lines_z<false, false><<<blocks, threads, shm, s>>>(m, Vc, acc);
+        if (energy) launch_chained(k_lines_z<true, false>, blocks, threads, shm, s, m, Vc, acc);
+        else launch_chained(k_lines_z<false, false>, blocks, threads, shm, s, m, Vc, acc);
     }
     PD_LAUNCHED();
     return PD_OK;
@@ -612,10 +622,10 @@ int fft_inverse(const FftMesh &m, int route, int nout, cudaStream_t s) {
         return PD_OK;
     }
     const dim3 g((m.K1h + FFT_LINES_C - 1) / FFT_LINES_C, m.ax[2].n, nout);
-    k_lines_y<true><<<g, fft_line_threads(m.ax[1]), fft_line_smem(m.ax[1]), s>>>(m);
+    launch_chained(k_lines_y<true>, g, fft_line_threads(m.ax[1]), fft_line_smem(m.ax[1]), s, m);
     PD_LAUNCHED();
     const int pairs = (m.ax[1].n + 1) / 2 * m.ax[2].n;
-    k_rows_inverse<<<dim3((pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, nout), FFT_RADIX_MAX * FFT_ROW_PAIRS, fft_rows_smem(m), s>>>(m);
+    launch_chained(k_rows_inverse, dim3((pairs + FFT_ROW_PAIRS - 1) / FFT_ROW_PAIRS, nout), FFT_RADIX_MAX * FFT_ROW_PAIRS, fft_rows_smem(m), s, m);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -626,7 +636,7 @@ int fft_batch(const FftBatch &f, const long long *st, cudaStream_t s) {
         PD_PLANE_LAUNCH(k_bplane_forward, k.inplace, k.threads, k.count, k.smem, s, (f.tab, f.planes + k.first, st));
         PD_LAUNCHED();
     }
-    k_blines_z<<<f.ncols, f.line_threads, f.line_smem, s>>>(f.tab, f.cols, st);
+    launch_chained(k_blines_z, f.ncols, f.line_threads, f.line_smem, s, f.tab, f.cols, st);
     PD_LAUNCHED();
     for (int c = 0; c < f.nclass; ++c) {
         const FftBatch::Class &k = f.cls[c];

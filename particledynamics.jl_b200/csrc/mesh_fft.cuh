@@ -11,6 +11,11 @@
 // Planes too large for shared memory go through k_rows_forward / k_lines_y / k_rows_inverse instead of the
 // plane kernels (five kernels).
 //
+// In principle L2-bound (20 bytes per mode and kernel), in fact latency-bound: a 120^3 mesh is 120 planes, one
+// CTA each, between whose passes stand barriers.  120^3, warm: planes 11.3 us each way, z lines 7.3 us (the
+// library's six kernels and the multiply: 54 us of a launch list with cold caches; with the planes' lines as
+// separate kernels the step of 64 000 ions takes 1 % more, of 18 302 ions on 70 x 70 x 112 16 % more).
+//
 // A line of length n = a b (a, b <= 16) takes two register passes: DFTs of length a over stride-b
 // elements, the twiddles exp(-2 pi i q k / n) from a table computed in FP64, DFTs of length b (the
 // Cooley-Tukey decomposition).  Inverse transforms run the forward code on values with real and

@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -175,7 +176,8 @@ constexpr int BRICK_WORDS = 40;   // shared words of chunk_brick: 4 per reportin
 
 // CH: particles of the chunk (threads t and t + CH, ... share particle t); NT: threads of the CTA; TILE: floats
 // of the shared brick.  The chunk's bounding box comes from warp reductions (the warps of the first CH threads
-// report, every thread combines): bound by latency, as one CTA's chunk is all that many SMs have.
+// report, every thread combines): bound by latency, as one CTA's chunk is all that many SMs have (shared-memory
+// atomics and synchronous brick copies: 14.6 us for the gather of 1000 ions, now 7.5).
 template <int P, int CH, int NT, int TILE = TILE_MAX>
 __device__ __forceinline__ void chunk_brick(bool valid, int k1, int k2, int k3, int K1, int K2, int K3, int &d1,
                                             int &d2, int &d3, Brick &b, int *sm /* BRICK_WORDS ints */,
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_spread(const
                                                          const int *__restrict__ nchunk_dev, float *__restrict__ grid,
                                                          int K1, int K2, int K3, float Lx, float Ly, float Lz,
                                                          WindowPoly wp) {
+    chain_begin();
     const int c = blockIdx.x;
     if (nchunk_dev && c >= *nchunk_dev) return;
     if (c >= nchunks) return;
@@ -489,6 +492,7 @@ __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_gather(const
                                                          const int *__restrict__ nchunk_dev, GatherGrids grids,
                                                          int K1, int K2, int K3, float Lx, float Ly, float Lz,
                                                          GatherOut o) {
+    chain_begin();
     const int c = blockIdx.x;
     if (nchunk_dev && c >= *nchunk_dev) return;
     if (c >= nchunks) return;
@@ -731,7 +735,7 @@ void launch_spread_t(int P, const float4 *xq, int nchunks, const int *ns_dev, fl
     switch (P) {
 #define PD_SPREAD_CASE(PP)                                                                                         \
     case PP:                                                                                                       \
-        k_spread<PP, WIN><<<nchunks, MESH_THREADS, 0, s>>>(xq, nchunks, ns_dev, grid, K1, K2, K3, Lx, Ly, Lz, wp); \
+        launch_chained(k_spread<PP, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, grid, K1, K2, K3, Lx, Ly, Lz, wp); \
         break;
         PD_MESH_ORDER_CASES(PD_SPREAD_CASE)
 #undef PD_SPREAD_CASE
@@ -747,10 +751,10 @@ void launch_gather_t(int P, bool energy, const float4 *xq, int nchunks, const in
 #define PD_GATHER_CASE(PP)                                                                                          \
     case PP:                                                                                                        \
         if (energy)                                                                                                 \
-            k_gather<PP, MODE, true, IK, WIN><<<nchunks, MESH_THREADS, 0, s>>>(xq, nchunks, ns_dev, g, K1, K2, K3, Lx, \
+            launch_chained(k_gather<PP, MODE, true, IK, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, g, K1, K2, K3, Lx, \
                                                                                Ly, Lz, o);                          \
         else                                                                                                        \
-            k_gather<PP, MODE, false, IK, WIN><<<nchunks, MESH_THREADS, 0, s>>>(xq, nchunks, ns_dev, g, K1, K2, K3,    \
+            launch_chained(k_gather<PP, MODE, false, IK, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, g, K1, K2, K3,    \
                                                                                 Lx, Ly, Lz, o);                     \
         break;
         PD_MESH_ORDER_CASES(PD_GATHER_CASE)

@@ -28,6 +28,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_mlp_forward(const __nv_bfloat
                                                               MlpWeights wt, float *__restrict__ out_s,
                                                               const float4 *__restrict__ V,
                                                               float4 *__restrict__ corr, int *__restrict__ err) {
+    chain_begin();
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ __align__(8) uint64_t bars[FW_WG];
     __shared__ uint32_t tmem_base;
@@ -652,7 +654,7 @@ int mlp_forward_launch(const pd_mlp *q, const void *X, int n, float *s, const fl
     if (n <= 0) return PD_OK;
     const int tiles = (n + MLP_TILE - 1) / MLP_TILE;
     const int ctas = std::min(sm_count(), (tiles + FW_WG - 1) / FW_WG);
-    k_mlp_forward<<<ctas, FW_THREADS, FW_BYTES, st>>>(static_cast<const __nv_bfloat16 *>(X), n, mlp_weights(q), s, V,
+    launch_chained(k_mlp_forward, ctas, FW_THREADS, FW_BYTES, st, static_cast<const __nv_bfloat16 *>(X), n, mlp_weights(q), s, V,
                                                         corr, q->err);
     PD_LAUNCHED();
     return PD_OK;

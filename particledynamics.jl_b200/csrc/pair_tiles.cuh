@@ -15,6 +15,7 @@
 #pragma once
 #include <algorithm>
 
+#include "chain.cuh"
 #include "cluster_pairs.cuh"
 #include "packed2.cuh"
 
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(128) k_pairs_force(const float4 *__restrict__ 
                                                      const int *__restrict__ nw, const int *__restrict__ counts,
                                                      const float *__restrict__ lj_table, float4 *__restrict__ fc,
                                                      int nsplit, const __grid_constant__ PairParams pp) {
+    chain_begin();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nwarp = blockDim.x >> 5;
     const int ti = lane & 7, q = lane >> 3;
     const int S = blockIdx.x / nsplit, part = blockIdx.x % nsplit;
@@ -244,6 +246,7 @@ __global__ void __launch_bounds__(64) k_pairs_energy(const float4 *__restrict__ 
                                                      const float *__restrict__ lj_table, float4 *__restrict__ fc,
                                                      float *__restrict__ vc, int nslot, int nsplit,
                                                      const __grid_constant__ PairParams pp) {
+    chain_begin();
     constexpr int NT = 64;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int ti = lane & 7, q = lane >> 3;
@@ -398,11 +401,11 @@ static void launch_tiles(pd_cluster *c, int energy, cudaStream_t s) {
     // the energy pass has two warps per part: as many warps as the force pass
     const int eparts = std::max(1, c->nsplit * c->pair_warps / 2);
     if (energy)
-        k_pairs_energy<LJK, COUL, NP><<<c->nsmax * eparts, 64, 0, s>>>(c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts,
+        launch_chained(k_pairs_energy<LJK, COUL, NP>, c->nsmax * eparts, 64, 0, s, c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts,
                                                                        c->lj_table, c->fc, c->vc, c->nslot, eparts,
                                                                        c->pp);
     else
-        k_pairs_force<LJK, COUL, NP><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
+        launch_chained(k_pairs_force<LJK, COUL, NP>, c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s, 
             c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts, c->lj_table, c->fc, c->nsplit, c->pp);
 }
 
