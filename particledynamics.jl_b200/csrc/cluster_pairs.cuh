@@ -56,9 +56,9 @@ __device__ __forceinline__ float horner(const float (&c)[NP], float x) {
     return acc;
 }
 
-// EXCL: working entries flagged by the prune (bit 17) carry 8 pair masks (one per i-cluster,
+// The pass with exclusion masks: working entries flagged by the prune (bit 17) carry 8 pair masks (one per i-cluster,
 // bit ti * 8 + tj) at xmask[8 (wxid[e] - 1)]; a masked pair takes the excluded branch of pair_force.
-template <int LJK, bool COUL, bool ENERGY, int NP, bool EXCL>
+template <int LJK, bool COUL, bool ENERGY, int NP>
 __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, const int *__restrict__ ts,
                                               const uint2 *__restrict__ cjw, const int *__restrict__ scio,
                                               const int *__restrict__ nw, const int *__restrict__ counts,
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
     // force (and with ENERGY its half energy and half virial).  `masked` drops the self
     // and double-counted pairs of the tile that holds the i-cluster itself; marked
     // (pbc) tiles take the compensated periodic difference (PeriodicDisplacement.jl:4-14).
-    // Padding atoms sit far away with zero charge and contribute exact zeros.  `excl` (EXCL only):
+    // Padding atoms sit far away with zero charge and contribute exact zeros.  `excl`:
     // the pair is an exception; its Coulomb term becomes minus the mesh part (the scaled term is
     // added outside the tiles) and, with bond exclusions, its LJ term is dropped.
     auto pair = [&](const int a, const float4 &pi, const float4 &pj, int tyi, int tyj, bool masked, bool pbc,
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
                 lrc2 = pp.lrc2;
                 esh = pp.esh;
             }
-            const bool use = r2 < lrc2 && !(EXCL && pp.lj_excl && excl);
+            const bool use = r2 < lrc2 && !(pp.lj_excl && excl);
             const float ir6 = rinv2 * rinv2 * rinv2;
             f += use ? (12.f * c12 * ir6 - 6.f * c6) * ir6 * rinv2 : 0.f;
             if (ENERGY) en += use ? (c12 * ir6 - c6) * ir6 - esh : 0.f;
@@ -150,12 +150,12 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
             const float rinv3 = rinv * rinv2;
             const float cq = pi.w * pj.w;
             float fq = inr ? rinv3 - pf : 0.f;
-            if (EXCL) fq = excl ? (inr ? -pf : (pp.has_mesh ? -rinv3 : 0.f)) : fq;
+            fq = excl ? (inr ? -pf : (pp.has_mesh ? -rinv3 : 0.f)) : fq;
             f = fmaf(cq, fq, f);
             if (ENERGY) {
                 const float pe = horner(cpe, x);
                 float eq = inr ? rinv + pe - pp.eshift : 0.f;
-                if (EXCL) eq = excl ? (inr ? pe : (pp.has_mesh ? -rinv : 0.f)) : eq;
+                eq = excl ? (inr ? pe : (pp.has_mesh ? -rinv : 0.f)) : eq;
                 en = fmaf(cq, eq, en);
             }
         }
@@ -239,9 +239,9 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
         const bool pbc = (word >> 16) & 1u;   // tile may cross a box face before the next prune
         const int cj = (int)__reduce_or_sync(0xffffffffu, cur.x);
         const int da = cj - S * 8;   // index of the i-cluster that is the j-cluster itself, if in [0, 8)
-        const bool hasx = EXCL && ((word >> 17) & 1u);
+        const bool hasx = (word >> 17) & 1u;
         size_t xb = 0;
-        if (EXCL && hasx) xb = (size_t)(__reduce_or_sync(0xffffffffu, (uint32_t)wxid[e]) - 1) * 8;
+        if (hasx) xb = (size_t)(__reduce_or_sync(0xffffffffu, (uint32_t)wxid[e]) - 1) * 8;
         float A[10], B[10];
 #pragma unroll
         for (int k = 0; k < 10; ++k) A[k] = B[k] = 0.f;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
                 const float4 pi = sxq[a * 8 + ti];
                 const int tyi = LJK == PD_LJ_TABLE ? sty[a * 8 + ti] : 0;
                 const bool self = da == a;
-                const unsigned long long mk = (EXCL && hasx) ? xmask[xb + a] : 0ull;
+                const unsigned long long mk = hasx ? xmask[xb + a] : 0ull;
                 const bool xa = (mk >> (ti * 8 + q)) & 1ull, xbb = (mk >> (ti * 8 + q + 4)) & 1ull;
                 if ((lo >> a) & 1u) pair(a, pi, ja, tyi, cta, self && !gtA, pbc, xa, A);
                 if ((hi >> a) & 1u) pair(a, pi, jb, tyi, ctb, self && !gtB, pbc, xbb, B);
@@ -294,43 +294,42 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
     }
 }
 
-template <int LJK, bool COUL, bool EN, int NP, bool EXCL>
+template <int LJK, bool COUL, bool EN, int NP>
 static void launch_pairs(pd_cluster *c, cudaStream_t s) {
-    k_pairs<LJK, COUL, EN, NP, EXCL><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
+    k_pairs<LJK, COUL, EN, NP><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
         c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts, c->lj_table, c->fc, c->vc, c->nslot, c->nsplit, c->pp,
         c->wxid, c->xmask);
 }
 
-template <int LJK, bool EN, bool EXCL>
+template <int LJK, bool EN>
 static void launch_pairs_poly(pd_cluster *c, cudaStream_t s) {
     const PairParams &pp = c->pp;
     if (!pp.coulomb) {
-        launch_pairs<LJK, false, EN, 1, EXCL>(c, s);
+        launch_pairs<LJK, false, EN, 1>(c, s);
         return;
     }
     const int n = EN ? (pp.nf > pp.ne ? pp.nf : pp.ne) : pp.nf;
-    if (n <= 8) launch_pairs<LJK, true, EN, 8, EXCL>(c, s);
-    else if (n <= 10) launch_pairs<LJK, true, EN, 10, EXCL>(c, s);
-    else if (n <= 12) launch_pairs<LJK, true, EN, 12, EXCL>(c, s);
-    else if (n <= 14) launch_pairs<LJK, true, EN, 14, EXCL>(c, s);
-    else if (n <= 16) launch_pairs<LJK, true, EN, 16, EXCL>(c, s);
-    else if (n <= 20) launch_pairs<LJK, true, EN, 20, EXCL>(c, s);
-    else launch_pairs<LJK, true, EN, 32, EXCL>(c, s);
+    if (n <= 8) launch_pairs<LJK, true, EN, 8>(c, s);
+    else if (n <= 10) launch_pairs<LJK, true, EN, 10>(c, s);
+    else if (n <= 12) launch_pairs<LJK, true, EN, 12>(c, s);
+    else if (n <= 14) launch_pairs<LJK, true, EN, 14>(c, s);
+    else if (n <= 16) launch_pairs<LJK, true, EN, 16>(c, s);
+    else if (n <= 20) launch_pairs<LJK, true, EN, 20>(c, s);
+    else launch_pairs<LJK, true, EN, 32>(c, s);
 }
 
 // The pair pass for the engine's LJ kind and energy flag.
-template <bool EXCL>
 static void pairs_dispatch(pd_cluster *c, int energy, cudaStream_t s) {
     switch (c->pp.lj_kind) {
         case PD_LJ_NONE:
-            energy ? launch_pairs_poly<PD_LJ_NONE, true, EXCL>(c, s) : launch_pairs_poly<PD_LJ_NONE, false, EXCL>(c, s);
+            energy ? launch_pairs_poly<PD_LJ_NONE, true>(c, s) : launch_pairs_poly<PD_LJ_NONE, false>(c, s);
             break;
         case PD_LJ_UNIFORM:
-            energy ? launch_pairs_poly<PD_LJ_UNIFORM, true, EXCL>(c, s)
-                   : launch_pairs_poly<PD_LJ_UNIFORM, false, EXCL>(c, s);
+            energy ? launch_pairs_poly<PD_LJ_UNIFORM, true>(c, s)
+                   : launch_pairs_poly<PD_LJ_UNIFORM, false>(c, s);
             break;
         default:
-            energy ? launch_pairs_poly<PD_LJ_TABLE, true, EXCL>(c, s) : launch_pairs_poly<PD_LJ_TABLE, false, EXCL>(c, s);
+            energy ? launch_pairs_poly<PD_LJ_TABLE, true>(c, s) : launch_pairs_poly<PD_LJ_TABLE, false>(c, s);
             break;
     }
 }

@@ -123,7 +123,7 @@ int cluster_exceptions_launch(pd_cluster *c, int energy, cudaStream_t s) {
 }
 
 int cluster_pairs_launch_excl(pd_cluster *c, int energy, cudaStream_t s) {
-    pairs_dispatch<true>(c, energy, s);
+    pairs_dispatch(c, energy, s);
     PD_LAUNCHED();
     return cluster_exceptions_launch(c, energy, s);
 }
