@@ -227,7 +227,8 @@ int pd_cluster_buffers(pd_cluster *c, const int **perm, const float **xq, const 
  * Mesh engine: ElectrostaticsSolver / MeshWorkspace (src/electrostatics/Solver.jl:17-158)
  * for SPME (B-spline window, exact deconvolution), P3M with the optimal influence
  * function for analytic (AD) or ik differentiation, and ESP (prolate split and window,
- * optimal AD influence or plain deconvolution).  cuFFT does the transforms.
+ * optimal AD influence or plain deconvolution).  Transforms run in the library's own
+ * kernels, or cuFFT where an axis is no product of two factors up to 16.
  * ====================================================================== */
 typedef struct pd_mesh pd_mesh;
 
@@ -525,7 +526,8 @@ typedef struct {
 int pd_batch_create(pd_batch **out, const pd_batch_replica *reps, int nrep, float skin, int cap, int lanes);
 int pd_batch_destroy(pd_batch *b);
 int pd_batch_count(pd_batch *b, int *n, int *ncell);
-/* Lanes per row of the pair kernel (1, 2, 4, 8), the autotuner's choice. */
+/* Lanes per row of the pair kernel (1, 2, 4, 8), the autotuner's choice.  One lane adds a row's
+ * terms in row order; charged rows take at least 8 lanes where they are long. */
 int pd_batch_set_lanes(pd_batch *b, int lanes);
 /* Displacement decision and the flag-gated rebuild at centred coordinates (all replicas). */
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t st);
@@ -552,8 +554,8 @@ typedef struct {
 int pd_batch_set_coulomb(pd_batch *b, const pd_batch_coulomb *c);
 /* One SPME or P3M-AD mesh per replica (meshes: nrep x (K1, K2, K3), the replica's own box at the
  * shared spacing), B-spline order 4..6, with its FP64 influence function from the single-system
- * setup (compute_influence!, Influence.jl:190-227).  The replicas' meshes are transformed by one
- * batched cuFFT plan per mesh size; spread, influence multiply and gather are one launch each over
+ * setup (compute_influence!, Influence.jl:190-227).  The replicas' meshes are transformed by the
+ * mesh engine's kernels over all of them (or by one batched cuFFT plan per mesh size); spread, influence multiply and gather are one launch each over
  * all replicas.  Neutral replicas only (net_charge = :error).  Host boundary: allocates. */
 int pd_batch_set_mesh(pd_batch *b, int kind, int order, double alpha, double C, const int *meshes);
 /* Spread tile of the batched meshes, the autotuner's choice: 32 or 64 particles (cell-order
