@@ -197,8 +197,9 @@ __global__ void k_batch_bin(const float *__restrict__ x, const float *__restrict
 }
 
 // Rows of the flagged replicas' cells, nsplit warps per global cell (rows.cuh): rows, their lengths and their
-// entries are in cell order (positions in `sorted`).
-__global__ void __launch_bounds__(32 * ROWS_WARPS, ROWS_BLOCKS) k_batch_rows(
+// entries are in cell order (positions in `sorted`).  Five blocks per SM, 96 registers: at the 80 of six the replica's
+// grid spills (96 replicas, five steps: 1588 us with six, 1359 with five; 12 melts 859, 818).
+__global__ void __launch_bounds__(32 * ROWS_WARPS, 5) k_batch_rows(
     const float4 *__restrict__ xq, int ncell, int nsplit, const int *__restrict__ cell_rep,
     const BatchRep *__restrict__ reps, const int *__restrict__ rep_flag, const int *__restrict__ sorted,
     const int *__restrict__ cell_off, float rl2, int cap, int *__restrict__ rows, int *__restrict__ counts,
