@@ -137,9 +137,13 @@ __device__ __forceinline__ int ell_reach(float rl, float L, int n) {
     return min(max(1, (int)ceilf(rl * (float)n / L - 1e-5f)), (n - 1) / 2);
 }
 
-// Rounds per block of a drift kernel of `blocks` blocks of 256 particles: one while the blocks are about a wave
-// (148 SMs, five blocks each), up to four beyond.
-inline int drift_items(int blocks) { return blocks <= 740 ? 1 : blocks <= 1480 ? 2 : 4; }
+// Rounds per block of a drift kernel of `blocks` blocks of 256 particles: as many as bring the blocks into one wave
+// (148 SMs, five blocks each), up to `most`: four for the NVE drifts, which wait on memory alone (4096 blocks in six
+// rounds: five steps of 1 048 576 atoms 1625 -> 1668 us).
+inline int drift_items(int blocks, int most = 4) {
+    const int rounds = (blocks + 739) / 740;
+    return rounds < 1 ? 1 : rounds > most ? most : rounds;
+}
 
 // ------------------------------------------------------------------ host side of ell.cu
 
