@@ -405,8 +405,10 @@ int pd_md_evaluate(pd_md *md, int energy, pd_stream_t sp) {
     const float *q = c->p.coulomb ? st.q : nullptr;
     int rc, h[W_LEN];
     if ((rc = cluster_decide_launch(c, st.x, st.y, st.z, 0, s))) return rc;
-    // With a list there is a slot order, and any slot order will do for the mesh: its transform starts before
-    // the host knows whether the list is kept, and runs while the decision is read back.
+    // With a list there is a slot order, and any order that holds every particle once will do for the mesh: its
+    // transform starts before the host knows whether the list is kept, and runs while the decision is read back.
+    // A build that met non-finite coordinates leaves an order with particles missing and its error word set (in an
+    // evaluation or in a captured step): the transform then runs again after the new build.
     const bool early = c->have_build;
     if (early) {
         if ((rc = pd_cluster_pack(c, st.x, st.y, st.z, q, st.type, sp))) return rc;
@@ -418,7 +420,8 @@ int pd_md_evaluate(pd_md *md, int energy, pd_stream_t sp) {
         return code;
     };
     if ((rc = cluster_read_counts(c, h, s))) return refused(rc);
-    if (h[W_BUILD] || !c->have_build) {
+    const bool failed = h[W_ERR] != 0;   // of the last build: there is no list to keep
+    if (h[W_BUILD] || failed || !c->have_build) {
         // the build packs the slots anew: after the spread has read them
         if (early && md->m) PD_CUDA(cudaStreamWaitEvent(s, md->ev_spread, 0));
         for (int attempt = 0; attempt < 8; ++attempt) {
@@ -445,7 +448,7 @@ int pd_md_evaluate(pd_md *md, int energy, pd_stream_t sp) {
         if ((rc = cluster_set_word(c, W_PRUNE, 1, s))) return rc;
     }
     if ((rc = fork_learned(md, s))) return rc;
-    if (!early && (rc = fork_mesh(md, energy, s))) return rc;
+    if ((!early || failed) && (rc = fork_mesh(md, energy, s))) return rc;
     if ((rc = cluster_prune_launch(c, 1, s))) return rc;
     return enqueue_forces(md, energy, 0.f, s);
 }
