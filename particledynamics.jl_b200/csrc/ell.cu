@@ -576,6 +576,7 @@ struct pd_ell {
     float rl2 = 0.f, threshold = 0.f;
     int lanes = 1;
     int cap = 0;
+    int epoch = 0;                      // counts the row storages: captured kernels hold their address, capacity and stride
     long long *st = nullptr;
     int *cell_of = nullptr, *cell_count = nullptr, *cell_off = nullptr, *sorted = nullptr, *tmp = nullptr;
     int *pos_of = nullptr;              // inverse of sorted
@@ -657,6 +658,8 @@ int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *
 }
 
 size_t ell_scan_part_len(int ncell) { return scan_part_len(ncell); }
+
+int ell_rows_epoch(const pd_ell *e) { return e->epoch; }
 
 EllRowsView ell_rows_view(const pd_ell *e) {
     EllRowsView v;
@@ -815,18 +818,19 @@ int ell_pack_launch(pd_ell *e, const float *x, const float *y, const float *z, c
 
 static int ell_alloc_rows(pd_ell *e, int cap) {
     PD_CHECK(cap > 0, PD_EINVAL, "Invalid ELL capacity");
+    ++e->epoch;
     PD_CHECK((long long)e->n * cap <= 0x7fffffffLL, PD_EINVAL,
              "Neighbor table of %d particles x cap %d exceeds the Int32 index range; lower `cap`", e->n, cap);
     dfree(e->rows);
     int rc = dalloc(&e->rows, (size_t)e->n * cap);
     if (rc) return rc;
     PD_CUDA(cudaMemset(e->rows, 0xff, sizeof(int) * (size_t)e->n * cap));
+    e->cap = cap;
     if (e->xrows) {
         dfree(e->xrows);
         if ((rc = dalloc(&e->xrows, (size_t)e->n * cap))) return rc;
         PD_CUDA(cudaMemset(e->xrows, 0xff, sizeof(int) * (size_t)e->n * cap));
     }
-    e->cap = cap;
     return PD_OK;
 }
 
@@ -979,6 +983,7 @@ int pd_ell_rows(pd_ell *e, int **rows, int **counts) {
     PD_CHECK(e && rows && counts, PD_EINVAL, "pd_ell_rows: null argument");
     if (!e->xrows) {   // from now on every rebuild refreshes them (captured steps are captured again)
         int rc;
+        dfree(e->xcounts);   // of rows that were lost in a resize
         if ((rc = dalloc(&e->xcounts, (size_t)e->n)) || (rc = dalloc(&e->xrows, (size_t)e->n * e->cap))) {
             dfree(e->xcounts);
             return rc;
@@ -1073,7 +1078,8 @@ struct EllStepArgs {
     float4 *xq;
     const int *pos_of;
     const float4 *ref;
-    const int *rows, *xrows;  // not read by the drift: part of the key that captured steps are matched on
+    const int *rows, *xrows;  // not read by the drift, as rows_epoch: part of the key that captured steps are matched on
+    int rows_epoch;           // a resized storage may come back at the old address with another capacity, the rows' stride
     float threshold;
 };
 
@@ -1273,6 +1279,7 @@ static EllStepArgs ell_step_args(pd_ell_md *md, float dt, float gamma, float kT,
     a.pos_of = e->pos_of;
     a.rows = e->rows;
     a.xrows = e->xrows;
+    a.rows_epoch = e->epoch;
     a.ref = e->ref;
     a.threshold = e->threshold;
     if (md->f0) {

@@ -161,6 +161,7 @@ struct pd_ell;
 namespace pdb {
 
 EllRowsView ell_rows_view(const ::pd_ell *e);
+int ell_rows_epoch(const ::pd_ell *e);   // changes with the rows' storage (address, capacity)
 int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *cell_off, int *part, int *sorted,
                     int *tmp, long long *st, cudaStream_t s);
 // Exclusive scan of a histogram into ncell + 1 offsets, the histogram set to zero; part: ell_scan_part_len(ncell)

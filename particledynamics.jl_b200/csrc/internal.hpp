@@ -233,6 +233,7 @@ int mlp_forward_launch(const pd_mlp *q, const void *X, int n, float *s, const fl
 int learned_correction_launch(pd_learned *h, const pd_mlp *net, const float *x, const float *y, const float *z,
                               const float *q, const int *type, float4 *corr, cudaStream_t s);
 const float4 *learned_corr(const pd_learned *h);
+int learned_rows_epoch(const pd_learned *h);   // of the neighbour rows, which captured steps hold
 const float4 *learned_radial(const pd_learned *h);
 
 // Batched meshes of charged replicas (batch_mesh.cu).  Replica r's real grids start at float

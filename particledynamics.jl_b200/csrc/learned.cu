@@ -281,6 +281,7 @@ int learned_correction_launch(pd_learned *h, const pd_mlp *net, const float *x, 
     return mlp_forward_launch(net, h->X, h->n, nullptr, h->V, corr ? corr : h->corr, s);
 }
 
+int learned_rows_epoch(const pd_learned *h) { return ell_rows_epoch(h->ell); }
 const float4 *learned_corr(const pd_learned *h) { return h->corr; }
 const float4 *learned_radial(const pd_learned *h) { return h->V; }
 

@@ -43,6 +43,7 @@ struct pd_md {
     cudaStream_t exec_stream[2] = {nullptr, nullptr};
     int exec_epoch[2] = {-1, -1};   // pair-kernel shape the graphs were captured with
     int exec_mepoch[2] = {-1, -1};  // mesh epoch the graphs were captured with
+    int exec_lepoch[2] = {-1, -1};  // row storage of the learned correction the graphs were captured with
     double *esum = nullptr;   // device FP64 energy sum
     float half_c_self = 0.f;
     // learned coarse-mesh correction: descriptors + network on a third stream
@@ -504,7 +505,8 @@ int pd_md_step(pd_md *md, int nsteps, float dt, int energy_last, int use_graph, 
             continue;
         }
         if (!md->exec[energy] || md->exec_dt[energy] != dt || md->exec_stream[energy] != s ||
-            md->exec_epoch[energy] != md->c->shape_epoch || (md->m && md->exec_mepoch[energy] != md->m->epoch)) {
+            md->exec_epoch[energy] != md->c->shape_epoch || (md->m && md->exec_mepoch[energy] != md->m->epoch) ||
+            (md->learned && md->exec_lepoch[energy] != learned_rows_epoch(md->learned))) {
             if (md->exec[energy]) {
                 cudaGraphExecDestroy(md->exec[energy]);
                 md->exec[energy] = nullptr;
@@ -535,6 +537,7 @@ int pd_md_step(pd_md *md, int nsteps, float dt, int energy_last, int use_graph, 
             md->exec_stream[energy] = s;
             md->exec_epoch[energy] = md->c->shape_epoch;
             if (md->m) md->exec_mepoch[energy] = md->m->epoch;
+            if (md->learned) md->exec_lepoch[energy] = learned_rows_epoch(md->learned);
         }
         PD_CUDA(cudaGraphLaunch(md->exec[energy], s));
     }
