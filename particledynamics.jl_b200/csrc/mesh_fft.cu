@@ -545,7 +545,8 @@ int fft_plane_class(const FftMesh &m) {
     return !fft_plane_inplace(m) ? 3 : nt <= 256 ? 0 : nt <= 512 ? 1 : 2;
 }
 
-int fft_line_threads(const FftAxis &a) { return FFT_LINES_C * std::max(a.a, a.b); }
+// Whole warps: the energy sums shuffle across all 32 lanes (a factor of 9 alone would give four and a half warps).
+int fft_line_threads(const FftAxis &a) { return (FFT_LINES_C * std::max(a.a, a.b) + 31) / 32 * 32; }
 size_t fft_line_smem(const FftAxis &a) { return sizeof(float2) * (size_t)a.n * FFT_LINES_C; }
 
 int fft_init() {

@@ -57,3 +57,32 @@ def test_batched_transform_routes(pd, ora, cuda, mesh):
         assert np.linalg.norm(F - ref["F"]) < 1e-5 * np.linalg.norm(ref["F"])
         assert abs(float(b.replica(k, b.epot).double().sum()) - ref["Etot"]) < 1e-5 * abs(ref["Etot"])
     b.close()
+
+
+# z axes whose larger factor is odd (a half-empty last warp) and even, on planes and on separate lines
+@pytest.mark.parametrize("influence", ["spme", "p3m_ik"])
+@pytest.mark.parametrize("mesh", [(16, 18, 20), (14, 15, 42), (16, 15, 45), (12, 14, 54), (16, 16, 64), (15, 16, 72),
+                                  (12, 12, 75), (10, 12, 81), (12, 10, 150), (8, 9, 225), (240, 256, 25)])
+def test_energy_and_virial_of_every_warp_shape(pd, ora, cuda, mesh, influence):
+    import torch
+    L, C, alpha, order = (14.0, 15.0, 16.0), 1.7, 0.9, 5
+    rng = np.random.default_rng(17)
+    n = 300
+    R = (rng.random((n, 3)) * np.array(L) - np.array(L) / 2).astype(np.float32).astype(float)
+    q = rng.standard_normal(n)
+    q = (q - q.mean()).astype(np.float32).astype(float)
+    spec = pd.ElectrostaticsSpec(coulomb_prefactor=C, real_cutoff=4.0, alpha=alpha, influence=influence, order=order,
+                                 mesh=mesh, net_charge="background")
+    s = pd.ElectrostaticsSolver(spec, L, q)
+    t = [torch.tensor(np.ascontiguousarray(a), dtype=torch.float32, device="cuda") for a in (*R.T, q)]
+    ref = ora.mesh(R, q, L, mesh, order, kind=influence, alpha=alpha, C=C, background=True)
+    for _ in range(3):
+        f = [torch.zeros(n, device="cuda") for _ in range(4)]
+        vg = torch.zeros(6, device="cuda")
+        s.transform(*t, energy=True)
+        s.gather(*t, *f[:3], epot=f[3], vglobal=vg, energy=True, set=influence != "p3m_ik")
+        torch.cuda.synchronize()
+        # FP64 sums over FP32 modes: the modes' rounding (a few 1e-7 of the energy) is all that is left
+        assert abs(s.mesh_energy()[0] - ref["Emesh"]) < 1e-6 * abs(ref["Emesh"])
+        assert np.max(np.abs(vg.double().cpu().numpy() - ref["W"])) < 2e-6 * abs(ref["Emesh"])
+    s.close()
