@@ -176,9 +176,9 @@ struct pd_mesh {
     float4 *packed = nullptr;  // particles packed in the caller's order (SoA entry points), or in the mesh's own
     // the mesh's own order of unordered particles (a transform without an order): columns of the box sorted
     // along z, serpentine, so that 64 consecutive particles lie together
-    int sort_n = 0;            // particles of the last such transform (0: none)
     int nbin = 0, ncx = 1, ncy = 1, nzb = 1;
-    int *bin = nullptr, *rank = nullptr, *order = nullptr;   // per particle
+    int *bin = nullptr, *rank = nullptr;   // per particle; a gather without an order keeps its particles' ids in bin
+    int *order = nullptr;                  // nmax_packed entries, then how many of them the last such transform wrote
     int *bin_count = nullptr, *bin_off = nullptr, *scan_part = nullptr;
     int route = 0;             // FFT_PLANES / FFT_LINES: this library's transforms; FFT_CUFFT: the plans below
     pdb::FftMesh fft{};

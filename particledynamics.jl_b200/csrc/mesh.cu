@@ -143,14 +143,16 @@ __global__ void k_self_table(const float *__restrict__ ghat, int K1, int K2, int
 __global__ void k_unit_node(float *grid) { grid[0] = 1.f; }
 
 __global__ void k_pack_order(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-                             const float *__restrict__ q, const int *__restrict__ order, int n, int ntot,
-                             float4 *__restrict__ out) {
+                             const float *__restrict__ q, const int *__restrict__ order,
+                             const int *__restrict__ written, int n, int ntot, float4 *__restrict__ out,
+                             int *__restrict__ ids) {
     chain_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntot) return;
     if (t < n) {
-        const int i = order ? order[t] : t;
+        const int i = order && (!written || *written == n) ? order[t] : t;
         out[t] = make_float4(x[i], y[i], z[i], q[i]);
+        if (ids) ids[t] = i;
     } else {
         out[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -182,11 +184,14 @@ __global__ void k_order_bin(const float *__restrict__ x, const float *__restrict
     rank[i] = atomicAdd(&count[b], 1);
 }
 
+// *written: the entries of the order are a permutation of the first n particles.  The count lives beside them, in
+// the stream's order: what the host has last enqueued may be in a graph that runs later, again, or never.
 __global__ void k_order_scatter(const int *__restrict__ bin, const int *__restrict__ rank, const int *__restrict__ off,
-                                int n, int *__restrict__ order) {
+                                int n, int *__restrict__ order, int *__restrict__ written) {
     chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) order[off[bin[i]] + rank[i]] = i;
+    if (i == 0) *written = n;
 }
 
 // Global virial plus background (_store_global_virial_kernel!, Solver.jl:382-388).
@@ -738,10 +743,11 @@ int make_order(pd_mesh *m, const double box[3]) {
     m->nzb = std::max(1, std::min(1024, (int)(n / (8.0 * m->ncx * m->ncy))));
     m->nbin = m->ncx * m->ncy * m->nzb;
     int rc;
-    if ((rc = dalloc(&m->bin, (size_t)n)) || (rc = dalloc(&m->rank, (size_t)n)) || (rc = dalloc(&m->order, (size_t)n)) ||
+    if ((rc = dalloc(&m->bin, (size_t)n)) || (rc = dalloc(&m->rank, (size_t)n)) || (rc = dalloc(&m->order, (size_t)n + 1)) ||
         (rc = dalloc(&m->bin_count, (size_t)m->nbin)) || (rc = dalloc(&m->bin_off, (size_t)m->nbin + 1)) ||
         (rc = dalloc(&m->scan_part, ell_scan_part_len(m->nbin))))
         return rc;
+    PD_CUDA(cudaMemset(m->order + n, 0, sizeof(int)));
     PD_CUDA(cudaMemset(m->bin_count, 0, sizeof(int) * (size_t)m->nbin));
     PD_CUDA(cudaMemset(m->scan_part, 0, sizeof(int) * ell_scan_part_len(m->nbin)));
     return PD_OK;
@@ -930,7 +936,6 @@ int pd_mesh_transform(pd_mesh *m, const float *x, const float *y, const float *z
     PD_CHECK(ntot <= m->nmax_packed, PD_EINVAL, "pd_mesh_transform: %d particles exceed nmax = %d of this solver", n,
              m->p.nmax);
     // more particles than one chunk, without an order: the mesh's own, which the gather takes again
-    m->sort_n = 0;
     if (!order && n > MESH_CHUNK) {
         const int blocks = (n + 255) / 256;
         launch_chained(k_order_bin, blocks, 256, 0, st, x, y, z, n, (float)m->box[0], (float)m->box[1], (float)m->box[2], m->ncx,
@@ -938,13 +943,14 @@ int pd_mesh_transform(pd_mesh *m, const float *x, const float *y, const float *z
         PD_LAUNCHED();
         const int rc = cell_scan_launch(m->bin_count, m->bin_off, m->nbin, m->scan_part, nullptr, st);
         if (rc) return rc;
-        launch_chained(k_order_scatter, blocks, 256, 0, st, m->bin, m->rank, m->bin_off, n, m->order);
+        launch_chained(k_order_scatter, blocks, 256, 0, st, m->bin, m->rank, m->bin_off, n, m->order,
+                       m->order + m->nmax_packed);
         PD_LAUNCHED();
-        m->sort_n = n;
         order = m->order;
     }
     if (ntot > 0) {
-        launch_chained(k_pack_order, (ntot + 255) / 256, 256, 0, st, x, y, z, q, order, n, ntot, m->packed);
+        launch_chained(k_pack_order, (ntot + 255) / 256, 256, 0, st, x, y, z, q, order, nullptr, n, ntot, m->packed,
+                       nullptr);
         PD_LAUNCHED();
     }
     return mesh_transform_packed(m, m->packed, nchunks, nullptr, energy, st);
@@ -957,11 +963,14 @@ int pd_mesh_gather(pd_mesh *m, const float *x, const float *y, const float *z, c
     cudaStream_t st = (cudaStream_t)s;
     const int nchunks = (n + MESH_CHUNK - 1) / MESH_CHUNK;
     PD_CHECK(m->nmax_packed >= nchunks * MESH_CHUNK, PD_ESTATE, "pd_mesh_gather: no transform of %d particles", n);
-    if (!order && n > 0 && n == m->sort_n) order = m->order;   // a permutation, whatever the positions are now
+    // without an order: the mesh's own if it is one of as many particles (a permutation, whatever the positions are
+    // now), which the device knows; the pack writes down which particle an entry got
+    const bool own = !order && n > MESH_CHUNK;
     // the packed staging buffer holds the particles of the last transform; refresh it (positions may differ)
     if (n > 0) {
-        launch_chained(k_pack_order, (nchunks * MESH_CHUNK + 255) / 256, 256, 0, st, x, y, z, q, order, n, nchunks * MESH_CHUNK,
-                                                                         m->packed);
+        launch_chained(k_pack_order, (nchunks * MESH_CHUNK + 255) / 256, 256, 0, st, x, y, z, q, own ? m->order : order,
+                       own ? m->order + m->nmax_packed : nullptr, n, nchunks * MESH_CHUNK, m->packed,
+                       own ? m->bin : nullptr);
         PD_LAUNCHED();
     }
     if (n > 0) {
@@ -971,7 +980,7 @@ int pd_mesh_gather(pd_mesh *m, const float *x, const float *y, const float *z, c
         o.fy = fy;
         o.fz = fz;
         o.epot = epot;
-        o.ids = order;
+        o.ids = own ? m->bin : order;
         o.n_entries = n;
         o.bg = m->bg;
         o.self_tab = m->self_tab;

@@ -42,3 +42,50 @@ def test_unordered_charges(pd, ora, cuda, n, L):
     s.gather(*m2, *g, set=True)
     assert float((torch.stack(g) - out[1][:, :half]).norm()) < 1e-6 * float(out[1].norm())
     s.close()
+
+
+def test_order_follows_the_stream(pd, cuda):
+    """The own order belongs to the last transform that ran: captured ones that have not run yet, and replays between
+    eager calls of other particle counts, leave every gather's particles complete."""
+    import torch
+    n, half, L = 3000, 1400, (14.0, 15.0, 16.0)
+    rng = np.random.default_rng(8)
+    R = rng.random((n, 3)) * np.array(L) - np.array(L) / 2
+    q = rng.standard_normal(n)
+    spec = pd.ElectrostaticsSpec(coulomb_prefactor=1.7, real_cutoff=4.0, alpha=0.9, influence="spme", order=5,
+                                 mesh=(14, 16, 16), net_charge="background")
+    s = pd.ElectrostaticsSolver(spec, L, q)
+    t = [torch.tensor(np.ascontiguousarray(a), dtype=torch.float32, device="cuda") for a in (*R.T, q)]
+    th = [a[:half].contiguous() for a in t]
+    ident = torch.arange(n, dtype=torch.int32, device="cuda")
+
+    def gather(x, order=None):
+        g = [torch.zeros(x[0].numel(), device="cuda") for _ in range(3)]
+        s.gather(*x, *g, order=order, set=True)
+        return torch.stack(g)
+
+    def agree(x):
+        a, b = gather(x), gather(x, ident[:x[0].numel()].contiguous())
+        # the same potential and stencils; only the FP32 brick offsets differ
+        assert float((a - b).norm()) < 1e-6 * float(b.norm()) and float(b.norm()) > 0
+
+    s.transform(*th)
+    out = [torch.zeros(n, device="cuda") for _ in range(3)]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):       # captured, not run
+        s.transform(*t)
+        s.gather(*t, *out, set=True)
+    agree(t)                            # no order of n particles exists yet
+    agree(th)
+    for _ in range(2):
+        graph.replay()                  # now the order holds n particles, though the last eager call had half
+        torch.cuda.synchronize()
+        b = gather(t, ident)
+        assert float((torch.stack(out) - b).norm()) < 1e-6 * float(b.norm())
+        agree(th)
+        agree(t)
+        s.transform(*th)
+        agree(t)
+        agree(th)
+    s.close()
