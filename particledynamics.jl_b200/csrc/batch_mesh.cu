@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(TP * CH, BMESH_CTAS_PER_SM) k_bspread(const fl
     const int c = blockIdx.x;
     const BMeshRep R = reps[chunk_rep[c]];
     spread_chunk<P, WIN_BSPLINE, CH, BTILE, TP>(mq + (size_t)c * CH, gridA + R.grid, R.K1, R.K2, R.K3, R.Lx, R.Ly, R.Lz,
-                                     WindowPoly{nullptr, 0});
+                                     WindowPoly{nullptr, 0}, bspline_peak3(P));
 }
 
 // spec *= G (the influence multiply of _solve_kernel!, MeshKernels.jl:57-81) over the concatenated

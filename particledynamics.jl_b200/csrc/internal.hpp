@@ -200,6 +200,7 @@ struct pd_mesh {
     float4 *self_tab = nullptr; // self-force table (T^3 samples of the fractional position), or null
     int self_T = 0;
     int epoch = 0;              // bumped when a change needs captured steps to be captured again
+    float wpeak3 = 1.f;         // prolate window: cube of its largest weight (the spread's fixed-point scale)
 };
 
 namespace pdb {

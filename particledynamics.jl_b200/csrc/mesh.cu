@@ -574,10 +574,10 @@ int mesh_transform_packed(pd_mesh *m, const float4 *xq, int nchunks, const int *
              m->p.order);
     if (m->prolate)
         launch_spread_t<WIN_PROLATE>(m->p.order, xq, nchunks, ns_dev, m->gridA, m->K1, m->K2, m->K3, Lx, Ly, Lz,
-                                     window_poly(m), s);
+                                     window_poly(m), m->wpeak3, s);
     else
         launch_spread_t<WIN_BSPLINE>(m->p.order, xq, nchunks, ns_dev, m->gridA, m->K1, m->K2, m->K3, Lx, Ly, Lz,
-                                     window_poly(m), s);
+                                     window_poly(m), 1.f, s);
     PD_LAUNCHED();
     if (ev_spread) PD_CUDA(cudaEventRecord(ev_spread, s));
     return mesh_solve_grids(m, energy, s, ev_r2c);
@@ -694,6 +694,15 @@ int copy_prolate(pd_mesh *m, const pd_prolate *w) {
     std::vector<float> poly((size_t)(w->deg + 1) * H);
     for (int k = 0; k <= w->deg; ++k)
         for (int h = 0; h < H; ++h) poly[(size_t)k * H + h] = (float)w->poly[k][h];
+    // the window's largest weight: sampled along every node's polynomial, rounded up by more than the samples miss
+    double peak = 0.0;
+    for (int h = 0; h < H; ++h)
+        for (int t = -500; t <= 500; ++t) {
+            double v = 0.0;
+            for (int k = w->deg; k >= 0; --k) v = v * (1e-3 * t) + w->poly[k][h];
+            peak = std::max(peak, std::fabs(v));
+        }
+    m->wpeak3 = (float)std::pow(1.0001 * peak, 3);
     int rc;
     if ((rc = dalloc(&m->xq, (size_t)w->nquad)) || (rc = dalloc(&m->wchi, (size_t)w->nquad)) ||
         (rc = dalloc(&m->wpoly, poly.size())))

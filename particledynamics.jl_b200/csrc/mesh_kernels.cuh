@@ -91,6 +91,14 @@ struct WindowPoly {
     int deg;
 };
 
+// Cube of a window's largest weight, which bounds what a charge gives to one node: the central value of the B-spline
+// of order P (rounded up in the fourth digit), or the value the host finds for a prolate window.
+__host__ __device__ constexpr float bspline_peak3(int P) {
+    constexpr float peak[13] = {1.f,     1.f,     1.f,     0.7501f, 0.6667f, 0.5990f, 0.5501f,
+                                0.5111f, 0.4794f, 0.4530f, 0.4305f, 0.4110f, 0.3940f};
+    return peak[P] * peak[P] * peak[P];
+}
+
 // First node and the weights (and du-derivatives) of the prolate stencil at grid coordinate u:
 // _prolate_cell (Windows.jl:158-167) for the base node and tau, then one Horner pass per node
 // giving the value and the tau-derivative of its polynomial (window_stencil(::ProlatePolyStencil),
@@ -325,7 +333,8 @@ __device__ __forceinline__ bool my_plane(int j3, int h) {
 // threads share the z planes of its stencil.
 template <int P, int WIN, int CH, int TILE = TILE_MAX, int TP = 2>
 __device__ __forceinline__ void spread_chunk(const float4 *__restrict__ chunk, float *__restrict__ grid, int K1,
-                                             int K2, int K3, float Lx, float Ly, float Lz, const WindowPoly &wp) {
+                                             int K2, int K3, float Lx, float Ly, float Lz, const WindowPoly &wp,
+                                             float peak3) {
     constexpr int NT = TP * CH;
     __shared__ __align__(16) float tile[TILE];
     __shared__ unsigned rowbase[ROWS_MAX];
@@ -347,25 +356,36 @@ __device__ __forceinline__ void spread_chunk(const float4 *__restrict__ chunk, f
     if (b.fits) {
         // The brick accumulates in 32-bit fixed point: integer shared-memory reductions are native
         // (a float reduction is not), and integer sums are exact, so a chunk's brick does not depend
-        // on the order of its atomics.  The window weights lie in [0, 1], so no node of the brick
-        // exceeds the chunk's sum of |q| in magnitude; the scale is the largest power of two that
-        // keeps that sum below 2^30.  Each contribution rounds to a step of at most sum|q| / 2^30.
-        __shared__ float s_qabs[NT / 32];
-        float qa = (valid && h == 0) ? fabsf(v.w) : 0.f;
+        // on the order of its atomics.  Partial sums may wrap, only a node's final sum has to fit: it lies between
+        // -Q(-) and Q(+) times the cube of the window's largest weight (peak3), Q(+-) the chunk's charge of either
+        // sign, so the scale takes the larger of the two to 2 147 000 000 (the rest of the 32 bits is left to the
+        // rounding of the sums).  Half a step per contribution, Q peak3 / 4.3e9, is at the rounding of FP32 sums: the
+        // charge grid of a melt, order 6 at spacing 1.2, differs from FP64 by 9.3e-8 (FP32 sums in random order 8.9e-8,
+        // a scale from the sum of all |q| to 2^30 with unit weights 9.1e-7).
+        __shared__ float s_qabs[NT / 32], s_qnet[NT / 32];
+        float qa = (valid && h == 0) ? fabsf(v.w) : 0.f, qn = (valid && h == 0) ? v.w : 0.f;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) qa += __shfl_xor_sync(0xffffffffu, qa, off);
-        if ((t & 31) == 0) s_qabs[t >> 5] = qa;
+        for (int off = 16; off > 0; off >>= 1) {
+            qa += __shfl_xor_sync(0xffffffffu, qa, off);
+            qn += __shfl_xor_sync(0xffffffffu, qn, off);
+        }
+        if ((t & 31) == 0) {
+            s_qabs[t >> 5] = qa;
+            s_qnet[t >> 5] = qn;
+        }
         const int nb4 = (b.e1 * b.e2 * b.e3 + 3) >> 2;
         int4 *itile4 = reinterpret_cast<int4 *>(tile);
         int *itile = reinterpret_cast<int *>(tile);
         for (int k = t; k < nb4; k += NT) itile4[k] = make_int4(0, 0, 0, 0);
         __syncthreads();
-        float qsum = 0.f;
+        float qsum = 0.f, qnet = 0.f;
 #pragma unroll
-        for (int k = 0; k < NT / 32; ++k) qsum += s_qabs[k];
-        qsum = fmaxf(qsum, 1e-30f);
-        const int ex = min(30 - (int)ceilf(log2f(qsum)), 126);   // qsum * 2^ex <= 2^30, 2^ex finite
-        const float scale = ldexpf(1.f, ex), inv_scale = ldexpf(1.f, -ex);
+        for (int k = 0; k < NT / 32; ++k) {
+            qsum += s_qabs[k];
+            qnet += s_qnet[k];
+        }
+        const float most = fmaxf(0.5f * (qsum + fabsf(qnet)) * peak3, 3e-29f);   // the scale stays finite
+        const float scale = 2.147e9f / most, inv_scale = 1.f / scale;
         if (valid) {
             const float qs = v.w * scale;
 #pragma unroll
@@ -419,12 +439,13 @@ template <int P, int WIN>
 __global__ void __launch_bounds__(MESH_THREADS, MESH_CTAS_PER_SM) k_spread(const float4 *__restrict__ xq, int nchunks,
                                                          const int *__restrict__ nchunk_dev, float *__restrict__ grid,
                                                          int K1, int K2, int K3, float Lx, float Ly, float Lz,
-                                                         WindowPoly wp) {
+                                                         WindowPoly wp, float peak3) {
     chain_begin();
     const int c = blockIdx.x;
     if (nchunk_dev && c >= *nchunk_dev) return;
     if (c >= nchunks) return;
-    spread_chunk<P, WIN, MESH_CHUNK>(xq + (size_t)c * MESH_CHUNK, grid, K1, K2, K3, Lx, Ly, Lz, wp);
+    spread_chunk<P, WIN, MESH_CHUNK>(xq + (size_t)c * MESH_CHUNK, grid, K1, K2, K3, Lx, Ly, Lz, wp,
+                                     WIN == WIN_BSPLINE ? bspline_peak3(P) : peak3);
 }
 
 // AD gather of chunks (the sums of _gather_ad_lines_sums, MeshKernels.jl:281-311,
@@ -731,11 +752,12 @@ constexpr int MESH_ORDER_MIN = 3, MESH_ORDER_MAX = 12;
 
 template <int WIN>
 void launch_spread_t(int P, const float4 *xq, int nchunks, const int *ns_dev, float *grid, int K1, int K2, int K3,
-                     float Lx, float Ly, float Lz, const WindowPoly &wp, cudaStream_t s) {
+                     float Lx, float Ly, float Lz, const WindowPoly &wp, float peak3, cudaStream_t s) {
     switch (P) {
 #define PD_SPREAD_CASE(PP)                                                                                         \
     case PP:                                                                                                       \
-        launch_chained(k_spread<PP, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, grid, K1, K2, K3, Lx, Ly, Lz, wp); \
+        launch_chained(k_spread<PP, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, grid, K1, K2, K3, Lx, Ly, Lz, wp, \
+                       peak3);                                                                                     \
         break;
         PD_MESH_ORDER_CASES(PD_SPREAD_CASE)
 #undef PD_SPREAD_CASE
@@ -768,7 +790,7 @@ void launch_gather_t(int P, bool energy, const float4 *xq, int nchunks, const in
                                                  int, int, int, float, float, float, const GatherOut &, cudaStream_t)
 #define PD_SPREAD_LAUNCHER(WIN)                                                                                 \
     template void launch_spread_t<WIN>(int, const float4 *, int, const int *, float *, int, int, int, float, float, \
-                                       float, const WindowPoly &, cudaStream_t)
+                                       float, const WindowPoly &, float, cudaStream_t)
 
 extern PD_SPREAD_LAUNCHER(WIN_BSPLINE);
 extern PD_SPREAD_LAUNCHER(WIN_PROLATE);
