@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
                                                            float *__restrict__ fy, float *__restrict__ fz,
                                                            float *__restrict__ epot, float4 *__restrict__ fc,
                                                            BatchKick kick, long long *__restrict__ st, int advance,
-                                                           const __grid_constant__ BatchCoul cp) {
+                                                           float face, const __grid_constant__ BatchCoul cp) {
     chain_begin();
     if (st[E_VALID] == 0) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,8 +358,9 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
             }
         });
     };
-    // the margin keeps the faces farther than the cutoff by more than the coordinates' rounding
-    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, 1.001f * sqrtf(cut2)))) walk(std::false_type{});
+    // face: 1.001 keeps the faces farther than the cutoff by more than the coordinates' rounding; infinite for
+    // coordinates that may lie beyond them
+    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, face * sqrtf(cut2)))) walk(std::false_type{});
     else walk(std::true_type{});
 #pragma unroll
     for (int off = G / 2; off > 0; off >>= 1) {
@@ -401,7 +402,8 @@ __global__ void __launch_bounds__(B_THREADS, 3) k_batch_pairs_seq(const float4 *
                                                                float *__restrict__ fx, float *__restrict__ fy,
                                                                float *__restrict__ fz, float *__restrict__ epot,
                                                                float4 *__restrict__ fc, BatchKick kick,
-                                                               long long *__restrict__ st, int advance) {
+                                                               long long *__restrict__ st, int advance,
+                                                               float face) {
     chain_begin();
     if (st[E_VALID] == 0) return;
     __shared__ int turn[B_THREADS / 32][32 * (SEQ_E + 1)];
@@ -464,7 +466,7 @@ __global__ void __launch_bounds__(B_THREADS, 3) k_batch_pairs_seq(const float4 *
             }
         }
     };
-    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, 1.001f * sqrtf(lj.rc2)))) walk(std::false_type{});
+    if (__all_sync(0xffffffffu, cnt == 0 || clear_of_faces<3>(pi, L, face * sqrtf(lj.rc2)))) walk(std::false_type{});
     else walk(std::true_type{});
     if (live) {
         if (SLOT) {
@@ -680,7 +682,8 @@ static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, con
 
 template <bool COUL, int NP = BATCH_NP>
 static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, float *epot, int energy,
-                               const BatchKick &kick, int advance, bool slot, cudaStream_t s) {
+                               const BatchKick &kick, int advance, bool slot, bool centred, cudaStream_t s) {
+    const float face = centred ? 1.001f : INFINITY;
     // Charged rows are long and every choice below 8 lanes reads their sectors several times; uncharged rows take
     // the caller's choice.
     const int G = COUL ? std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8) : b->lanes;
@@ -689,7 +692,7 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
         if (G == 1) {
 #define PD_BS(EE, SS)                                                                                               \
     launch_chained(k_batch_pairs_seq<EE, SS>, blocks, B_THREADS, 0, s, b->xq, b->n, b->cap, b->rows, b->counts,     \
-                   b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, b->fc, kick, b->st, advance)
+                   b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, b->fc, kick, b->st, advance, face)
             if (slot) {
                 if (energy) PD_BS(true, true);
                 else PD_BS(false, true);
@@ -704,7 +707,7 @@ static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, flo
 #define PD_BP2(GG, EE, SS)                                                                                            \
     launch_chained(k_batch_pairs<GG, EE, COUL, SS, NP>, blocks, B_THREADS, 0, s, b->xq, b->n, b->cap, b->rows, b->counts,         \
                                                                      b->sorted, b->rep_of, b->reps, fx, fy, fz, epot, \
-                                                                     b->fc, kick, b->st, advance, b->cp)
+                                                                     b->fc, kick, b->st, advance, face, b->cp)
 #define PD_BP(GG)                                                                                                     \
     if (slot) {                                                                                                       \
         if (energy) PD_BP2(GG, true, true);                                                                           \
@@ -790,20 +793,22 @@ static int batch_mesh_transform(pd_batch *b, cudaStream_t s) {
 // below it the extra launch costs more than the scattered stores.
 constexpr int BATCH_SLOT_MIN = 32768;
 
-// The force pass: pack (unless the drift has packed the coordinates), then the row pair kernel; with charges and meshes the pair kernel runs on s
+// The force pass: pack (unless the drift has packed the coordinates), then the row pair kernel; with charges and meshes
+// the pair kernel runs on s
 // while the mesh branch runs on the batch's mesh stream (forked and joined by events, so the same
 // code is captured into the step graph), and the gather joins both and applies the closing kick.
 static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const float *z, float *fx, float *fy,
-                              float *fz, float *epot, int energy, BatchKick kick, int advance, bool packed,
+                              float *fz, float *epot, int energy, BatchKick kick, int advance, bool drifted,
                               cudaStream_t s) {
+    const bool centred = drifted;   // a caller's own coordinates may have crossed a face since the update
     if (!b->coul) {
         const int blocks = (b->n + B_THREADS - 1) / B_THREADS;
-        if (!packed) {
+        if (!drifted) {
             launch_chained(k_batch_pack<false>, blocks, B_THREADS, 0, s, x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
             PD_LAUNCHED();
         }
         const bool slot = b->n >= BATCH_SLOT_MIN;
-        launch_batch_pairs<false>(b, fx, fy, fz, epot, energy, kick, slot ? 0 : advance, slot, s);
+        launch_batch_pairs<false>(b, fx, fy, fz, epot, energy, kick, slot ? 0 : advance, slot, centred, s);
         PD_LAUNCHED();
         if (!slot) return PD_OK;
         if (energy)
@@ -828,9 +833,9 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
     nokick.on = 0;
     // the polynomial's coefficient bucket: the fitted force coefficients, and the energy's with energy
     if (std::max(b->coul_nf, energy ? b->coul_ne : 0) <= 14)
-        launch_batch_pairs<true, 14>(b, fx, fy, fz, epot, energy, nokick, advance, true, s);
+        launch_batch_pairs<true, 14>(b, fx, fy, fz, epot, energy, nokick, advance, true, centred, s);
     else
-        launch_batch_pairs<true, BATCH_NP>(b, fx, fy, fz, epot, energy, nokick, advance, true, s);
+        launch_batch_pairs<true, BATCH_NP>(b, fx, fy, fz, epot, energy, nokick, advance, true, centred, s);
     PD_LAUNCHED();
     PD_CUDA(cudaStreamWaitEvent(s, b->ev_join, 0));
     BMeshKick mk;

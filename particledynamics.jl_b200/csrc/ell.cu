@@ -414,7 +414,7 @@ __global__ void k_ell_export(const int *__restrict__ rows, const int *__restrict
 struct EllModel {
     int kind;        // PD_PAIR_LJ or PD_PAIR_WCA
     float eps, sig2, rc2, eshift;
-    float rc_clear;  // a particle farther than this from every face has no pair across one
+    float rc_clear;  // a particle farther than this from every face has no pair across one (coordinates centred)
 };
 
 struct EllKick {     // closing half kick fused into the pair kernel (step engine)
@@ -744,10 +744,11 @@ int ell_decide_launch(pd_ell *e, const float *x, const float *y, const float *z,
 }
 
 template <int D, int G, bool UNIT>
-static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
+static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy, bool centred,
                         const EllKick &kick, cudaStream_t s) {
     const int blocks = (int)(((long long)e->n * G + ELL_THREADS - 1) / ELL_THREADS);
-    const EllModel m = ell_model(e);
+    EllModel m = ell_model(e);
+    if (!centred) m.rc_clear = INFINITY;
     const EllRowsView v = ell_rows_view(e);
 #define PD_ELL_PAIRS(EN, OO)                                                                                      \
     launch_chained(k_ell_pairs<D, G, UNIT, EN, OO>, blocks, ELL_THREADS, 0, s, e->xq, e->n, v.rows, v.counts, v.sorted, v.sk, v.st, \
@@ -770,37 +771,38 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
 }
 
 template <int D>
-static void ell_pairs_d(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
+static void ell_pairs_d(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy, bool centred,
                         const EllKick &kick, cudaStream_t s) {
     if (e->dense) {
         // the caller's lanes, or a whole warp per row where the rows alone leave SMs idle (4000 LJ atoms: 63 blocks
         // of four lanes per row, 16 us; 500 blocks of a warp, 8 us); a million atoms take 4 and 8 lanes alike and 16
         // a third longer
         if (e->p.lanes == 0 && e->n < 16384) {
-            ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, kick, s);
+            ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s);
             return;
         }
         switch (e->lanes) {
-            case 1: ell_pairs_g<D, 1, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-            case 2: ell_pairs_g<D, 2, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-            case 4: ell_pairs_g<D, 4, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-            default: ell_pairs_g<D, 8, true>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+            case 1: ell_pairs_g<D, 1, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+            case 2: ell_pairs_g<D, 2, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+            case 4: ell_pairs_g<D, 4, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+            default: ell_pairs_g<D, 8, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
         }
         return;
     }
     switch (e->lanes) {
-        case 1: ell_pairs_g<D, 1, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        case 2: ell_pairs_g<D, 2, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        case 4: ell_pairs_g<D, 4, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
-        default: ell_pairs_g<D, 8, false>(e, fx, fy, fz, epot, vir, energy, kick, s); break;
+        case 1: ell_pairs_g<D, 1, false>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+        case 2: ell_pairs_g<D, 2, false>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+        case 4: ell_pairs_g<D, 4, false>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
+        default: ell_pairs_g<D, 8, false>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
     }
 }
 
-// The pair kernel over packed coordinates that are already in e->xq.
-int ell_pairs_launch(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy,
+// The pair kernel over packed coordinates that are already in e->xq.  centred: the coordinates have passed the
+// list's decision or come from its drift; a caller's own may have crossed a face since the update.
+int ell_pairs_launch(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy, bool centred,
                      const EllKick &kick, cudaStream_t s) {
-    if (e->dim == 3) ell_pairs_d<3>(e, fx, fy, fz, epot, vir, energy, kick, s);
-    else ell_pairs_d<2>(e, fx, fy, fz, epot, vir, energy, kick, s);
+    if (e->dim == 3) ell_pairs_d<3>(e, fx, fy, fz, epot, vir, energy, centred, kick, s);
+    else ell_pairs_d<2>(e, fx, fy, fz, epot, vir, energy, centred, kick, s);
     PD_LAUNCHED();
     return PD_OK;
 }
@@ -957,7 +959,7 @@ int pd_ell_forces(pd_ell *e, const float *x, const float *y, const float *z, flo
     if ((rc = ell_pack_launch(e, x, y, z, s))) return rc;
     EllKick kick;
     memset(&kick, 0, sizeof kick);
-    return ell_pairs_launch(e, fx, fy, fz, epot, vir, energy, kick, s);
+    return ell_pairs_launch(e, fx, fy, fz, epot, vir, energy, false, kick, s);
 }
 
 int pd_ell_status(pd_ell *e, pd_ell_stats *out) {
@@ -1329,7 +1331,7 @@ static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int e
     memset(&kick, 0, sizeof kick);
     if (mode == 2) {
         // GJF: forces without a kick, then the velocity update (which advances the step)
-        if ((rc = ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, kick, s)))
+        if ((rc = ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, true, kick, s)))
             return rc;
         if (e->dim == 3) k_ell_gjf_vel<3><<<blocks, ELL_THREADS, 0, s>>>(a, e->st);
         else k_ell_gjf_vel<2><<<blocks, ELL_THREADS, 0, s>>>(a, e->st);
@@ -1348,7 +1350,7 @@ static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int e
     // the closing half kick: dt / 2 (NVE, BAOAB), none for BAOA (its B1 kicked the full 2 dt / 2)
     kick.half_dt = mode == 1 ? 0.5f * (2.f * a.dt - a.kick) : 0.5f * a.dt;
     kick.advance = 1;
-    return ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, kick, s);
+    return ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, true, kick, s);
 }
 
 static int ell_run(pd_ell_md *md, int mode, int nsteps, float dt, float gamma, float kT, unsigned long long seed,
@@ -1440,7 +1442,7 @@ int pd_ell_md_evaluate(pd_ell_md *md, int energy, pd_stream_t sp) {
     if ((rc = ell_pack_launch(e, md->st.x, md->st.y, md->st.z, s))) return rc;
     EllKick kick;
     memset(&kick, 0, sizeof kick);
-    return ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, kick, s);
+    return ell_pairs_launch(e, md->st.fx, md->st.fy, md->st.fz, md->st.epot, md->st.vir6, energy, true, kick, s);
 }
 
 int pd_ell_md_step(pd_ell_md *md, int nsteps, float dt, int energy_last, int use_graph, pd_stream_t s) {

@@ -106,3 +106,70 @@ def test_batch_outputs_match_single_systems(pd, cuda, nrep, n_hi):
         for a, c in zip((b.fx, b.fy, b.fz), f):
             assert float((b.replica(k, a) - c).norm()) < 1e-5 * float(torch.stack(f).norm())
         eng.close()
+
+
+def _ell_forces(eng, x, n, dim=3, energy=False):
+    import torch
+    f = [torch.zeros(n, device="cuda") for _ in range(dim)] + [None] * (3 - dim)
+    e, w = torch.zeros(n, device="cuda"), torch.zeros((n, 6 if dim == 3 else 3), device="cuda")
+    eng.forces(*x, *f, epot=e if energy else None, vir=w if energy else None, energy=energy)
+    torch.cuda.synchronize()
+    return torch.stack(f[:dim], 1).double().cpu().numpy()
+
+
+# dense rows, sparse rows, 2D; direct and by-position force stores
+@pytest.mark.parametrize("dim,n,rho", [(3, 1500, 0.8), (3, 33000, 0.8), (3, 9000, 0.08), (2, 9000, 0.85)])
+@pytest.mark.parametrize("energy", [False, True])
+def test_forces_at_uncentred_coordinates(pd, ora, cuda, dim, n, rho, energy):
+    """Forces between updates take coordinates that have drifted over a face, or come as another image of the box."""
+    import torch
+    pos, box = _fluid(n, rho, 5 + n, dim)
+    L = np.array(box)
+    eng = pd.ELLEngine(n, box, dim=dim, model="lj", cutoff=2.5, skin=0.3, capacity=160)
+
+    def dev(p):
+        return [torch.tensor(np.ascontiguousarray(p[:, d]), dtype=torch.float32, device="cuda") for d in range(dim)] + \
+               [None] * (3 - dim)
+
+    eng.update(*dev(pos))
+    rng = np.random.default_rng(4)
+    moved = pos + 0.1 * rng.uniform(-1, 1, pos.shape) / np.sqrt(dim)      # within half the skin, not wrapped
+    image = moved + L * (rng.random(pos.shape) < 0.2) * np.where(moved > 0, -1.0, 0.0)
+    for p in (moved, image):
+        p = p.astype(np.float32).astype(float)
+        F = _ell_forces(eng, dev(p), n, dim, energy)
+        p3 = p if dim == 3 else np.concatenate([p, np.zeros((n, 1))], 1)
+        b3 = box if dim == 3 else (*box, 50.0)
+        ref = ora.pairs_cells(p3 - np.array(b3) * np.round(p3 / np.array(b3)), b3, kind=1, sigma=1.0, eps=1.0, rc_lj=2.5)
+        # FP32 coordinates up to a box from the centre: their rounding, through a force constant of about 1e3
+        assert np.linalg.norm(F - ref["F"][:, :dim]) < 1e-4 * np.linalg.norm(ref["F"])
+    eng.close()
+
+
+@pytest.mark.parametrize("lanes", [1, 4])
+@pytest.mark.parametrize("nrep,n_hi", [(3, 1500), (12, 6000)])
+def test_batch_forces_at_uncentred_coordinates(pd, cuda, lanes, nrep, n_hi):
+    """The same for the batched pass: another image of a particle, or one that has crossed a face, has the same pairs."""
+    import torch
+    specs = pd.synthetic.replica_set(nrep, n_lo=1200 if nrep < 5 else 3000, n_hi=n_hi, seed=21)
+    b = pd.batch.BatchedReplicas(pd.batch.make_systems(specs), skin=0.3, cap=160, lanes=lanes)
+    b.evaluate()
+    b.synchronize()
+    ref = torch.stack([b.fx, b.fy, b.fz]).double()
+    rng = np.random.default_rng(3)
+    img = []
+    for d, a in enumerate((b.x, b.y, b.z)):
+        t = a.clone()
+        for k, s in enumerate(b.systems):
+            v = b.replica(k, t)
+            pick = torch.tensor(rng.random(s["n"]) < 0.2, device="cuda") & (v > 0)
+            v -= pick * float(np.float32(s["box"][d]))
+        img.append(t)
+    f = [torch.zeros(b.n, device="cuda") for _ in range(3)]
+    N = pd._native
+    torch.cuda.synchronize()
+    N.call("pd_batch_forces", b.handle, *[a.data_ptr() for a in img], *[a.data_ptr() for a in f], 0, 0, 0)
+    torch.cuda.synchronize()
+    # shifting a coordinate by a box rounds it to an ulp of the box, about 1e-6; force constants reach 1e3
+    assert float((torch.stack(f).double() - ref).norm()) < 1e-4 * float(ref.norm())
+    b.close()
