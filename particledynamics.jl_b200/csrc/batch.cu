@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_pairs(const float4 *__restr
             }
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
+                if (!(r2[c] > 0.f && r2[c] < cut2)) continue;   // a difference that is not finite adds nothing
                 a[0] = fmaf(f[c], dx[c], a[0]);
                 a[1] = fmaf(f[c], dy[c], a[1]);
                 a[2] = fmaf(f[c], dz[c], a[2]);
@@ -456,12 +457,11 @@ __global__ void __launch_bounds__(B_THREADS, 3) k_batch_pairs_seq(const float4 *
                 if (ENERGY) unpk(un, v[0], v[1]);
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
-                    const bool in = r2[c] > 0.f && r2[c] < lj.rc2;
-                    const float fv = in ? f[c] : 0.f;
-                    a[0] = fmaf(fv, dx[c], a[0]);
-                    a[1] = fmaf(fv, dy[c], a[1]);
-                    a[2] = fmaf(fv, dz[c], a[2]);
-                    if (ENERGY) e += in ? 0.5f * v[c] : 0.f;
+                    if (!(r2[c] > 0.f && r2[c] < lj.rc2)) continue;   // a difference that is not finite adds nothing
+                    a[0] = fmaf(f[c], dx[c], a[0]);
+                    a[1] = fmaf(f[c], dy[c], a[1]);
+                    a[2] = fmaf(f[c], dz[c], a[2]);
+                    if (ENERGY) e += 0.5f * v[c];
                 }
             }
         }

@@ -485,13 +485,13 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
             if (ENERGY) unpk(un, u[0], u[1]);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const bool in = r2[c] > 0.f && r2[c] < lj.rc2;
-                const float fv = in ? f[c] : 0.f;
+                if (!(r2[c] > 0.f && r2[c] < lj.rc2)) continue;   // a difference that is not finite adds nothing
+                const float fv = f[c];
                 a[0] = fmaf(fv, dx[c], a[0]);
                 a[1] = fmaf(fv, dy[c], a[1]);
                 if (D == 3) a[2] = fmaf(fv, dz[c], a[2]);
                 if (ENERGY) {
-                    e += in ? 0.5f * u[c] : 0.f;
+                    e += 0.5f * u[c];
                     const float hx = 0.5f * fv * dx[c], hy = 0.5f * fv * dy[c];
                     w[0] = fmaf(hx, dx[c], w[0]);
                     w[1] = fmaf(hy, dy[c], w[1]);

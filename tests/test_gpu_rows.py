@@ -173,3 +173,48 @@ def test_batch_forces_at_uncentred_coordinates(pd, cuda, lanes, nrep, n_hi):
     # shifting a coordinate by a box rounds it to an ulp of the box, about 1e-6; force constants reach 1e3
     assert float((torch.stack(f).double() - ref).norm()) < 1e-4 * float(ref.norm())
     b.close()
+
+
+@pytest.mark.parametrize("lanes", [0, 1, 4])
+def test_non_finite_neighbour_leaves_the_rest(pd, ora, cuda, lanes):
+    """A particle whose coordinate is not finite has no pairs: the other particles' forces stay finite."""
+    import torch
+    n = 1500
+    pos, box = _fluid(n, 0.8, 12)
+    eng = pd.ELLEngine(n, box, model="lj", cutoff=2.5, skin=0.3, capacity=160, lanes=lanes)
+    x = [torch.tensor(np.ascontiguousarray(pos[:, d]), dtype=torch.float32, device="cuda") for d in range(3)]
+    eng.update(*x)
+    for bad in (float("nan"), float("inf")):
+        y = [a.clone() for a in x]
+        y[1][7] = bad
+        for energy in (False, True):
+            F = _ell_forces(eng, y, n, 3, energy)
+            ref = ora.pairs_cells(np.delete(pos, 7, 0), box, kind=1, sigma=1.0, eps=1.0, rc_lj=2.5)
+            assert np.linalg.norm(np.delete(F, 7, 0) - ref["F"]) < 2e-5 * np.linalg.norm(ref["F"])
+    eng.close()
+
+
+@pytest.mark.parametrize("lanes,charged", [(1, False), (4, False), (8, False), (1, True)])
+def test_batch_non_finite_neighbour_leaves_the_rest(pd, cuda, lanes, charged):
+    import torch
+    if charged:
+        el = dict(alpha=pd.splits.alpha_from_tolerance(9.0, 1e-5), C=pd.synthetic.COULOMB_EV_A, rc=9.0, order=5,
+                  kind="spme", spacing=1.0)
+        b = pd.batch.BatchedReplicas(pd.batch.melt_systems([1000, 1200], seed=3), skin=1.0, lanes=lanes, electrostatics=el)
+    else:
+        b = pd.batch.BatchedReplicas(pd.batch.make_systems(pd.synthetic.replica_set(3, n_lo=1200, n_hi=1500, seed=21)),
+                                     skin=0.3, cap=160, lanes=lanes)
+    b.evaluate()
+    b.synchronize()
+    for bad in (float("nan"), float("inf")):
+        y = b.y.clone()
+        y[700] = bad
+        f = [torch.zeros(b.n, device="cuda") for _ in range(3)]
+        torch.cuda.synchronize()
+        pd._native.call("pd_batch_forces", b.handle, b.x.data_ptr(), y.data_ptr(), b.z.data_ptr(),
+                        *[a.data_ptr() for a in f], 0, 0, 0)
+        torch.cuda.synchronize()
+        F = torch.stack(f)
+        F[:, 700] = 0.0
+        assert bool(torch.isfinite(F).all())
+    b.close()
