@@ -17,8 +17,8 @@
 //   * the displacement maximum and the rebuild decision run in one kernel
 //     (the last block decides), fused with the drift in the step engine;
 //   * the pair kernel reads packed (x, y, z, 0) coordinates, G lanes per row
-//     reduced by shuffles; without energies it stores forces by position, and the closing
-//     half kick carries them to particle order (with energies it is fused into the kernel).
+//     reduced by shuffles; the closing half kick is fused into it for small systems and
+//     runs in particle order after it for large ones.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -431,14 +431,20 @@ struct EllKick {     // closing half kick fused into the pair kernel (step engin
 // u = 4 eps (s12 - s6) - shift (LJ) or + eps (WCA) inside (0, rc^2); each row gets half of every
 // pair energy and half of its dyadic virial.  Forces are stored (not added): by position for k_ell_finish
 // (OUT_SLOT: a particle's force and velocity are nine scattered 32-byte sectors, a position's force is one coalesced
-// record), or with energies by particle (OUT_FORCE) and with the closing half kick (OUT_KICK).
+// record), by particle (OUT_FORCE), or by particle with the closing half kick (OUT_KICK).
 enum { OUT_FORCE = 0, OUT_KICK = 1, OUT_SLOT = 2 };
 
-__device__ __forceinline__ void ell_kick(const EllKick &kick, int i, int D, const float *a) {
-    const float im = kick.inv_mass ? kick.inv_mass[i] : kick.inv_mass_uniform;
-    const float c = kick.half_dt * im;
-    const float v0 = fmaf(c, a[0], kick.vx[i]), v1 = fmaf(c, a[1], kick.vy[i]);
-    const float v2 = D == 3 ? fmaf(c, a[2], kick.vz[i]) : 0.f;
+struct EllVel {   // what the closing kick of a particle reads
+    float im, v[3];
+};
+__device__ __forceinline__ EllVel ell_velocity(const EllKick &kick, int i, int D) {
+    return {kick.inv_mass ? kick.inv_mass[i] : kick.inv_mass_uniform,
+            {kick.vx[i], kick.vy[i], D == 3 ? kick.vz[i] : 0.f}};
+}
+__device__ __forceinline__ void ell_kick(const EllKick &kick, int i, int D, const EllVel &u, const float *a) {
+    const float im = u.im, c = kick.half_dt * im;
+    const float v0 = fmaf(c, a[0], u.v[0]), v1 = fmaf(c, a[1], u.v[1]);
+    const float v2 = D == 3 ? fmaf(c, a[2], u.v[2]) : 0.f;
     kick.vx[i] = v0;
     kick.vy[i] = v1;
     if (D == 3) kick.vz[i] = v2;
@@ -469,6 +475,14 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
     for (int t = 0; t < NV; ++t) w[t] = 0.f;
     const float4 pi = k < n ? xq[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int cnt = k < n ? counts[k] : 0;
+    // the particle's id and velocity are loaded under the row's walk: after it, they were two more memory latencies at
+    // the end of a small step (five Langevin steps of 3 000 to 12 000 2D disks 119 to 125 us, now 106)
+    int i = 0;
+    EllVel vel = {};
+    if (OUT != OUT_SLOT && lane == 0 && k < n) {
+        i = sorted[k];
+        if (OUT == OUT_KICK) vel = ell_velocity(kick, i, D);
+    }
     const LjRow lj = lj_row(m.eps, m.sig2, m.rc2, m.kind == PD_PAIR_WCA ? m.eps : -m.eshift);
     auto walk = [&](auto wrap) {
         constexpr bool WRAP = decltype(wrap)::value;
@@ -524,7 +538,6 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
         if (OUT == OUT_SLOT) {
             fc[k] = make_float4(a[0], a[1], a[2], 0.f);
         } else {
-            const int i = sorted[k];
             fx[i] = a[0];
             fy[i] = a[1];
             if (D == 3) fz[i] = a[2];
@@ -533,7 +546,7 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_pairs(const float4 *__restr
 #pragma unroll
                 for (int t = 0; t < NV; ++t) vir[(size_t)i * NV + t] = w[t];
             }
-            if (OUT == OUT_KICK) ell_kick(kick, i, D, a);
+            if (OUT == OUT_KICK) ell_kick(kick, i, D, vel, a);
         }
     }
     if (OUT == OUT_KICK && kick.advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
@@ -550,12 +563,14 @@ __global__ void __launch_bounds__(ELL_THREADS) k_ell_finish(const float4 *__rest
     if (st[E_VALID] == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
+        EllVel vel = {};
+        if (KICK) vel = ell_velocity(kick, i, D);
         const float4 f = fc[pos_of[i]];
         const float a[3] = {f.x, f.y, f.z};
         fx[i] = a[0];
         fy[i] = a[1];
         if (D == 3) fz[i] = a[2];
-        if (KICK) ell_kick(kick, i, D, a);
+        if (KICK) ell_kick(kick, i, D, vel, a);
     }
     if (KICK && kick.advance && blockIdx.x == 0 && threadIdx.x == 0) st[E_STEP] += 1;
 }
@@ -588,6 +603,12 @@ struct pd_ell {
 };
 
 namespace pdb {
+
+// From this size the pair kernel stores its forces by position and k_ell_finish carries them to particle order; below
+// it the launch costs more than the scattered stores.  Five steps, by particle / by position: 2D disks 24 000: 105 /
+// 115 us, 50 000: 110 / 116, 100 000: 117 / 117, 250 000: 189 / 159; dilute 3D fluid 24 000: 169 / 178, 40 000: 178 /
+// 174; dense LJ 32 000: 170 / 175, 70 000: 251 / 244, 1 048 576: 1729 / 1649.
+constexpr int ELL_SLOT_MIN = 32768;
 
 static void ell_free(pd_ell *e) {
     dfree(e->pos_of);
@@ -753,11 +774,10 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
     if (energy) {
         if (kick.vx) PD_ELL_PAIRS(true, OUT_KICK);
         else PD_ELL_PAIRS(true, OUT_FORCE);
+    } else if (e->n < ELL_SLOT_MIN) {
+        if (kick.vx) PD_ELL_PAIRS(false, OUT_KICK);
+        else PD_ELL_PAIRS(false, OUT_FORCE);
     } else {
-        // By position at every size: particles' forces and velocities are scattered loads and stores at the end of the
-        // longest chain, and cost more than a launch that takes them in order.  Five Langevin steps of 6 000 to 30 000
-        // 2D disks 116 us (stored by particle: 125 to 129), five NVE steps of 20 000 to 32 000 LJ atoms 171 (191); below
-        // 6 000 particles the two are within 3 %.
         PD_ELL_PAIRS(false, OUT_SLOT);
         const int fb = (e->n + ELL_THREADS - 1) / ELL_THREADS;
         count_launch();
@@ -899,7 +919,7 @@ int pd_ell_create(pd_ell **out, const pd_ell_params *p, const double box[3]) {
         (rc = dalloc(&e->counts, (size_t)e->n)) || (rc = dalloc(&e->ref, (size_t)e->n)) ||
         (rc = dalloc(&e->xq, (size_t)e->n)) || (rc = dalloc(&e->pos_of, (size_t)e->n)) ||
         (rc = dalloc(&e->scan_part, scan_part_len(e->ncell))) ||
-        (rc = dalloc(&e->fc, (size_t)e->n)) || (rc = ell_alloc_rows(e, p->cap))) {
+        (rc = dalloc(&e->fc, e->n < ELL_SLOT_MIN ? 1 : (size_t)e->n)) || (rc = ell_alloc_rows(e, p->cap))) {
         ell_free(e);
         delete e;
         return rc;
@@ -1110,6 +1130,7 @@ __global__ void __launch_bounds__(ELL_THREADS, MODE == 1 ? 5 : 1)
     for (int it = 0; it < items && valid; ++it) {
         const int i = (blockIdx.x * items + it) * ELL_THREADS + threadIdx.x;
         if (i >= a.n) break;
+        const int at = a.pos_of[i];   // loaded with the rest: the stores below might alias it
         const float im = a.inv_mass ? a.inv_mass[i] : a.inv_mass_uniform;
         float p[3] = {a.x[i], a.y[i], D == 3 ? a.z[i] : 0.f};
         float v[3] = {a.vx[i], a.vy[i], D == 3 ? a.vz[i] : 0.f};
@@ -1180,7 +1201,7 @@ __global__ void __launch_bounds__(ELL_THREADS, MODE == 1 ? 5 : 1)
             a.z[i] = p[2];
             a.vz[i] = v[2];
         }
-        a.xq[a.pos_of[i]] = make_float4(p[0], p[1], p[2], 0.f);
+        a.xq[at] = make_float4(p[0], p[1], p[2], 0.f);
         disp = fmaxf(disp, ell_displacement<D>(p, a.ref[i], a.L, true));
     }
     if (ell_block_max_last(__float_as_uint(disp), st, E_DMAX, E_TICKET_D)) {

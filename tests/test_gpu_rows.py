@@ -16,8 +16,8 @@ def _fluid(n, rho, seed, dim=3):
     return pos.astype(np.float32).astype(float), (float(np.float32(L)),) * dim
 
 
-# 3D, dense cells: a warp per row, then the engine's lanes; four and two warps per cell.
-# Sparse cells: one thread per row; 2D: the one-block and the tiled cell scan.
+# 3D, dense cells: a warp per row, the engine's lanes, forces by position; four and two warps per cell.
+# Sparse cells: one thread per row, by particle and by position; 2D: the one-block and the tiled cell scan.
 CASES = [(3, 1500, 0.8), (3, 17000, 0.8), (3, 33000, 0.8), (3, 9000, 0.08), (3, 40000, 0.08), (2, 9000, 0.85),
          (2, 60000, 0.85)]
 
@@ -117,7 +117,7 @@ def _ell_forces(eng, x, n, dim=3, energy=False):
     return torch.stack(f[:dim], 1).double().cpu().numpy()
 
 
-# dense rows, sparse rows, 2D; forces by position, and by particle with energies
+# dense rows, sparse rows, 2D; forces by particle and by position
 @pytest.mark.parametrize("dim,n,rho", [(3, 1500, 0.8), (3, 33000, 0.8), (3, 9000, 0.08), (2, 9000, 0.85)])
 @pytest.mark.parametrize("energy", [False, True])
 def test_forces_at_uncentred_coordinates(pd, ora, cuda, dim, n, rho, energy):
