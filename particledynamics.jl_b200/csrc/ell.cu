@@ -245,6 +245,18 @@ __global__ void k_ell_scatter(const int *__restrict__ cell_of, int n, const int 
     sorted[cell_off[c] + atomicAdd(&cursor[c], 1)] = i;
 }
 
+// The n ids at sorted[a] in ascending order, by one warp: every id's rank among them.
+__device__ __forceinline__ void cell_ranks(int *__restrict__ sorted, int *__restrict__ tmp, int a, int n, int lane) {
+    for (int k = lane; k < n; k += 32) {
+        const int id = sorted[a + k];
+        int r = 0;
+        for (int j = 0; j < n; ++j) r += sorted[a + j] < id ? 1 : 0;
+        tmp[a + r] = id;
+    }
+    __syncwarp();
+    for (int k = lane; k < n; k += 32) sorted[a + k] = tmp[a + k];
+}
+
 // Particles of a cell in ascending id (one warp per cell), which makes the rows and the pair
 // sums independent of the atomic cursor order.  Cells above 32 entries rank through `tmp`.
 // The cell's scatter cursor is reset to zero for the next build's histogram.
@@ -265,31 +277,36 @@ __global__ void k_ell_cellsort(const int *__restrict__ cell_off, int ncell, int 
         if (lane < n) sorted[a + r] = id;
         return;
     }
-    for (int k = lane; k < n; k += 32) {
-        const int id = sorted[a + k];
-        int r = 0;
-        for (int j = 0; j < n; ++j) r += sorted[a + j] < id ? 1 : 0;
-        tmp[a + r] = id;
-    }
-    __syncwarp();
-    for (int k = lane; k < n; k += 32) sorted[a + k] = tmp[a + k];
+    cell_ranks(sorted, tmp, a, n, lane);
 }
 
 // The same order for sparse cells, one thread per cell: insertion by id (a warp per cell left 30 lanes idle,
-// 72 us for the 506 944 cells of a million 2D disks).
+// 72 us for the 506 944 cells of a million 2D disks).  Cells of a cluster in an otherwise sparse box go through the
+// ranks of a whole warp: insertion takes the square of their particles in dependent steps of one thread.
+constexpr int SPARSE_SORT_MAX = 32;
 __global__ void k_ell_cellsort_sparse(const int *__restrict__ cell_off, int ncell, int *__restrict__ sorted,
-                                      int *__restrict__ cell_count, const long long *__restrict__ st) {
+                                      int *__restrict__ tmp, int *__restrict__ cell_count,
+                                      const long long *__restrict__ st) {
     chain_begin();
     if (!ell_requested(st)) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    cell_count[c] = 0;
-    const int a = cell_off[c], b = cell_off[c + 1];
-    for (int k = a + 1; k < b; ++k) {
-        const int id = sorted[k];
-        int j = k;
-        for (; j > a && sorted[j - 1] > id; --j) sorted[j] = sorted[j - 1];
-        sorted[j] = id;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    int a = 0, n = 0;
+    if (c < ncell) {
+        cell_count[c] = 0;
+        a = cell_off[c];
+        n = cell_off[c + 1] - a;
+    }
+    if (n <= SPARSE_SORT_MAX) {
+        for (int k = a + 1; k < a + n; ++k) {
+            const int id = sorted[k];
+            int j = k;
+            for (; j > a && sorted[j - 1] > id; --j) sorted[j] = sorted[j - 1];
+            sorted[j] = id;
+        }
+    }
+    for (unsigned heavy = __ballot_sync(0xffffffffu, n > SPARSE_SORT_MAX); heavy; heavy &= heavy - 1) {
+        const int src = __ffs(heavy) - 1;
+        cell_ranks(sorted, tmp, __shfl_sync(0xffffffffu, a, src), __shfl_sync(0xffffffffu, n, src), lane);
     }
 }
 
@@ -669,7 +686,8 @@ int ell_sort_launch(const int *cell_of, int n, int ncell, int *cell_count, int *
         launch_chained(k_ell_cellsort, (int)(((long long)ncell * 32 + 255) / 256), 256, 0, s, cell_off, ncell, sorted, tmp,
                                                                                   cell_count, st);
     else
-        launch_chained(k_ell_cellsort_sparse, (ncell + 127) / 128, 128, 0, s, cell_off, ncell, sorted, cell_count, st);
+        launch_chained(k_ell_cellsort_sparse, (ncell + 127) / 128, 128, 0, s, cell_off, ncell, sorted, tmp, cell_count,
+                       st);
     PD_LAUNCHED();
     return PD_OK;
 }

@@ -218,3 +218,40 @@ def test_batch_non_finite_neighbour_leaves_the_rest(pd, cuda, lanes, charged):
         F[:, 700] = 0.0
         assert bool(torch.isfinite(F).all())
     b.close()
+
+
+@pytest.mark.parametrize("dim,clump", [(3, 33), (3, 900), (2, 32), (2, 257)])
+def test_rows_of_a_clump_in_a_sparse_box(pd, ora, cuda, dim, clump):
+    """One crowded cell among sparse ones: its particles are in id order too, and every row is complete."""
+    import torch
+    n, L, rl = 6000, (60.0 if dim == 3 else 160.0), 2.8
+    rng = np.random.default_rng(clump)
+    pos = rng.uniform(-L / 2, L / 2, (n, dim))
+    nc = int(L / rl)
+    pos[rng.permutation(n)[:clump]] = (nc // 3 + 0.5) * (L / nc) - L / 2 + rng.uniform(-1.0, 1.0, (clump, dim))
+    pos = pos.astype(np.float32).astype(float)
+    eng = pd.ELLEngine(n, (L,) * dim, dim=dim, model="lj", cutoff=2.5, skin=0.3, capacity=1024)
+    x = [torch.tensor(np.ascontiguousarray(pos[:, d]), dtype=torch.float32, device="cuda") for d in range(dim)]
+    x += [None] * (3 - dim)
+    eng.update(*x)
+    assert eng.status()["error"] == 0
+    rows, counts = eng.rows_host()
+    p3 = pos if dim == 3 else np.concatenate([pos, np.zeros((n, 1))], 1)
+    want = ora.neighbor_rows(p3, (L,) * 3, float(np.float32(2.5) + np.float32(0.3)), cap=1024)
+    border = 0
+    for i in range(n):
+        got = sorted(rows[i].tolist())
+        assert len(set(got)) == len(got) == counts[i]
+        if got != want[i]:   # a pair whose distance is the list radius within an FP32 ulp
+            for j in set(got) ^ set(want[i]):
+                d = p3[i] - p3[j]
+                r = np.linalg.norm(d - L * np.round(d / L))
+                assert abs(r - rl) < 1e-5
+                border += 1
+    assert border < 20
+    assert max(counts) >= clump // 2
+    eng.request()   # id order inside a cell: a second build gives the same rows, entry by entry
+    eng.update(*x)
+    again, _ = eng.rows_host()
+    assert all(np.array_equal(r, t) for r, t in zip(rows, again))
+    eng.close()
