@@ -1024,6 +1024,14 @@ static void free_geometry(pd_cluster *c) {
     dfree(c->vc);
 }
 
+// Parts of four warps, about 12 to an SM: the force pass of 1000 ions takes 5.4 us (two warps, 32 parts: 6.8), of
+// 18 302 ions 20.2 us (15 parts of two warps: 21.7), of 64 000 ions 52.7 us (5 x 2: 55.3), of 512 000 ions 303 us
+// (1 x 2: 314).  With exceptions the same shape is the better one too: 1000 ions 16.4 us (17.0), 18 302 30.2 (32.2),
+// 64 000 74.5 (76.5), 512 000 402 (411).
+int cluster_default_split(int nsmax, int num_sms) {
+    return std::max(1, std::min(32, (12 * num_sms + nsmax / 2) / std::max(nsmax, 1)));
+}
+
 int cluster_build_launch(pd_cluster *c, const float *x, const float *y, const float *z, const float *q,
                          const int *type, int conditional, cudaStream_t s) {
     const int N = c->n, g = conditional ? 1 : 0;
@@ -1255,10 +1263,7 @@ int pd_cluster_setup(pd_cluster *c, const double box[3]) {
     c->pp.Lx = c->L[0];
     c->pp.Ly = c->L[1];
     c->pp.Lz = c->L[2];
-    // Parts of four warps, about 12 to an SM: the force pass of 1000 ions takes 5.4 us (two warps, 32 parts: 6.8), of
-    // 18 302 ions 20.2 us (15 parts of two warps: 21.7), of 64 000 ions 52.7 us (5 x 2: 55.3), of 512 000 ions 303 us
-    // (1 x 2: 314).
-    c->nsplit = std::max(1, std::min(32, (12 * c->num_sms + nsmax / 2) / std::max(nsmax, 1)));
+    c->nsplit = cluster_default_split(nsmax, c->num_sms);
     if (!same_geom) {
         free_geometry(c);
         c->ncs = ncs;

@@ -227,6 +227,8 @@ int cluster_read_counts(pd_cluster *c, int *host, cudaStream_t s);
 int cluster_exceptions_launch(pd_cluster *c, int energy, cudaStream_t s);
 // Frees an engine's exception buffers.
 void cluster_free_exceptions(pd_cluster *c);
+// Parts per super-cluster of the pair pass, for the default of four warps per part.
+int cluster_default_split(int nsmax, int num_sms);
 int cluster_set_word(pd_cluster *c, int word, int value, cudaStream_t s);
 // ELL, network and learned-correction internals used by the learned form and the step engine.
 int mlp_forward_launch(const pd_mlp *q, const void *X, int n, float *s, const float4 *V, float4 *corr,

@@ -117,7 +117,7 @@ extern "C" int pd_cluster_compute_static(const pd_cluster_params *p, const doubl
     int dev = 0;
     PD_CUDA(cudaGetDevice(&dev));
     PD_CUDA(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, dev));
-    c.nsplit = std::max(1, std::min(32, (32 * c.num_sms + c.nsmax - 1) / std::max(c.nsmax, 1)));
+    c.nsplit = cluster_default_split(c.nsmax, c.num_sms);
     cluster_pair_params(p, box, &c.pp);
 
     // carve every buffer of the list out of the arena
