@@ -4,7 +4,7 @@
 // Semantics: _cluster_pair_kernel! of
 // src/clusterpairs/Kernels.jl (ParticleDynamics.jl) with the pair physics of
 // pair_force (src/clusterpairs/PairFunctor.jl:127-156).  Layout of this
-// library: one CTA of 1, 2 or 4 warps (two by default; the tuned shape) per super-cluster part; thread
+// library: one CTA of 1, 2 or 4 warps (four by default; the tuned shape) per super-cluster part; thread
 // (ti, tj) = (tid & 7, tid >> 3) pairs i-atom ti of each of the 8 i-clusters
 // with j-atom tj of the current j-cluster.  The 64 i-atoms live in shared
 // memory as packed float4 (x, y, z, C q); j-atoms are read as one float4 each,
@@ -13,6 +13,8 @@
 // added with three fence-free reductions; i-forces stay in registers and are
 // reduced once per CTA.
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.hpp"
 
@@ -296,7 +298,11 @@ __global__ void __launch_bounds__(128) k_pairs(const float4 *__restrict__ xq, co
 
 template <int LJK, bool COUL, bool EN, int NP>
 static void launch_pairs(pd_cluster *c, cudaStream_t s) {
-    k_pairs<LJK, COUL, EN, NP><<<c->nsmax * c->nsplit, 32 * c->pair_warps, 0, s>>>(
+    // With energies a warp keeps ten sums per i-atom; where a super-cluster is one part already, four warps that share
+    // it only add up more of them at its end: 128 000 ions 649 us with two (683), 512 000 ions 2379 (2505).  With more
+    // parts the four are the better ones (18 302 ions in six parts 138.6 us, 138.8 with two).
+    const int warps = EN && c->nsplit == 1 ? std::min(2, c->pair_warps) : c->pair_warps;
+    k_pairs<LJK, COUL, EN, NP><<<c->nsmax * c->nsplit, 32 * warps, 0, s>>>(
         c->xq, c->ts, c->cjw, c->scio, c->nw, c->counts, c->lj_table, c->fc, c->vc, c->nslot, c->nsplit, c->pp,
         c->wxid, c->xmask);
 }

@@ -248,3 +248,19 @@ def test_workflow_exceptions_through_steps(pd, ora, cuda):
     s = st.cluster.statistics()
     assert s["builds"] >= 2 and s["error"] == 0 and s["mask_entries"] > 0
     assert math.isfinite(E)
+
+
+def test_exceptions_in_every_pair_shape(pd, cuda):
+    """Forces, energies and virials do not depend on how a super-cluster is shared among CTAs and warps."""
+    rc = 9.0
+    pos, q, box = _melt(pd)
+    eng = _engine(pd, len(pos), box, rc)
+    eng.set_exceptions(_pick_pairs(pos, box, rc, rc + 1.0, seed=11))
+    F0, E0, W0 = _compute(eng, pos, q)
+    for shape in ((1, 1), (1, 2), (1, 4), (3, 1), (3, 4)):
+        eng.set_pair_shape(*shape)
+        F, E, W = _compute(eng, pos, q)
+        assert np.max(np.abs(F - F0)) < 1e-4 and np.max(np.abs(E - E0)) < 5e-4 and np.max(np.abs(W - W0)) < 5e-4
+        F, _, _ = _compute(eng, pos, q, energy=False)
+        assert np.max(np.abs(F - F0)) < 1e-4   # the tolerances of the other order of the sums above
+    eng.close()
