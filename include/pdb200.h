@@ -527,7 +527,8 @@ int pd_batch_create(pd_batch **out, const pd_batch_replica *reps, int nrep, floa
 int pd_batch_destroy(pd_batch *b);
 int pd_batch_count(pd_batch *b, int *n, int *ncell);
 /* Lanes per row of the pair kernel (1, 2, 4, 8), the autotuner's choice.  One lane adds a row's
- * terms in row order; charged rows take at least 8 lanes where they are long. */
+ * terms in row order; charged rows take at least 8 lanes where they are long (4 from 4 entries on average, 8
+ * from 12), and pd_batch_status reports the lanes in use. */
 int pd_batch_set_lanes(pd_batch *b, int lanes);
 /* Displacement decision and the flag-gated rebuild at centred coordinates (all replicas). */
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t st);

@@ -188,13 +188,18 @@ class BatchedReplicas:
     def autotune(self, dt: float, lanes=(1, 2, 4, 8), tiles=((32, 2), (64, 2), (64, 4)), steps: int = 10) -> dict:
         """Time the captured step for every (lanes per row, spread tile) pair on this batch and keep the
         fastest (the step's pair pass and mesh branch overlap, so whole steps are timed); a spread tile is
-        (ions per CTA, threads per ion).  The state is restored afterwards."""
+        (ions per CTA, threads per ion).  Choices that run the same kernels (a charged batch takes at least
+        8 lanes on long rows) are timed once and share that time.  The state is restored afterwards."""
         saved = [t.clone() for t in (self.x, self.y, self.z, self.vx, self.vy, self.vz, self.fx, self.fy, self.fz)]
         s = self.stream
-        times = {}
+        times, timed = {}, {}
         for g in lanes:
             for tile in (tiles if self.electrostatics is not None else (self.spread_tile,)):
                 self.set_lanes(g)
+                in_use = (self.status()["lanes"], tile)
+                if in_use in timed:
+                    times[(g, tile)] = timed[in_use]
+                    continue
                 if self.electrostatics is not None:
                     self.set_spread_tile(*tile)
                 self.step(2, dt)
@@ -204,7 +209,7 @@ class BatchedReplicas:
                     self.step(steps, dt)
                     b.record(s)
                 b.synchronize()
-                times[(g, tile)] = a.elapsed_time(b) / steps
+                times[(g, tile)] = timed[in_use] = a.elapsed_time(b) / steps
         best = min(times, key=times.get)
         self.set_lanes(best[0])
         if self.electrostatics is not None:

@@ -680,13 +680,17 @@ static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, con
     return PD_OK;
 }
 
+// Lanes per row that the pair kernel runs with.  Charged rows are long and every choice below 8 lanes reads their
+// sectors several times; uncharged rows take the caller's choice.
+static int batch_lanes(const pd_batch *b) {
+    return b->coul ? std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8) : b->lanes;
+}
+
 template <bool COUL, int NP = BATCH_NP>
 static void launch_batch_pairs(pd_batch *b, float *fx, float *fy, float *fz, float *epot, int energy,
                                const BatchKick &kick, int advance, bool slot, bool centred, cudaStream_t s) {
     const float face = centred ? 1.001f : INFINITY;
-    // Charged rows are long and every choice below 8 lanes reads their sectors several times; uncharged rows take
-    // the caller's choice.
-    const int G = COUL ? std::max(b->lanes, b->mean_row < 4.0 ? 1 : b->mean_row < 12.0 ? 4 : 8) : b->lanes;
+    const int G = batch_lanes(b);
     const int blocks = (int)(((long long)b->n * G + B_THREADS - 1) / B_THREADS);
     if constexpr (!COUL) {
         if (G == 1) {
@@ -1048,7 +1052,7 @@ int pd_batch_status(pd_batch *b, pd_ell_stats *out) {
     out->builds = h[E_BUILDS];
     out->required = h[E_REQUIRED];
     out->cap = b->cap;
-    out->lanes = b->lanes;
+    out->lanes = batch_lanes(b);
     return PD_OK;
 }
 

@@ -168,3 +168,19 @@ def test_the_64_melt_set_at_full_size(pd, ora, cuda):
         F = np.stack([b.replica(k, t).cpu().numpy() for t in (b.fx, b.fy, b.fz)], 1).astype(float)
         ref = _oracle(pd, ora, s, b.meshes[k], alpha, pos)
         assert np.linalg.norm(F - ref["F"]) / np.linalg.norm(ref["F"]) < 1e-5, (k, s["n"])
+
+
+def test_autotuner_times_a_kernel_once(pd, cuda):
+    """Lanes that run the same kernel share one timing, and the lanes in use are reported."""
+    b, _, _ = _batch(pd, [1000, 1400], lanes=1)
+    b.evaluate()
+    assert b.status()["lanes"] == 8      # about 150 entries per row
+    res = b.autotune(1.0 / pd.synthetic.TIME_UNIT_FS, steps=4)
+    assert len(res["ms"]) == 12 and res["lanes"] == b.lanes
+    for tile in ("32x2", "64x2", "64x4"):
+        assert len({res["ms"][f"lanes {g}, tile {tile}"] for g in (1, 2, 4, 8)}) == 1
+    b.close()
+    specs = pd.synthetic.replica_set(3, n_lo=500, n_hi=900, seed=21)
+    u = pd.batch.BatchedReplicas(pd.batch.make_systems(specs), skin=0.3, lanes=2)
+    assert u.status()["lanes"] == 2      # uncharged rows take the caller's
+    u.close()
