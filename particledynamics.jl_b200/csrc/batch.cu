@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(B_THREADS) k_batch_finish(const float4 *__rest
 
 struct pd_batch {
     int nrep = 0, n = 0, ncell = 0, cap = 0, lanes = 4;
+    int num_sms = device_sms();
     double mean_row = 0.0;           // expected entries per row at the replicas' densities
     float rl2 = 0.f, threshold = 0.f;
     std::vector<BatchRep> hreps;
@@ -665,9 +666,7 @@ static int batch_rebuild_launch(pd_batch *b, const float *x, const float *y, con
         return rc;
     launch_chained(k_batch_pack<true>, blocks, B_THREADS, 0, s, x, y, z, nullptr, b->sorted, b->n, b->pos_of, b->xq, b->st);
     PD_LAUNCHED();
-    // few cells: several warps per cell, until the chip has about 16 warps per SM
-    int nsplit = 1;
-    while (nsplit < 8 && (long long)b->ncell * nsplit < 148 * 16) nsplit *= 2;
+    const int nsplit = rows_split(b->ncell, b->num_sms);
     const int grid = (int)(((long long)b->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
     launch_chained(k_batch_rows, grid, 32 * ROWS_WARPS, sizeof(float4) * ROWS_WARPS * ROWS_CAP, s, 
         b->xq, b->ncell, nsplit, b->cell_rep, b->reps, b->rep_flag, b->sorted, b->cell_off, b->rl2, b->cap, b->rows,
@@ -854,7 +853,7 @@ static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const
 
 static int batch_enqueue_step(pd_batch *b, float dt, cudaStream_t s, int cond) {
     const pd_md_state &S = b->state;
-    const int blocks = batch_blocks(b), items = drift_items(blocks);
+    const int blocks = batch_blocks(b), items = drift_items(blocks, b->num_sms);
     cudaGraphConditionalHandle h = 0;
     if (cond) {
         cudaStreamCaptureStatus status;
@@ -1020,8 +1019,9 @@ int pd_batch_set_lanes(pd_batch *b, int lanes) {
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t sp) {
     PD_CHECK(b && x && y && z, PD_EINVAL, "pd_batch_update: null argument");
     cudaStream_t s = (cudaStream_t)sp;
-    launch_chained(k_batch_drift<false, false>, (batch_blocks(b) + drift_items(batch_blocks(b)) - 1) / drift_items(batch_blocks(b)), B_THREADS, 0, s,
-        b->n, drift_items(batch_blocks(b)), const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
+    const int blocks = batch_blocks(b), items = drift_items(blocks, b->num_sms);
+    launch_chained(k_batch_drift<false, false>, (blocks + items - 1) / items, B_THREADS, 0, s,
+        b->n, items, const_cast<float *>(x), const_cast<float *>(y), const_cast<float *>(z), nullptr, nullptr, nullptr,
         nullptr, nullptr, nullptr, nullptr, 0.f, b->rep_of, b->reps, b->ref, b->threshold, nullptr, nullptr, b->rep_dmax,
         b->rep_flag, b->nrep, b->st, 0);
     PD_LAUNCHED();

@@ -607,6 +607,7 @@ struct pd_ell {
     bool allpairs = false;
     float rl2 = 0.f, threshold = 0.f;
     int lanes = 1;
+    int num_sms = device_sms();
     int cap = 0;
     int epoch = 0;                      // counts the row storages: captured kernels hold their address, capacity and stride
     long long *st = nullptr;
@@ -743,9 +744,7 @@ int ell_rebuild_launch(pd_ell *e, const float *x, const float *y, const float *z
                                                       e->ny, e->nz, e->rl2, e->cap, e->rows, e->counts, e->ref, e->st)
     if (e->dense) {
         const RowGrid g{{Lx, Ly, Lz}, e->nx, e->ny, e->nz, 0};
-        // few cells: several warps per cell, until the chip has about 16 warps per SM
-        int nsplit = 1;
-        while (nsplit < 8 && (long long)e->ncell * nsplit < 148 * 16) nsplit *= 2;
+        const int nsplit = rows_split(e->ncell, e->num_sms);
         const int grid = (int)(((long long)e->ncell * nsplit + ROWS_WARPS - 1) / ROWS_WARPS);
         const size_t shm = sizeof(float4) * ROWS_WARPS * ROWS_CAP;
         if (e->dim == 3)
@@ -1333,7 +1332,7 @@ static EllStepArgs ell_step_args(pd_ell_md *md, float dt, float gamma, float kT,
 static int ell_enqueue_step(pd_ell_md *md, const EllStepArgs &a, int mode, int energy, cudaStream_t s, int cond) {
     pd_ell *e = md->e;
     const int blocks = (e->n + ELL_THREADS - 1) / ELL_THREADS;
-    const int items = drift_items(blocks, mode == 1 ? 8 : 4);
+    const int items = drift_items(blocks, e->num_sms, mode == 1 ? 8 : 4);
     cudaGraphConditionalHandle h = 0;
     if (cond) {
         cudaStreamCaptureStatus status;

@@ -137,12 +137,28 @@ __device__ __forceinline__ int ell_reach(float rl, float L, int n) {
     return min(max(1, (int)ceilf(rl * (float)n / L - 1e-5f)), (n - 1) / 2);
 }
 
-// Rounds per block of a drift kernel of `blocks` blocks of 256 particles: as many as bring the blocks into one wave
-// (148 SMs, five blocks each), up to `most`: four for the NVE drifts, which wait on memory alone (4096 blocks in six
-// rounds: five steps of 1 048 576 atoms 1625 -> 1668 us).
-inline int drift_items(int blocks, int most = 4) {
-    const int rounds = (blocks + 739) / 740;
+// Rounds per block of a drift kernel of `blocks` blocks of 256 particles: as many as bring the blocks into what five
+// per SM take at once, up to `most`.  For the Langevin drift, whose launch bounds hold five blocks per SM, that is one
+// wave.  The other drifts have no such bound (NVE in 3D takes 76 registers, three blocks per SM; the batched one 32,
+// eight): their rounds, at most four, only share out the fence and the atomic that end a block (4096 blocks in six
+// rounds instead of four: five steps of 1 048 576 atoms 1625 -> 1668 us).
+inline int drift_items(int blocks, int num_sms, int most = 4) {
+    const int at_once = 5 * num_sms, rounds = (blocks + at_once - 1) / at_once;
     return rounds < 1 ? 1 : rounds > most ? most : rounds;
+}
+
+// Warps per cell of a row build by cells: one, or as many as give the chip about 16 warps per SM where cells are few.
+inline int rows_split(int ncell, int num_sms) {
+    int nsplit = 1;
+    while (nsplit < 8 && (long long)ncell * nsplit < 16LL * num_sms) nsplit *= 2;
+    return nsplit;
+}
+
+inline int device_sms() {   // of the current device
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
 }
 
 // ------------------------------------------------------------------ host side of ell.cu
