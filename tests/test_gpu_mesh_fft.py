@@ -6,9 +6,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # planes in shared memory in place: smallest mesh, odd and unequal axes, radix 16 on every axis, a radix-1 factor;
-# 736 threads on a plane; planes in two buffers (more items than threads); separate lines: large planes, odd rows; cuFFT: a prime factor 11
+# 736 threads on a plane; planes in two buffers (more items than threads); separate lines: large planes, odd rows and
+# lines; cuFFT: 245 = 5 x 7 x 7, a prime factor 11
 MESHES = [(5, 6, 7), (27, 25, 21), (16, 32, 256), (7, 120, 14), (120, 120, 6), (128, 128, 9), (160, 150, 7), (240, 256, 8),
-          (225, 245, 6), (240, 225, 9), (22, 26, 24)]
+          (225, 225, 6), (240, 225, 9), (225, 245, 6), (22, 26, 24)]
 
 
 @pytest.mark.parametrize("influence", ["spme", "p3m_ik"])

@@ -255,3 +255,43 @@ def test_rows_of_a_clump_in_a_sparse_box(pd, ora, cuda, dim, clump):
     again, _ = eng.rows_host()
     assert all(np.array_equal(r, t) for r, t in zip(rows, again))
     eng.close()
+
+
+@pytest.mark.parametrize("form", ["rows", "batch1", "batch4"])
+def test_isolated_pairs_to_rounding(pd, cuda, form):
+    """Every particle has one neighbour, so a force is one term.  With u = 2^-24: the differences and r^2 are within
+    4 u, 1/r^2 (the refined approximation) adds 2 u, s2 u, so s6 is within 23 u, s12 within 47 u, and their products with
+    1/r^2 and the difference within 58 u of the two terms' sizes."""
+    import torch
+    m, L = 1000, 60.0
+    rng = np.random.default_rng(6)
+    g = np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3) * 6.0 - 27.0
+    d = rng.normal(size=(m, 3))
+    d *= (np.linspace(0.72, 2.49, m) / np.linalg.norm(d, axis=1))[:, None]
+    pos = np.stack([g + d / 2, g - d / 2], 1).reshape(-1, 3).astype(np.float32).astype(float)
+    n = 2 * m
+    x = [torch.tensor(np.ascontiguousarray(pos[:, k]), dtype=torch.float32, device="cuda") for k in range(3)]
+    f = [torch.zeros(n, device="cuda") for _ in range(3)]
+    e = torch.zeros(n, device="cuda")
+    if form == "rows":
+        eng = pd.ELLEngine(n, (L,) * 3, model="lj", cutoff=2.5, skin=0.3, capacity=8)
+        eng.update(*x)
+        eng.forces(*x, *f, epot=e, vir=torch.zeros((n, 6), device="cuda"), energy=True)
+    else:
+        eng = pd.batch.BatchedReplicas([dict(n=n, box=(L,) * 3, kind="lj", positions=pos, velocities=np.zeros((n, 3)),
+                                             masses=1.0, eps=1.0, sigma=1.0, rc=2.5)], skin=0.3, cap=8,
+                                       lanes=int(form[-1]))
+        eng.evaluate(energy=True)
+        eng.synchronize()
+        f, e = [eng.fx, eng.fy, eng.fz], eng.epot
+    torch.cuda.synchronize()
+    F, E = torch.stack(f, 1).double().cpu().numpy(), e.double().cpu().numpy()
+    r = pos[0::2] - pos[1::2]
+    r2 = (r * r).sum(1)
+    s6 = r2 ** -3
+    u = 2.0 ** -24
+    ref = (24.0 * (2.0 * s6 * s6 - s6) / r2)[:, None] * r
+    size = 24.0 * (2.0 * s6 * s6 + s6) / np.sqrt(r2)
+    assert np.all(np.abs(F[0::2] - ref) <= 58 * u * size[:, None]) and np.all(F[1::2] == -F[0::2])
+    assert np.all(np.abs(E[0::2] - 2.0 * (s6 * s6 - s6)) <= 50 * u * 2.0 * (s6 * s6 + s6))
+    eng.close()
