@@ -228,7 +228,8 @@ int pd_cluster_buffers(pd_cluster *c, const int **perm, const float **xq, const 
  * for SPME (B-spline window, exact deconvolution), P3M with the optimal influence
  * function for analytic (AD) or ik differentiation, and ESP (prolate split and window,
  * optimal AD influence or plain deconvolution).  Transforms run in the library's own
- * kernels, or cuFFT where an axis is no product of two factors up to 16.
+ * kernels, or cuFFT where an axis is no product of two factors of 1 to 10, 12, 14, 15 or 16
+ * (with a factor 11 or 13; 125, 147, 162, 175, 189, 200, 216, 243, 245, 250, 252; most axes above 256).
  * ====================================================================== */
 typedef struct pd_mesh pd_mesh;
 
@@ -360,8 +361,8 @@ int pd_md_step_host(pd_md *md, float *host_xyz, float *host_v, int nsteps, float
  * ELL route: cell list + fixed-capacity neighbour rows (the reference's default `CellList`
  * route for LJ / WCA, src/neighbors/DeviceNeighborCUDA.jl, src/neighbors/DenseNeighborCUDA.jl)
  * and the row pair kernels (src/engine/PairTraversal.jl:66-125, src/engine/PairModels.jl:13-49,
- * src/nonbonded/LJELLEngineKernels.jl).  2D and 3D; rows are slot-major (slot t of particle i
- * at t * n + i, _ell_index, src/neighbors/NeighborTypes.jl:31), 0-based ids.
+ * src/nonbonded/LJELLEngineKernels.jl).  2D and 3D; pd_ell_rows exports the rows slot-major
+ * (slot t of particle i at t * n + i, _ell_index, src/neighbors/NeighborTypes.jl:31), 0-based ids.
  * ====================================================================== */
 typedef struct pd_ell pd_ell;
 
@@ -397,18 +398,22 @@ int pd_ell_destroy(pd_ell *e);
 int pd_ell_update(pd_ell *e, const float *x, const float *y, const float *z, pd_stream_t s);
 /* request_device_rebuild!: invalidate the list so that the next update rebuilds it. */
 int pd_ell_request(pd_ell *e, pd_stream_t s);
-/* The row pair kernel: f (stored), with energy = 1 the per-particle energy (half of each pair) and
+/* The row pair kernel at coordinates within half the skin of the last update's, centred or any other
+ * image up to a box away: f (stored), with energy = 1 the per-particle energy (half of each pair) and
  * the per-particle half virial (3D: n x 6 xx yy zz xy xz yz; 2D: n x 3 xx yy xy).  z / fz may be
  * NULL in 2D.  No forces are written while the list is invalid. */
 int pd_ell_forces(pd_ell *e, const float *x, const float *y, const float *z, float *fx, float *fy, float *fz,
                   float *epot, float *vir, int energy, pd_stream_t s);
 /* device_neighbor_status (DeviceNeighborCUDA.jl:624-637): boundary readback. */
 int pd_ell_status(pd_ell *e, pd_ell_stats *out);
-/* Device pointers of the rows (cap * n ints) and the row lengths (n ints). */
+/* Device pointers of the rows (cap * n ints) and the row lengths (n ints), by particle id.  Host
+ * boundary: the first call (and the first after a resize that ran out of memory) allocates them,
+ * waits for the device and copies the current rows, so it cannot run inside a stream capture.  From
+ * then on every rebuild refreshes them, and captured steps are captured again. */
 int pd_ell_rows(pd_ell *e, int **rows, int **counts);
 /* resize_capacity! + rearm_capacity_rebuild! (DeviceNeighborCUDA.jl:606-620): new row storage of
  * capacity cap, a latched capacity error cleared and a rebuild requested.  Captured graphs that
- * hold the old storage must be re-captured (the step engine does so when its key changes). */
+ * hold the old storage or capacity must be re-captured (the step engines do so by themselves). */
 int pd_ell_resize(pd_ell *e, int cap);
 
 /* Step engine on the ELL route (src/engine/Run.jl:162-294, src/engine/Langevin.jl): drift with the
@@ -532,13 +537,16 @@ int pd_batch_count(pd_batch *b, int *n, int *ncell);
 int pd_batch_set_lanes(pd_batch *b, int lanes);
 /* Displacement decision and the flag-gated rebuild at centred coordinates (all replicas). */
 int pd_batch_update(pd_batch *b, const float *x, const float *y, const float *z, pd_stream_t st);
-/* Forces (stored) and, with energy, the per-particle energy (half of each pair). */
+/* Forces (stored) and, with energy, the per-particle energy (half of each pair), at coordinates
+ * within half the skin of the last update's, centred or any other image up to a box away. */
 int pd_batch_forces(pd_batch *b, const float *x, const float *y, const float *z, float *fx, float *fy, float *fz,
                     float *epot, int energy, pd_stream_t st);
 int pd_batch_status(pd_batch *b, pd_ell_stats *out);
 /* Device pointers of the rows (cap x n ints, slot t of the particle at cell-order position k at
  * t * n + k, entries are cell-order positions), their lengths (n, by position) and the cell order
- * (n particle indices). */
+ * (n particle indices).  Host boundary: the first call allocates the rows, waits for the device and
+ * copies the current ones, so it cannot run inside a stream capture; every later rebuild refreshes
+ * them, and the captured step is captured again. */
 int pd_batch_rows(pd_batch *b, int **rows, int **counts, int **order);
 
 /* Charged replicas (the batched ionic melts): every replica's real-space Coulomb term is the
@@ -556,8 +564,9 @@ int pd_batch_set_coulomb(pd_batch *b, const pd_batch_coulomb *c);
 /* One SPME or P3M-AD mesh per replica (meshes: nrep x (K1, K2, K3), the replica's own box at the
  * shared spacing), B-spline order 4..6, with its FP64 influence function from the single-system
  * setup (compute_influence!, Influence.jl:190-227).  The replicas' meshes are transformed by the
- * mesh engine's kernels over all of them (or by one batched cuFFT plan per mesh size); spread, influence multiply and gather are one launch each over
- * all replicas.  Neutral replicas only (net_charge = :error).  Host boundary: allocates. */
+ * mesh engine's kernels over all of them; if one replica's mesh does not fit those (an axis that
+ * takes cuFFT, or planes beyond shared memory), the whole batch runs one batched cuFFT plan per
+ * mesh size instead.  Spread, influence multiply and gather are one launch each over all replicas.  Neutral replicas only (net_charge = :error).  Host boundary: allocates. */
 int pd_batch_set_mesh(pd_batch *b, int kind, int order, double alpha, double C, const int *meshes);
 /* Spread tile of the batched meshes, the autotuner's choice: 32 or 64 particles (cell-order
  * neighbours of one replica) per spread / gather CTA, with 2 threads per ion sharing its stencil's

@@ -4,7 +4,8 @@ Hundreds of independent 3D LJ / WCA systems of uneven size run as one device bat
 particles are concatenated, every stage of the NVE step is one launch over all replicas and the
 step is captured into one CUDA graph.  Charged replicas (ionic melts) add the real-space Coulomb
 polynomial to the pair kernel and one SPME / P3M-AD mesh per replica, spread, multiplied and
-gathered in one launch each over all replicas, transformed by the mesh kernels over all of them.
+gathered in one launch each over all replicas, transformed by the mesh kernels over all of them
+(if every replica's mesh fits those; one that does not puts the whole batch on batched cuFFT plans).
 ``autotune_lanes`` picks the pair kernel's lanes per row, ``autotune`` the lanes per row and the
 spread tile of charged batches, by timing the candidates on the batch itself.  The reference steps
 one system per engine; looping the single-system engines is the comparison.

@@ -16,16 +16,17 @@
 //      stencil staged in shared memory, rows identical to the single-system kernels'), the
 //      capacity commit by the last block;
 //   3. k_batch_pack (coordinates in cell order) and k_batch_pairs<G>: G lanes per row (G chosen by
-//      the caller's autotuner), the replica's LJ or WCA model, the closing half kick fused, the
-//      device step advanced.
-// Rows live in cell order (slot t of the particle at position k of the cell order at t * N + k,
-// entries are cell-order positions), so row stores and loads are contiguous per warp and the
-// neighbours' packed records of a row sit in nearby cells.
+//      the caller's autotuner), the replica's LJ or WCA model; the closing half kick is fused into
+//      it for small batches, and runs in k_batch_finish for those of BATCH_SLOT_MIN particles or
+//      more and in the meshes' gather for charged ones; the device step advances.
+// Rows live in cell order (entry t of the particle at position k of the cell order at k * cap + t,
+// entries are cell-order positions), so a row's entries are contiguous and the neighbours' packed
+// records of a row sit in nearby cells.
 //
 // Charged replicas (the batched ionic melts) add the real-space Coulomb polynomial to the pair kernel
 // and a mesh per replica (batch_mesh.cu): the step's force pass packs coordinates and charges once,
-// runs the pair kernel while the mesh branch (spread, batched transforms per mesh size, influence
-// multiply) runs on a second stream, and the gather joins both and applies the closing half kick.
+// runs the pair kernel while the mesh branch (spread, transforms with the influence multiply) runs on
+// a second stream, and the gather joins both and applies the closing half kick.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -792,14 +793,14 @@ static int batch_mesh_transform(pd_batch *b, cudaStream_t s) {
     return batch_fft_all(b, false, s);
 }
 
-// From this size the pair kernel stores its forces by position and k_batch_finish carries them to particle order:
-// below it the extra launch costs more than the scattered stores.
+// From this size the pair kernel stores its forces by position and k_batch_finish carries them to particle order. Below
+// it the two are within 4 % of each other either way (five steps, by particle / by position: 4757 atoms 242 / 251 us,
+// 17 316 atoms 318 / 307), and the launch is saved.
 constexpr int BATCH_SLOT_MIN = 32768;
 
 // The force pass: pack (unless the drift has packed the coordinates), then the row pair kernel; with charges and meshes
-// the pair kernel runs on s
-// while the mesh branch runs on the batch's mesh stream (forked and joined by events, so the same
-// code is captured into the step graph), and the gather joins both and applies the closing kick.
+// the pair kernel runs on s while the mesh branch runs on the batch's mesh stream (forked and joined by events, so the
+// same code is captured into the step graph), and the gather joins both and applies the closing kick.
 static int batch_pairs_launch(pd_batch *b, const float *x, const float *y, const float *z, float *fx, float *fy,
                               float *fz, float *epot, int energy, BatchKick kick, int advance, bool drifted,
                               cudaStream_t s) {
@@ -1213,8 +1214,9 @@ static int batch_make_plans(pd_batch *b, int prio_hi) {
     return PD_OK;
 }
 
-// Every replica's mesh on this library's transforms, when every mesh's planes fit in shared memory:
-// the table of meshes and the work of every CTA, the replicas' planes largest first.
+// Every replica's mesh on this library's transforms, when every mesh's planes fit in shared memory (all or none: one
+// replica whose mesh does not leaves the whole batch on the cuFFT groups): the table of meshes and the work of every
+// CTA, the replicas' planes largest first.
 static int batch_make_transforms(pd_batch *b) {
     std::vector<FftMesh> tab((size_t)b->nrep);
     for (int r = 0; r < b->nrep; ++r) {

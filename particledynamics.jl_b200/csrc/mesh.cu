@@ -6,11 +6,12 @@
 // (Splits.jl:21-240), influence functions and virial coefficients in FP64
 // (Influence.jl:24-227), the solve with the FP64 energy/virial reduction
 // (MeshKernels.jl:34-81), the ik field (MeshKernels.jl:84-102) and the AD / ik
-// gathers (MeshKernels.jl:105-147, 281-333); cuFFT does the transforms
-// (Solver.jl:34-65, 305-347).  The spread and gather kernels are in
-// mesh_kernels.cuh.  The charge grid is kept zero between transforms: the solve
-// clears it after the forward transform has consumed it, and the inverse
-// transform writes the potential into a second grid.
+// gathers (MeshKernels.jl:105-147, 281-333).  The transforms (Solver.jl:34-65,
+// 305-347) run in the kernels of mesh_fft.cu, which multiply between them, or in
+// cuFFT for axes that those do not take.  The spread and gather kernels are in
+// mesh_kernels.cuh.  The charge grid is kept zero between transforms: the forward
+// transform clears it (the solve on the cuFFT route), and the inverse transform
+// writes the potential into a second grid.
 #include <cufft.h>
 
 #include <algorithm>

@@ -339,7 +339,7 @@ __device__ __forceinline__ void lines_z(const FftMesh &m, int col0, float2 *S, c
 
 // Planes come in three CTA sizes (up to 256, 512 or FFT_PLANE_THREADS threads): the registers are capped so that
 // four, two or one of them share an SM, as a plane alone leaves most of an SM waiting on its own barriers (12 melts of
-// 3 600 to 12 000 ions, 10 steps: 926 us with one size, 814 with three).
+// 2050 to 16 282 ions, 5 steps: 926 us with one size, 814 with three).
 constexpr int fft_plane_blocks(int maxt) { return maxt <= 256 ? 4 : maxt <= 512 ? 2 : 1; }
 
 template <bool INPLACE, int MAXT>

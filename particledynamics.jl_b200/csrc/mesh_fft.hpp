@@ -10,8 +10,9 @@ constexpr int FFT_LINES_C = 16;          // adjacent lines per CTA of the line k
 constexpr int FFT_PLANE_THREADS = 768;
 constexpr size_t FFT_PLANE_SMEM_MAX = 220 * 1024;
 
-// How a mesh is transformed: cuFFT (an axis is not a product of two supported lengths), whole z planes in
-// shared memory, or separate x and y lines.
+// How a mesh is transformed: cuFFT (an axis is no product of two lengths of 1 to 10, 12, 14, 15 or 16: those with a
+// factor 11 or 13, 125, 147, 162, 175, 189, 200, 216, 243, 245, 250, 252 and most above 256), whole z planes in shared
+// memory, or separate x and y lines.
 enum { FFT_CUFFT = 0, FFT_PLANES = 1, FFT_LINES = 2 };
 
 // One axis: n = a b, w[k] = exp(-2 pi i k / n).

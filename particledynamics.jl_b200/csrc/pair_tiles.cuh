@@ -21,8 +21,6 @@
 
 namespace pdb {
 
-
-
 template <int NP>
 __device__ __forceinline__ f2 horner2(const f2 (&c)[NP], f2 x) {
     f2 acc = c[NP - 1];

@@ -34,7 +34,8 @@ struct RowGrid {
 // ROWS_GROUP particles: the accepted ones are appended in visiting order by ballot.  Bound by the issue of the
 // tests (12 instructions per 32 candidates and particle); a lane-per-particle scan of the same stage left the
 // lanes beyond the cell's particles idle and scattered its row stores (1 048 576 LJ atoms, 19 per cell: 3.34 ms
-// per build, now 0.56).  NOWRAP: no pair of the stencil crosses a periodic face, the nearest-image shift is the identity.
+// per build, now 0.56).  Without WRAP no pair of the
+// stencil crosses a periodic face: the nearest-image shift is the identity.
 template <int D, bool WRAP>
 __device__ __forceinline__ void rows_test(const RowGrid &g, float4 *sw, int fill, int np, float xi, float yi, float zi,
                                           int k0, float rl2, int cap, int *__restrict__ rows, int &found) {
@@ -276,7 +277,7 @@ __device__ __forceinline__ bool clear_of_faces(const float4 &pi, const float *L,
 }
 
 // One row's LJ / WCA sums of two neighbours at a time: f/r = 24 eps (2 s12 - s6) / r^2 and u = 4 eps (s12 - s6) + eoff
-// inside (0, rc2); ea, eb: whether the pair counts.
+// inside (0, rc2), which the caller tests.
 struct LjRow {
     f2 sig2, eps24, eps4, eoff, two, minus1;
     float rc2;
