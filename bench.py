@@ -1236,9 +1236,9 @@ def main():
     nsm = torch.cuda.get_device_properties(0).multi_processor_count
     fp32_peak = nsm * 128 * 2 * float(peaks.get("sm_max_mhz", 1965.0)) * 1e6 / 1e12   # TFLOP/s (no measured FP32 figure)
     achieved = flops / (pair_ms * 1e-3) / 1e12
-    roofline = {"kernel": "k_pairs<LJ uniform, Coulomb polynomial, force only>", "bound": "fp32",
+    roofline = {"kernel": "k_pairs_force<LJ uniform, Coulomb polynomial>", "bound": "fp32",
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
-                "traffic": profiled_traffic("k_pairs_melt64k.md"), "per_launch_ms": pair_ms,
+                "traffic": profiled_traffic("k_pairs_force_melt64k.md"), "per_launch_ms": pair_ms,
                 "pairs_within_rc": npairs, "flop_per_pair": flop_pair,
                 "peak_source": "nominal FP32 FMA rate at sm_max_mhz (MEASURED_PEAKS.json has no FP32 figure)"}
 
