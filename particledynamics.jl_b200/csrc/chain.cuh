@@ -1,7 +1,8 @@
 // Launches of kernels that follow one another in a stream: a chained kernel may be set up while its predecessor
 // still runs, and its blocks wait at chain_begin() until that one is complete and its writes are visible
 // (programmatic dependent launch).  Chains of short kernels are otherwise bound by the gaps between them (mesh sum of 99 998 charges in nine
-// kernels 148 -> 136 us, learned correction of 64 000 ions in seven 90 -> 70 us).
+// kernels 148 -> 136 us, learned correction of 64 000 ions in seven 90 -> 70 us).  Not for a kernel whose few long blocks
+// have to spread over the chip (launch_gather_t in mesh_kernels.cuh).
 #pragma once
 
 #include <cuda_runtime.h>

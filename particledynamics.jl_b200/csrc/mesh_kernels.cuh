@@ -765,7 +765,10 @@ void launch_spread_t(int P, const float4 *xq, int nchunks, const int *ns_dev, fl
     }
 }
 
-// MODE 0 (add), 1 (set) or 2 (the join of the step).
+// MODE 0 (add), 1 (set) or 2 (the join of the step).  Not chained: set up while the transforms still run, one CTA to an
+// SM, the gather's blocks pile up on the SMs that those leave free, and wait there until their turn.  Mesh sums outside
+// captures, chained / not: 4000 charges at order 8: 146 / 98 us, 20 000 at order 12: 858 / 466, 50 000 ordered ones at
+// order 6 with energies: 189 / 123; 99 998 unordered: 126 / 128.
 template <int WIN, bool IK, int MODE>
 void launch_gather_t(int P, bool energy, const float4 *xq, int nchunks, const int *ns_dev, const GatherGrids &g,
                      int K1, int K2, int K3, float Lx, float Ly, float Lz, const GatherOut &o, cudaStream_t s) {
@@ -773,10 +776,10 @@ void launch_gather_t(int P, bool energy, const float4 *xq, int nchunks, const in
 #define PD_GATHER_CASE(PP)                                                                                          \
     case PP:                                                                                                        \
         if (energy)                                                                                                 \
-            launch_chained(k_gather<PP, MODE, true, IK, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, g, K1, K2, K3, Lx, \
+            k_gather<PP, MODE, true, IK, WIN><<<nchunks, MESH_THREADS, 0, s>>>(xq, nchunks, ns_dev, g, K1, K2, K3, Lx, \
                                                                                Ly, Lz, o);                          \
         else                                                                                                        \
-            launch_chained(k_gather<PP, MODE, false, IK, WIN>, nchunks, MESH_THREADS, 0, s, xq, nchunks, ns_dev, g, K1, K2, K3,    \
+            k_gather<PP, MODE, false, IK, WIN><<<nchunks, MESH_THREADS, 0, s>>>(xq, nchunks, ns_dev, g, K1, K2, K3,    \
                                                                                 Lx, Ly, Lz, o);                     \
         break;
         PD_MESH_ORDER_CASES(PD_GATHER_CASE)
