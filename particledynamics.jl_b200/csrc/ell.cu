@@ -402,16 +402,17 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS, ROWS_BLOCKS) k_ell_rows_cells
 }
 
 // Packed coordinates (x, y, z, 0) in cell order.  REBUILD: inside a rebuild, after the sort (the particles'
-// positions in the new order are written too); otherwise the pack of a force evaluation.
+// positions in the new order are written too); otherwise the pack of a force evaluation, by particle: coalesced loads and
+// one scattered 16-byte store instead of two or three scattered loads (forces of 1 000 000 2D disks 37.7 -> 31.9 us).
 template <int D, bool REBUILD>
 __global__ void k_ell_pack(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                            const int *__restrict__ sorted, int n, int *__restrict__ pos_of, float4 *__restrict__ xq,
                            const long long *__restrict__ st) {
     chain_begin();
     if (REBUILD && !ell_requested(st)) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int i = sorted[k];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int i = REBUILD ? sorted[t] : t, k = REBUILD ? t : pos_of[t];
     xq[k] = make_float4(x[i], y[i], D == 3 ? z[i] : 0.f, 0.f);
     if (REBUILD) pos_of[i] = k;
 }
