@@ -386,7 +386,8 @@ typedef struct {
     int valid, error, requested;   /* error: 0, 1 capacity (rows longer than cap), 2 coordinates */
     long long step, last_build, interval, checks, builds;
     long long required;            /* longest row of the last build attempt */
-    int cap, lanes, allpairs;      /* allpairs: box below three cells per dimension, rows from all pairs */
+    int cap, lanes, allpairs;      /* lanes: per row, in use; allpairs: box below three cells per dimension, rows from
+                                    * all pairs */
 } pd_ell_stats;
 
 /* DeviceNeighborWorkspace(T, N, box; cutoff, skin, cap, interval) (DeviceNeighborCUDA.jl:64-88) */

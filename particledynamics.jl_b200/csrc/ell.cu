@@ -805,18 +805,17 @@ static void ell_pairs_g(pd_ell *e, float *fx, float *fy, float *fz, float *epot,
 #undef PD_ELL_PAIRS
 }
 
+// Lanes per row that the pair kernel runs with: the caller's, the density's, or on dense rows a whole warp where the rows
+// alone leave SMs idle (4000 LJ atoms: 63 blocks of four lanes per row, 16 us; 500 blocks of a warp, 8 us); a million
+// atoms take 4 and 8 lanes alike and 16 a third longer.
+static int ell_lanes(const pd_ell *e) { return e->dense && e->p.lanes == 0 && e->n < 16384 ? 32 : e->lanes; }
+
 template <int D>
 static void ell_pairs_d(pd_ell *e, float *fx, float *fy, float *fz, float *epot, float *vir, int energy, bool centred,
                         const EllKick &kick, cudaStream_t s) {
     if (e->dense) {
-        // the caller's lanes, or a whole warp per row where the rows alone leave SMs idle (4000 LJ atoms: 63 blocks
-        // of four lanes per row, 16 us; 500 blocks of a warp, 8 us); a million atoms take 4 and 8 lanes alike and 16
-        // a third longer
-        if (e->p.lanes == 0 && e->n < 16384) {
-            ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s);
-            return;
-        }
-        switch (e->lanes) {
+        switch (ell_lanes(e)) {
+            case 32: ell_pairs_g<D, 32, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
             case 1: ell_pairs_g<D, 1, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
             case 2: ell_pairs_g<D, 2, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
             case 4: ell_pairs_g<D, 4, true>(e, fx, fy, fz, epot, vir, energy, centred, kick, s); break;
@@ -1011,7 +1010,7 @@ int pd_ell_status(pd_ell *e, pd_ell_stats *out) {
     out->builds = h[E_BUILDS];
     out->required = h[E_REQUIRED];
     out->cap = e->cap;
-    out->lanes = e->lanes;
+    out->lanes = ell_lanes(e);
     out->allpairs = e->allpairs ? 1 : 0;
     return PD_OK;
 }

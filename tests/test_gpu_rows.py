@@ -295,3 +295,11 @@ def test_isolated_pairs_to_rounding(pd, cuda, form):
     assert np.all(np.abs(F[0::2] - ref) <= 58 * u * size[:, None]) and np.all(F[1::2] == -F[0::2])
     assert np.all(np.abs(E[0::2] - 2.0 * (s6 * s6 - s6)) <= 50 * u * 2.0 * (s6 * s6 + s6))
     eng.close()
+
+
+@pytest.mark.parametrize("n,rho,asked,used", [(1500, 0.8, 0, 32), (1500, 0.8, 2, 2), (17000, 0.8, 0, 4), (9000, 0.08, 0, 1)])
+def test_status_gives_the_lanes_in_use(pd, cuda, n, rho, asked, used):
+    _, box = _fluid(n, rho, 3)
+    eng = pd.ELLEngine(n, box, model="lj", cutoff=2.5, skin=0.3, capacity=160, lanes=asked)
+    assert eng.status()["lanes"] == used
+    eng.close()
